@@ -393,13 +393,18 @@ __device__ bool remove_node(Patch &p, uint32_t x, uint32_t ins[2], uint32_t un[2
 // ---- batched best-first search: one warp per item -------------------------------------------
 //
 // The frontier (up to 128 entries, unordered) lives in registers, 4 slots per lane, entry
-// e = slot * 32 + lane; slots at or past `used` are empty. Each round the warp evaluates every
-// entry whose bound passes (up to four per lane, their loads issued together), reduces the best
-// total (ties: the entry first in (cost, node) order) and gathers the children of the expanded
-// entries into the warp's shared buffer, which becomes the next frontier. Only when more than 128
-// children arrive are the 128 lowest in (cost, node) order selected (a radix selection by warp
-// ballots) and kept, the rest counted as overflow. The records of the next round's slot 0 are loaded as soon as it is known.
-// oracle/bittner.c (gpu_find_node_batched) restates the same rounds.
+// e = slot * 32 + lane. Each round the warp evaluates every entry, reduces the best total and
+// gathers the children of the expanded entries into the warp's shared buffer, which becomes the
+// next frontier. Only when more than 128 children arrive are the 128 lowest in (cost, node) order
+// selected (a radix selection by warp sums) and kept, the rest counted as overflow. The best
+// position (ties: the earliest round, then the entry first in (cost, node) order) is kept per lane
+// and resolved after the last round. oracle/bittner.c (gpu_find_node_batched) restates the same
+// rounds.
+// Bound: the dependent chain of a round (a record's L2 round trip, the evaluation, the reduction,
+// the gather); a search takes 16 to 18 rounds, 6 to 14 entries each. Keeping the patch's keys in
+// registers, the best per lane and no bound test per entry shortened the chain: a chunk's launch
+// went from 29.6 to about 20.5 us on 65,536 triangles (41 items), from 51.7 to about 38 us on
+// 4.19M (2,621 items).
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kFrontier = 4;  // slots per lane (128 entries)
 constexpr uint32_t kFrontierCap = 32u * kFrontier;
@@ -462,138 +467,164 @@ __device__ __forceinline__ uint32_t warp_select_kth(const uint32_t (&key)[S], ui
   return res;
 }
 
-// Per-warp buffer of a round's children (up to 256 entries; blocks of up to kRankWarps warps).
-constexpr int kRankWarps = 8;
-__device__ __forceinline__ uint2 *child_buffer() {
-  __shared__ uint2 buf[kRankWarps][2 * kFrontierCap];
-  return buf[(threadIdx.x >> 5) & (kRankWarps - 1)];
+constexpr int kWarpItemsPerBlock = 4;
+
+// Per-warp buffer of a round's expanded entries (up to 128: the induced cost and the left child, the
+// induced cost and the right child), read back as up to 256 children of 8 bytes.
+__device__ __forceinline__ uint4 *child_buffer() {
+  __shared__ uint4 buf[kWarpItemsPerBlock][kFrontierCap];
+  return buf[(threadIdx.x >> 5) & (kWarpItemsPerBlock - 1)];
 }
 
-// State of one batched search (warp-uniform except the per-lane frontier entries and records).
+// The patch as the search looks it up, one copy of the keys in every lane's registers: the nodes of
+// get_subset (slot 1 empty: only slot 0 is looked at) and of the patched boxes. A search meets a
+// patched node in a few rounds only, so an entry costs eight compares and the shared-memory patch
+// is read behind one rarely taken branch.
+struct PatchKeys {
+  uint32_t node[4], box[4];
+  __device__ __forceinline__ explicit PatchKeys(const PatchData *d) {
+    const bool more = d->idx[1] != kNone;
+    node[0] = d->idx[0];
+#pragma unroll
+    for (int k = 1; k < 4; ++k) node[k] = more ? d->idx[k] : kNone;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) box[k] = d->apath[k];
+  }
+  __device__ __forceinline__ bool patched(uint32_t x) const {
+    bool hit = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) hit |= x == node[k] || x == box[k];
+    return hit;
+  }
+};
+
+// One batched search. The frontier's entry e = slot * 32 + lane is live when e < m; the per-lane
+// best is the lane's first entry of its smallest total, the lowest (cost, node) within a round.
 struct BatchedSearch {
   float fc[kFrontier];
   uint32_t fn[kFrontier];
-  uint32_t used;     // slots holding entries
-  bool haveRec;      // slot 0's tree records are already in rec[]
-  float4 rec[3];
-  float bestCost;
-  uint32_t best;
+  uint32_t m;         // entries in the frontier (every one is within the bound)
+  uint32_t round;
+  float4 rec[3];      // the tree record of slot 0's entry
+  float bestCost;     // warp-uniform
+  float myCost, myEntry;
+  uint32_t myRound, myNode;
 };
 
-// One round over the first S slots (S >= used). Returns false when no entry passed the bound.
+// The record of entry x (of the root where x is no node: the entry is flagged when it is evaluated).
+__device__ __forceinline__ void load_entry(const Patch &p, uint32_t x, float4 (&rec)[3]) {
+  const float4 *q = reinterpret_cast<const float4 *>(p.t + (x < p.numNodes ? x : p.root));
+  rec[0] = __ldg(q);
+  rec[1] = __ldg(q + 1);
+  rec[2] = __ldg(q + 2);
+}
+
+// One round over S slots (32 S >= m): evaluates every entry, updates the bound and makes the
+// children of the expanded entries the next frontier. The bound only changes here and an entry's
+// two children share its induced cost, so every child passes the bound when its round comes: no
+// entry is tested against it again. Which entry reached the best total is resolved once, after the
+// last round (find_node_batched): a round needs the minimum itself only.
 template <int S>
-__device__ __forceinline__ bool batched_round(const Patch &p, BatchedSearch &st, const Box &nbox, float sarea,
-                                              uint2 *buf, SearchCounters &ctr) {
+__device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &keys, BatchedSearch &st, const Box &nbox,
+                                              float sarea, uint4 *buf, SearchCounters &ctr) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t ltMask = (1u << lane) - 1u;
   const float kInf = __int_as_float(0x7f800000);
-  bool cand[S];
-  uint32_t nc = 0;
+  ctr.visits += st.m;
+  float induced[S];
+  uint32_t left[S], right[S];
+  uint32_t inner = 0;  // bit s: this lane's slot s holds an inner node
+  float roundCost = kInf, roundEntry = kInf;
+  uint32_t roundNode = kNone;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    cand[s] = st.fc[s] != kInf && fadd(st.fc[s], sarea) < st.bestCost;
-    nc += __popc(__ballot_sync(kFull, cand[s]));
-  }
-  if (nc == 0) return false;
-  ctr.visits += nc;
-  NodeP cn[S];
-  float total[S], induced[S];
-#pragma unroll
-  for (int s = 0; s < S; ++s) {
-    total[s] = induced[s] = kInf;
-    if (!cand[s]) continue;
-    const uint32_t xs = p.chk(st.fn[s]);
-    float4 q0, q1, q2;
-    if (s == 0 && st.haveRec) {
-      q0 = st.rec[0]; q1 = st.rec[1]; q2 = st.rec[2];
+    induced[s] = kInf;
+    left[s] = right[s] = kNone;
+    if (S > 1 && (uint32_t)s * 32u + lane >= st.m) continue;
+    if (S == 1 && lane >= st.m) continue;
+    const uint32_t x = st.fn[s];
+    float4 q[3];
+    if (s == 0) {
+      q[0] = st.rec[0]; q[1] = st.rec[1]; q[2] = st.rec[2];
     } else {
-      const float4 *q = reinterpret_cast<const float4 *>(p.t + xs);
-      q0 = __ldg(q); q1 = __ldg(q + 1); q2 = __ldg(q + 2);
+      load_entry(p, x, q);
     }
+    if (x >= p.numNodes) p.bad = true;
     Box b;
-    p.subset_aabb_from(st.fn[s], q0, q1, q2, cn[s], b);
+    b.mn[0] = q[0].x; b.mn[1] = q[0].y; b.mn[2] = q[0].z;
+    b.mx[0] = q[0].w; b.mx[1] = q[1].x; b.mx[2] = q[1].y;
+    left[s] = __float_as_uint(q[1].w);
+    right[s] = __float_as_uint(q[2].x);
+    bool leaf = (__float_as_uint(q[2].y) & 0xFFFFu) != 0u;
+    if (keys.patched(x)) {
+      NodeP n;
+      p.subset_aabb_from(x, q[0], q[1], q[2], n, b);
+      left[s] = n.left;
+      right[s] = n.right;
+      leaf = n.isLeafFlag != 0;
+    }
     const float ind = fmul(-1.0f, surface_area(b));
     merge_into(b, nbox);
-    total[s] = fadd(st.fc[s], surface_area(b));
-    induced[s] = fadd(ind, total[s]);
+    const float total = fadd(st.fc[s], surface_area(b));
+    induced[s] = fadd(ind, total);
+    inner |= (leaf ? 0u : 1u) << s;
+    if (S == 1) {
+      roundCost = total;
+      roundEntry = st.fc[s];
+      roundNode = x;
+    } else if (total < roundCost ||
+               (total == roundCost && (st.fc[s] < roundEntry || (st.fc[s] == roundEntry && x < roundNode)))) {
+      roundCost = total;
+      roundEntry = st.fc[s];
+      roundNode = x;
+    }
   }
-  // Best of the round: smallest total, then smallest (cost, node) of the entry.
-  uint32_t kl = 0xFFFFFFFFu;
-#pragma unroll
-  for (int s = 0; s < S; ++s)
-    if (cand[s]) kl = min(kl, f2ord(total[s]));
-  const uint32_t kmin = __reduce_min_sync(kFull, kl);
-  uint32_t rnode;
-  uint32_t tieMask = 0;  // this lane's slots that reach kmin
-#pragma unroll
-  for (int s = 0; s < S; ++s)
-    if (cand[s] && f2ord(total[s]) == kmin) tieMask |= 1u << s;
-  const uint32_t tieLanes = __ballot_sync(kFull, tieMask != 0);
-  if (__popc(tieLanes) == 1 && (S == 1 || __popc(__shfl_sync(kFull, tieMask, __ffs(tieLanes) - 1)) == 1)) {
-    uint32_t mine = kNone;
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-      if (tieMask & (1u << s)) mine = st.fn[s];
-    rnode = __shfl_sync(kFull, mine, __ffs(tieLanes) - 1);
-  } else {
-    uint32_t cl = 0xFFFFFFFFu;
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-      if (tieMask & (1u << s)) cl = min(cl, f2ord(st.fc[s]));
-    const uint32_t cmin = __reduce_min_sync(kFull, cl);
-    uint32_t nl = 0xFFFFFFFFu;
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-      if ((tieMask & (1u << s)) && f2ord(st.fc[s]) == cmin) nl = min(nl, st.fn[s]);
-    rnode = __reduce_min_sync(kFull, nl);
-  }
-  const float rbest = ord2f(kmin);
-  if (rbest < st.bestCost) {
-    st.bestCost = rbest;
-    st.best = rnode;
+  const float kmin = ord2f(__reduce_min_sync(kFull, f2ord(roundCost)));
+  if (kmin < st.bestCost) st.bestCost = kmin;
+  if (roundCost < st.myCost) {
+    st.myCost = roundCost;
+    st.myEntry = roundEntry;
+    st.myNode = roundNode;
+    st.myRound = st.round;
   }
   // Children of the expanded entries: the k-th expanded entry (slot-major, then lane) writes
   // children 2k and 2k + 1 to the warp's buffer.
   uint32_t m = 0;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    const bool kids = cand[s] && !cn[s].isLeafFlag && fadd(induced[s], sarea) < st.bestCost;
+    const bool kids = ((inner >> s) & 1u) && fadd(induced[s], sarea) < st.bestCost;
     const uint32_t kmask = __ballot_sync(kFull, kids);
     const uint32_t mk = 2u * __popc(kmask);
     if (kids) {
-      const uint32_t k = m / 2 + __popc(kmask & ltMask);
-      buf[2 * k] = make_uint2(__float_as_uint(induced[s]), cn[s].left);
-      buf[2 * k + 1] = make_uint2(__float_as_uint(induced[s]), cn[s].right);
+      buf[m / 2 + __popc(kmask & ltMask)] = make_uint4(__float_as_uint(induced[s]), left[s], __float_as_uint(induced[s]), right[s]);
       if (m + mk > 32u) {  // children past slot 0: warm their records in L2
-        if (cn[s].left < p.numNodes) prefetch_node(p.t, cn[s].left);
-        if (cn[s].right < p.numNodes) prefetch_node(p.t, cn[s].right);
+        if (left[s] < p.numNodes) prefetch_node(p.t, left[s]);
+        if (right[s] < p.numNodes) prefetch_node(p.t, right[s]);
       }
     }
     m += mk;
   }
   __syncwarp();
-  st.haveRec = false;
-  if (m <= kFrontierCap) {
-    st.used = (m + 31u) / 32u;
+  const uint2 *child = reinterpret_cast<const uint2 *>(buf);
+  if (S <= 2 || m <= kFrontierCap) {
+    st.m = m;
+    if (lane < m) {  // slot 0 first: its records are on their way while the other slots are read
+      const uint2 v = child[lane];
+      st.fc[0] = __uint_as_float(v.x);
+      st.fn[0] = v.y;
+      load_entry(p, v.y, st.rec);
+    }
+    if (m > 32u) {
 #pragma unroll
-    for (int s = 0; s < kFrontier; ++s) {
-      const uint32_t e = (uint32_t)s * 32u + lane;
-      if ((uint32_t)s < st.used) {
-        const uint2 v = e < m ? buf[e] : make_uint2(__float_as_uint(kInf), kNone);
-        st.fc[s] = __uint_as_float(v.x);
-        st.fn[s] = v.y;
-      } else {
-        st.fc[s] = kInf;
-        st.fn[s] = kNone;
+      for (int s = 1; s < kFrontier; ++s) {
+        const uint32_t e = (uint32_t)s * 32u + lane;
+        if (e < m) {
+          const uint2 v = child[e];
+          st.fc[s] = __uint_as_float(v.x);
+          st.fn[s] = v.y;
+        }
       }
     }
-    if (lane < m) {  // slot 0's records for the next round (an index out of range: the root's)
-      const float4 *q = reinterpret_cast<const float4 *>(p.t + (st.fn[0] < p.numNodes ? st.fn[0] : p.root));
-      st.rec[0] = __ldg(q);
-      st.rec[1] = __ldg(q + 1);
-      st.rec[2] = __ldg(q + 2);
-    }
-    st.haveRec = true;
   } else {
     // Overflow: keep the 128 lowest children in (cost, node) order. The frontier is unordered, so
     // only that set matters: select the 128th smallest cost, then, among the children at that cost
@@ -604,7 +635,7 @@ __device__ __forceinline__ bool batched_round(const Patch &p, BatchedSearch &st,
 #pragma unroll
     for (int s = 0; s < 2 * kFrontier; ++s) {
       const uint32_t e = (uint32_t)s * 32u + lane;
-      const uint2 v = e < m ? buf[e] : make_uint2(0u, kNone);
+      const uint2 v = e < m ? child[e] : make_uint2(0u, kNone);
       in |= (e < m ? 1u : 0u) << s;
       key[s] = f2ord(__uint_as_float(v.x));
       nd[s] = v.y;
@@ -634,62 +665,74 @@ __device__ __forceinline__ bool batched_round(const Patch &p, BatchedSearch &st,
       }
     }
     uint32_t pos = 0;
+    uint2 *kept = reinterpret_cast<uint2 *>(buf);
 #pragma unroll
     for (int s = 0; s < 2 * kFrontier; ++s) {
       const bool keep = ((in >> s) & 1u) && (key[s] < tc || (((tie >> s) & 1u) && nd[s] <= tn));
       const uint32_t km = __ballot_sync(kFull, keep);
-      if (keep) buf[pos + __popc(km & ltMask)] = make_uint2(__float_as_uint(ord2f(key[s])), nd[s]);
+      if (keep) kept[pos + __popc(km & ltMask)] = make_uint2(__float_as_uint(ord2f(key[s])), nd[s]);
       pos += __popc(km);
     }
     __syncwarp();
 #pragma unroll
     for (int s = 0; s < kFrontier; ++s) {
-      const uint2 v = buf[(uint32_t)s * 32u + lane];
+      const uint2 v = child[(uint32_t)s * 32u + lane];
       st.fc[s] = __uint_as_float(v.x);
       st.fn[s] = v.y;
     }
+    load_entry(p, st.fn[0], st.rec);
     ctr.overflow += m - kFrontierCap;
-    st.used = kFrontier;
+    st.m = kFrontierCap;
   }
   __syncwarp();
-  return true;
 }
 
 // findNode1's cost model in batched rounds (every lane of the warp calls it with the same patch).
-__device__ uint32_t find_node_batched(const Patch &p, uint32_t n, SearchCounters &ctr) {
+__device__ __forceinline__ uint32_t find_node_batched(const Patch &p, uint32_t n, SearchCounters &ctr) {
   const uint32_t lane = threadIdx.x & 31u;
   __syncwarp();  // the warp's patch writes are visible to every lane
   const float kInf = __int_as_float(0x7f800000);
   const Box nbox = tree_box(p.t, p.chk(n));
   const float sarea = tree_sa(p.t, p.chk(n));
+  const PatchKeys keys(p.d);
   BatchedSearch st;
 #pragma unroll
   for (int s = 0; s < kFrontier; ++s) {
-    st.fc[s] = kInf;
-    st.fn[s] = kNone;
+    st.fc[s] = 0.0f;
+    st.fn[s] = p.root;
   }
-  if (lane == 0) {
-    st.fc[0] = 0.0f;
-    st.fn[0] = p.root;
-  }
-  st.used = 1;
-  st.haveRec = false;
+  load_entry(p, p.root, st.rec);
+  st.m = sarea < kInf ? 1u : 0u;  // the root's bound: 0 + sarea against no best yet
   st.bestCost = kInf;
-  st.best = 0;
-  uint2 *buf = child_buffer();
-  for (uint32_t round = 0;; ++round) {
-    if (round > p.numNodes) {  // bounded: every round evaluates at least one node
+  st.myCost = st.myEntry = kInf;
+  st.myNode = 0;
+  st.myRound = 0xFFFFFFFFu;
+  uint4 *buf = child_buffer();
+  for (st.round = 0; st.m != 0u; ++st.round) {
+    if (st.round > p.numNodes) {  // bounded: every round evaluates at least one node
       p.bad = true;
       break;
     }
-    const bool more = st.used <= 1   ? batched_round<1>(p, st, nbox, sarea, buf, ctr)
-                      : st.used <= 2 ? batched_round<2>(p, st, nbox, sarea, buf, ctr)
-                                     : batched_round<kFrontier>(p, st, nbox, sarea, buf, ctr);
-    if (!more) break;
+    if (st.m <= 32u) batched_round<1>(p, keys, st, nbox, sarea, buf, ctr);
+    else if (st.m <= 64u) batched_round<2>(p, keys, st, nbox, sarea, buf, ctr);
+    else batched_round<kFrontier>(p, keys, st, nbox, sarea, buf, ctr);
   }
+  // The first round that reached the best total, and its lowest (cost, node).
+  const uint32_t cost = f2ord(st.myCost);
+  uint32_t tied = __ballot_sync(kFull, cost == __reduce_min_sync(kFull, cost));
+  if (__popc(tied) > 1) {
+    const bool in0 = (tied >> lane) & 1u;
+    const uint32_t r = __reduce_min_sync(kFull, in0 ? st.myRound : 0xFFFFFFFFu);
+    const bool in1 = in0 && st.myRound == r;
+    const uint32_t c = __reduce_min_sync(kFull, in1 ? f2ord(st.myEntry) : 0xFFFFFFFFu);
+    const bool in2 = in1 && f2ord(st.myEntry) == c;
+    const uint32_t node = __reduce_min_sync(kFull, in2 ? st.myNode : 0xFFFFFFFFu);
+    tied = __ballot_sync(kFull, in2 && st.myNode == node);
+  }
+  const uint32_t best = __shfl_sync(kFull, st.myNode, __ffs(tied) - 1);
   __syncwarp();  // every lane is done reading the patch before it changes again
   p.bad = __any_sync(kFull, p.bad);
-  return st.best;
+  return best;
 }
 
 // reinsert (Bittner13CUDA.cu:308-358).
@@ -735,8 +778,6 @@ __device__ bool reinsert(Patch &p, uint32_t x, uint32_t unused, bool update, con
 // ---- per-item steps shared by the single-tree and the batched kernels ---------------------------
 // (t, root, numNodes) describe one tree; owner / counter point at that tree's entries; rank is the
 // item's position in its tree's chunk (lower rank wins a conflict).
-
-constexpr int kWarpItemsPerBlock = 4;
 
 // The patch storage of this warp (blocks of kWarpItemsPerBlock warps).
 __device__ __forceinline__ PatchData *warp_patch_data() {
