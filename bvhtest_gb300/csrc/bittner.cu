@@ -299,11 +299,9 @@ __global__ void __launch_bounds__(kWarpItemsPerBlock * 32) gain_warp_kernel(
   SearchCounters ctr = {0u, 0u};
   uint32_t ins[2], un[2], g = kNone;
   const uint32_t x = __ldg(cand + k);
-  const Heap unused{nullptr, nullptr};
   bool ok = x < numNodes;
   ok = ok && remove_node(p, x, ins, un, g);
-  ok = ok && reinsert<BVHGB_SEARCH_BATCHED>(p, ins[0], un[0], true, unused, 0, ctr);
-  ok = ok && reinsert<BVHGB_SEARCH_BATCHED>(p, ins[1], un[1], false, unused, 0, ctr);
+  ok = ok && reinsert_both(p, ins, un, ctr);
   if (p.bad) ok = false;
   float v = 0.0f;
   if (ok) v = isolated_gain(p, g, un[0], un[1], ok);

@@ -57,6 +57,25 @@ __device__ __forceinline__ Box tree_box(const bvhgb_node *t, uint32_t x) {
   r.mx[0] = a.w; r.mx[1] = b.x; r.mx[2] = b.y;
   return r;
 }
+// Links and box of a node, loaded together.
+struct NodeRec {
+  NodeP n;
+  Box b;
+};
+__device__ __forceinline__ NodeRec tree_rec(const bvhgb_node *t, uint32_t x) {
+  const float4 *p = reinterpret_cast<const float4 *>(t + x);
+  const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+  NodeRec r;
+  r.b.mn[0] = a.x; r.b.mn[1] = a.y; r.b.mn[2] = a.z;
+  r.b.mx[0] = a.w; r.b.mx[1] = b.x; r.b.mx[2] = b.y;
+  r.n.parent = __float_as_uint(b.z);
+  r.n.left = __float_as_uint(b.w);
+  r.n.right = __float_as_uint(c.x);
+  const uint32_t fl = __float_as_uint(c.y);
+  r.n.isLeafFlag = (uint16_t)(fl & 0xFFFFu);
+  r.n.isLeft = (uint16_t)(fl >> 16);
+  return r;
+}
 __device__ __forceinline__ float tree_sa(const bvhgb_node *t, uint32_t x) { return __ldg(&t[x].surfaceArea); }
 __device__ __forceinline__ bool tree_leaf(const bvhgb_node *t, uint32_t x) { return __ldg(&t[x].isLeafFlag) != 0; }
 
@@ -98,10 +117,16 @@ struct Patch {
     if (d->idx[3] == x) return 3;
     return kNone;
   }
-  __device__ uint32_t index(uint32_t x) const {
-    for (uint32_t i = 0; i < NSLOT; ++i)
-      if (d->idx[i] == x) return i;
-    return kNone;
+  // The first slot of x; every slot is read before the first compare (no chain of loads and exits).
+  __device__ __forceinline__ uint32_t index(uint32_t x) const {
+    uint32_t v[NSLOT];
+#pragma unroll
+    for (int i = 0; i < NSLOT; ++i) v[i] = d->idx[i];
+    uint32_t r = kNone;
+#pragma unroll
+    for (int i = NSLOT - 1; i >= 0; --i)
+      if (v[i] == x) r = (uint32_t)i;
+    return r;
   }
   __device__ NodeP get(uint32_t x) const {
     uint32_t i = index(x);
@@ -361,28 +386,46 @@ __device__ uint32_t find_node2(const Patch &p, uint32_t n, SearchCounters &ctr) 
   return best;
 }
 
-// removeNode (Bittner13CUDA.cu:267-305).
-__device__ bool remove_node(Patch &p, uint32_t x, uint32_t ins[2], uint32_t un[2], uint32_t &g_out) {
-  if (tree_leaf(p.t, p.chk(x)) || x == p.root) return false;
-  const uint32_t sn = p.patch_node(x, P_NODE);
-  const uint32_t s = p.sibling(p.d->nd[sn]);
-  const uint32_t pi = p.d->nd[sn].parent;
+// removeNode (Bittner13CUDA.cu:267-305) with patchAABBFrom(grand parent) written out. Every record is
+// loaded once and as soon as its index is known, all loads of a step before the first use of one:
+// node, parent, then grand parent and sibling, then the boxes around the grand parent are four
+// dependent round trips (slot by slot they were eight).
+__device__ __forceinline__ bool remove_node(Patch &p, uint32_t x, uint32_t ins[2], uint32_t un[2], uint32_t &g_out) {
+  NodeP nx = tree_node(p.t, p.chk(x));
+  if (nx.isLeafFlag || x == p.root) return false;
+  const uint32_t l = nx.left, r = nx.right, pi = nx.parent;
+  const NodeP np = tree_node(p.t, p.chk(pi));
+  const float sl = tree_sa(p.t, p.chk(l)), sr = tree_sa(p.t, p.chk(r));
   if (pi == p.root) return false;
-  const uint32_t ss = p.patch_node(s, P_SIBLING);
-  const uint32_t sp = p.patch_node(pi, P_PARENT);
-  const uint32_t gi = p.d->nd[sp].parent;
-  const uint32_t sg = p.patch_node(gi, P_GRAND_PARENT);
-  if (p.d->nd[sp].isLeft) {
-    p.d->nd[sg].left = s;
-    p.d->nd[ss].isLeft = 1;
-  } else {
-    p.d->nd[sg].right = s;
-    p.d->nd[ss].isLeft = 0;
+  const uint32_t s = nx.isLeft == 0 ? np.left : np.right, gi = np.parent;
+  NodeRec rs = tree_rec(p.t, p.chk(s));
+  NodeP ng = tree_node(p.t, p.chk(gi));
+  const uint32_t other = np.isLeft ? ng.right : ng.left;  // the grand parent's other child
+  const uint32_t ggi = ng.parent;
+  const Box ob = tree_box(p.t, p.chk(other));
+  const NodeP ngg = tree_node(p.t, p.chk(ggi));
+  if (np.isLeft) ng.left = s;
+  else ng.right = s;
+  rs.n.isLeft = np.isLeft ? 1 : 0;
+  rs.n.parent = gi;
+  Box b = np.isLeft ? rs.b : ob;  // the left child's box merged with the right's
+  merge_into(b, np.isLeft ? ob : rs.b);
+  p.d->idx[P_NODE] = x;
+  p.d->nd[P_NODE] = nx;
+  p.d->idx[P_SIBLING] = s;
+  p.d->nd[P_SIBLING] = rs.n;
+  p.d->idx[P_PARENT] = pi;
+  p.d->nd[P_PARENT] = np;
+  p.d->idx[P_GRAND_PARENT] = gi;
+  p.d->nd[P_GRAND_PARENT] = ng;
+  p.d->apath[0] = gi;
+  p.d->abox[0] = b;
+  if (gi != p.root) {
+    merge_into(b, tree_box(p.t, p.chk(ng.isLeft ? ngg.right : ngg.left)));
+    p.d->apath[1] = ggi;
+    p.d->abox[1] = b;
   }
-  p.d->nd[ss].parent = gi;
-  p.patch_aabb_from(gi, 0);
-  const uint32_t l = p.d->nd[sn].left, r = p.d->nd[sn].right;
-  if (tree_sa(p.t, p.chk(l)) > tree_sa(p.t, p.chk(r))) { ins[0] = l; ins[1] = r; }
+  if (sl > sr) { ins[0] = l; ins[1] = r; }
   else { ins[0] = r; ins[1] = l; }
   un[0] = x;
   un[1] = pi;
@@ -401,10 +444,10 @@ __device__ bool remove_node(Patch &p, uint32_t x, uint32_t ins[2], uint32_t un[2
 // and resolved after the last round. oracle/bittner.c (gpu_find_node_batched) restates the same
 // rounds.
 // Bound: the dependent chain of a round (a record's L2 round trip, the evaluation, the reduction,
-// the gather); a search takes 16 to 18 rounds, 6 to 14 entries each. Keeping the patch's keys in
-// registers, the best per lane and no bound test per entry shortened the chain: a chunk's launch
-// went from 29.6 to about 20.5 us on 65,536 triangles (41 items), from 51.7 to about 38 us on
-// 4.19M (2,621 items).
+// the gather); a search takes 16 to 18 rounds of 6 to 14 entries. With the patch's keys in
+// registers, the best per lane, no bound test per entry, records loaded side by side and one copy
+// of the search's code for both reinsertions a chunk's launch went from 29.6 to 18 us on 65,536
+// triangles (41 items) and from 51.7 to 35 us on 4.19M (2,621 items).
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kFrontier = 4;  // slots per lane (128 entries)
 constexpr uint32_t kFrontierCap = 32u * kFrontier;
@@ -531,32 +574,30 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
   const uint32_t ltMask = (1u << lane) - 1u;
   const float kInf = __int_as_float(0x7f800000);
   ctr.visits += st.m;
-  float induced[S];
-  uint32_t left[S], right[S];
+  float induced[S] = {};
+  uint32_t left[S] = {}, right[S] = {};
   uint32_t inner = 0;  // bit s: this lane's slot s holds an inner node
   float roundCost = kInf, roundEntry = kInf;
   uint32_t roundNode = kNone;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    induced[s] = kInf;
-    left[s] = right[s] = kNone;
-    if (S > 1 && (uint32_t)s * 32u + lane >= st.m) continue;
-    if (S == 1 && lane >= st.m) continue;
+    const bool live = (uint32_t)s * 32u + lane < st.m;  // other lanes compute on what they hold
     const uint32_t x = st.fn[s];
     float4 q[3];
     if (s == 0) {
       q[0] = st.rec[0]; q[1] = st.rec[1]; q[2] = st.rec[2];
     } else {
+      if (!live) continue;
       load_entry(p, x, q);
     }
-    if (x >= p.numNodes) p.bad = true;
+    if (live && x >= p.numNodes) p.bad = true;
     Box b;
     b.mn[0] = q[0].x; b.mn[1] = q[0].y; b.mn[2] = q[0].z;
     b.mx[0] = q[0].w; b.mx[1] = q[1].x; b.mx[2] = q[1].y;
     left[s] = __float_as_uint(q[1].w);
     right[s] = __float_as_uint(q[2].x);
     bool leaf = (__float_as_uint(q[2].y) & 0xFFFFu) != 0u;
-    if (keys.patched(x)) {
+    if (live && keys.patched(x)) {
       NodeP n;
       p.subset_aabb_from(x, q[0], q[1], q[2], n, b);
       left[s] = n.left;
@@ -567,13 +608,13 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
     merge_into(b, nbox);
     const float total = fadd(st.fc[s], surface_area(b));
     induced[s] = fadd(ind, total);
-    inner |= (leaf ? 0u : 1u) << s;
+    inner |= (live && !leaf ? 1u : 0u) << s;
     if (S == 1) {
-      roundCost = total;
+      roundCost = live ? total : kInf;
       roundEntry = st.fc[s];
       roundNode = x;
-    } else if (total < roundCost ||
-               (total == roundCost && (st.fc[s] < roundEntry || (st.fc[s] == roundEntry && x < roundNode)))) {
+    } else if (live && (total < roundCost || (total == roundCost && (st.fc[s] < roundEntry ||
+                                                                 (st.fc[s] == roundEntry && x < roundNode))))) {
       roundCost = total;
       roundEntry = st.fc[s];
       roundNode = x;
@@ -589,18 +630,22 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
   }
   // Children of the expanded entries: the k-th expanded entry (slot-major, then lane) writes
   // children 2k and 2k + 1 to the warp's buffer.
+  // Rounds of one slot use the buffer's first two quarters in turn, so a round's writes never meet
+  // the previous round's reads; wider rounds wait for those reads.
+  if (S > 1) __syncwarp();
+  else buf += (st.round & 1u) * 32u;
   uint32_t m = 0;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const bool kids = ((inner >> s) & 1u) && fadd(induced[s], sarea) < st.bestCost;
     const uint32_t kmask = __ballot_sync(kFull, kids);
     const uint32_t mk = 2u * __popc(kmask);
-    if (kids) {
-      buf[m / 2 + __popc(kmask & ltMask)] = make_uint4(__float_as_uint(induced[s]), left[s], __float_as_uint(induced[s]), right[s]);
-      if (m + mk > 32u) {  // children past slot 0: warm their records in L2
-        if (left[s] < p.numNodes) prefetch_node(p.t, left[s]);
-        if (right[s] < p.numNodes) prefetch_node(p.t, right[s]);
-      }
+    if (kids)
+      buf[m / 2 + __popc(kmask & ltMask)] =
+          make_uint4(__float_as_uint(induced[s]), left[s], __float_as_uint(induced[s]), right[s]);
+    if (m + mk > 32u && kids) {  // children past slot 0: warm their records in L2
+      if (left[s] < p.numNodes) prefetch_node(p.t, left[s]);
+      if (right[s] < p.numNodes) prefetch_node(p.t, right[s]);
     }
     m += mk;
   }
@@ -684,7 +729,8 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
     ctr.overflow += m - kFrontierCap;
     st.m = kFrontierCap;
   }
-  __syncwarp();
+  // A one-slot round may follow and write either quarter before every lane has read this one.
+  if (S > 1) __syncwarp();
 }
 
 // findNode1's cost model in batched rounds (every lane of the warp calls it with the same patch).
@@ -739,19 +785,27 @@ __device__ __forceinline__ uint32_t find_node_batched(const Patch &p, uint32_t n
 // MODE: BVHGB_SEARCH_BATCHED (warp-cooperative), BVHGB_SEARCH_HEAP (findNode1) or
 // BVHGB_SEARCH_ALT (findNode2).
 template <int MODE>
-__device__ bool reinsert(Patch &p, uint32_t x, uint32_t unused, bool update, const Heap &pq, uint32_t cap,
-                         SearchCounters &ctr) {
+__device__ __forceinline__ bool reinsert(Patch &p, uint32_t x, uint32_t unused, bool update, const Heap &pq,
+                                         uint32_t cap, SearchCounters &ctr) {
   const uint32_t best = MODE == BVHGB_SEARCH_BATCHED ? find_node_batched(p, x, ctr)
                         : MODE == BVHGB_SEARCH_ALT   ? find_node2(p, x, ctr)
                                                      : find_node(p, x, pq, cap, ctr);
   if (best == p.root) return false;
+  const NodeP nx = tree_node(p.t, p.chk(x)), nb = tree_node(p.t, p.chk(best));
   const uint32_t bpi = p.index(best);
-  uint32_t sb;
-  if (bpi == kNone) sb = p.patch_node(best, update ? P_1ST_BEST : P_2ND_BEST);
-  else if (bpi == P_GRAND_PARENT) sb = P_GRAND_PARENT;
-  else sb = p.move(bpi, update ? P_1ST_BEST : P_2ND_BEST);
-  const uint32_t sx = p.patch_node(x, update ? P_1ST_INSERT : P_2ND_INSERT);
+  uint32_t sb = update ? P_1ST_BEST : P_2ND_BEST;
+  const uint32_t sx = update ? P_1ST_INSERT : P_2ND_INSERT;
   const uint32_t su = update ? P_NODE : P_PARENT;
+  if (bpi == kNone) {
+    p.d->idx[sb] = best;
+    p.d->nd[sb] = nb;
+  } else if (bpi == P_GRAND_PARENT) {
+    sb = P_GRAND_PARENT;
+  } else {
+    p.move(bpi, sb);
+  }
+  p.d->idx[sx] = x;
+  p.d->nd[sx] = nx;
   const uint32_t ri = p.d->nd[sb].parent;
   const uint32_t rpi = p.index(ri);
   const uint32_t sr = rpi == kNone ? p.patch_node(ri, update ? P_1ST_ROOT : P_2ND_ROOT)
@@ -774,6 +828,15 @@ __device__ bool reinsert(Patch &p, uint32_t x, uint32_t unused, bool update, con
   return true;
 }
 
+// Both reinsertions of a removed node on a whole warp: one copy of the search's code for the two
+// (a launch starts with cold instruction caches).
+__device__ __forceinline__ bool reinsert_both(Patch &p, const uint32_t ins[2], const uint32_t un[2], SearchCounters &ctr) {
+  const Heap unused{nullptr, nullptr};
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k)
+    if (!reinsert<BVHGB_SEARCH_BATCHED>(p, k ? ins[1] : ins[0], k ? un[1] : un[0], k == 0, unused, 0, ctr)) return false;
+  return true;
+}
 
 // ---- per-item steps shared by the single-tree and the batched kernels ---------------------------
 // (t, root, numNodes) describe one tree; owner / counter point at that tree's entries; rank is the
@@ -801,24 +864,23 @@ __device__ __forceinline__ void warp_patch_item(const bvhgb_node *__restrict__ t
   p.clear();
   SearchCounters ctr = {0u, 0u};
   uint32_t ins[2], un[2], g = kNone;
-  const Heap unused{nullptr, nullptr};
   ok = ok && remove_node(p, node, ins, un, g);
-  ok = ok && reinsert<BVHGB_SEARCH_BATCHED>(p, ins[0], un[0], true, unused, 0, ctr);
-  ok = ok && reinsert<BVHGB_SEARCH_BATCHED>(p, ins[1], un[1], false, unused, 0, ctr);
+  ok = ok && reinsert_both(p, ins, un, ctr);
+  p.bad = __any_sync(kFull, p.bad);
   if (p.bad) ok = false;
   __syncwarp();
+  if (lane < NSLOT) {  // a lane per slot
+    const uint32_t y = ok ? p.d->idx[lane] : kNone;
+    out->idx[lane] = y;
+    out->nd[lane] = p.d->nd[lane];
+    if (y != kNone) atomicMin(&owner[y], rank);
+  }
   if (lane != 0) return;
   if (p.bad) atomicOr(err, kErrBadIndex);
   *valid = ok ? 1u : 0u;
   toFix3[0] = ok ? g : kNone;
   toFix3[1] = ok ? un[0] : kNone;
   toFix3[2] = ok ? un[1] : kNone;
-#pragma unroll
-  for (int s = 0; s < NSLOT; ++s) {
-    out->nd[s] = p.d->nd[s];
-    out->idx[s] = ok ? p.d->idx[s] : kNone;
-    if (ok && p.d->idx[s] != kNone) atomicMin(&owner[p.d->idx[s]], rank);
-  }
   if (!ok) atomicAdd(&stats[S_INVALID], 1ull);
   if (ctr.overflow) atomicAdd(&stats[S_OVERFLOW], (unsigned long long)ctr.overflow);
   atomicAdd(&stats[S_VISITS], (unsigned long long)ctr.visits);
