@@ -26,21 +26,17 @@ namespace {
 constexpr int kIn = kMlpIn, kH = kMlpHidden;
 constexpr int oW1 = 0, oB1 = oW1 + kH * kIn, oW2 = oB1 + kH, oB2 = oW2 + kH * kH, oW3 = oB2 + kH, oB3 = oW3 + kH;
 static_assert(oB3 + 1 == kMlpParams, "parameter layout");
-constexpr int kWPad = (kMlpParams + 3) & ~3;
 
 constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2 / pi)
 constexpr float kGeluA = 0.044715f;
 
-__device__ __forceinline__ float gelu(float z) {
-  const float u = kGeluC * (z + kGeluA * z * z * z);
-  return 0.5f * z * (1.0f + tanhf(u));
-}
-__device__ __forceinline__ float gelu_grad(float z) {
+// gelu(z) and gelu'(z) from one tanh.
+__device__ __forceinline__ float gelu_both(float z, float &slope) {
   const float u = kGeluC * (z + kGeluA * z * z * z);
   const float t = tanhf(u);
-  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * z * z);
+  slope = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * z * z);
+  return 0.5f * z * (1.0f + t);
 }
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Inference GELU: tanh(u) = 1 - 2 / (1 + e^(2u)), e^(2u) = 2^(2u / ln 2) from the hardware's
 // approximate base-2 exponential and 1 / (1 + e^(2u)) from its approximate reciprocal (relative
@@ -61,24 +57,6 @@ __device__ __forceinline__ float gelu_fast(float z) {
 __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
   const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t *>(&p);
-}
-
-__device__ __forceinline__ void load_row(const uint16_t *__restrict__ x, size_t row, float in[kIn]) {
-  const uint4 *p = reinterpret_cast<const uint4 *>(x + row * kIn);
-#pragma unroll
-  for (int w = 0; w < 3; ++w) {
-    const uint4 v = __ldg(p + w);
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      in[w * 8 + h * 2 + 0] = __uint_as_float(u[h] << 16);
-      in[w * 8 + h * 2 + 1] = __uint_as_float(u[h] & 0xFFFF0000u);
-    }
-  }
-}
-
-__device__ __forceinline__ void load_weights(const __nv_bfloat16 *__restrict__ w, float *W) {
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) W[i] = __bfloat162float(w[i]);
 }
 
 // ---- inference on the 5th-generation tensor cores (tcgen05) ----------------------------------------
@@ -343,12 +321,23 @@ __global__ void __launch_bounds__(128, 4) mlp_forward_tc_kernel(const __nv_bfloa
 // The two gradient rounding points (dZ2, dZ1 to BF16) are the tensor cores' operand type; the FP64
 // oracle (oracle/mlp.py) rounds at the same places. Sums over the tile run in a fixed order, so a
 // training step repeats bit for bit.
-constexpr int kTile = 128;                 // samples per block, 4 warps
+//
+// Bound: the latency of one tile's chain at 64 CTAs (batch 8,192), one per SM, so the warps of a
+// tile matter, not their number on the chip: eight warps (a 16-sample row tile each; two warps per
+// 16 units of the weight gradients) and 16-byte weight loads. A sum keeps its order whatever warp
+// makes it, so the gradients are those of four warps bit for bit.
+constexpr int kTile = 128;                 // samples per block
+constexpr int kTrainThreads = 256;
+constexpr int kTrainWarps = kTrainThreads / 32;
 constexpr int kK1 = 32;                    // layer-1 K: 24 features + 8 zeros
 constexpr int kSX = 40;                    // bf16 row strides chosen so fragment loads hit distinct banks
 constexpr int kSH = 72;
-constexpr int kSZ = 68;                    // fp32 row stride of the pre-activations
-constexpr size_t kTrainSmem = sizeof(float) * (kWPad + 2 * kTile * kSZ + kTile) +
+constexpr int kSZ = 68;                    // fp32 row stride of the GELU slopes
+constexpr int kBias = 3 * kH + 1;          // b1, b2, W3, b3 as FP32
+constexpr int kBiasPad = (kBias + 3) & ~3;
+static_assert(kTile == 16 * kTrainWarps && kH == 64, "one row tile per warp, two warps per 16 units");
+static_assert(oW2 % 8 == 0 && oB1 % 8 == 0 && kIn % 8 == 0, "16-byte weight loads");
+constexpr size_t kTrainSmem = sizeof(float) * (kBiasPad + 2 * kTile * kSZ + kTile) + sizeof(uint32_t) * kTile +
                               sizeof(uint16_t) * (kH * kSX + 2 * kH * kSH + kTile * kSX + 3 * kTile * kSH);
 
 __device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], const uint32_t b[2]) {
@@ -391,19 +380,39 @@ __device__ __forceinline__ void frag_b_t(const uint16_t *m, int stride, int k0, 
   b[1] = pack2(p[8 * stride], p[9 * stride]);
 }
 
-__global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *__restrict__ w,
-                                                          const uint16_t *__restrict__ x, const float *__restrict__ tgt,
-                                                          const uint32_t *__restrict__ index, uint32_t n, float scaleN,
-                                                          float *__restrict__ part, float *__restrict__ lossBase,
-                                                          const uint32_t *__restrict__ stepDev, uint32_t step0,
-                                                          uint32_t lossCap) {
+// Row of position i in the batch of step t: SplitMix64 of (seed, t, i), reduced modulo the samples.
+__device__ __forceinline__ uint32_t batch_row(uint64_t seed, uint64_t t, uint32_t batch, uint32_t i, uint32_t numSamples) {
+  uint64_t z = seed + 0x9E3779B97F4A7C15ull * (t * (uint64_t)batch + i + 1);
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  z ^= z >> 31;
+  return (uint32_t)(z % numSamples);
+}
+
+// The next launch of the stream may start now; what it needs of this one it waits for itself.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Everything the launches before this one wrote is visible from here on.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// n samples; with numSamples > 0 sample s is row batch_row(seed, step, n, s, numSamples) of x,
+// otherwise row s. The tile's loss goes to *loss.
+__global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const __nv_bfloat16 *__restrict__ w,
+                                                                  const uint16_t *__restrict__ x,
+                                                                  const float *__restrict__ tgt, uint32_t n,
+                                                                  uint32_t numSamples, uint64_t seed, uint64_t step,
+                                                                  float scaleN, float *__restrict__ part,
+                                                                  float *__restrict__ loss) {
   extern __shared__ __align__(16) float sm[];
   float *grad = part + (size_t)blockIdx.x * kMlpParams;
-  float *W = sm;                       // fp32 copy of the (BF16) parameters: biases and W3
-  float *Z1 = W + kWPad;               // [q][j] pre-activations
-  float *Z2 = Z1 + kTile * kSZ;
-  float *dY = Z2 + kTile * kSZ;
-  uint16_t *sW1 = reinterpret_cast<uint16_t *>(dY + kTile);  // [j][f], f padded to 32
+  float *B1 = sm;                      // fp32 copies of the (BF16) biases and W3
+  float *B2 = B1 + kH;
+  float *W3 = B2 + kH;
+  float *B3 = W3 + kH;
+  float *G1 = sm + kBiasPad;           // [q][j] gelu'(Z1)
+  float *G2 = G1 + kTile * kSZ;        // [q][j] gelu'(Z2)
+  float *dY = G2 + kTile * kSZ;
+  uint32_t *rows = reinterpret_cast<uint32_t *>(dY + kTile);
+  uint16_t *sW1 = reinterpret_cast<uint16_t *>(rows + kTile);  // [j][f], f padded to 32
   uint16_t *sW2 = sW1 + kH * kSX;                             // [j][i]
   uint16_t *sW2T = sW2 + kH * kSH;                            // [i][j]
   uint16_t *sX = sW2T + kH * kSH;                             // [q][f]
@@ -413,45 +422,51 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const int g = (int)(lane >> 2), t = (int)(lane & 3u);
   const uint16_t *wb = reinterpret_cast<const uint16_t *>(w);
-  for (int i = tid; i < kMlpParams; i += kTile) W[i] = bf16_val(__ldg(wb + i));
-  for (int i = tid; i < kH * kK1; i += kTile) {
-    const int j = i / kK1, f = i % kK1;
-    sW1[j * kSX + f] = f < kIn ? __ldg(wb + oW1 + j * kIn + f) : (uint16_t)0;
-  }
-  for (int i = tid; i < kH * kH; i += kTile) {
-    const int j = i / kH, k = i % kH;
-    const uint16_t v = __ldg(wb + oW2 + i);
-    sW2[j * kSH + k] = v;
-    sW2T[k * kSH + j] = v;
-  }
-  {
+  grid_release();
+  // The samples do not depend on earlier steps: they are gathered before the weights are waited for.
+  if (tid < (uint32_t)kTile) {
     const uint32_t s = blockIdx.x * kTile + tid;
     const bool live = s < n;
-    const uint32_t row = live ? (index ? __ldg(index + s) : s) : 0u;
+    const uint32_t row = live ? (numSamples ? batch_row(seed, step, n, s, numSamples) : s) : 0u;
+    rows[tid] = row;
     const uint4 *p = reinterpret_cast<const uint4 *>(x + (size_t)row * kIn);
-    uint32_t *dst = reinterpret_cast<uint32_t *>(sX + tid * kSX);
+    uint4 *dst = reinterpret_cast<uint4 *>(sX + tid * kSX);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const uint4 v = live ? __ldg(p + c) : make_uint4(0u, 0u, 0u, 0u);
-      dst[4 * c + 0] = v.x;
-      dst[4 * c + 1] = v.y;
-      dst[4 * c + 2] = v.z;
-      dst[4 * c + 3] = v.w;
-    }
-#pragma unroll
-    for (int c = 12; c < kK1 / 2; ++c) dst[c] = 0u;
+    for (int c = 0; c < 3; ++c) dst[c] = live ? __ldg(p + c) : make_uint4(0u, 0u, 0u, 0u);
+    dst[3] = make_uint4(0u, 0u, 0u, 0u);
   }
+  grid_wait();
+  for (int i = tid; i < kH * kIn / 8; i += kTrainThreads) {
+    const int j = i / (kIn / 8), c = i % (kIn / 8);
+    *reinterpret_cast<uint4 *>(sW1 + j * kSX + 8 * c) = __ldcg(reinterpret_cast<const uint4 *>(wb + oW1) + i);
+    if (c == 0) *reinterpret_cast<uint4 *>(sW1 + j * kSX + kIn) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  for (int i = tid; i < kH * kH / 8; i += kTrainThreads) {
+    const int j = i / (kH / 8), c = i % (kH / 8);
+    const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(wb + oW2) + i);
+    *reinterpret_cast<uint4 *>(sW2 + j * kSH + 8 * c) = v;
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      sW2T[(8 * c + 2 * h) * kSH + j] = (uint16_t)u[h];
+      sW2T[(8 * c + 2 * h + 1) * kSH + j] = (uint16_t)(u[h] >> 16);
+    }
+  }
+  if (tid < (uint32_t)kBias) {
+    const int i = (int)tid;
+    B1[i] = bf16_val(__ldcg(wb + (i < kH ? oB1 + i : oB2 + (i - kH))));  // b2, W3 and b3 lie in a row
+  }
+  static_assert(oW3 == oB2 + kH && oB3 == oW3 + kH, "b2, W3 and b3 lie in a row");
   __syncthreads();
 
-  // ---- forward: warp w owns samples [32w, 32w + 32), two 16-row tiles ----
-  const int q0 = 32 * (int)warp;
-  float yPart[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};  // [tile][row g / g + 8]
-  for (int mt = 0; mt < 2; ++mt) {
-    const int r0 = q0 + 16 * mt;
+  // ---- forward: warp w owns samples [16w, 16w + 16) ----
+  const int r0 = 16 * (int)warp;
+  float yPart[2] = {0.0f, 0.0f};  // rows g, g + 8
+  {
     float acc[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      const float b0 = W[oB1 + 8 * nt + 2 * t], b1v = W[oB1 + 8 * nt + 2 * t + 1];
+      const float b0 = B1[8 * nt + 2 * t], b1v = B1[8 * nt + 2 * t + 1];
       acc[nt][0] = b0;
       acc[nt][1] = b1v;
       acc[nt][2] = b0;
@@ -473,20 +488,19 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int q = r0 + g + 8 * h, j = 8 * nt + 2 * t;
-        Z1[q * kSZ + j] = acc[nt][2 * h];
-        Z1[q * kSZ + j + 1] = acc[nt][2 * h + 1];
-        sA1[q * kSH + j] = bf16_u16(gelu(acc[nt][2 * h]));
-        sA1[q * kSH + j + 1] = bf16_u16(gelu(acc[nt][2 * h + 1]));
+        float s0, s1;
+        const float a0 = gelu_both(acc[nt][2 * h], s0), a1 = gelu_both(acc[nt][2 * h + 1], s1);
+        *reinterpret_cast<float2 *>(G1 + q * kSZ + j) = make_float2(s0, s1);
+        *reinterpret_cast<uint32_t *>(sA1 + q * kSH + j) = pack2(bf16_u16(a0), bf16_u16(a1));
       }
     }
   }
   __syncwarp();
-  for (int mt = 0; mt < 2; ++mt) {
-    const int r0 = q0 + 16 * mt;
+  {
     float acc[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-      const float b0 = W[oB2 + 8 * nt + 2 * t], b1v = W[oB2 + 8 * nt + 2 * t + 1];
+      const float b0 = B2[8 * nt + 2 * t], b1v = B2[8 * nt + 2 * t + 1];
       acc[nt][0] = b0;
       acc[nt][1] = b1v;
       acc[nt][2] = b0;
@@ -508,55 +522,49 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int q = r0 + g + 8 * h, j = 8 * nt + 2 * t;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float z = acc[nt][2 * h + e];
-          Z2[q * kSZ + j + e] = z;
-          const uint16_t a2 = bf16_u16(gelu(z));
-          sD1[q * kSH + j + e] = a2;  // the layer-2 activations, until dZ1 takes the buffer
-          yPart[mt][h] += W[oW3 + j + e] * bf16_val(a2);
-        }
+        float s0, s1;
+        const uint16_t a0 = bf16_u16(gelu_both(acc[nt][2 * h], s0)), a1 = bf16_u16(gelu_both(acc[nt][2 * h + 1], s1));
+        *reinterpret_cast<float2 *>(G2 + q * kSZ + j) = make_float2(s0, s1);
+        *reinterpret_cast<uint32_t *>(sD1 + q * kSH + j) = pack2(a0, a1);  // until dZ1 takes the buffer
+        yPart[h] += W3[j] * bf16_val(a0);
+        yPart[h] += W3[j + 1] * bf16_val(a1);
       }
     }
   }
   // y of each row: the four lanes of a quad hold its 64 columns
   float lsum = 0.0f;
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float v = yPart[mt][h];
-      v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-      v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-      const int q = q0 + 16 * mt + g + 8 * h;
-      const uint32_t s = blockIdx.x * kTile + q;
-      const bool live = s < n;
-      const uint32_t row = live ? (index ? __ldg(index + s) : s) : 0u;
-      const float yv = W[oB3] + v;
-      const float diff = live ? yv - __ldg(tgt + row) : 0.0f;
-      if (t == 0) {
-        dY[q] = 2.0f * diff / scaleN;
-        lsum += diff * diff / scaleN;
-      }
+  for (int h = 0; h < 2; ++h) {
+    float v = yPart[h];
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+    const int q = r0 + g + 8 * h;
+    const bool live = blockIdx.x * kTile + q < n;
+    const float yv = B3[0] + v;
+    const float diff = live ? yv - __ldg(tgt + rows[q]) : 0.0f;
+    if (t == 0) {
+      dY[q] = 2.0f * diff / scaleN;
+      lsum += diff * diff / scaleN;
     }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xFFFFFFFFu, lsum, o);
-  if (lane == 0) {
-    uint32_t slot = 0;
-    if (stepDev) slot = *stepDev - step0;
-    if (slot < lossCap) atomicAdd(lossBase + slot, lsum);
-  }
+  if (lane == 0) atomicAdd(loss, lsum);
   __syncwarp();
   // dZ2 of the warp's rows
-  for (int i = lane; i < 32 * kH; i += 32) {
-    const int q = q0 + i / kH, j = i % kH;
-    sD2[q * kSH + j] = bf16_u16(dY[q] * W[oW3 + j] * gelu_grad(Z2[q * kSZ + j]));
+#pragma unroll 4
+  for (int i = lane; i < 16 * kH / 2; i += 32) {
+    const int q = r0 + i / (kH / 2), j = 2 * (i % (kH / 2));
+    const float2 s = *reinterpret_cast<const float2 *>(G2 + q * kSZ + j);
+    *reinterpret_cast<uint32_t *>(sD2 + q * kSH + j) =
+        pack2(bf16_u16(dY[q] * W3[j] * s.x), bf16_u16(dY[q] * W3[j + 1] * s.y));
   }
   __syncthreads();
   // dW3[j] = sum_q dY[q] A2[q][j], db3 = sum_q dY[q]: a warp per unit, lanes over samples
-  for (int j = warp; j < kH; j += kTile / 32) {
+#pragma unroll 4
+  for (int j = warp; j < kH; j += kTrainWarps) {
     float gsum = 0.0f;
+#pragma unroll
     for (int q = lane; q < kTile; q += 32) gsum += dY[q] * bf16_val(sD1[q * kSH + j]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xFFFFFFFFu, gsum, o);
@@ -571,62 +579,56 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
   }
   // dA1 = dZ2 . W2 for the warp's rows (registers), then dZ1 once every warp has read the
   // activations out of sD1
-  float dacc[2][8][4];
+  float dacc[8][4];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
-    const int r0 = q0 + 16 * mt;
+  for (int nt = 0; nt < 8; ++nt) dacc[nt][0] = dacc[nt][1] = dacc[nt][2] = dacc[nt][3] = 0.0f;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) dacc[mt][nt][0] = dacc[mt][nt][1] = dacc[mt][nt][2] = dacc[mt][nt][3] = 0.0f;
-#pragma unroll
-    for (int k0 = 0; k0 < kH; k0 += 16) {
-      uint32_t a[4];
-      frag_a(sD2, kSH, r0, k0, g, t, a);
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        uint32_t b[2];
-        frag_b(sW2T, kSH, k0, 8 * nt, g, t, b);
-        mma16816(dacc[mt][nt], a, b);
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
+  for (int k0 = 0; k0 < kH; k0 += 16) {
+    uint32_t a[4];
+    frag_a(sD2, kSH, r0, k0, g, t, a);
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = q0 + 16 * mt + g + 8 * h, i = 8 * nt + 2 * t;
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          sD1[q * kSH + i + e] = bf16_u16(dacc[mt][nt][2 * h + e] * gelu_grad(Z1[q * kSZ + i + e]));
-      }
+      uint32_t b[2];
+      frag_b(sW2T, kSH, k0, 8 * nt, g, t, b);
+      mma16816(dacc[nt], a, b);
     }
   }
   __syncthreads();
-  // ---- weight gradients: warp w owns units [16w, 16w + 16), K = the tile's samples ----
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = r0 + g + 8 * h, i = 8 * nt + 2 * t;
+      const float2 s = *reinterpret_cast<const float2 *>(G1 + q * kSZ + i);
+      *reinterpret_cast<uint32_t *>(sD1 + q * kSH + i) =
+          pack2(bf16_u16(dacc[nt][2 * h] * s.x), bf16_u16(dacc[nt][2 * h + 1] * s.y));
+    }
+  }
+  __syncthreads();
+  // ---- weight gradients: warps w and w + 4 own units [16w, 16w + 16) (w < 4), each half of the
+  // columns; K = the tile's samples ----
   {
-    const int j0 = 16 * (int)warp;
-    float g2[8][4], g1[4][4];
+    const int j0 = 16 * (int)(warp & 3u), half = (int)(warp >> 2);
+    float g2[4][4], g1[2][4];
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) g2[nt][0] = g2[nt][1] = g2[nt][2] = g2[nt][3] = 0.0f;
+    for (int nt = 0; nt < 4; ++nt) g2[nt][0] = g2[nt][1] = g2[nt][2] = g2[nt][3] = 0.0f;
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) g1[nt][0] = g1[nt][1] = g1[nt][2] = g1[nt][3] = 0.0f;
-#pragma unroll 2
+    for (int nt = 0; nt < 2; ++nt) g1[nt][0] = g1[nt][1] = g1[nt][2] = g1[nt][3] = 0.0f;
+#pragma unroll 4
     for (int k0 = 0; k0 < kTile; k0 += 16) {
       uint32_t a2[4], a1[4];
       frag_a_t(sD2, kSH, j0, k0, g, t, a2);
       frag_a_t(sD1, kSH, j0, k0, g, t, a1);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
+      for (int nt = 0; nt < 4; ++nt) {
         uint32_t b[2];
-        frag_b_t(sA1, kSH, k0, 8 * nt, g, t, b);
+        frag_b_t(sA1, kSH, k0, 32 * half + 8 * nt, g, t, b);
         mma16816(g2[nt], a2, b);
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < 2; ++nt) {
         uint32_t b[2];
-        frag_b_t(sX, kSX, k0, 8 * nt, g, t, b);
+        frag_b_t(sX, kSX, k0, 16 * half + 8 * nt, g, t, b);
         mma16816(g1[nt], a1, b);
       }
     }
@@ -634,23 +636,25 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
     for (int h = 0; h < 2; ++h) {
       const int j = j0 + g + 8 * h;
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        grad[oW2 + j * kH + 8 * nt + 2 * t] = g2[nt][2 * h];
-        grad[oW2 + j * kH + 8 * nt + 2 * t + 1] = g2[nt][2 * h + 1];
+      for (int nt = 0; nt < 4; ++nt) {
+        grad[oW2 + j * kH + 32 * half + 8 * nt + 2 * t] = g2[nt][2 * h];
+        grad[oW2 + j * kH + 32 * half + 8 * nt + 2 * t + 1] = g2[nt][2 * h + 1];
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int f = 8 * nt + 2 * t + e;
+          const int f = 16 * half + 8 * nt + 2 * t + e;
           if (f < kIn) grad[oW1 + j * kIn + f] = g1[nt][2 * h + e];
         }
       }
     }
   }
   // bias gradients: a warp per unit, lanes over samples
-  for (int j = warp; j < kH; j += kTile / 32) {
+#pragma unroll 4
+  for (int j = warp; j < kH; j += kTrainWarps) {
     float b2 = 0.0f, b1 = 0.0f;
+#pragma unroll
     for (int q = lane; q < kTile; q += 32) {
       b2 += bf16_val(sD2[q * kSH + j]);
       b1 += bf16_val(sD1[q * kSH + j]);
@@ -667,57 +671,63 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const __nv_bfloat16 *_
   }
 }
 
-// g = the sum of the tiles' gradient rows, in tile order.
-__global__ void grad_reduce_kernel(const float *__restrict__ part, uint32_t tiles, float *__restrict__ g) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (uint32_t)kMlpParams) return;
+// Parameter i's gradient: the sum of the tiles' rows in tile order (the loads of 32 tiles are in
+// flight together).
+__device__ __forceinline__ float tile_sum(const float *part, uint32_t tiles, uint32_t i) {
   float acc = 0.0f;
-  for (uint32_t b = 0; b < tiles; ++b) acc += part[(size_t)b * kMlpParams + i];
-  g[i] = acc;
+  uint32_t b = 0;
+  for (; b + 32 <= tiles; b += 32) {
+    float v[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = __ldcg(part + (size_t)(b + k) * kMlpParams + i);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) acc += v[k];
+  }
+  for (; b < tiles; ++b) acc += __ldcg(part + (size_t)b * kMlpParams + i);
+  return acc;
 }
 
-// AdamW (Loshchilov and Hutter) on all parameters in one block: moments, bias correction with the
-// step count t = *stepDev + 1, decoupled weight decay on weights only; refreshes the BF16 copy,
-// clears the gradient and advances the device step counter.
-__global__ void __launch_bounds__(1024) adamw_kernel(float *__restrict__ p, __nv_bfloat16 *__restrict__ pb,
-                                                     float *__restrict__ g, float *__restrict__ m,
-                                                     float *__restrict__ v, uint32_t *stepDev, float lr, float wd) {
+__global__ void grad_reduce_kernel(const float *__restrict__ part, uint32_t tiles, float *__restrict__ g) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < (uint32_t)kMlpParams) g[i] = tile_sum(part, tiles, i);
+}
+
+// AdamW (Loshchilov and Hutter), step t (from 1), on the tiles' gradient rows: one thread per
+// parameter sums its gradient, advances the moments and the parameter (bias correction, decoupled
+// weight decay on weights only) and refreshes the BF16 copy. 92 blocks of two warps: the kernel is
+// one parameter's chain of loads. A step of batch 8,192 takes 18 us in two overlapping launches; in
+// four (batch rows, a four-warp tile, the sum, a one-block update) it took 43.
+constexpr int kAdamThreads = 64;
+__global__ void __launch_bounds__(kAdamThreads) adamw_kernel(const float *__restrict__ part, uint32_t tiles,
+                                                             float *__restrict__ p, __nv_bfloat16 *__restrict__ pb,
+                                                             float *__restrict__ m, float *__restrict__ v,
+                                                             uint32_t *__restrict__ stepDev, uint32_t step, float lr,
+                                                             float wd) {
+  grid_release();
+  grid_wait();
+  const uint32_t i = blockIdx.x * kAdamThreads + threadIdx.x;
+  if (i == 0) *stepDev = step;
+  if (i >= (uint32_t)kMlpParams) return;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float t = (float)(*stepDev + 1u);
+  const float t = (float)step;
   const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const bool bias = (i >= oB1 && i < oW2) || (i >= oB2 && i < oW3) || i == oB3;
-    float pi = p[i];
-    if (!bias) pi -= lr * wd * pi;
-    pi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    p[i] = pi;
-    pb[i] = __float2bfloat16_rn(pi);
-    g[i] = 0.0f;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) *stepDev += 1u;
+  const float m0 = m[i], v0 = v[i];
+  float pi = p[i];
+  const float gi = tile_sum(part, tiles, i);
+  // one fused rounding each, written out: the trained weights must not depend on how they are compiled
+  const float mi = __fmaf_rn(1.0f - b1, gi, __fmul_rn(b1, m0));
+  const float vi = __fmaf_rn(__fmul_rn(1.0f - b2, gi), gi, __fmul_rn(b2, v0));
+  m[i] = mi;
+  v[i] = vi;
+  const bool bias = ((int)i >= oB1 && (int)i < oW2) || ((int)i >= oB2 && (int)i < oW3) || (int)i == oB3;
+  if (!bias) pi -= lr * wd * pi;
+  pi -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = pi;
+  pb[i] = __float2bfloat16_rn(pi);
 }
 
 __global__ void to_bf16_kernel(const float *__restrict__ p, __nv_bfloat16 *__restrict__ pb, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) pb[i] = __float2bfloat16_rn(p[i]);
-}
-
-// Batch rows for step t = *stepDev + 1: SplitMix64 of (seed, t, i), reduced modulo numSamples.
-__global__ void batch_index_kernel(uint32_t *__restrict__ idx, uint32_t batch, uint32_t numSamples, uint64_t seed,
-                                   const uint32_t *__restrict__ stepDev) {
-  const uint64_t t = (uint64_t)*stepDev + 1u;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
-    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (t * (uint64_t)batch + i + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    idx[i] = (uint32_t)(z % numSamples);
-  }
 }
 
 // ---- features ----------------------------------------------------------------------------------
@@ -1074,8 +1084,7 @@ struct bvhgb_mlp {
   __nv_bfloat16 *pb = nullptr;
   uint32_t *stepDev = nullptr;
   uint32_t *err = nullptr;  // error bits of the inference kernel (kErrTimeout)
-  uint32_t *idx = nullptr;
-  uint32_t idxCap = 0, lossCap = 0;
+  uint32_t lossCap = 0;
   float *part = nullptr;  // per-tile gradient rows [partCap][kMlpParams]
   uint32_t partCap = 0;
 };
@@ -1181,7 +1190,6 @@ extern "C" BVHGB_API int bvhgb_mlp_destroy(bvhgb_mlp *m) {
   cudaFree(m->pb);
   cudaFree(m->stepDev);
   cudaFree(m->err);
-  cudaFree(m->idx);
   delete m;
   return BVHGB_OK;
 }
@@ -1225,7 +1233,7 @@ extern "C" BVHGB_API int bvhgb_mlp_gradient(bvhgb_mlp *m, const uint16_t *x, con
   if (st) return st;
   cudaStream_t s = as_stream(stream);
   BVHGB_CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4, s));
-  mlp_train_kernel<<<tiles, kTile, kTrainSmem, s>>>(m->pb, x, t, nullptr, n, (float)n, m->part, m->loss, nullptr, 0, 1);
+  mlp_train_kernel<<<tiles, kTrainThreads, kTrainSmem, s>>>(m->pb, x, t, n, 0u, 0ull, 0ull, (float)n, m->part, m->loss);
   BVHGB_LAUNCH_CHECK("mlp gradient");
   grad_reduce_kernel<<<ceil_div((uint32_t)kMlpParams, 256u), 256, 0, s>>>(m->part, tiles, m->g);
   BVHGB_LAUNCH_CHECK("mlp gradient reduce");
@@ -1247,46 +1255,37 @@ extern "C" BVHGB_API int bvhgb_mlp_train(bvhgb_mlp *m, const uint16_t *x, const 
   if (!st) st = ensure_part(m, tiles);
   if (st) return st;
   cudaStream_t s = as_stream(stream);
-  if (m->idxCap < batch) {
-    cudaFree(m->idx);
-    m->idx = nullptr;
-    m->idxCap = 0;
-    BVHGB_CUDA_TRY(dev_malloc(&m->idx, 4ull * batch));
-    m->idxCap = batch;
-  }
   uint32_t step0 = 0;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(&step0, m->stepDev, 4, cudaMemcpyDeviceToHost, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   BVHGB_CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4ull * steps, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
-  // Capture one step (batch rows, forward + backward, AdamW) and replay it; the kernels read the
-  // step number from device memory so every replay is the next step.
-  cudaStream_t cap = nullptr;
-  BVHGB_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    batch_index_kernel<<<ceil_div(batch, 256), 256, 0, cap>>>(m->idx, batch, numSamples, seed, m->stepDev);
-    mlp_train_kernel<<<tiles, kTile, kTrainSmem, cap>>>(m->pb, x, t, m->idx, batch, (float)batch, m->part, m->loss,
-                                                         m->stepDev, step0, steps);
-    grad_reduce_kernel<<<ceil_div((uint32_t)kMlpParams, 256u), 256, 0, cap>>>(m->part, tiles, m->g);
-    adamw_kernel<<<1, 1024, 0, cap>>>(m->p, m->pb, m->g, m->m, m->v, m->stepDev, lr, weightDecay);
-    e = cudaStreamEndCapture(cap, &graph);
+  // Two launches per step, each started while the one before drains (it gathers its samples, then
+  // waits for the weights).
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t train{}, adam{};
+  train.gridDim = dim3(tiles);
+  train.blockDim = dim3(kTrainThreads);
+  train.dynamicSmemBytes = kTrainSmem;
+  adam.gridDim = dim3(ceil_div((uint32_t)kMlpParams, (uint32_t)kAdamThreads));
+  adam.blockDim = dim3(kAdamThreads);
+  train.stream = adam.stream = s;
+  train.attrs = adam.attrs = &early;
+  train.numAttrs = adam.numAttrs = 1;
+  cudaError_t e = cudaSuccess;
+  for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k) {
+    const uint32_t step = step0 + k + 1u;
+    e = cudaLaunchKernelEx(&train, mlp_train_kernel, (const __nv_bfloat16 *)m->pb, x, t, batch, numSamples, seed,
+                           (uint64_t)step, (float)batch, m->part, m->loss + k);
+    if (e == cudaSuccess)
+      e = cudaLaunchKernelEx(&adam, adamw_kernel, (const float *)m->part, tiles, m->p, m->pb, m->m, m->v, m->stepDev,
+                             step, lr, weightDecay);
+    if (e == cudaSuccess) count_launch(2);
   }
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-  if (graph) cudaGraphDestroy(graph);
-  cudaStreamDestroy(cap);
-  if (e != cudaSuccess) {
-    set_last_error("bvhgb_mlp_train capture", e);
-    if (exec) cudaGraphExecDestroy(exec);
-    return BVHGB_CUDA_ERROR;
-  }
-  for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k) e = cudaGraphLaunch(exec, s);
-  count_launch(4u * steps);  // (the capture itself recorded none: its launches are not counted)
   if (e == cudaSuccess && lossHistory) e = cudaMemcpyAsync(lossHistory, m->loss, 4ull * steps, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaGraphExecDestroy(exec);
   if (e != cudaSuccess) {
     set_last_error("bvhgb_mlp_train", e);
     return BVHGB_CUDA_ERROR;
