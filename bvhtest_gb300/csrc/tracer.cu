@@ -62,18 +62,24 @@ struct TraceParams {
   uint32_t cull;
 };
 
-// Camera::genRays (Camera.cpp:67-88): pixel coordinates in double, the rest in float.
-__device__ __forceinline__ void camera_ray(const CamParams &cam, uint32_t x, uint32_t y, RayPre &r) {
-  const double qx = __ddiv_rn(__dadd_rn((double)x, 0.5), (double)cam.w);
-  const double qy = __ddiv_rn(__dadd_rn((double)y, 0.5), (double)cam.h);
-  const float px = (float)__dmul_rn(__dmul_rn(__dsub_rn(__dmul_rn(2.0, qx), 1.0), (double)cam.scale), (double)cam.ratio);
-  const float py = (float)__dmul_rn(__dsub_rn(1.0, __dmul_rn(2.0, qy)), (double)cam.scale);
+// Camera::genRays (Camera.cpp:67-88): pixel coordinates in double, the rest in float. The image-plane
+// coordinate of column x (py of row y) in the camera's basis.
+__device__ __forceinline__ float camera_axis(const CamParams &cam, bool row, uint32_t v) {
+  const double q = __ddiv_rn(__dadd_rn((double)v, 0.5), (double)(row ? cam.h : cam.w));
+  const double c = __dsub_rn(__dmul_rn(2.0, q), 1.0);  // a row's 1 - 2q is its exact negative
+  const double s = __dmul_rn(row ? -c : c, (double)cam.scale);
+  return row ? (float)s : (float)__dmul_rn(s, (double)cam.ratio);
+}
+__device__ __forceinline__ void camera_ray_at(const CamParams &cam, float px, float py, RayPre &r) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     r.o[k] = cam.pos[k];
     r.d[k] = fadd(fadd(fmul(cam.s[k], px), fmul(cam.u[k], py)), cam.f[k]);
   }
   normalize3(r.d);
+}
+__device__ __forceinline__ void camera_ray(const CamParams &cam, uint32_t x, uint32_t y, RayPre &r) {
+  camera_ray_at(cam, camera_axis(cam, false, x), camera_axis(cam, true, y), r);
   setup_ray(r);
 }
 
@@ -89,36 +95,17 @@ __device__ __forceinline__ float uniform01(uint64_t seed, uint64_t idx, uint32_t
 // One cosine-weighted diffuse bounce from every primary hit (an addition: the reference traces
 // primary rays only). The bounce starts on the hit point, offset along the normal that faces the
 // incoming ray; the direction follows Malley's method around that normal in the orthonormal basis
-// of Duff et al. (JCGT 2017).
-// Incoherent rays (bounce, random) are bound by the latency of their record and triangle loads:
-// at most 48 registers keep 40 warps per SM resident instead of 36 (2.5% faster bounce phase).
-template <bool REC>
-__global__ void __launch_bounds__(128, 10) trace_bounce_kernel(const bvhgb_node *__restrict__ nodes,
-                                                           const TravNode *__restrict__ trav, uint32_t numNodes,
-                                                           uint32_t root, const float *__restrict__ vert,
-                                                           const uint32_t *__restrict__ faces, CamParams cam,
-                                                           TraceParams tp, uint64_t seed, float offset,
-                                                           const bvhgb_hit *__restrict__ primary,
-                                                           bvhgb_hit *__restrict__ out, float *__restrict__ rayOrg,
-                                                           float *__restrict__ rayDir) {
-  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= cam.w || y >= cam.h) return;
+// of Duff et al. (JCGT 2017). False: the pixel's primary ray hit nothing.
+// px, py: the pixel's image-plane coordinates (camera_axis).
+__device__ __forceinline__ bool bounce_ray(const CamParams &cam, uint32_t x, uint32_t y, float px, float py,
+                                           const float *__restrict__ vert, const uint32_t *__restrict__ faces,
+                                           uint64_t seed, float offset, const bvhgb_hit *__restrict__ primary,
+                                           RayPre &r) {
   const size_t pix = (size_t)y * cam.w + x;
   const bvhgb_hit ph = primary[pix];
-  bvhgb_hit o;
-  o.primId = kNone;
-  o.t = __int_as_float(0x7f800000);
-  if (ph.primId == kNone) {
-    out[pix] = o;
-    if (rayOrg) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) rayOrg[3 * pix + k] = rayDir[3 * pix + k] = 0.0f;
-    }
-    return;
-  }
+  if (ph.primId == kNone) return false;
   RayPre cr;
-  camera_ray(cam, x, y, cr);
+  camera_ray_at(cam, px, py, cr);
   float v0[3], v1[3], v2[3];
   load_tri(vert, faces, ph.primId, v0, v1, v2);
   float e1[3], e2[3], n[3];
@@ -144,13 +131,38 @@ __global__ void __launch_bounds__(128, 10) trace_bounce_kernel(const bvhgb_node 
   float sn, cs;
   sincosf(phi, &sn, &cs);
   const float lx = rr * cs, ly = rr * sn, lz = sqrtf(fmaxf(0.0f, 1.0f - u1));
-  RayPre r;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const float hp = fadd(cr.o[k], fmul(ph.t, cr.d[k]));
     r.o[k] = hp + offset * n[k];
     r.d[k] = lx * tv[k] + ly * bv[k] + lz * n[k];
   }
+  return true;
+}
+
+__device__ __forceinline__ void store_hit(bvhgb_hit *out, const Hit &h) {
+  bvhgb_hit o;
+  o.primId = h.prim;
+  o.t = h.prim == kNone ? __int_as_float(0x7f800000) : h.t;
+  *out = o;
+}
+
+// On the node array. Incoherent rays are bound by the latency of their node and triangle loads: at
+// most 48 registers keep 40 warps per SM resident.
+__global__ void __launch_bounds__(128, 10) trace_bounce_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes,
+                                                           uint32_t root, const float *__restrict__ vert,
+                                                           const uint32_t *__restrict__ faces, CamParams cam,
+                                                           TraceParams tp, uint64_t seed, float offset,
+                                                           const bvhgb_hit *__restrict__ primary,
+                                                           bvhgb_hit *__restrict__ out, float *__restrict__ rayOrg,
+                                                           float *__restrict__ rayDir) {
+  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= cam.w || y >= cam.h) return;
+  const size_t pix = (size_t)y * cam.w + x;
+  RayPre r = {};
+  const bool live = bounce_ray(cam, x, y, camera_axis(cam, false, x), camera_axis(cam, true, y), vert, faces, seed,
+                               offset, primary, r);
   if (rayOrg) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -158,13 +170,56 @@ __global__ void __launch_bounds__(128, 10) trace_bounce_kernel(const bvhgb_node 
       rayDir[3 * pix + k] = r.d[k];
     }
   }
-  setup_ray(r);
-  Hit h;
-  if (REC) traverse_records(r, nodes, trav, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
-  else traverse(r, nodes, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
-  o.primId = h.prim;
-  o.t = h.prim == kNone ? __int_as_float(0x7f800000) : h.t;
-  out[pix] = o;
+  Hit h = {kNone, 0.0f};
+  if (live) {
+    setup_ray(r);
+    traverse(r, nodes, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
+  }
+  store_hit(out + pix, h);
+}
+
+// On a prepared tracer's wide records: a warp takes a run of pixels, tile by tile of 8 x 4 (the
+// order of the pixels does not matter to the hits, neighbours keep the records they share in L1).
+constexpr uint32_t kTileW = 8, kTileH = 4;
+static_assert(kTileW * kTileH == kWideRays && kTileW + kTileH <= 32, "one tile per set-up");
+__global__ void __launch_bounds__(32, kWideWarps) trace_bounce_wide_kernel(
+    const __grid_constant__ WideScene sc, const __grid_constant__ CamParams cam, uint64_t seed, float offset,
+    uint32_t tilesX, uint32_t tilesY, uint32_t run, const bvhgb_hit *__restrict__ primary,
+    bvhgb_hit *__restrict__ out, float *__restrict__ rayOrg, float *__restrict__ rayDir) {
+  auto pixel = [&](uint32_t i, uint32_t &x, uint32_t &y) {
+    const uint32_t tile = i / (kTileW * kTileH), k = i % (kTileW * kTileH);
+    x = tile % tilesX * kTileW + k % kTileW;
+    y = tile / tilesX * kTileH + k / kTileW;
+    return x < cam.w && y < cam.h;
+  };
+  trace_wide(
+      sc, tilesX * tilesY * kTileW * kTileH, run,
+      [&](uint32_t i, bool valid, RayPre &r) {
+        // 32 rays are one tile: lanes 0-7 make its columns' coordinates, lanes 8-11 its rows'.
+        const uint32_t lane = threadIdx.x & 31u, tile = (i - lane) / (kTileW * kTileH);
+        const bool row = lane >= kTileW;
+        const float axis = camera_axis(cam, row, row ? tile / tilesX * kTileH + (lane - kTileW) % kTileH
+                                                     : tile % tilesX * kTileW + lane);
+        const float px = __shfl_sync(0xFFFFFFFFu, axis, lane % kTileW);
+        const float py = __shfl_sync(0xFFFFFFFFu, axis, kTileW + lane / kTileW);
+        uint32_t x, y;
+        if (!valid || !pixel(i, x, y)) return false;
+        const bool live = bounce_ray(cam, x, y, px, py, sc.vert, sc.faces, seed, offset, primary, r);
+        if (rayOrg) {
+          const size_t pix = (size_t)y * cam.w + x;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            rayOrg[3 * pix + k] = r.o[k];
+            rayDir[3 * pix + k] = r.d[k];
+          }
+        }
+        return live;
+      },
+      [&](uint32_t i, const Hit &h) {
+        uint32_t x, y;
+        if (pixel(i, x, y)) store_hit(out + (size_t)y * cam.w + x, h);
+      },
+      &g_trace_errors);
 }
 
 // BUNDLE: the warp traverses as one bundle of rays (traverse_bundle, the reference's rayBundles);
@@ -176,12 +231,21 @@ __global__ void __launch_bounds__(128) trace_image_kernel(const bvhgb_node *__re
                                                           const uint32_t *__restrict__ faces, CamParams cam,
                                                           TraceParams tp, bvhgb_pixel *__restrict__ img,
                                                           bvhgb_hit *__restrict__ hits) {
-  const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
+  // The block's 16 x 8 pixels: a warp takes an 8 x 4 tile of them, a bundle two rows of 16 (its visit
+  // count belongs to those 32 pixels). The columns' and rows' coordinates, which are computed in
+  // double at a sixty-fourth of the float rate, are made once per block: 24 instead of 256.
+  const uint32_t tid = threadIdx.y * 16u + threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t bx = BUNDLE ? threadIdx.x : (warp & 1u) * 8u + (lane & 7u);
+  const uint32_t by = BUNDLE ? threadIdx.y : (warp >> 1) * 4u + (lane >> 3);
+  const uint32_t x = blockIdx.x * 16u + bx, y = blockIdx.y * 8u + by;
+  __shared__ float axis[24];
+  if (tid < 24u) axis[tid] = camera_axis(cam, tid >= 16u, tid < 16u ? blockIdx.x * 16u + tid : blockIdx.y * 8u + (tid - 16u));
+  __syncthreads();
   const bool active = x < cam.w && y < cam.h;
   if (!BUNDLE && !active) return;  // a bundle keeps its whole warp in the traversal
   RayPre r;
-  camera_ray(cam, active ? x : 0u, active ? y : 0u, r);
+  camera_ray_at(cam, axis[bx], axis[16u + by], r);
+  setup_ray(r);
   Hit h;
   const uint32_t visits =
       BUNDLE ? traverse_bundle<REC>(r, active, nodes, trav, numNodes, root, vert, faces, tp.tmin, tp.tmax,
@@ -210,9 +274,16 @@ __global__ void __launch_bounds__(128) trace_image_kernel(const bvhgb_node *__re
   }
 }
 
-template <bool REC>
-__global__ void __launch_bounds__(128, 10) trace_rays_kernel(const bvhgb_node *__restrict__ nodes,
-                                                         const TravNode *__restrict__ trav, uint32_t numNodes,
+__device__ __forceinline__ void load_ray(const float *__restrict__ org, const float *__restrict__ dir, uint32_t i,
+                                         RayPre &r) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.o[k] = __ldg(org + 3 * (size_t)i + k);
+    r.d[k] = __ldg(dir + 3 * (size_t)i + k);
+  }
+}
+
+__global__ void __launch_bounds__(128, 10) trace_rays_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes,
                                                          uint32_t root, const float *__restrict__ vert,
                                                          const uint32_t *__restrict__ faces,
                                                          const float *__restrict__ org, const float *__restrict__ dir,
@@ -220,19 +291,23 @@ __global__ void __launch_bounds__(128, 10) trace_rays_kernel(const bvhgb_node *_
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   RayPre r;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    r.o[k] = __ldg(org + 3 * (size_t)i + k);
-    r.d[k] = __ldg(dir + 3 * (size_t)i + k);
-  }
+  load_ray(org, dir, i, r);
   setup_ray(r);
   Hit h;
-  if (REC) traverse_records(r, nodes, trav, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
-  else traverse(r, nodes, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
-  bvhgb_hit o;
-  o.primId = h.prim;
-  o.t = h.prim == kNone ? __int_as_float(0x7f800000) : h.t;
-  hits[i] = o;
+  traverse(r, nodes, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0, h, &g_trace_errors);
+  store_hit(hits + i, h);
+}
+
+__global__ void __launch_bounds__(32, kWideWarps) trace_rays_wide_kernel(
+    const __grid_constant__ WideScene sc, const float *__restrict__ org, const float *__restrict__ dir, uint32_t n,
+    uint32_t run, bvhgb_hit *__restrict__ hits) {
+  trace_wide(
+      sc, n, run,
+      [&](uint32_t i, bool valid, RayPre &r) {
+        if (valid) load_ray(org, dir, i, r);
+        return valid;
+      },
+      [&](uint32_t i, const Hit &h) { store_hit(hits + i, h); }, &g_trace_errors);
 }
 
 // The reference's Ray (lib/base/Ray.hpp:38-80): origin, direction, 1 / direction, sign of the
@@ -312,9 +387,12 @@ __global__ void __launch_bounds__(128) trace_ray_image_kernel(const bvhgb_node *
   }
 }
 
-__global__ void build_trav_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, TravNode *__restrict__ out) {
-  for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < numNodes; x += gridDim.x * blockDim.x)
+__global__ void build_trav_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, TravNode *__restrict__ out,
+                                  WideNode *__restrict__ wide) {
+  for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < numNodes; x += gridDim.x * blockDim.x) {
     build_trav(nodes, numNodes, x, out, &g_trace_errors);
+    if (wide) build_wide(nodes, numNodes, x, wide, &g_trace_errors);
+  }
 }
 
 // Host mirror of the device normalise (each operation rounds once; this file's host code is
@@ -378,7 +456,20 @@ TraceParams make_trace_params(const bvhgb_trace_config *cfg) {
   return tp;
 }
 
-// The three traces, on the node array (trav == nullptr) or on a prepared tracer's records.
+WideScene make_wide_scene(const bvhgb_node *nodes, const WideNode *wide, uint32_t numNodes, uint32_t root,
+                          const float *vert, const uint32_t *faces, const bvhgb_trace_config *cfg) {
+  const TraceParams tp = make_trace_params(cfg);
+  return WideScene{nodes, wide, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0};
+}
+
+// Rays of a block's run: kWideRun, or fewer (a multiple of the 32 that are set up at a time) where
+// that would leave warps of the chip without a run.
+uint32_t wide_run(uint64_t rays) {
+  const uint64_t warps = (uint64_t)sm_count() * kWideWarps;
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rays / warps / kWideRays, 1u) * kWideRays, kWideRun);
+}
+
+// The three traces, on the node array (no records given) or on a prepared tracer's records.
 int launch_image(const bvhgb_node *nodes, const TravNode *trav, uint32_t numNodes, uint32_t root, const float *vert,
                  const uint32_t *faces, const bvhgb_camera *cam, const bvhgb_trace_config *cfg, bvhgb_pixel *img,
                  bvhgb_hit *hits, cudaStream_t s) {
@@ -400,38 +491,43 @@ int launch_image(const bvhgb_node *nodes, const TravNode *trav, uint32_t numNode
   return BVHGB_OK;
 }
 
-int launch_rays(const bvhgb_node *nodes, const TravNode *trav, uint32_t numNodes, uint32_t root, const float *vert,
+int launch_rays(const bvhgb_node *nodes, const WideNode *wide, uint32_t numNodes, uint32_t root, const float *vert,
                 const uint32_t *faces, const float *org, const float *dir, uint32_t n, const bvhgb_trace_config *cfg,
                 bvhgb_hit *hits, cudaStream_t s) {
   if (n == 0) return BVHGB_OK;
   if (!org || !dir || !hits) return BVHGB_INVALID_ARGUMENT;
-  if (trav)
-    trace_rays_kernel<true><<<ceil_div(n, 128), 128, 0, s>>>(nodes, trav, numNodes, root, vert, faces, org, dir, n,
-                                                             make_trace_params(cfg), hits);
-  else
-    trace_rays_kernel<false><<<ceil_div(n, 128), 128, 0, s>>>(nodes, trav, numNodes, root, vert, faces, org, dir, n,
-                                                              make_trace_params(cfg), hits);
+  if (wide && n < (1u << 31)) {  // the runs count rays in 32 bits
+    const uint32_t run = wide_run(n);
+    trace_rays_wide_kernel<<<ceil_div(n, run), 32, 0, s>>>(
+        make_wide_scene(nodes, wide, numNodes, root, vert, faces, cfg), org, dir, n, run, hits);
+  } else {
+    trace_rays_kernel<<<ceil_div(n, 128), 128, 0, s>>>(nodes, numNodes, root, vert, faces, org, dir, n,
+                                                       make_trace_params(cfg), hits);
+  }
   BVHGB_LAUNCH_CHECK("trace rays");
   return BVHGB_OK;
 }
 
-int launch_bounce(const bvhgb_node *nodes, const TravNode *trav, uint32_t numNodes, uint32_t root, const float *vert,
+int launch_bounce(const bvhgb_node *nodes, const WideNode *wide, uint32_t numNodes, uint32_t root, const float *vert,
                   const uint32_t *faces, const bvhgb_camera *cam, const bvhgb_trace_config *cfg, uint64_t seed,
                   float offset, const bvhgb_hit *primary, bvhgb_hit *bounce, float *rayOrg, float *rayDir,
                   cudaStream_t s) {
   if (!primary || !bounce || (rayOrg == nullptr) != (rayDir == nullptr)) return BVHGB_INVALID_ARGUMENT;
   if (cam->width == 0 || cam->height == 0) return BVHGB_OK;
   const CamParams cp = make_cam_params(cam);
-  dim3 block(16, 8);
-  dim3 grid(ceil_div(cam->width, 16), ceil_div(cam->height, 8));
-  if (trav)
-    trace_bounce_kernel<true><<<grid, block, 0, s>>>(nodes, trav, numNodes, root, vert, faces, cp,
-                                                     make_trace_params(cfg), seed, offset, primary, bounce, rayOrg,
-                                                     rayDir);
-  else
-    trace_bounce_kernel<false><<<grid, block, 0, s>>>(nodes, trav, numNodes, root, vert, faces, cp,
-                                                      make_trace_params(cfg), seed, offset, primary, bounce, rayOrg,
-                                                      rayDir);
+  const uint32_t tx = ceil_div(cam->width, kTileW), ty = ceil_div(cam->height, kTileH);
+  const uint64_t rays = (uint64_t)tx * ty * (kTileW * kTileH);
+  if (wide && rays < (1ull << 31)) {  // the runs count rays in 32 bits
+    const uint32_t run = wide_run(rays);
+    trace_bounce_wide_kernel<<<ceil_div(rays, run), 32, 0, s>>>(
+        make_wide_scene(nodes, wide, numNodes, root, vert, faces, cfg), cp, seed, offset, tx, ty, run, primary, bounce,
+        rayOrg, rayDir);
+  } else {
+    dim3 block(16, 8);
+    dim3 grid(ceil_div(cam->width, 16), ceil_div(cam->height, 8));
+    trace_bounce_kernel<<<grid, block, 0, s>>>(nodes, numNodes, root, vert, faces, cp, make_trace_params(cfg), seed,
+                                               offset, primary, bounce, rayOrg, rayDir);
+  }
   BVHGB_LAUNCH_CHECK("trace bounce");
   return BVHGB_OK;
 }
@@ -444,7 +540,8 @@ struct bvhgb_tracer {
   uint32_t maxNodes = 0;
   const bvhgb_node *nodes = nullptr;
   uint32_t numNodes = 0, root = 0;
-  bvhgb::TravNode *trav = nullptr;
+  bvhgb::TravNode *trav = nullptr;  // both children per record: images (their pixels count the visits)
+  bvhgb::WideNode *wide = nullptr;  // four grandchildren per record: rays that only want the hit
 };
 
 using namespace bvhgb;
@@ -478,9 +575,14 @@ extern "C" BVHGB_API int bvhgb_tracer_create(uint32_t maxNodes, bvhgb_tracer **o
   auto *tr = new bvhgb_tracer();
   tr->maxNodes = maxNodes;
   const cudaError_t e = dev_malloc(&tr->trav, sizeof(TravNode) * (size_t)maxNodes);
+  // Where the wide records do not fit, rays and bounces go through the node array.
+  if (e == cudaSuccess && dev_malloc(&tr->wide, sizeof(WideNode) * (size_t)maxNodes) != cudaSuccess) {
+    tr->wide = nullptr;
+    cudaGetLastError();
+  }
   if (e != cudaSuccess) {
     set_last_error("bvhgb_tracer_create", e);
-    delete tr;
+    bvhgb_tracer_destroy(tr);
     return e == cudaErrorMemoryAllocation ? BVHGB_OUT_OF_MEMORY : BVHGB_CUDA_ERROR;
   }
   *out = tr;
@@ -490,6 +592,7 @@ extern "C" BVHGB_API int bvhgb_tracer_create(uint32_t maxNodes, bvhgb_tracer **o
 extern "C" BVHGB_API int bvhgb_tracer_destroy(bvhgb_tracer *tr) {
   if (!tr) return BVHGB_OK;
   cudaFree(tr->trav);
+  cudaFree(tr->wide);
   delete tr;
   return BVHGB_OK;
 }
@@ -502,7 +605,7 @@ extern "C" BVHGB_API int bvhgb_tracer_update(bvhgb_tracer *tr, const bvhgb_node 
   tr->numNodes = numNodes;
   tr->root = root;
   build_trav_kernel<<<std::min(ceil_div(numNodes, 256), (uint32_t)sm_count() * 16), 256, 0, as_stream(stream)>>>(
-      nodes, numNodes, tr->trav);
+      nodes, numNodes, tr->trav, tr->wide);
   BVHGB_LAUNCH_CHECK("tracer records");
   return BVHGB_OK;
 }
@@ -518,7 +621,7 @@ extern "C" BVHGB_API int bvhgb_tracer_trace_rays(const bvhgb_tracer *tr, const f
                                                  const float *org, const float *dir, uint32_t n,
                                                  const bvhgb_trace_config *cfg, bvhgb_hit *hits, bvhgb_stream stream) {
   if (!tr || !tr->nodes || !vert || !faces) return BVHGB_INVALID_ARGUMENT;
-  return launch_rays(tr->nodes, tr->trav, tr->numNodes, tr->root, vert, faces, org, dir, n, cfg, hits,
+  return launch_rays(tr->nodes, tr->wide, tr->numNodes, tr->root, vert, faces, org, dir, n, cfg, hits,
                      as_stream(stream));
 }
 
@@ -527,7 +630,7 @@ extern "C" BVHGB_API int bvhgb_tracer_trace_bounce(const bvhgb_tracer *tr, const
                                                    float offset, const bvhgb_hit *primary, bvhgb_hit *bounce,
                                                    float *rayOrg, float *rayDir, bvhgb_stream stream) {
   if (!tr || !tr->nodes || !vert || !faces || !cam) return BVHGB_INVALID_ARGUMENT;
-  return launch_bounce(tr->nodes, tr->trav, tr->numNodes, tr->root, vert, faces, cam, cfg, seed, offset, primary,
+  return launch_bounce(tr->nodes, tr->wide, tr->numNodes, tr->root, vert, faces, cam, cfg, seed, offset, primary,
                        bounce, rayOrg, rayDir, as_stream(stream));
 }
 

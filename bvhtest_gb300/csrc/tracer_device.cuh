@@ -18,6 +18,24 @@ struct RayPre {
   int kx, ky, kz;
 };
 
+// Two single-precision operations in one instruction, each half rounded on its own.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n"
+      " mov.b64 {%0, %1}, z;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n"
+      " mov.b64 {%0, %1}, z;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
 __device__ __forceinline__ void setup_ray(RayPre &r) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) r.inv[k] = fdiv(1.0f, r.d[k]);
@@ -37,20 +55,16 @@ __device__ __forceinline__ void setup_ray(RayPre &r) {
 
 __device__ __forceinline__ float pick(const float *v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); }
 
-// Watertight ray/triangle test; every operation rounds once (matches the oracle bit for bit).
+// Watertight ray/triangle test; every operation rounds once (matches the oracle bit for bit). The
+// vertices come with their components in the ray's order (kx, ky, kz), which is how they are loaded:
+// nothing is selected here.
 __device__ __forceinline__ bool ray_tri(const RayPre &r, const float *v0, const float *v1, const float *v2, float tmin,
                                         float tmax, bool cull, float &tout) {
-  float A[3], B[3], C[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    A[k] = fsub(v0[k], r.o[k]);
-    B[k] = fsub(v1[k], r.o[k]);
-    C[k] = fsub(v2[k], r.o[k]);
-  }
-  const float Akz = pick(A, r.kz), Bkz = pick(B, r.kz), Ckz = pick(C, r.kz);
-  const float Ax = fsub(pick(A, r.kx), fmul(r.sx, Akz)), Ay = fsub(pick(A, r.ky), fmul(r.sy, Akz));
-  const float Bx = fsub(pick(B, r.kx), fmul(r.sx, Bkz)), By = fsub(pick(B, r.ky), fmul(r.sy, Bkz));
-  const float Cx = fsub(pick(C, r.kx), fmul(r.sx, Ckz)), Cy = fsub(pick(C, r.ky), fmul(r.sy, Ckz));
+  const float ox = pick(r.o, r.kx), oy = pick(r.o, r.ky), oz = pick(r.o, r.kz);
+  const float Akz = fsub(v0[2], oz), Bkz = fsub(v1[2], oz), Ckz = fsub(v2[2], oz);
+  const float Ax = fsub(fsub(v0[0], ox), fmul(r.sx, Akz)), Ay = fsub(fsub(v0[1], oy), fmul(r.sy, Akz));
+  const float Bx = fsub(fsub(v1[0], ox), fmul(r.sx, Bkz)), By = fsub(fsub(v1[1], oy), fmul(r.sy, Bkz));
+  const float Cx = fsub(fsub(v2[0], ox), fmul(r.sx, Ckz)), Cy = fsub(fsub(v2[1], oy), fmul(r.sy, Ckz));
   float U = fsub(fmul(Cx, By), fmul(Cy, Bx));
   float V = fsub(fmul(Ax, Cy), fmul(Ay, Cx));
   float W = fsub(fmul(Bx, Ay), fmul(By, Ax));
@@ -74,20 +88,27 @@ __device__ __forceinline__ bool ray_tri(const RayPre &r, const float *v0, const 
   return true;
 }
 
-// Robust slab test; sign-selected planes make 0 * inf NaNs drop out of the min/max.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
+      " fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+// Robust slab test; sign-selected planes make 0 * inf NaNs drop out of the min/max. The six plane
+// distances are three packed subtractions and products over the box's words as they are loaded; the
+// far distances are scaled once, after their minimum (rounding is monotonic, so the minimum of the
+// scaled distances is the scaled minimum). 18 instructions instead of 27.
 __device__ __forceinline__ bool box_hit(const RayPre &r, float4 a, float4 b, float tmin, float tmax, float &tn) {
-  const float mn[3] = {a.x, a.y, a.z};
-  const float mx[3] = {a.w, b.x, b.y};
-  float t0 = tmin, t1 = tmax;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const bool neg = r.inv[k] < 0.0f || (r.inv[k] == 0.0f && signbit(r.inv[k]));
-    const float nearP = neg ? mx[k] : mn[k], farP = neg ? mn[k] : mx[k];
-    const float tNear = fmul(fsub(nearP, r.o[k]), r.inv[k]);
-    const float tFar = fmul(fmul(fsub(farP, r.o[k]), r.inv[k]), kFarScale);
-    t0 = fmaxf(t0, tNear);
-    t1 = fminf(t1, tFar);
-  }
+  const float2 p = mul2(add2(make_float2(a.x, a.y), make_float2(-r.o[0], -r.o[1])), make_float2(r.inv[0], r.inv[1]));
+  const float2 q = mul2(add2(make_float2(a.z, a.w), make_float2(-r.o[2], -r.o[0])), make_float2(r.inv[2], r.inv[0]));
+  const float2 w = mul2(add2(make_float2(b.x, b.y), make_float2(-r.o[1], -r.o[2])), make_float2(r.inv[1], r.inv[2]));
+  const bool nx = __float_as_int(r.inv[0]) < 0, ny = __float_as_int(r.inv[1]) < 0, nz = __float_as_int(r.inv[2]) < 0;
+  const float t0 = fmaxf(fmaxf(fmaxf(nx ? q.y : p.x, ny ? w.x : p.y), nz ? w.y : q.x), tmin);
+  const float tf = fminf(fminf(nx ? p.x : q.y, ny ? p.y : w.x), nz ? q.x : w.y);
+  const float t1 = fminf(fmul(tf, kFarScale), tmax);
   tn = t0;
   return t0 <= t1;
 }
@@ -108,12 +129,26 @@ __device__ __forceinline__ void load_tri(const float *__restrict__ vert, const u
   }
 }
 
+// The same triangle with every vertex's components in the ray's order.
+__device__ __forceinline__ void load_tri_permuted(const RayPre &r, const float *__restrict__ vert,
+                                                  const uint32_t *__restrict__ faces, uint32_t f, float *v0, float *v1,
+                                                  float *v2) {
+  const uint32_t a = __ldg(faces + 3 * (size_t)f), b = __ldg(faces + 3 * (size_t)f + 1), c = __ldg(faces + 3 * (size_t)f + 2);
+  const int k[3] = {r.kx, r.ky, r.kz};
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v0[j] = __ldg(vert + 3 * (size_t)a + k[j]);
+    v1[j] = __ldg(vert + 3 * (size_t)b + k[j]);
+    v2[j] = __ldg(vert + 3 * (size_t)c + k[j]);
+  }
+}
+
 __device__ __forceinline__ void test_leaf(const RayPre &r, const float *__restrict__ vert,
                                           const uint32_t *__restrict__ faces, uint32_t first, uint32_t count,
                                           float tmin, float tmax, bool cull, Hit &h) {
   for (uint32_t f = first; f < first + count; ++f) {
     float v0[3], v1[3], v2[3], t;
-    load_tri(vert, faces, f, v0, v1, v2);
+    load_tri_permuted(r, vert, faces, f, v0, v1, v2);
     if (ray_tri(r, v0, v1, v2, tmin, tmax, cull, t)) {
       if (h.prim == kNone || t < h.t || (t == h.t && f < h.prim)) {
         h.t = t;
@@ -123,80 +158,69 @@ __device__ __forceinline__ void test_leaf(const RayPre &r, const float *__restri
   }
 }
 
-// Closest hit through the 48-byte node array. Returns the number of inner nodes visited.
+// Closest hit through the 48-byte node array. Returns the number of inner nodes visited. A stack entry
+// holds the far child's links, which were loaded with its box: taking it off needs no load.
 __device__ __forceinline__ uint32_t traverse(const RayPre &r, const bvhgb_node *__restrict__ nodes, uint32_t numNodes,
                                              uint32_t root, const float *__restrict__ vert,
                                              const uint32_t *__restrict__ faces, float tmin, float tmax, bool cull,
                                              Hit &h, uint32_t *err) {
-  uint2 stack[kStack];
+  uint4 stack[kStack];  // left, right, leaf, entry distance
   int sp = 0;
   uint32_t visits = 0;
   h.prim = kNone;
   h.t = tmax;
+  float lim = tmax;
   float4 a, b, c;
   load_node(nodes, root, a, b, c);
   float tn;
   if (!box_hit(r, a, b, tmin, tmax, tn)) return 0;
   uint32_t left = __float_as_uint(b.w), right = __float_as_uint(c.x);
   bool leaf = (__float_as_uint(c.y) & 0xFFFFu) != 0;
-  // A tree visits each node at most once; the bound turns a cyclic (corrupted) input into an error.
-  for (uint32_t it = 0;; ++it) {
-    if (it > numNodes) {
-      atomicOr(err, kErrBadIndex);
-      break;
-    }
+  for (;;) {
+    bool go = false;
     if (leaf) {
       test_leaf(r, vert, faces, left, right, tmin, tmax, cull, h);
+      if (h.prim != kNone) lim = fmul(h.t, kBestSlack);
     } else {
-      ++visits;
+      // A tree visits each node at most once; the bound turns a cyclic (corrupted) input into an error.
+      if (++visits > numNodes) {
+        atomicOr(err, kErrBadIndex);
+        break;
+      }
       if (left >= numNodes || right >= numNodes) {
         atomicOr(err, kErrBadIndex);
       } else {
         float4 la, lb, lc, ra, rb, rc;
         load_node(nodes, left, la, lb, lc);
         load_node(nodes, right, ra, rb, rc);
-        const float lim = h.prim == kNone ? tmax : fmul(h.t, kBestSlack);
         float tl, tr;
         const bool hl = box_hit(r, la, lb, tmin, lim, tl);
         const bool hr = box_hit(r, ra, rb, tmin, lim, tr);
+        const bool lfirst = hl && (!hr || tl <= tr);
         if (hl && hr) {
-          const bool lfirst = tl <= tr;
-          const uint32_t farIdx = lfirst ? right : left;
-          if (sp < kStack) stack[sp++] = make_uint2(farIdx, __float_as_uint(lfirst ? tr : tl));
-          else atomicOr(err, kErrStackOverflow);
-          const float4 &nb = lfirst ? lb : rb;
-          const float4 &nc = lfirst ? lc : rc;
-          left = __float_as_uint(nb.w);
-          right = __float_as_uint(nc.x);
-          leaf = (__float_as_uint(nc.y) & 0xFFFFu) != 0;
-          continue;
+          if (sp < kStack)
+            stack[sp++] = lfirst ? make_uint4(__float_as_uint(rb.w), __float_as_uint(rc.x), __float_as_uint(rc.y), __float_as_uint(tr))
+                                 : make_uint4(__float_as_uint(lb.w), __float_as_uint(lc.x), __float_as_uint(lc.y), __float_as_uint(tl));
+          else
+            atomicOr(err, kErrStackOverflow);
         }
-        if (hl || hr) {
-          const float4 &nb = hl ? lb : rb;
-          const float4 &nc = hl ? lc : rc;
-          left = __float_as_uint(nb.w);
-          right = __float_as_uint(nc.x);
-          leaf = (__float_as_uint(nc.y) & 0xFFFFu) != 0;
-          continue;
+        go = hl || hr;
+        if (go) {
+          left = __float_as_uint(lfirst ? lb.w : rb.w);
+          right = __float_as_uint(lfirst ? lc.x : rc.x);
+          leaf = (__float_as_uint(lfirst ? lc.y : rc.y) & 0xFFFFu) != 0;
         }
       }
     }
     // Pop the next subtree whose entry distance can still beat the best hit.
-    bool found = false;
-    while (sp > 0) {
-      const uint2 e = stack[--sp];
-      const float lim = h.prim == kNone ? tmax : fmul(h.t, kBestSlack);
-      if (__uint_as_float(e.y) <= lim) {
-        const float4 *p = reinterpret_cast<const float4 *>(nodes + e.x);
-        const float4 nb = __ldg(p + 1), nc = __ldg(p + 2);
-        left = __float_as_uint(nb.w);
-        right = __float_as_uint(nc.x);
-        leaf = (__float_as_uint(nc.y) & 0xFFFFu) != 0;
-        found = true;
-        break;
-      }
+    while (!go && sp > 0) {
+      const uint4 e = stack[--sp];
+      go = __uint_as_float(e.w) <= lim;
+      left = e.x;
+      right = e.y;
+      leaf = (e.z & 0xFFFFu) != 0;
     }
-    if (!found) break;
+    if (!go) break;
   }
   return visits;
 }
@@ -268,54 +292,486 @@ __device__ __forceinline__ uint32_t traverse_records(const RayPre &r, const bvhg
     return 0;
   }
   uint32_t cur = root;
-  for (uint32_t it = 0;; ++it) {
-    if (it > numNodes) {  // a tree visits each node at most once: a cyclic (corrupted) input
+  float lim = tmax;
+  for (;;) {
+    if (++visits > numNodes) {  // a tree visits each node at most once: a cyclic (corrupted) input
       atomicOr(err, kErrBadIndex);
       break;
     }
-    ++visits;
     const float4 *q = reinterpret_cast<const float4 *>(trav + cur);
     const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
     const uint4 q3 = __ldg(reinterpret_cast<const uint4 *>(q + 3));
-    float lim = h.prim == kNone ? tmax : fmul(h.t, kBestSlack);
     float tl, tr;
     bool hl = box_hit(r, q0, make_float4(q1.x, q1.y, 0.0f, 0.0f), tmin, lim, tl);
     bool hr = box_hit(r, make_float4(q1.z, q1.w, q2.x, q2.y), make_float4(q2.z, q2.w, 0.0f, 0.0f), tmin, lim, tr);
-    if (hl && q3.z) {
-      test_leaf(r, vert, faces, q3.x, q3.z, tmin, tmax, cull, h);
-      hl = false;
+    // Leaf children: the lanes of a warp test their next one together, whichever side it is on.
+    bool ll = hl && q3.z != 0u, rl = hr && q3.w != 0u;
+    hl = hl && !ll;
+    hr = hr && !rl;
+    if (ll || rl) {
+      do {
+        test_leaf(r, vert, faces, ll ? q3.x : q3.y, ll ? q3.z : q3.w, tmin, tmax, cull, h);
+        rl = rl && ll;
+        ll = false;
+      } while (rl);
+      if (h.prim != kNone) lim = fmul(h.t, kBestSlack);
+      hl = hl && tl <= lim;
+      hr = hr && tr <= lim;
     }
-    if (hr && q3.w) {
-      test_leaf(r, vert, faces, q3.y, q3.w, tmin, tmax, cull, h);
-      hr = false;
-    }
-    if (hl || hr) lim = h.prim == kNone ? tmax : fmul(h.t, kBestSlack);
-    hl = hl && tl <= lim;
-    hr = hr && tr <= lim;
+    const bool lfirst = hl && (!hr || tl <= tr);
     if (hl && hr) {
-      const bool lfirst = tl <= tr;
       if (sp < kStack) stack[sp++] = make_uint2(lfirst ? q3.y : q3.x, __float_as_uint(lfirst ? tr : tl));
       else atomicOr(err, kErrStackOverflow);
-      cur = lfirst ? q3.x : q3.y;
-      continue;
     }
-    if (hl || hr) {
-      cur = hl ? q3.x : q3.y;
-      continue;
-    }
+    bool go = hl || hr;
+    cur = lfirst ? q3.x : q3.y;
     // Pop the next subtree whose entry distance can still beat the best hit.
-    bool found = false;
-    while (sp > 0) {
+    while (!go && sp > 0) {
       const uint2 e = stack[--sp];
-      if (__uint_as_float(e.y) <= (h.prim == kNone ? tmax : fmul(h.t, kBestSlack))) {
-        cur = e.x;
-        found = true;
-        break;
-      }
+      go = __uint_as_float(e.y) <= lim;
+      cur = e.x;
     }
-    if (!found) break;
+    if (!go) break;
   }
   return visits;
+}
+
+// ---- four-wide records ---------------------------------------------------------------------------
+// Record of an inner node for rays whose visits are not counted (bounce, given and random rays): the
+// boxes of its up to four grandchildren (a leaf child stands for itself), quantised to 8 bits per
+// plane on a power-of-two grid of the record's own, in one 64-byte line. A ray reads one such line
+// where it reads three of the binary records (192 bytes), and its chain of dependent loads halves.
+// Every plane is rounded outwards, so a box only grows and the closest hit, which does not depend
+// on which further boxes are opened, stays the same (the smallest t, then the smallest primitive).
+struct __align__(64) WideNode {
+  float o[3];       // the grid's origin
+  uint32_t meta;    // byte k < 3: the exponent of axis k's grid step (biased); bits 24-27: slots with an
+                    // inner node, bits 28-31: slots with a leaf
+  uint32_t lo[3];   // byte j: slot j's lower plane on the axis
+  uint32_t hi[3];
+  uint32_t ref[4];  // an inner slot: the node; a leaf: its only face, or the leaf node | kLeafNode
+  uint32_t pad[2];
+};
+static_assert(sizeof(WideNode) == 64, "one line");
+constexpr uint32_t kLeafNode = 0x80000000u;
+// Stack of the wide traversal: at most three entries are pushed per two levels, so this holds every
+// tree that kStack holds for the binary one.
+constexpr int kWideSteps = 8;       // records per lane between two rounds of leaf tests
+constexpr int kWideStack = kStack * 3 / 2 + 3 * kWideSteps;
+
+// Node x's wide record (none for a leaf).
+__device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, uint32_t x,
+                                           WideNode *__restrict__ out, uint32_t *err) {
+  const float4 *p = reinterpret_cast<const float4 *>(nodes + x);
+  const float4 xb = __ldg(p + 1), xc = __ldg(p + 2);
+  if (__float_as_uint(xc.y) & 0xFFFFu) return;
+  const uint32_t child[2] = {__float_as_uint(xb.w), __float_as_uint(xc.x)};
+  float mn[4][3], mx[4][3];
+  uint32_t ref[4] = {0u, 0u, 0u, 0u}, kinds = 0;
+  bool ok = child[0] < numNodes && child[1] < numNodes;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (!ok) break;
+    const float4 *q = reinterpret_cast<const float4 *>(nodes + child[c]);
+    const float4 a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
+    const uint32_t l = __float_as_uint(b.w), r = __float_as_uint(d.x);
+    if (__float_as_uint(d.y) & 0xFFFFu) {
+      mn[2 * c][0] = a.x; mn[2 * c][1] = a.y; mn[2 * c][2] = a.z;
+      mx[2 * c][0] = a.w; mx[2 * c][1] = b.x; mx[2 * c][2] = b.y;
+      if (r != 0u) {
+        kinds |= 16u << (2 * c);
+        ref[2 * c] = r == 1u && l < kLeafNode ? l : child[c] | kLeafNode;
+      }
+      continue;
+    }
+    const uint32_t g[2] = {l, r};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (g[k] >= numNodes) {
+        ok = false;
+        break;
+      }
+      const float4 *w = reinterpret_cast<const float4 *>(nodes + g[k]);
+      const float4 e = __ldg(w), f = __ldg(w + 1), h = __ldg(w + 2);
+      const int s = 2 * c + k;
+      mn[s][0] = e.x; mn[s][1] = e.y; mn[s][2] = e.z;
+      mx[s][0] = e.w; mx[s][1] = f.x; mx[s][2] = f.y;
+      const uint32_t count = __float_as_uint(h.x);
+      if (!(__float_as_uint(h.y) & 0xFFFFu)) {
+        kinds |= 1u << s;
+        ref[s] = g[k];
+      } else if (count != 0u) {
+        kinds |= 16u << s;
+        ref[s] = count == 1u && __float_as_uint(f.w) < kLeafNode ? __float_as_uint(f.w) : g[k] | kLeafNode;
+      }
+    }
+  }
+  if (!ok) {  // no slot is ever opened
+    atomicOr(err, kErrBadIndex);
+    kinds = 0;
+  }
+  WideNode n;
+  n.meta = kinds << 24;
+  n.pad[0] = n.pad[1] = 0u;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) n.ref[s] = ref[s];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float lo = __int_as_float(0x7f800000), hi = -lo;
+    bool finite = true;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (!(kinds & (17u << s))) continue;
+      lo = fminf(lo, mn[s][k]);
+      hi = fmaxf(hi, mx[s][k]);
+      finite = finite && isfinite(mn[s][k]) && isfinite(mx[s][k]);
+    }
+    // The step: 240 of them span the boxes, and none is finer than two units in the last place of
+    // the largest coordinate, so that the differences below are exact to a fraction of a step.
+    const float need = fmaxf((hi - lo) * (1.0f / 240.0f), fmaxf(fabsf(lo), fabsf(hi)) * 4.76837158e-7f);
+    uint32_t e = (__float_as_uint(need) >> 23) + 1u;  // the next power of two above
+    n.lo[k] = n.hi[k] = 0u;
+    if (!finite || !(need < 1e37f) || kinds == 0u) {
+      // Not on any grid: a step of infinity makes every plane distance NaN, which drops out of the
+      // slab test, so the slots pass on this axis.
+      n.o[k] = 0.0f;
+      n.meta |= 255u << (8 * k);
+      continue;
+    }
+    e = e < 32u ? 32u : e;
+    const float step = __uint_as_float(e << 23), inv = __uint_as_float((254u - e) << 23);
+    n.o[k] = lo - 4.0f * step;
+    n.meta |= e << (8 * k);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (!(kinds & (17u << s))) continue;
+      // an eighth of a step beyond the plane: more than every rounding on the way back
+      const int ql = (int)floorf((mn[s][k] - n.o[k]) * inv - 0.125f), qh = (int)ceilf((mx[s][k] - n.o[k]) * inv + 0.125f);
+      n.lo[k] |= (uint32_t)min(max(ql, 0), 255) << (8 * s);
+      n.hi[k] |= (uint32_t)min(max(qh, 0), 255) << (8 * s);
+    }
+  }
+  const uint4 *src = reinterpret_cast<const uint4 *>(&n);
+  uint4 *dst = reinterpret_cast<uint4 *>(out + x);
+#pragma unroll
+  for (int w = 0; w < 4; ++w) dst[w] = src[w];
+}
+
+// A plane's byte in the middle of the mantissa of 1.0: 1 + q 2^-15, exactly, in one byte permute.
+__device__ __forceinline__ float wide_plane(uint32_t packed, int slot) {
+  return __uint_as_float(__byte_perm(packed, 0x3F800000u, 0x7604u | ((uint32_t)slot << 4)));
+}
+
+// A warp traces a run of rays through the wide records and keeps its lanes busy. Rays differ in
+// length by more than the mean (33.5M-triangle scene: 34 records on average, 152 for the longest of
+// a warp), so a lane that is done takes the next ray of the run at once; and since a ray tests two
+// triangles per 30 records, one lane's test would stop the others each time: leaves wait in a queue
+// of the lane's own, and the lanes test theirs together every few records. Rays are made (or read)
+// and set up 32 at a time by the whole warp and wait in shared memory until lanes take them. Neither
+// changes a hit: the closest one does not depend on when a triangle is tested, only on which
+// records are skipped, and those lie behind a hit already found.
+//
+// Bound: the latency of the record loads (long scoreboard 9.6 of 15 cycles per instruction; L1 hits
+// 53%, shared with the stacks). 4.19M rays in 33.5M triangles / the 1080p bounce in 4.19M, in ms:
+// one thread per ray on binary records 8.6 / 4.2; four-wide records alone 8.4 / 4.3; with refill and
+// queued leaves 4.9 / 2.7 (128 rays per run; 64: 5.4 / 2.9, 256: 5.2 / 2.9; 4 or 12 records between
+// leaf tests: 5.0 / 2.9, 4.9 / 2.7); with stolen runs 5.0 / 2.5; with 24 warps per SM and 12 stack
+// entries in shared memory instead of 32 warps and a local stack 4.4 / 2.5 (the stacks' sectors had
+// pushed the records out of L1; 16 and 28 warps: 4.4 / 2.7, 4.7 / 2.5).
+constexpr uint32_t kWideWarps = 24; // warps per SM
+constexpr int kWideRays = 32;       // rays set up at a time
+constexpr uint32_t kWideRun = 128;  // most rays of a block's run
+constexpr int kWideQueue = 6;       // leaves a lane can hold; it pauses when four more would not fit
+constexpr int kWideTop = 12;        // stack entries per lane in shared memory, the deeper ones are in local memory
+constexpr uint32_t kWideRefill = 8; // idle lanes that make a refill worth its instructions
+
+// Work stealing: a block is one warp with one run of rays, and a warp whose run is used up takes the
+// run of a block that has not been launched yet (clusterlaunchcontrol) instead of ending, so its
+// lanes drain once per launch, not once per run. The request for the next run travels while the
+// warp works on this one. A request that finds no block left is the last one made.
+struct __align__(16) StolenRun {
+  unsigned long long reply[2];
+  unsigned long long bar;
+};
+__device__ __forceinline__ uint32_t shared_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void steal_request(StolenRun &st) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the last reply was read
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(shared_addr(&st.bar)) : "memory");
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   shared_addr(st.reply)),
+               "r"(shared_addr(&st.bar))
+               : "memory");
+}
+
+// Waits (bounded) for the reply of phase 'parity': true and the block's index, or false. One lane
+// waits and reads the reply, so that its own fence orders the read before the next request.
+__device__ __forceinline__ bool steal_wait(StolenRun &st, uint32_t parity, uint32_t &block, uint32_t *err) {
+  uint32_t taken = 0, x = 0;
+  if ((threadIdx.x & 31u) == 0u) {
+    uint32_t ok = 0;
+    for (uint32_t i = 0; i < (1u << 18) && !ok; ++i) {
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(ok)
+          : "r"(shared_addr(&st.bar)), "r"(parity)
+          : "memory");
+    }
+    if (ok) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile(
+          "{\n .reg .pred p;\n .reg .b128 h;\n .reg .b64 a, b;\n ld.shared.v2.b64 {a, b}, [%2];\n mov.b128 h, {a, b};\n"
+          " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n selp.u32 %0, 1, 0, p;\n mov.u32 %1, 0;\n"
+          " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n}\n"
+          : "=r"(taken), "=r"(x)
+          : "r"(shared_addr(st.reply))
+          : "memory");
+    } else {
+      atomicOr(err, kErrTimeout);
+    }
+  }
+  block = __shfl_sync(0xFFFFFFFFu, x, 0);
+  return __shfl_sync(0xFFFFFFFFu, taken, 0) != 0u;
+}
+
+struct WideShared {
+  StolenRun steal;
+  float org[3][kWideRays], inv[3][kWideRays], shear[3][kWideRays];
+  uint32_t axes[kWideRays];  // kx | ky << 2 | kz << 4
+  uint32_t index[kWideRays];
+  uint32_t leaf[kWideQueue][32];
+  uint2 stack[kWideTop][32];  // the lanes' first stack entries (node, entry distance)
+};
+
+__device__ __forceinline__ WideShared &wide_shared() {
+  __shared__ WideShared sm;
+  return sm;
+}
+
+struct WideScene {
+  const bvhgb_node *nodes;
+  const WideNode *wide;
+  uint32_t numNodes, root;
+  const float *vert;
+  const uint32_t *faces;
+  float tmin, tmax;
+  bool cull;
+};
+
+// Block b's run is rays [b * run, ...) of 'total' (< 2^31). gen(i, valid, r), which
+// the whole warp calls for 32 rays in a row from a multiple of 32, sets r.o and r.d of a valid ray and
+// returns whether there is one to trace; emit(i, hit) takes every ray's result (no hit for those gen
+// refused). A block is one warp; every lane calls it.
+template <typename Gen, typename Emit>
+__device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, uint32_t run, const Gen &gen, const Emit &emit,
+                                           uint32_t *err) {
+  const uint32_t lane = threadIdx.x & 31u, ltMask = (1u << lane) - 1u;
+  const bvhgb_node *__restrict__ nodes = sc.nodes;
+  const WideNode *__restrict__ wide = sc.wide;
+  WideShared &sm = wide_shared();
+  const bool anyT = sc.tmin < 0.0f;  // negative distances: entries are not pruned by their distance
+  uint2 deep[kWideStack - kWideTop];
+  int sp = 0;
+  uint32_t cur = kNone, ray = kNone, steps = 0, pend = 0;
+  RayPre r = {};
+  Hit h = {kNone, 0.0f};
+  float lim = 0.0f;
+  // warp-uniform: the rays waiting, the run's position and end, the steal's state
+  uint32_t head = 0, count = 0, next = blockIdx.x * run, end = min(total, next + run), parity = 0;
+  bool more = true;  // a request is on its way
+  if (lane == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&sm.steal.bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    steal_request(sm.steal);
+  }
+  __syncwarp();
+  for (;;) {
+    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, ray == kNone);
+    if (__popc(idle) >= (int)kWideRefill) {
+      if (head == count && next >= end && more) {
+        uint32_t block;
+        more = steal_wait(sm.steal, parity, block, err);
+        parity ^= 1u;
+        if (more) {
+          next = block * run;
+          end = min(total, next + run);
+          if (lane == 0) steal_request(sm.steal);
+        }
+        __syncwarp();
+      }
+      if (head == count && next < end) {
+        const uint32_t i = next + lane;
+        RayPre g = {};
+        bool live = gen(i, i < end, g);
+        if (live) {
+          setup_ray(g);
+          float4 a, b, c;
+          load_node(nodes, sc.root, a, b, c);
+          float tn;
+          live = box_hit(g, a, b, sc.tmin, sc.tmax, tn);
+          if (live && (__float_as_uint(c.y) & 0xFFFFu)) {  // the tree is one leaf
+            Hit o = {kNone, sc.tmax};
+            test_leaf(g, sc.vert, sc.faces, __float_as_uint(b.w), __float_as_uint(c.x), sc.tmin, sc.tmax, sc.cull, o);
+            emit(i, o);
+            live = false;
+          } else if (!live) {
+            emit(i, Hit{kNone, sc.tmax});
+          }
+        } else if (i < end) {
+          emit(i, Hit{kNone, sc.tmax});
+        }
+        const uint32_t have = __ballot_sync(0xFFFFFFFFu, live);
+        __syncwarp();
+        if (live) {
+          const uint32_t s = __popc(have & ltMask);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            sm.org[k][s] = g.o[k];
+            // A direction component near zero counts as 2^-80: products with the reciprocal stay
+            // finite, so a ray parallel to an axis is still kept out of the slabs beside it.
+            sm.inv[k][s] = fabsf(g.d[k]) < 8.271806e-25f ? copysignf(1.2089258e24f, g.d[k]) : g.inv[k];
+          }
+          sm.shear[0][s] = g.sx;
+          sm.shear[1][s] = g.sy;
+          sm.shear[2][s] = g.sz;
+          sm.axes[s] = (uint32_t)g.kx | ((uint32_t)g.ky << 2) | ((uint32_t)g.kz << 4);
+          sm.index[s] = i;
+        }
+        head = 0;
+        count = __popc(have);
+        next = end - next > (uint32_t)kWideRays ? next + kWideRays : end;
+        __syncwarp();
+      }
+      if (head == count && next >= end && !more && idle == 0xFFFFFFFFu) break;
+      const uint32_t s = head + __popc(idle & ltMask);
+      if (ray == kNone && s < count) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          r.o[k] = sm.org[k][s];
+          r.inv[k] = sm.inv[k][s];
+        }
+        r.sx = sm.shear[0][s];
+        r.sy = sm.shear[1][s];
+        r.sz = sm.shear[2][s];
+        const uint32_t ax = sm.axes[s];
+        r.kx = (int)(ax & 3u);
+        r.ky = (int)((ax >> 2) & 3u);
+        r.kz = (int)(ax >> 4);
+        ray = sm.index[s];
+        cur = sc.root;
+        sp = 0;
+        steps = 0;
+        pend = 0;
+        h.prim = kNone;
+        h.t = lim = sc.tmax;
+      }
+      head = min(count, head + (uint32_t)__popc(idle));
+      __syncwarp();  // the next 32 rays may overwrite these
+    }
+    if (sp > kWideStack - 3 * kWideSteps || steps > sc.numNodes) {
+      // A deeper stack than any the binary traversal can hold, or a cyclic (corrupted) tree: a tree
+      // visits each node at most once.
+      if (ray != kNone) atomicOr(err, steps > sc.numNodes ? kErrBadIndex : kErrStackOverflow);
+      cur = kNone;
+      sp = 0;
+      steps = 0;
+    }
+#pragma unroll 1
+    for (int step = 0; step < kWideSteps; ++step) {
+      // the next subtree, if its entry distance can still beat the best hit
+      if (cur == kNone && sp > 0) {
+        --sp;
+        uint2 e;
+        if (sp < kWideTop) e = sm.stack[sp][lane];
+        else e = deep[sp - kWideTop];
+        if (__uint_as_float(e.y) <= lim || anyT) cur = e.x;
+      }
+      if (cur == kNone || pend > (uint32_t)kWideQueue - 4u) continue;
+      ++steps;
+      const uint4 *q = reinterpret_cast<const uint4 *>(wide + cur);
+      const uint4 w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
+      const uint2 w3 = __ldg(reinterpret_cast<const uint2 *>(q + 3));
+      const uint32_t ref[4] = {w2.z, w2.w, w3.x, w3.y};
+      const float o[3] = {__uint_as_float(w0.x), __uint_as_float(w0.y), __uint_as_float(w0.z)};
+      const uint32_t lo[3] = {w1.x, w1.y, w1.z}, hi[3] = {w1.w, w2.x, w2.y};
+      float scale[3], base[3];
+      uint32_t pn[3], pf[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float gridStep = __uint_as_float(((w0.w >> (8 * k)) & 0xFFu) << 23);
+        scale[k] = (gridStep * 32768.0f) * r.inv[k];
+        base[k] = (o[k] - r.o[k]) * r.inv[k] - scale[k];
+        const bool neg = __float_as_int(r.inv[k]) < 0;
+        pn[k] = neg ? hi[k] : lo[k];
+        pf[k] = neg ? lo[k] : hi[k];
+      }
+      // A slot's near and far plane distances are one packed operation per axis. What follows is
+      // predicated, not branched (a slot's outcome differs per lane), but for the leaves: two in
+      // thirty records.
+      uint32_t key[4], leaves = 0;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        float2 t[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          t[k] = fma2(make_float2(wide_plane(pn[k], s), wide_plane(pf[k], s)), make_float2(scale[k], scale[k]),
+                      make_float2(base[k], base[k]));
+        const float t0 = fmaxf(fmaxf(fmaxf(t[0].x, t[1].x), t[2].x), sc.tmin);
+        const float tf = fminf(fminf(t[0].y, t[1].y), t[2].y);
+        const bool hit = t0 <= fminf(fmaf(fabsf(tf), 9.5367432e-7f, tf), lim);
+        // ordered by entry distance (a negative one is 0), the slot in the low bits
+        const uint32_t k = (__float_as_uint(fmaxf(t0, 0.0f)) & ~3u) | (uint32_t)s;
+        key[s] = hit && (w0.w & (1u << (24 + s))) ? k : 0xFFFFFFFFu;
+        leaves |= hit ? w0.w & (1u << (28 + s)) : 0u;
+      }
+      while (leaves) {
+        const int s = __ffs(leaves) - 29;
+        leaves &= leaves - 1u;
+        sm.leaf[pend][lane] = s == 0 ? ref[0] : s == 1 ? ref[1] : s == 2 ? ref[2] : ref[3];
+        ++pend;
+      }
+#define BVHGB_ORDER(a, b)                                                             \
+  {                                                                                   \
+    const uint32_t x_ = min(key[a], key[b]), y_ = max(key[a], key[b]);                \
+    key[a] = x_;                                                                      \
+    key[b] = y_;                                                                      \
+  }
+      BVHGB_ORDER(0, 1) BVHGB_ORDER(2, 3) BVHGB_ORDER(0, 2) BVHGB_ORDER(1, 3) BVHGB_ORDER(1, 2)
+#undef BVHGB_ORDER
+      // The nearest is next, the others go onto the stack, farthest first.
+#pragma unroll
+      for (int j = 3; j >= 0; --j) {
+        const bool live = key[j] != 0xFFFFFFFFu;
+        const uint32_t ra = key[j] & 1u ? ref[1] : ref[0], rb = key[j] & 1u ? ref[3] : ref[2];
+        const uint32_t rf = key[j] & 2u ? rb : ra;
+        if (j == 0) {
+          cur = live ? rf : kNone;
+        } else {
+          const uint2 e = make_uint2(rf, key[j] & ~3u);
+          if (live && sp < kWideTop) sm.stack[sp][lane] = e;
+          if (live && sp >= kWideTop) deep[sp - kWideTop] = e;
+          sp += live ? 1 : 0;
+        }
+      }
+    }
+    // The leaves found meanwhile, one per lane at a time.
+    while (__any_sync(0xFFFFFFFFu, pend != 0u)) {
+      if (pend == 0u) continue;
+      const uint32_t e = sm.leaf[--pend][lane];
+      uint32_t first = e, faceCount = 1u;
+      if (e & kLeafNode) {
+        const float4 *p = reinterpret_cast<const float4 *>(nodes + (e & ~kLeafNode));
+        first = __float_as_uint(__ldg(p + 1).w);
+        faceCount = __float_as_uint(__ldg(p + 2).x);
+      }
+      test_leaf(r, sc.vert, sc.faces, first, faceCount, sc.tmin, sc.tmax, sc.cull, h);
+      if (h.prim != kNone) lim = fmul(h.t, kBestSlack);
+    }
+    if (ray != kNone && cur == kNone && sp == 0) {
+      emit(ray, h);
+      ray = kNone;
+    }
+  }
 }
 
 // ---- ray bundles ---------------------------------------------------------------------------------

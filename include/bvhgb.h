@@ -480,10 +480,11 @@ BVHGB_API int bvhgb_trace_bounce(const bvhgb_node *nodes, uint32_t numNodes, uin
                                  uint64_t seed, float offset, const bvhgb_hit *primary, bvhgb_hit *bounce,
                                  float *rayOrg, float *rayDir, bvhgb_stream stream);
 /* A tracer prepared for one tree (no counterpart in the reference, whose tracer reads the node
- * array): bvhgb_tracer_update builds traversal records (both children's boxes and references per
- * inner node, 64 bytes each, maxNodes of them allocated at create) once, and every trace call on
- * the tracer reuses them, loading one record per visit instead of two 48-byte nodes. The node
- * array must stay as it was at the last update while traces run. Same hits as the calls above. */
+ * array): bvhgb_tracer_update builds traversal records once, and every trace call on the tracer
+ * reuses them: for images both children's boxes and references per inner node, for rays and bounces
+ * its grandchildren's, 64 bytes each, maxNodes of either kind allocated at create (the second kind
+ * where there is memory for it). The node array must stay as it was at the last update while traces
+ * run. Same hits as the calls above. */
 typedef struct bvhgb_tracer bvhgb_tracer;
 BVHGB_API int bvhgb_tracer_create(uint32_t maxNodes, bvhgb_tracer **out);
 BVHGB_API int bvhgb_tracer_destroy(bvhgb_tracer *tr);
