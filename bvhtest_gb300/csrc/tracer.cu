@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(32, kWideWarps) trace_bounce_wide_kernel(
         const float py = __shfl_sync(0xFFFFFFFFu, axis, kTileW + lane / kTileW);
         uint32_t x, y;
         if (!valid || !pixel(i, x, y)) return false;
-        const bool live = bounce_ray(cam, x, y, px, py, sc.vert, sc.faces, seed, offset, primary, r);
+        const bool live = bounce_ray(cam, x, y, px, py, sc.vert, sc.facesOf, seed, offset, primary, r);
         if (rayOrg) {
           const size_t pix = (size_t)y * cam.w + x;
 #pragma unroll
@@ -459,14 +459,7 @@ TraceParams make_trace_params(const bvhgb_trace_config *cfg) {
 WideScene make_wide_scene(const bvhgb_node *nodes, const WideNode *wide, uint32_t numNodes, uint32_t root,
                           const float *vert, const uint32_t *faces, const bvhgb_trace_config *cfg) {
   const TraceParams tp = make_trace_params(cfg);
-  return WideScene{nodes, wide, numNodes, root, vert, faces, tp.tmin, tp.tmax, tp.cull != 0};
-}
-
-// Rays of a block's run: kWideRun, or fewer (a multiple of the 32 that are set up at a time) where
-// that would leave warps of the chip without a run.
-uint32_t wide_run(uint64_t rays) {
-  const uint64_t warps = (uint64_t)sm_count() * kWideWarps;
-  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rays / warps / kWideRays, 1u) * kWideRays, kWideRun);
+  return WideScene{nodes, wide, faces, vert, numNodes, root, tp.tmin, tp.tmax, tp.cull != 0};
 }
 
 // The three traces, on the node array (no records given) or on a prepared tracer's records.

@@ -548,26 +548,33 @@ __device__ __forceinline__ WideShared &wide_shared() {
   return sm;
 }
 
+// What the rays are traced against, one tree for all of them.
 struct WideScene {
-  const bvhgb_node *nodes;
-  const WideNode *wide;
-  uint32_t numNodes, root;
+  static constexpr bool kMany = false;  // several trees: a lane keeps the pointers of its ray's own
+  const bvhgb_node *nodesOf;
+  const WideNode *wideOf;
+  const uint32_t *facesOf;
   const float *vert;
-  const uint32_t *faces;
+  uint32_t nodeCount, rootNode;
   float tmin, tmax;
   bool cull;
+  __device__ __forceinline__ const bvhgb_node *nodes(uint32_t) const { return nodesOf; }
+  __device__ __forceinline__ const WideNode *wide(uint32_t) const { return wideOf; }
+  __device__ __forceinline__ const uint32_t *faces(uint32_t) const { return facesOf; }
+  __device__ __forceinline__ uint32_t numNodes() const { return nodeCount; }
+  __device__ __forceinline__ uint32_t root() const { return rootNode; }
 };
 
 // Block b's run is rays [b * run, ...) of 'total' (< 2^31). gen(i, valid, r), which
 // the whole warp calls for 32 rays in a row from a multiple of 32, sets r.o and r.d of a valid ray and
 // returns whether there is one to trace; emit(i, hit) takes every ray's result (no hit for those gen
 // refused). A block is one warp; every lane calls it.
-template <typename Gen, typename Emit>
-__device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, uint32_t run, const Gen &gen, const Emit &emit,
+template <typename Scene, typename Gen, typename Emit>
+__device__ __forceinline__ void trace_wide(const Scene &sc, uint32_t total, uint32_t run, const Gen &gen, const Emit &emit,
                                            uint32_t *err) {
   const uint32_t lane = threadIdx.x & 31u, ltMask = (1u << lane) - 1u;
-  const bvhgb_node *__restrict__ nodes = sc.nodes;
-  const WideNode *__restrict__ wide = sc.wide;
+  const WideNode *laneWide = nullptr;
+  const uint32_t *laneFaces = nullptr;
   WideShared &sm = wide_shared();
   const bool anyT = sc.tmin < 0.0f;  // negative distances: entries are not pruned by their distance
   uint2 deep[kWideStack - kWideTop];
@@ -606,12 +613,12 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
         if (live) {
           setup_ray(g);
           float4 a, b, c;
-          load_node(nodes, sc.root, a, b, c);
+          load_node(sc.nodes(i), sc.root(), a, b, c);
           float tn;
           live = box_hit(g, a, b, sc.tmin, sc.tmax, tn);
           if (live && (__float_as_uint(c.y) & 0xFFFFu)) {  // the tree is one leaf
             Hit o = {kNone, sc.tmax};
-            test_leaf(g, sc.vert, sc.faces, __float_as_uint(b.w), __float_as_uint(c.x), sc.tmin, sc.tmax, sc.cull, o);
+            test_leaf(g, sc.vert, sc.faces(i), __float_as_uint(b.w), __float_as_uint(c.x), sc.tmin, sc.tmax, sc.cull, o);
             emit(i, o);
             live = false;
           } else if (!live) {
@@ -658,7 +665,11 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
         r.ky = (int)((ax >> 2) & 3u);
         r.kz = (int)(ax >> 4);
         ray = sm.index[s];
-        cur = sc.root;
+        if (Scene::kMany) {
+          laneWide = sc.wide(ray);
+          laneFaces = sc.faces(ray);
+        }
+        cur = sc.root();
         sp = 0;
         steps = 0;
         pend = 0;
@@ -668,10 +679,10 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
       head = min(count, head + (uint32_t)__popc(idle));
       __syncwarp();  // the next 32 rays may overwrite these
     }
-    if (sp > kWideStack - 3 * kWideSteps || steps > sc.numNodes) {
+    if (sp > kWideStack - 3 * kWideSteps || steps > sc.numNodes()) {
       // A deeper stack than any the binary traversal can hold, or a cyclic (corrupted) tree: a tree
       // visits each node at most once.
-      if (ray != kNone) atomicOr(err, steps > sc.numNodes ? kErrBadIndex : kErrStackOverflow);
+      if (ray != kNone) atomicOr(err, steps > sc.numNodes() ? kErrBadIndex : kErrStackOverflow);
       cur = kNone;
       sp = 0;
       steps = 0;
@@ -688,7 +699,7 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
       }
       if (cur == kNone || pend > (uint32_t)kWideQueue - 4u) continue;
       ++steps;
-      const uint4 *q = reinterpret_cast<const uint4 *>(wide + cur);
+      const uint4 *q = reinterpret_cast<const uint4 *>((Scene::kMany ? laneWide : sc.wide(0)) + cur);
       const uint4 w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
       const uint2 w3 = __ldg(reinterpret_cast<const uint2 *>(q + 3));
       const uint32_t ref[4] = {w2.z, w2.w, w3.x, w3.y};
@@ -760,11 +771,11 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
       const uint32_t e = sm.leaf[--pend][lane];
       uint32_t first = e, faceCount = 1u;
       if (e & kLeafNode) {
-        const float4 *p = reinterpret_cast<const float4 *>(nodes + (e & ~kLeafNode));
+        const float4 *p = reinterpret_cast<const float4 *>(sc.nodes(ray) + (e & ~kLeafNode));
         first = __float_as_uint(__ldg(p + 1).w);
         faceCount = __float_as_uint(__ldg(p + 2).x);
       }
-      test_leaf(r, sc.vert, sc.faces, first, faceCount, sc.tmin, sc.tmax, sc.cull, h);
+      test_leaf(r, sc.vert, Scene::kMany ? laneFaces : sc.faces(0), first, faceCount, sc.tmin, sc.tmax, sc.cull, h);
       if (h.prim != kNone) lim = fmul(h.t, kBestSlack);
     }
     if (ray != kNone && cur == kNone && sp == 0) {
@@ -772,6 +783,13 @@ __device__ __forceinline__ void trace_wide(const WideScene &sc, uint32_t total, 
       ray = kNone;
     }
   }
+}
+
+// Rays of a block's run: kWideRun, or fewer (a multiple of the 32 that are set up at a time) where
+// that would leave warps of the chip without a run.
+inline uint32_t wide_run(uint64_t rays) {
+  const uint64_t warps = (uint64_t)sm_count() * kWideWarps, per = rays / warps / kWideRays * kWideRays;
+  return (uint32_t)(per < (uint64_t)kWideRays ? (uint64_t)kWideRays : per < kWideRun ? per : kWideRun);
 }
 
 // ---- ray bundles ---------------------------------------------------------------------------------

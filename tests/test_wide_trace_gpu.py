@@ -147,6 +147,30 @@ def test_bounce(gpu, width, height):
     assert gpu.trace_errors() == 0
 
 
+@pytest.mark.parametrize("rays", [1, 33, 500, 5000])
+def test_batch(gpu, rays):
+    """Meshes of 1, 2, 3 and more triangles in one launch, below and above the rule's line (a ray per
+    eight inner nodes), against the single-mesh traversal on the node array."""
+    import torch
+    counts = np.array([1, 700, 2, 3, 5000, 64], np.uint32)
+    parts = [scenes.uniform_soup(int(n), sigma=0.05, seed=60 + k)[0] for k, n in enumerate(counts)]
+    vert = np.concatenate(parts)
+    faces = np.arange(vert.shape[0], dtype=np.uint32).reshape(-1, 3)
+    v = torch.from_numpy(vert).cuda()
+    f = torch.from_numpy(faces.view(np.int32)).cuda()
+    b = gpu.Batch(counts)
+    nodes = b.empty_nodes()
+    b.build(v, f, nodes)
+    b.optimize(nodes, 2)
+    hits, org, d = b.trace_random(nodes, v, f, rays, seed=9, with_rays=True)
+    for m in range(len(counts)):
+        sl = slice(m * rays, (m + 1) * rays)
+        fo = f[int(b.face_offsets[m]): int(b.face_offsets[m + 1])].contiguous()
+        ref = gpu.trace_rays(b.mesh_nodes(nodes, m).contiguous(), v, fo, org[sl].contiguous(), d[sl].contiguous())
+        assert torch.equal(hits[sl], ref), m
+    assert b.stats()[1] == 0
+
+
 def test_without_memory_for_the_records(gpu):
     """No memory for the wide records: the tracer is made all the same and traces on the node array."""
     import ctypes as C
