@@ -31,10 +31,11 @@ struct HeapItem {
   float cost;
 };
 
-struct PatchOut {  // what the apply kernel needs
+struct alignas(16) PatchOut {  // what the apply kernel needs
   NodeP nd[NSLOT];
-  uint32_t idx[NSLOT];
+  uint32_t idx[NSLOT];  // then two words of padding: both arrays are read in 16-byte words
 };
+static_assert(sizeof(NodeP) == 16 && sizeof(PatchOut) == 208, "16-byte words");
 
 // Read-only view of the tree during the patch kernel (nothing writes the tree in that launch).
 __device__ __forceinline__ NodeP tree_node(const bvhgb_node *t, uint32_t x) {
@@ -924,42 +925,68 @@ __device__ __forceinline__ void apply_item(bvhgb_node *t, const PatchOut &in, ui
 // the claims are final before this launch) wins, i.e. owns every node of its own patch: a higher
 // rank that also claimed y does not own y, so it cannot win. The claims are released later, by
 // the refit launch.
-__device__ __forceinline__ bool item_wins(const PatchOut &in, const uint32_t *__restrict__ owner, uint32_t rank) {
+struct PatchIdx {
+  uint32_t v[NSLOT];
+};
+__device__ __forceinline__ PatchIdx patch_idx(const PatchOut &in) {
+  const uint4 *q = reinterpret_cast<const uint4 *>(in.idx);
+  const uint4 a = __ldg(q), b = __ldg(q + 1);
+  const uint2 c = __ldg(reinterpret_cast<const uint2 *>(q + 2));
+  return {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y}};
+}
+__device__ __forceinline__ bool item_wins(const PatchIdx &in, const uint32_t *__restrict__ owner, uint32_t rank) {
+  uint32_t o[NSLOT];  // all loads before the first compare
+#pragma unroll
+  for (int s = 0; s < NSLOT; ++s) o[s] = in.v[s] != kNone ? __ldg(owner + in.v[s]) : rank;
   bool win = true;
 #pragma unroll
-  for (int s = 0; s < NSLOT; ++s) {
-    const uint32_t x = in.idx[s];
-    if (x != kNone && owner[x] != rank) win = false;
-  }
+  for (int s = 0; s < NSLOT; ++s) win = win && o[s] == rank;
   return win;
 }
 
-// The parent of y in the tree being patched, given y's owner o and its parent p before the patch.
-__device__ __forceinline__ uint32_t new_parent(const PatchOut *__restrict__ in, const uint32_t *__restrict__ owner,
-                                               uint32_t y, uint32_t o, uint32_t p) {
-  if (o == kNone) return p;
-  const PatchOut &po = in[o];
-  if (!item_wins(po, owner, o)) return p;
+// Parent and left link of y in the tree being patched, given y's owner o and its links before the
+// patch. (A node's patched links are read from the patch of the winner that owns it.)
+__device__ __forceinline__ uint2 new_links(const PatchOut *__restrict__ in, const uint32_t *__restrict__ owner,
+                                           uint32_t y, uint32_t o, uint2 links) {
+  if (o == kNone) return links;
+  const PatchIdx idx = patch_idx(in[o]);
+  if (!item_wins(idx, owner, o)) return links;
+  uint32_t s = kNone;
 #pragma unroll
-  for (int s = 0; s < NSLOT; ++s)
-    if (po.idx[s] == y) return po.nd[s].parent;
-  return p;
+  for (int k = NSLOT - 1; k >= 0; --k)
+    if (idx.v[k] == y) s = (uint32_t)k;
+  if (s == kNone) return links;
+  return make_uint2(in[o].nd[s].parent, in[o].nd[s].left);
+}
+
+// The arrivals a node's refit waits for are marked in its counter word: one bit per child that lies on
+// a dirty path and one for a node that starts a path. Marks are set without reading them back (an
+// atomic or whose result nobody waits for), so a level of a climb is one load round trip: owner,
+// links and the marks set so far go out together. A climb that finds marks leaves the rest of the
+// way to the climb that set the first one; two that find none go on both, and set the same bits.
+// (With counts, a level was one atomic round trip: a chunk's launch took 7.8 us on 65,536 triangles
+// and 11.2 us on 4.19M, with marks 7.0 and 10.0; the refit of the latter went from 17.6 to 16.3.)
+constexpr uint32_t kMarkLeft = 1u, kMarkRight = 2u, kMarkStart = 4u, kMarks = 7u;
+
+__device__ __forceinline__ uint2 ld_links(const bvhgb_node *t, uint32_t x) {  // parent, left
+  return __ldcg(reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(t + x) + 24));
 }
 
 // Climb j of item k: all three decide the item's outcome (the owner array is final; valid[k], the
 // patch kernel's decision, is only read here, so the three climbs see the same value); climb 0
-// writes the patch and the statistics, climb j counts the arrivals along the item's j-th dirty
-// path (kFixTree3_1) in the new tree. The start node gets bit 31 as in count_path.
+// writes the patch and the statistics, climb j marks the item's j-th dirty path (kFixTree3_1) in
+// the new tree.
 __device__ __forceinline__ void apply_count_path(bvhgb_node *t, uint32_t root, uint32_t numNodes,
                                                  const PatchOut *__restrict__ in, uint32_t k, uint32_t j,
                                                  const uint32_t *__restrict__ valid, uint32_t *__restrict__ toFix,
                                                  const uint32_t *__restrict__ owner, uint32_t *__restrict__ counter,
                                                  unsigned long long *__restrict__ stats, uint32_t *__restrict__ err) {
-  if (!valid[k]) return;  // refused by removeNode or the search: it claimed nothing
+  const uint32_t isValid = __ldg(valid + k);
   uint32_t x = toFix[3 * k + j];
   const PatchOut &me = in[k];
-  const bool win = item_wins(me, owner, k);
-  if (!win) {
+  const PatchIdx idx = patch_idx(me);
+  if (!isValid) return;  // refused by removeNode or the search: it claimed nothing
+  if (!item_wins(idx, owner, k)) {
     toFix[3 * k + j] = kNone;  // the refit skips a lost item's paths
     if (j == 0) atomicAdd(&stats[S_CONFLICT], 1ull);
     return;
@@ -967,7 +994,7 @@ __device__ __forceinline__ void apply_count_path(bvhgb_node *t, uint32_t root, u
   if (j == 0) {
 #pragma unroll
     for (int s = 0; s < NSLOT; ++s) {
-      const uint32_t y = me.idx[s];
+      const uint32_t y = idx.v[s];
       if (y == kNone) continue;
       const NodeP n = me.nd[s];
       t[y].parent = n.parent;
@@ -978,20 +1005,19 @@ __device__ __forceinline__ void apply_count_path(bvhgb_node *t, uint32_t root, u
     atomicAdd(&stats[S_APPLIED], 1ull);
   }
   if (x == kNone) return;
-  uint32_t add = 0x80000001u;
+  uint32_t from = kNone;
   for (uint32_t steps = 0;; ++steps) {
     if (x >= numNodes || steps > numNodes) {
       atomicOr(err, kErrBadIndex);
       break;
     }
-    // owner, old parent and the counter update go out together: one round trip per level where
-    // no patch touched the node
-    const uint32_t o = owner[x];
-    const uint32_t p = __ldcg(&t[x].parent);  // discarded if a winner rewrites it in this launch
-    if (atomicAdd(&counter[x], add) != 0u) break;
-    if (x == root) break;
-    add = 1u;
-    x = new_parent(in, owner, x, o, p);
+    const uint32_t o = __ldg(owner + x), marks = __ldcg(&counter[x]);
+    uint2 links = ld_links(t, x);  // discarded if a winner rewrites them in this launch
+    links = new_links(in, owner, x, o, links);
+    atomicOr(&counter[x], from == kNone ? kMarkStart : links.y == from ? kMarkLeft : kMarkRight);
+    if (marks != 0u || x == root) break;
+    from = x;
+    x = links.x;
   }
 }
 
@@ -1003,38 +1029,35 @@ __device__ __forceinline__ void release_claims(const PatchOut &in, uint32_t j, u
   }
 }
 
-// Release a third of an item's claims and count the arrivals along one dirty path (kFixTree3_1);
-// the parent link is loaded together with the counter update, so a level costs one round trip.
-// The path's own start node gets bit 31 as well (the refit below must know its start nodes).
+// Release a third of an item's claims and mark one dirty path (kFixTree3_1), links final.
 __device__ __forceinline__ void count_path(const bvhgb_node *__restrict__ t, uint32_t root, uint32_t numNodes,
                                           const PatchOut &in, uint32_t j, uint32_t x, uint32_t *__restrict__ owner,
                                           uint32_t *__restrict__ counter, uint32_t *__restrict__ err) {
-  for (uint32_t s = j; s < (uint32_t)NSLOT; s += 3) {
-    const uint32_t y = in.idx[s];
-    if (y != kNone) owner[y] = kNone;
-  }
+  release_claims(in, j, owner);
   if (x == kNone) return;
-  uint32_t add = 0x80000001u;
+  uint32_t from = kNone;
   for (uint32_t steps = 0;; ++steps) {
     if (x >= numNodes || steps > numNodes) {
       atomicOr(err, kErrBadIndex);
       break;
     }
-    const uint32_t px = t[x].parent;  // issued before the update; the links are final here
-    if (atomicAdd(&counter[x], add) != 0u) break;
-    if (x == root) break;
-    add = 1u;
-    x = px;
+    const uint32_t marks = __ldcg(&counter[x]);
+    const uint2 links = ld_links(t, x);
+    atomicOr(&counter[x], from == kNone ? kMarkStart : links.y == from ? kMarkLeft : kMarkRight);
+    if (marks != 0u || x == root) break;
+    from = x;
+    x = links.x;
   }
 }
 
 // ---- dirty-path refit (kFixTree3_2) ------------------------------------------------------------
-// The last path to arrive at a node recomputes its box. A node's counter (set by the count pass)
-// holds the arrivals still expected in its low 16 bits and bit 31 for a start node (grand parent or
-// reused node: its children were relinked, so it is always recomputed). Each arrival subtracts one
-// and, for the child it comes from (side 0 left, 1 right), sets bit 16 + side if it rewrote that
-// child's box in this launch and bit 18 + side if the child changed (rewritten, or a start node,
-// which may have moved under a new parent). A side arrives at most once, so the bits never carry.
+// The last path to arrive at a node recomputes its box. A node's counter word (set by the count pass)
+// holds the arrivals to expect as marks: a dirty left or right child, a path that starts here (grand
+// parent or reused node: its children were relinked, so it is always recomputed). Each arrival sets
+// its own arrival bit (the mark shifted by 8) and, for the child it comes from (side 0 left, 1
+// right), bit 16 + side if it rewrote that child's box in this launch and bit 18 + side if the child
+// changed (rewritten, or a start node, which may have moved under a new parent). The arrival that
+// completes the marks is the last.
 //
 // Every counter update is relaxed: a rewritten box does not travel through the node record, whose
 // visibility would need a release by the writer and an acquire by the reader (fences that cost
@@ -1049,7 +1072,7 @@ __device__ __forceinline__ void count_path(const bvhgb_node *__restrict__ t, uin
 //
 // Links do not change in this launch and a node's box is written only by its last arrival, so the
 // climb reads one level ahead: while it handles node x it loads the parent's record and counter. A
-// node whose counter already shows this path as the only arrival left needs no update at all.
+// node whose word already shows this path as the only arrival left needs no update at all.
 constexpr unsigned long long kMailEmpty = 0xFFFFFFFFFFFFFFFFull;
 
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
@@ -1135,19 +1158,20 @@ __device__ __forceinline__ void refit_path(bvhgb_node *t, uint32_t root, uint32_
       ncnt = __ldcg(&counter[parent]);
     }
     uint32_t old = cnt;
-    if ((cnt & 0x7FFFFFFFu) != 1u) {  // other arrivals are (or were) expected here
+    const uint32_t mark = from == kNone ? kMarkStart : side ? kMarkRight : kMarkLeft;
+    if ((cnt & kMarks & ~(cnt >> 8)) != mark) {  // other arrivals are still expected here
       const bool post = from != kNone && written;
       if (post) mail_post(mail, from, cur);
-      uint32_t add = 0xFFFFFFFFu;  // one arrival less
-      if (from != kNone) add += (written ? (1u << (16 + side)) : 0u) + (changed ? (1u << (18 + side)) : 0u);
-      old = atomicAdd(&counter[x], add);
-      if ((old & 0xFFFFu) != 1u) return;  // not the last arrival
+      uint32_t add = mark << 8;
+      if (from != kNone) add |= (written ? (1u << (16 + side)) : 0u) | (changed ? (1u << (18 + side)) : 0u);
+      old = atomicOr(&counter[x], add);
+      if ((old & kMarks & ~(old >> 8)) != mark) return;  // not the last arrival
       if (post) mail_clear(mail, from);   // posted for nobody
-      if (from != l && ((old >> 16) & 1u)) lb = mail_take(mail, l, err);
-      if (from != r && ((old >> 17) & 1u)) rb = mail_take(mail, r, err);
     }
+    if (from != l && ((old >> 16) & 1u)) lb = mail_take(mail, l, err);
+    if (from != r && ((old >> 17) & 1u)) rb = mail_take(mail, r, err);
     counter[x] = 0u;
-    const bool start = (old >> 31) != 0u;  // x started a path (this one or an earlier arrival)
+    const bool start = (old & kMarkStart) != 0u;  // x started a path (this one or an earlier arrival)
     const bool anyChanged = changed || start || ((old >> 18) & 3u) != 0u;
     Box b;
     b.mn[0] = w0.x; b.mn[1] = w0.y; b.mn[2] = w0.z;
