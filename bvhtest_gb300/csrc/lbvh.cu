@@ -8,12 +8,14 @@
 //                  workspace has them, writes each triangle's box as a 32-byte record in face order
 //                  (the build then gathers one sector per leaf instead of a face and three vertices).
 //   sort         : sort.cu (replaces cub::DeviceRadixSort, LBVH_CUDA.cu:185-193).
-//   lbvh_build   : one thread per sorted leaf writes the leaf and climbs (Apetrei 2014 style): at each
-//                  step it picks the parent from the two neighbouring key deltas, meets its sibling
-//                  at the split, and the second thread to arrive merges the boxes and writes the
-//                  parent with the Karras node index the reference assigns (kGenLeafNodes +
-//                  kBuildTree + kFixAABBTree, LBVH_CUDA.cu:273-374), meeting its sibling through one
-//                  acq_rel exchange on the split's slot.
+//   lbvh_build   : a block makes the inner nodes among its 256 sorted leaves in shared memory and lists
+//                  the roots of its subtrees (treelet_build).
+//   lbvh_roots   : climbs from those roots (Apetrei 2014 style): at each step a climb picks the parent
+//                  from the two neighbouring key deltas, meets its sibling through one acq_rel exchange
+//                  on the split's slot, and the second to arrive merges the boxes and writes the parent.
+//                  Both give the nodes the Karras index the reference assigns (kGenLeafNodes +
+//                  kBuildTree + kFixAABBTree, LBVH_CUDA.cu:273-374).
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -24,7 +26,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t maxFaces = 0;
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
-  uint32_t *scene = nullptr;  // 6 order-mapped floats + error word
+  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, root counter
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -41,7 +43,6 @@ namespace {
 
 constexpr int kBoundsThreads = 256;
 constexpr int kMortonThreads = 256;
-constexpr int kBuildThreads = 128;
 
 __global__ void lbvh_init_kernel(uint32_t *scene) {
   if (threadIdx.x < 6) scene[threadIdx.x] = f2ord(0.0f);  // origin box [(0,0,0),(0,0,0)]
@@ -89,12 +90,13 @@ __global__ void __launch_bounds__(kBoundsThreads) lbvh_bounds_kernel(const float
 template <int BITS>
 __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float *__restrict__ vert,
                                                                      const uint32_t *__restrict__ faces, uint32_t n,
-                                                                     const uint32_t *__restrict__ scene, void *keysOut,
+                                                                     uint32_t *__restrict__ scene, void *keysOut,
                                                                      uint32_t *__restrict__ vals,
                                                                      uint32_t *__restrict__ slots,
                                                                      float4 *__restrict__ boxes) {
   float off[3], sc[3];
   morton_params(scene, off, sc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) scene[7] = 0;  // the build's root counter
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     Box b;
     float c[3];
@@ -110,45 +112,280 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
   }
 }
 
-template <int MODE, typename K>
-__global__ void __launch_bounds__(kBuildThreads) lbvh_build_kernel(const float *__restrict__ vert,
-                                                                   const uint32_t *__restrict__ faces,
-                                                                   const K *__restrict__ keys,
-                                                                   const uint32_t *__restrict__ idx, uint32_t n,
-                                                                   const float4 *__restrict__ boxes,
-                                                                   bvhgb_node *nodes, uint32_t *slots,
-                                                                   uint32_t *err) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t face = __ldg(idx + i);
-  Box box;
-  if (boxes) {
-    const float4 a = __ldg(boxes + 2 * (size_t)face), c = __ldg(boxes + 2 * (size_t)face + 1);
-    box.mn[0] = a.x; box.mn[1] = a.y; box.mn[2] = a.z;
-    box.mx[0] = a.w; box.mx[1] = c.x; box.mx[2] = c.y;
-  } else {
-    tri_box(vert, faces, face, box, nullptr);
+// ---- tree of a block of leaves ----------------------------------------------------------------------
+//
+// A block takes T consecutive sorted leaves, one per thread, and makes every inner node whose range
+// lies among them, all at once: thread t finds the range [l, r] of the node that splits between
+// leaves t and t + 1 (the leaves that share as long a prefix with it as its two neighbours do: a
+// binary search in the block's keys, or a mask of the index in refCompat mode), its Karras index and
+// its children, and takes its box from two overlapping windows of 2^j leaves (W_j[l] and
+// W_j[r - 2^j + 1]); the windows double level by level, in the order the queries need them. The
+// records are staged in shared memory and written in 16-byte words, neighbours together. What is
+// left, the roots of the block's subtrees (about 2 log2 T of them, at most kTreeletRoots), goes to a
+// list that a second launch climbs from through the global exchange slots (lbvh_climb_from).
+//
+// Why: with one climb per leaf every inner node cost an acquire-release exchange, a sibling's box
+// from L2 and three scattered stores in one dependent chain (4.19M leaves: 413 us at 24% of DRAM
+// throughput); here all but one node in seventeen costs none of them. Climbing from the block
+// itself cost more than it saved (450 us): its fences wait for all the records it has just written.
+// Measured, block of 256 / 512 / 1,024 leaves without the climbs: 186 / 209 / 295 us; the climbs of
+// the second launch 79 us (33.5M leaves: 3,050 us as one climb per leaf, 1,413 + 360 now).
+//
+// Windows overlap, so a box is a plain minimum and maximum over its leaves. The climb's merge differs
+// from that only where a coordinate is NaN (its result then depends on the order): a block with a NaN
+// among its boxes climbs leaf by leaf.
+constexpr int kTreelet = 256;
+// Between two neighbouring roots of a block the delta is a strict prefix minimum of the block's deltas
+// or a strict suffix minimum, and a delta is at most 96.
+constexpr int kTreeletRoots = 193;
+
+template <int T, typename K>
+struct TreeletSmem {
+  union {
+    float box[2][6][T];      // window boxes, ping-pong
+    float4 record[3 * T];    // node records on their way out
+  };
+  K key[T + 2];              // leaf B0 + i at [i + 1]
+  uint32_t parInner[T], parLeaf[T];  // parent | is-left << 31 (an index has 31 bits); kNone: not in this block
+  uint8_t gap[T + 1];        // delta of the leaves B0 + i - 1 and B0 + i
+  uint8_t made[T];           // inner record i of the block is one of its own
+};
+
+// The block's leaves are B0 .. B0 + cnt - 1; every thread of the T calls it. box: the thread's leaf's box
+// (t < cnt). keys: the tree's sorted keys (karras mode).
+template <int MODE, int T, typename K>
+__device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0, uint32_t n, uint32_t face, const Box &box,
+                                              const K *__restrict__ keys, bvhgb_node *nodes, uint32_t *slots,
+                                              uint2 *__restrict__ roots, uint32_t *rootCount, uint32_t *err) {
+  __shared__ int top;
+  constexpr int kBits = 8 * (int)sizeof(K);
+  const int t = (int)threadIdx.x;
+  const int cnt = (int)min((uint32_t)T, n - B0);
+  const bool live = t < cnt;
+  const uint32_t i = B0 + (uint32_t)t;
+  if (MODE == BVHGB_TOPO_KARRAS) {
+    if (live) sm.key[t + 1] = __ldg(keys + i);
+    if (t == 0 && B0 > 0) sm.key[0] = __ldg(keys + B0 - 1);
+    if (t == 0 && B0 + cnt < n) sm.key[cnt + 1] = __ldg(keys + B0 + cnt);
   }
-  lbvh_climb<MODE, K>(i, n, keys, face, box, nodes, slots, err);
+  sm.parInner[t] = sm.parLeaf[t] = kNone;
+  sm.made[t] = 0;
+  bool nan = false;
+  if (live) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      sm.box[0][k][t] = box.mn[k];
+      sm.box[0][3 + k][t] = box.mx[k];
+      nan = nan || isnan(box.mn[k]) || isnan(box.mx[k]);
+    }
+  }
+  if (__syncthreads_or(nan)) {
+    if (live) lbvh_climb<MODE, K>(i, n, keys, face, box, nodes, slots, err);
+    return;
+  }
+  // Deltas of the gaps around the block's leaves: gap g (local) at [g + 1], between leaves g and g + 1.
+  auto pair_delta = [&](int a) {  // leaves a and a + 1 (local), both in the tree
+    if (MODE == BVHGB_TOPO_REFCOMPAT) return __clz((int)((B0 + a) ^ (B0 + a + 1)));
+    const K x = sm.key[a + 1] ^ sm.key[a + 2];
+    if (x != 0) return sizeof(K) == 8 ? __clzll((long long)x) : __clz((int)x);
+    return kBits + __clz((int)((B0 + a) ^ (B0 + a + 1)));
+  };
+  if (live && B0 + t + 1 < n) sm.gap[t + 1] = (uint8_t)pair_delta(t);
+  if (t == 0 && B0 > 0) sm.gap[0] = (uint8_t)pair_delta(-1);
+  __syncthreads();
+  // The node of gap t: its range, if that lies in the block.
+  int l = t, r = t;
+  bool local = live && t + 1 < cnt;
+  if (local) {
+    const int d = sm.gap[t + 1];
+    r = t + 1;
+    if (MODE == BVHGB_TOPO_REFCOMPAT) {
+      const uint32_t mask = (2u << (31 - d)) - 1u;  // the range is the aligned block of that size (31 - d < 31)
+      const uint32_t gl = i & ~mask, gr = min(i | mask, n - 1u);
+      local = gl >= B0 && gr < B0 + (uint32_t)cnt;
+      l = (int)(gl - B0);
+      r = (int)(gr - B0);
+    } else {
+      const K mine = sm.key[t + 1];
+      const K bound = d < kBits ? (K)1 << (kBits - d) : (K)1;
+      auto same = [&](int c) {  // leaf c shares d bits with this gap's leaves (c may be a halo leaf)
+        if ((K)(sm.key[c + 1] ^ mine) >= bound) return false;
+        return d < kBits || __clz((int)((B0 + c) ^ i)) >= d - kBits;
+      };
+#pragma unroll
+      for (int step = T / 2; step > 0; step >>= 1) {
+        if (l - step >= 0 && same(l - step)) l -= step;
+        if (r + step < cnt && same(r + step)) r += step;
+      }
+      if (l == 0 && B0 > 0 && same(-1)) local = false;
+      if (r == cnt - 1 && B0 + cnt < n && same(cnt)) local = false;
+    }
+  }
+  const bool root = local && B0 + l == 0 && B0 + r == n - 1;
+  bool right = false;  // the node is its parent's left child: the parent splits at r
+  int slot = 0;        // its Karras index, less B0
+  if (local) {
+    right = B0 + l == 0 ? true : B0 + r == n - 1 ? false : sm.gap[r + 1] > sm.gap[l];
+    slot = root ? 0 : right ? r : l;
+    sm.made[slot] = 1;
+    const uint32_t parent = B0 + (uint32_t)slot;
+    if (l == t) sm.parLeaf[t] = parent | 0x80000000u;
+    else sm.parInner[t] = parent | 0x80000000u;
+    if (t + 1 == r) sm.parLeaf[t + 1] = parent;
+    else sm.parInner[t + 1] = parent;
+  }
+  // Boxes: windows of 1, 2, 4 ... leaves.
+  Box nb = box;
+  const int level = local ? 31 - __clz(r - l + 1) : -1;
+  int levels = 0;  // block-uniform: the highest level any node needs
+  {
+    if (t == 0) top = 0;
+    __syncthreads();
+    const int warpTop = __reduce_max_sync(0xFFFFFFFFu, level);
+    if ((t & 31) == 0 && warpTop > 0) atomicMax(&top, warpTop);
+    __syncthreads();
+    levels = top;
+  }
+  Box w = box;  // this thread's window W_j[t]
+  for (int j = 0; j < levels; ++j) {
+    const int half = 1 << j;
+    const float(*cur)[T] = sm.box[j & 1];
+    float(*nxt)[T] = sm.box[(j + 1) & 1];
+    if (t + half < cnt) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        w.mn[k] = fminf(w.mn[k], cur[k][t + half]);
+        w.mx[k] = fmaxf(w.mx[k], cur[3 + k][t + half]);
+      }
+    }
+    if (live) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        nxt[k][t] = w.mn[k];
+        nxt[3 + k][t] = w.mx[k];
+      }
+    }
+    __syncthreads();
+    if (level == j + 1) {
+      const int e = r - 2 * half + 1;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        nb.mn[k] = fminf(nxt[k][l], nxt[k][e]);
+        nb.mx[k] = fmaxf(nxt[3 + k][l], nxt[3 + k][e]);
+      }
+    }
+  }
+  __syncthreads();  // the windows make room for the records
+  auto stage = [&](int at, const Box &b, uint32_t par, uint32_t left, uint32_t rightLink, uint32_t leaf, uint32_t level) {
+    const uint32_t isLeft = par == kNone ? 0u : par >> 31, parent = par == kNone ? kNone : par & 0x7FFFFFFFu;
+    sm.record[3 * at] = make_float4(b.mn[0], b.mn[1], b.mn[2], b.mx[0]);
+    sm.record[3 * at + 1] = make_float4(b.mx[1], b.mx[2], __uint_as_float(parent), __uint_as_float(left));
+    sm.record[3 * at + 2] = make_float4(__uint_as_float(rightLink), __uint_as_float(leaf | (isLeft << 16)),
+                                        __uint_as_float(level), surface_area(b));
+  };
+  if (local)
+    stage(slot, nb, root ? 0u : sm.parInner[slot], l == t ? n - 1 + i : i, t + 1 == r ? n + i : i + 1, 0u, 0u);
+  __syncthreads();
+  float4 *out = reinterpret_cast<float4 *>(nodes + B0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int q = c * T + t;
+    if (q < 3 * cnt && sm.made[q / 3]) out[q] = sm.record[q];
+  }
+  __syncthreads();
+  if (live) stage(t, box, n == 1 ? 0u : sm.parLeaf[t], face, 1u, 1u, 255u);
+  __syncthreads();
+  out = reinterpret_cast<float4 *>(nodes + (size_t)n - 1 + B0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int q = c * T + t;
+    if (q < 3 * cnt) out[q] = sm.record[q];
+  }
+  // The roots of the block's subtrees: (l, r | is-left << 31).
+  const bool innerRoot = local && !root && sm.parInner[slot] == kNone;
+  const bool leafRoot = live && n > 1 && sm.parLeaf[t] == kNone;
+  if (t == 0) top = 0;
+  __syncthreads();
+  const uint32_t mine = (innerRoot ? 1u : 0u) + (leafRoot ? 1u : 0u);
+  uint32_t at = mine ? (uint32_t)atomicAdd(&top, (int)mine) : 0u;
+  __syncthreads();
+  if (t == 0 && top > 0) top = (int)atomicAdd(rootCount, (uint32_t)top);
+  __syncthreads();
+  if (mine) at += (uint32_t)top;
+  if (innerRoot) roots[at++] = make_uint2(B0 + l, (B0 + r) | (right ? 0x80000000u : 0u));
+  if (leafRoot) {
+    const bool leafRight = i == 0 ? true : i == n - 1 ? false : sm.gap[t + 1] > sm.gap[t];
+    roots[at] = make_uint2(i, i | (leafRight ? 0x80000000u : 0u));
+  }
 }
 
-template <int MODE>
-int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n,
-                 bvhgb_node *nodes, cudaStream_t s) {
-  // The exchange slots are re-armed by the Morton kernel; a second build from the same sorted keys
-  // re-arms them here.
-  if (!ws->slotsArmed) BVHGB_CUDA_TRY(cudaMemsetAsync(ws->slots, 0xFF, 4ull * n, s));
+// Climbs from the listed subtree roots.
+constexpr int kRootThreads = 128;
+template <int MODE, typename K>
+__global__ void __launch_bounds__(kRootThreads) lbvh_roots_kernel(const uint2 *__restrict__ roots,
+                                                                  const uint32_t *__restrict__ rootCount, uint32_t n,
+                                                                  const K *__restrict__ keys, bvhgb_node *nodes,
+                                                                  uint32_t *slots, uint32_t *err) {
+  const uint32_t count = min(*rootCount, n);
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+    const uint2 e = __ldg(roots + q);
+    const uint32_t l = e.x, r = e.y & 0x7FFFFFFFu;
+    const bool right = (e.y >> 31) != 0u;
+    const uint32_t node = l == r ? n - 1 + l : right ? r : l;
+    lbvh_climb_from<MODE, K>(l, r, right, load_box_cg(nodes + node), n, keys, nodes, slots, err);
+  }
+}
+
+
+template <int MODE, typename K>
+__global__ void __launch_bounds__(kTreelet) lbvh_build_kernel(const float *__restrict__ vert,
+                                                              const uint32_t *__restrict__ faces,
+                                                              const K *__restrict__ keys,
+                                                              const uint32_t *__restrict__ idx, uint32_t n,
+                                                              const float4 *__restrict__ boxes, bvhgb_node *nodes,
+                                                              uint32_t *slots, uint2 *__restrict__ roots,
+                                                              uint32_t *rootCount, uint32_t *err) {
+  __shared__ TreeletSmem<kTreelet, K> sm;
+  const uint32_t B0 = blockIdx.x * kTreelet, i = B0 + threadIdx.x;
+  uint32_t face = 0;
+  Box box = {};
+  if (i < n) {
+    face = __ldg(idx + i);
+    if (boxes) {
+      const float4 a = __ldg(boxes + 2 * (size_t)face), c = __ldg(boxes + 2 * (size_t)face + 1);
+      box.mn[0] = a.x; box.mn[1] = a.y; box.mn[2] = a.z;
+      box.mx[0] = a.w; box.mx[1] = c.x; box.mx[2] = c.y;
+    } else {
+      tri_box(vert, faces, face, box, nullptr);
+    }
+  }
+  treelet_build<MODE, kTreelet, K>(sm, B0, n, face, box, keys, nodes, slots, roots, rootCount, err);
+}
+
+// Roots a build of n leaves can list at most.
+size_t max_roots(uint32_t n) { return std::min<size_t>(n, (size_t)ceil_div(n, kTreelet) * kTreeletRoots); }
+
+template <int MODE, typename K>
+int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n, bvhgb_node *nodes,
+                 cudaStream_t s) {
+  // The exchange slots and the root counter are re-armed by the Morton kernel; a second build from the
+  // same sorted keys re-arms them here.
+  uint32_t *rootCount = ws->scene + 7;
+  if (!ws->slotsArmed) {
+    BVHGB_CUDA_TRY(cudaMemsetAsync(ws->slots, 0xFF, 4ull * n, s));
+    BVHGB_CUDA_TRY(cudaMemsetAsync(rootCount, 0, 4, s));
+  }
   ws->slotsArmed = false;
-  dim3 grid(ceil_div(n, kBuildThreads));
-  if (ws->keyBytes == 4)
-    lbvh_build_kernel<MODE, uint32_t><<<grid, kBuildThreads, 0, s>>>(
-        vert, faces, static_cast<const uint32_t *>(ws->keysSorted), ws->valsSorted, n, ws->triBoxes, nodes, ws->slots,
-        ws->scene + 6);
-  else
-    lbvh_build_kernel<MODE, uint64_t><<<grid, kBuildThreads, 0, s>>>(
-        vert, faces, static_cast<const uint64_t *>(ws->keysSorted), ws->valsSorted, n, ws->triBoxes, nodes, ws->slots,
-        ws->scene + 6);
+  // The list takes the place of the sort's alternate buffers, which nothing reads after the sort.
+  uint2 *roots = static_cast<uint2 *>(sort_alternate(ws->sortTemp, n, ws->keyBytes, 0, ws->cfg.mortonBits));
+  const K *keys = static_cast<const K *>(ws->keysSorted);
+  lbvh_build_kernel<MODE, K><<<ceil_div(n, kTreelet), kTreelet, 0, s>>>(
+      vert, faces, keys, ws->valsSorted, n, ws->triBoxes, nodes, ws->slots, roots, rootCount, ws->scene + 6);
   BVHGB_LAUNCH_CHECK("lbvh build");
+  if (n <= (uint32_t)kTreelet) return BVHGB_OK;  // one block makes the whole tree
+  const uint32_t grid = std::min(ceil_div(max_roots(n), kRootThreads), (uint32_t)sm_count() * 16);
+  lbvh_roots_kernel<MODE, K><<<grid, kRootThreads, 0, s>>>(roots, rootCount, n, keys, nodes, ws->slots, ws->scene + 6);
+  BVHGB_LAUNCH_CHECK("lbvh roots");
   return BVHGB_OK;
 }
 
@@ -256,9 +493,13 @@ extern "C" BVHGB_API int bvhgb_lbvh_build_tree(bvhgb_lbvh_workspace *ws, const f
   if (st) return st;
   if (n == 0) return BVHGB_OK;
   if (!vert || !faces || !nodes) return BVHGB_INVALID_ARGUMENT;
+  cudaStream_t s = as_stream(stream);
+  const bool wide = ws->keyBytes == 8;
   if (ws->cfg.topology == BVHGB_TOPO_REFCOMPAT)
-    return launch_build<BVHGB_TOPO_REFCOMPAT>(ws, vert, faces, n, nodes, as_stream(stream));
-  return launch_build<BVHGB_TOPO_KARRAS>(ws, vert, faces, n, nodes, as_stream(stream));
+    return wide ? launch_build<BVHGB_TOPO_REFCOMPAT, uint64_t>(ws, vert, faces, n, nodes, s)
+                : launch_build<BVHGB_TOPO_REFCOMPAT, uint32_t>(ws, vert, faces, n, nodes, s);
+  return wide ? launch_build<BVHGB_TOPO_KARRAS, uint64_t>(ws, vert, faces, n, nodes, s)
+              : launch_build<BVHGB_TOPO_KARRAS, uint32_t>(ws, vert, faces, n, nodes, s);
 }
 
 extern "C" BVHGB_API int bvhgb_lbvh_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces,

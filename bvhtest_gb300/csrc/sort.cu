@@ -388,6 +388,10 @@ uint32_t *sort_error_word(void *temp, uint32_t n, uint32_t keyBytes, uint32_t be
   return reinterpret_cast<uint32_t *>(static_cast<char *>(temp) + L.err);
 }
 
+void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit) {
+  return static_cast<char *>(temp) + make_layout(n, keyBytes, beginBit, endBit).altKeys;
+}
+
 int sort_pairs(void *temp, const void *keysIn, void *keysOut, const uint32_t *valsIn, uint32_t *valsOut, uint32_t n,
                uint32_t keyBytes, uint32_t beginBit, uint32_t endBit, cudaStream_t s, uint32_t tileKeys) {
   if (keyBytes == 4)

@@ -1,0 +1,61 @@
+"""The block-wise tree build gives the nodes of the leaf-by-leaf climb (which the batched build still
+is), byte for byte, around the block size, on equal and comb-like keys, and where a coordinate is
+infinite or no number (a block with one climbs); 63-bit keys against the oracle."""
+import numpy as np
+import pytest
+
+from bvhtest_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+SIZES = [1, 2, 3, 31, 255, 256, 257, 511, 513, 4096, 66049]
+
+
+def _vert(kind, n, seed):
+    vert, faces = scenes.uniform_soup(n, sigma=0.01, seed=seed)
+    tri = vert.reshape(n, 3, 3)
+    if kind == "equal":
+        tri[:] = tri[0]
+    elif kind == "runs":  # long runs of equal keys
+        tri[:] = tri[np.arange(n) // 300 * 300 % n]
+    elif kind == "comb":  # cells at powers of two on a line: a deep, one-sided tree
+        tri[:] = 0.0
+        tri[:, :, 0] = (0.5 ** (np.arange(n) % 22))[:, None]
+    elif kind in ("nan", "inf"):
+        g = np.random.default_rng(seed)
+        pick = g.integers(0, n, max(1, n // 400))
+        tri[pick, g.integers(0, 3, pick.size), g.integers(0, 3, pick.size)] = np.nan if kind == "nan" else np.inf
+    return tri.reshape(-1, 3).astype(np.float32), faces
+
+
+@pytest.mark.parametrize("topo", ["refCompat", "karras"])
+@pytest.mark.parametrize("kind", ["soup", "equal", "runs", "comb", "nan", "inf"])
+@pytest.mark.parametrize("n", SIZES)
+def test_equals_the_climb(gpu, n, kind, topo):
+    import torch
+    vert, faces = _vert(kind, n, n)
+    v = torch.from_numpy(vert).cuda()
+    f = torch.from_numpy(faces.view(np.int32)).cuda()
+    one = gpu.LBVH(n, 30, topo)
+    got = one.build(v, f)
+    again = gpu.empty_nodes(2 * n - 1)
+    one.build_tree(v, f, again)  # from the same sorted keys: slots and root counter re-armed
+    batch = gpu.Batch([n], topology=topo)
+    ref = batch.empty_nodes()
+    batch.build(v, f, ref)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref) and torch.equal(again, ref)
+    assert one.errors() == 0
+
+
+@pytest.mark.parametrize("topo", ["refCompat", "karras"])
+@pytest.mark.parametrize("kind", ["soup", "equal", "runs", "comb"])
+@pytest.mark.parametrize("n", [2, 255, 257, 5000, 66049])
+def test_long_keys(gpu, orc, n, kind, topo):
+    import torch
+    vert, faces = _vert(kind, n, n + 1)
+    b = gpu.LBVH(n, 63, topo)
+    got = b.build(torch.from_numpy(vert).cuda(), torch.from_numpy(faces.view(np.int32)).cuda())
+    torch.cuda.synchronize()
+    ref, _, _ = orc.lbvh_build(vert, faces, 63, 0 if topo == "refCompat" else 1)
+    assert np.array_equal(gpu.nodes_to_numpy(got).view(np.uint8), ref.view(np.uint8))
+    assert b.errors() == 0
