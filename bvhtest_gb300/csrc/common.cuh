@@ -109,6 +109,11 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
+// The next launch of the stream may start now; what it needs of this one it waits for itself.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Everything the launches before this one wrote is visible from here on.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 }  // namespace bvhgb
@@ -123,6 +128,23 @@ inline cudaStream_t as_stream(bvhgb_stream s) { return reinterpret_cast<cudaStre
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 int sm_count();
 uint64_t context_id();
+// Launch; early: it may start while the stream's previous kernel drains, and the kernel calls grid_wait()
+// before it touches anything that kernel (or one before it) wrote or reads.
+template <typename... P, typename... A>
+inline void launch_kernel(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, bool early,
+                          A &&...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 // cudaMalloc through the library's allocation-failure injection (bvhgb_debug_fail_allocations).
 cudaError_t dev_malloc(void **p, size_t bytes);
 template <typename T>

@@ -26,7 +26,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t maxFaces = 0;
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
-  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, root counter
+  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, root counter, sort gate
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -483,6 +483,10 @@ extern "C" BVHGB_API int bvhgb_lbvh_calc_morton(bvhgb_lbvh_workspace *ws, const 
 extern "C" BVHGB_API int bvhgb_lbvh_sort(bvhgb_lbvh_workspace *ws, uint32_t n, bvhgb_stream stream) {
   int st = check_ws(ws, n);
   if (st) return st;
+  if (ws->keyBytes == 8) {
+    return sort_morton(ws->sortTemp, static_cast<const uint64_t *>(ws->keys), static_cast<uint64_t *>(ws->keysSorted),
+                       ws->vals, ws->valsSorted, n, ws->scene + 8, as_stream(stream));
+  }
   return sort_pairs(ws->sortTemp, ws->keys, ws->keysSorted, ws->vals, ws->valsSorted, n, ws->keyBytes, 0,
                     ws->cfg.mortonBits, as_stream(stream));
 }

@@ -389,11 +389,6 @@ __device__ __forceinline__ uint32_t batch_row(uint64_t seed, uint64_t t, uint32_
   return (uint32_t)(z % numSamples);
 }
 
-// The next launch of the stream may start now; what it needs of this one it waits for itself.
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Everything the launches before this one wrote is visible from here on.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // n samples; with numSamples > 0 sample s is row batch_row(seed, step, n, s, numSamples) of x,
 // otherwise row s. The tile's loss goes to *loss.
 __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(const __nv_bfloat16 *__restrict__ w,

@@ -72,10 +72,21 @@ Layout make_layout(uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t en
   return L;
 }
 
+// A kernel given a gate word does its work only where that is not zero (null: always). The launches of a
+// gated sort start while the one before is still draining, so that a closed gate costs little.
+__device__ __forceinline__ bool gate_closed(const uint32_t *gate) {
+  if (!gate) return false;
+  grid_release();
+  grid_wait();
+  return __ldcg(gate) == 0u;
+}
+
 template <typename K>
 __global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict__ keys, uint32_t n,
                                                              uint32_t beginBit, uint32_t endBit, uint32_t passes,
-                                                             uint32_t *__restrict__ hist) {
+                                                             uint32_t *__restrict__ hist,
+                                                             const uint32_t *gate) {
+  if (gate_closed(gate)) return;
   extern __shared__ uint32_t sh[];  // passes * 256
   for (uint32_t i = threadIdx.x; i < passes * kRadix; i += blockDim.x) sh[i] = 0;
   __syncthreads();
@@ -93,7 +104,8 @@ __global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict
 }
 
 // Exclusive scan of each pass's 256 counts, in place. One CTA per pass.
-__global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist) {
+__global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint32_t *gate) {
+  if (gate_closed(gate)) return;
   __shared__ uint32_t s[kRadix];
   uint32_t *h = hist + blockIdx.x * kRadix;
   uint32_t v = h[threadIdx.x];
@@ -108,6 +120,10 @@ __global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist) {
   h[threadIdx.x] = s[threadIdx.x] - v;
 }
 
+// CTAs per SM of a tile shape.
+template <int ITEMS>
+constexpr int kSortCtas = ITEMS <= 8 ? 3 : 2;
+
 template <typename K, int THREADS, int ITEMS>
 struct OnesweepSmem {
   static constexpr int kWarps = THREADS / 32;
@@ -117,179 +133,237 @@ struct OnesweepSmem {
   uint32_t globalBase[kRadix];
   uint32_t scanTot[kRadix / 32];
   uint32_t tileIdx;
+  // The tile in digit order; its values beside the keys or, where two CTAs would not fit then, in their
+  // place once the keys are written.
+  static constexpr bool kSplit = sizeof(K) == 8 && THREADS == 512;
   K keys[kTile];
-  uint32_t vals[kTile];
+  uint32_t valsOwn[kSplit ? 1 : kTile];
+  __device__ __forceinline__ uint32_t *vals() { return kSplit ? reinterpret_cast<uint32_t *>(keys) : valsOwn; }
 };
 
+// CTAs take tiles from the counter until none is left. Bound: a tile's phases (load, rank, look back,
+// stage, write) are a chain of latencies with barriers between them, so a second CTA per SM is what
+// fills them: 64 registers per thread (ranks kept as 16-bit pairs, values read when the keys are out
+// of the way) and one staging buffer for keys and then values (82 KB for 8,192 64-bit keys). A pass of
+// 4.19M / 33.5M pairs of 64-bit keys: 45 / 310 us; with one CTA per SM and 124 registers 49 / 336;
+// with the look-back before the staging 50 / 298, in the lower warps while the upper ones stage 48 /
+// 374; 32 predecessors per round trip 46 / 334; digits matched by match.any 58 / 397.
 template <typename K, int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? 2 : 1) onesweep_kernel(const K *__restrict__ keysIn, K *__restrict__ keysOut,
-                                                            const uint32_t *__restrict__ valsIn,
-                                                            uint32_t *__restrict__ valsOut, uint32_t n,
-                                                            uint32_t shift, uint32_t mask,
-                                                            const uint32_t *__restrict__ offsets,
-                                                            uint32_t *tileCounter, uint32_t *status, uint32_t *err) {
+__global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
+    const K *__restrict__ keysIn, K *__restrict__ keysOut, const uint32_t *__restrict__ valsIn,
+    uint32_t *__restrict__ valsOut, uint32_t n, uint32_t tiles, uint32_t shift, uint32_t mask,
+    const uint32_t *__restrict__ offsets, uint32_t *tileCounter, uint32_t *status, uint32_t *err,
+    const uint32_t *gate) {
+  if (gate_closed(gate)) return;
   using Smem = OnesweepSmem<K, THREADS, ITEMS>;
-  constexpr int kWarps = Smem::kWarps, kTile = Smem::kTile, kItems = ITEMS, kThreads = THREADS;
+  constexpr int kWarps = Smem::kWarps, kTile = Smem::kTile;
+  constexpr bool kSplit = Smem::kSplit, kLate = THREADS == 512;
   static_assert(THREADS >= kRadix, "one thread per digit in the look-back");
+  static_assert(ITEMS % 4 == 0 && kTile <= 65536, "ranks in groups of four, as 16-bit pairs");
   extern __shared__ __align__(16) unsigned char smraw[];
   Smem &sm = *reinterpret_cast<Smem *>(smraw);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-
-  if (threadIdx.x == 0) sm.tileIdx = atomicAdd(tileCounter, 1u);
-  for (uint32_t i = lane; i < kBins; i += 32) sm.warpHist[warp][i] = 0;
-  __syncthreads();
-  const uint32_t tile = sm.tileIdx;
-  const uint64_t base = (uint64_t)tile * kTile;
-  const uint32_t valid = (uint32_t)min((uint64_t)kTile, (uint64_t)n - base);
-
-  // Warp-striped load: warp w owns keys [w*kItems*32, (w+1)*kItems*32) of the tile.
-  K key[kItems];
-  uint32_t val[kItems], dig[kItems], loc[kItems];
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    uint32_t t = warp * (kItems * 32) + j * 32 + lane;
-    if (t < valid) {
-      key[j] = keysIn[base + t];
-      val[j] = valsIn[base + t];
-      dig[j] = (uint32_t)(key[j] >> shift) & mask;
-    } else {
-      key[j] = 0;
-      val[j] = 0;
-      dig[j] = kRadix;  // padding bin
-    }
-  }
-  // Stable rank within the warp: items in order, lanes in order. Peers of an item are the lanes
-  // with the same digit (9 ballots: 8 digit bits + the padding bin); the lowest of them advances
-  // the warp's counter for that digit by their number. All atomics are issued first, in item
-  // order (__syncwarp orders them), and their results are used afterwards.
   const uint32_t ltMask = (1u << lane) - 1u;
-  uint32_t old[kItems], peersOf[kItems];
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    uint32_t peers = 0xFFFFFFFFu;
-#pragma unroll
-    for (int bit = 0; bit < 9; ++bit) {
-      const bool on = (dig[j] >> bit) & 1u;
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
-      peers &= on ? bal : ~bal;
-    }
-    peersOf[j] = peers;
-    old[j] = 0;
-    if ((peers & ltMask) == 0) old[j] = atomicAdd(&sm.warpHist[warp][dig[j]], (uint32_t)__popc(peers));
-    __syncwarp();
-  }
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    const uint32_t leader = __ffs(peersOf[j]) - 1u;
-    loc[j] = __shfl_sync(0xFFFFFFFFu, old[j], leader) + __popc(peersOf[j] & ltMask);
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) sm.tileIdx = atomicAdd(tileCounter, 1u);
+  for (;;) {
+    for (uint32_t i = lane; i < kBins; i += 32) sm.warpHist[warp][i] = 0;
+    __syncthreads();
+    const uint32_t tile = sm.tileIdx;
+    if (tile >= tiles) return;
+    const uint64_t base = (uint64_t)tile * kTile;
+    const uint32_t valid = (uint32_t)min((uint64_t)kTile, (uint64_t)n - base);
+    const uint32_t t0 = warp * (ITEMS * 32) + lane;  // warp-striped: item j of the thread is key t0 + 32 j
 
-  // Per digit (one thread each): exclusive over warps, tile count, publish, look back; the tile's
-  // exclusive scan over digits runs at the same time (a warp scan per 32 digits).
-  uint32_t count = 0, incl = 0;
-  if (threadIdx.x < kRadix) {
-    const uint32_t d = threadIdx.x;
+    K key[ITEMS];
+    uint32_t val[ITEMS];
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      uint32_t c = sm.warpHist[w][d];
-      sm.warpHist[w][d] = count;
-      count += c;
+    for (int j = 0; j < ITEMS; ++j) {
+      key[j] = t0 + 32 * j < valid ? keysIn[base + t0 + 32 * j] : (K)0;
+      if (!kSplit) val[j] = t0 + 32 * j < valid ? valsIn[base + t0 + 32 * j] : 0u;
     }
-    uint32_t *st = status + (size_t)tile * kRadix + d;
-    st_relaxed(st, (tile == 0 ? kFlagInc : kFlagAgg) | count);
-    incl = count;
+    // Stable rank within the warp: items in order, lanes in order. Peers of an item are the lanes
+    // with the same digit (8 ballots, and one for the padding bin in the last tile); the lowest of
+    // them advances the warp's counter for that digit by their number. The atomics of four items are
+    // issued, in item order (__syncwarp orders them), before their results are used.
+    uint32_t rank[ITEMS / 2];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
+    for (int j0 = 0; j0 < ITEMS; j0 += 4) {
+      uint32_t old[4], peers[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = j0 + q;
+        const bool in = t0 + 32 * j < valid;
+        const uint32_t d = in ? (uint32_t)(key[j] >> shift) & mask : (uint32_t)kRadix;
+        uint32_t p = 0xFFFFFFFFu;
+        if (valid != (uint32_t)kTile) {
+          const uint32_t bal = __ballot_sync(0xFFFFFFFFu, in);
+          p = in ? bal : ~bal;
+        }
+#pragma unroll
+        for (int bit = 0; bit < 8; ++bit) {
+          const bool on = (d >> bit) & 1u;
+          const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+          p &= on ? bal : ~bal;
+        }
+        peers[q] = p;
+        old[q] = 0;
+        if ((p & ltMask) == 0) old[q] = atomicAdd(&sm.warpHist[warp][d], (uint32_t)__popc(p));
+        __syncwarp();
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q += 2) {
+        const uint32_t a = __shfl_sync(0xFFFFFFFFu, old[q], __ffs(peers[q]) - 1) + __popc(peers[q] & ltMask);
+        const uint32_t b = __shfl_sync(0xFFFFFFFFu, old[q + 1], __ffs(peers[q + 1]) - 1) + __popc(peers[q + 1] & ltMask);
+        rank[(j0 + q) / 2] = a | (b << 16);
+      }
     }
-    if (lane == 31) sm.scanTot[warp] = incl;
-    uint32_t excl = 0;
-    if (tile > 0) {
-      int64_t pred = (int64_t)tile - 1;
-      bool done = false;
-      while (!done) {
-        uint32_t v[kLook];
+    __syncthreads();
+
+    // Per digit (one thread each): the tile's count, published; its place in the tile (a warp scan per
+    // 32 digits) and from it every warp's. Staging needs no more, so for the large tile the
+    // look-back comes after it: the predecessors' counts arrive meanwhile and the keys' registers are
+    // free for it. The smaller tiles look back at once (65,536 30-bit pairs in tiles of 2,048: 51 us
+    // against 58; 4.19M in tiles of 8,192: 213 against 191).
+    auto look_back = [&](uint32_t d, uint32_t count) {
+      uint32_t excl = 0;
+      if (tile > 0) {
+        int64_t pred = (int64_t)tile - 1;
+        bool done = false;
+        while (!done) {
+          uint32_t v[kLook];
 #pragma unroll
-        for (int q = 0; q < kLook; ++q) v[q] = pred - q >= 0 ? ld_relaxed(status + (size_t)(pred - q) * kRadix + d) : kFlagInc;
+          for (int q = 0; q < kLook; ++q) v[q] = pred - q >= 0 ? ld_relaxed(status + (size_t)(pred - q) * kRadix + d) : kFlagInc;
 #pragma unroll
-        for (int q = 0; q < kLook; ++q) {
-          if (done) break;
-          if (pred - q < 0) {
-            done = true;
-            break;
-          }
-          const uint32_t *ps = status + (size_t)(pred - q) * kRadix + d;
-          uint32_t spins = 0;
-          while ((v[q] & kFlagMask) == 0u) {
-            if (++spins > g_lookback_spin_limit) {
-              atomicOr(err, kErrTimeout);
+          for (int q = 0; q < kLook; ++q) {
+            if (done) break;
+            if (pred - q < 0) {
+              done = true;
               break;
             }
-            __nanosleep(32);
-            v[q] = ld_relaxed(ps);
+            const uint32_t *ps = status + (size_t)(pred - q) * kRadix + d;
+            uint32_t spins = 0;
+            while ((v[q] & kFlagMask) == 0u) {
+              if (++spins > g_lookback_spin_limit) {
+                atomicOr(err, kErrTimeout);
+                break;
+              }
+              __nanosleep(32);
+              v[q] = ld_relaxed(ps);
+            }
+            if ((v[q] & kFlagMask) == 0u) {
+              done = true;
+              break;
+            }
+            excl += v[q] & kValMask;
+            if (v[q] & kFlagInc) done = true;
           }
-          if ((v[q] & kFlagMask) == 0u) {
-            done = true;
-            break;
-          }
-          excl += v[q] & kValMask;
-          if (v[q] & kFlagInc) done = true;
+          pred -= kLook;
         }
-        pred -= kLook;
+        st_relaxed(status + (size_t)tile * kRadix + d, kFlagInc | (excl + count));
       }
-      st_relaxed(st, kFlagInc | (excl + count));
-    }
-    sm.globalBase[d] = offsets[d] + excl;
-  }
-  __syncthreads();
-  if (threadIdx.x < kRadix) {
-    uint32_t prefix = 0;
-    for (uint32_t w = 0; w < warp; ++w) prefix += sm.scanTot[w];
-    sm.tileStart[threadIdx.x] = prefix + incl - count;
-  }
-  __syncthreads();
-  // Stage the tile in digit order.
+      sm.globalBase[d] = offsets[d] + excl;
+    };
+    uint32_t count = 0, incl = 0;
+    if (threadIdx.x < kRadix) {
+      const uint32_t d = threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    if (dig[j] < kRadix) {
-      uint32_t pos = sm.tileStart[dig[j]] + sm.warpHist[warp][dig[j]] + loc[j];
-      sm.keys[pos] = key[j];
-      sm.vals[pos] = val[j];
+      for (int w = 0; w < kWarps; ++w) count += sm.warpHist[w][d];
+      st_relaxed(status + (size_t)tile * kRadix + d, (tile == 0 ? kFlagInc : kFlagAgg) | count);
+      incl = count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      if (lane == 31) sm.scanTot[warp] = incl;
+      if (!kLate) look_back(d, count);
     }
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < valid; i += kThreads) {
-    K k = sm.keys[i];
-    uint32_t d = (uint32_t)(k >> shift) & mask;
-    uint32_t dst = sm.globalBase[d] + (i - sm.tileStart[d]);
-    // Always true for a consistent sort; after a look-back timeout (err set) a later pass reads a
-    // permuted, partly stale key array whose digits no longer match the histogram, and this keeps
-    // its writes inside the arrays.
-    if (dst < n) {
-      keysOut[dst] = k;
-      valsOut[dst] = sm.vals[i];
+    __syncthreads();
+    if (threadIdx.x < kRadix) {
+      const uint32_t d = threadIdx.x;
+      uint32_t at = incl - count;
+      for (uint32_t w = 0; w < warp; ++w) at += sm.scanTot[w];
+      sm.tileStart[d] = at;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const uint32_t c = sm.warpHist[w][d];
+        sm.warpHist[w][d] = at;
+        at += c;
+      }
     }
+    __syncthreads();
+    // Stage the tile's keys in digit order; a rank becomes the place in the tile.
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (t0 + 32 * j < valid) {
+        const uint32_t d = (uint32_t)(key[j] >> shift) & mask;
+        const uint32_t pos = sm.warpHist[warp][d] + ((rank[j / 2] >> (16 * (j & 1))) & 0xFFFFu);
+        sm.keys[pos] = key[j];
+        if (!kSplit) sm.valsOwn[pos] = val[j];
+        if (kSplit) rank[j / 2] = j & 1 ? (rank[j / 2] & 0xFFFFu) | (pos << 16) : (rank[j / 2] & 0xFFFF0000u) | pos;
+      }
+    }
+    if (kLate && threadIdx.x < kRadix) look_back(threadIdx.x, count);
+    // The next tile (every thread has read this one's index), if there are more tiles than CTAs. Tiles
+    // are taken in order and a CTA's tile waits for lower ones only, so the lowest unfinished tile is
+    // always being worked on.
+    const bool more = gridDim.x < tiles;
+    if (more && threadIdx.x == THREADS - 1) sm.tileIdx = atomicAdd(tileCounter, 1u);
+    if (kSplit) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) val[j] = t0 + 32 * j < valid ? valsIn[base + t0 + 32 * j] : 0u;
+    }
+    __syncthreads();
+    uint32_t dst[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t i = j * THREADS + threadIdx.x;
+      dst[j] = n;
+      if (i < valid) {
+        const K k = sm.keys[i];
+        const uint32_t d = (uint32_t)(k >> shift) & mask;
+        dst[j] = sm.globalBase[d] + (i - sm.tileStart[d]);
+        // Always true for a consistent sort; after a look-back timeout (err set) a later pass reads a
+        // permuted, partly stale key array whose digits no longer match the histogram, and this keeps
+        // its writes inside the arrays.
+        if (dst[j] < n) {
+          keysOut[dst[j]] = k;
+          if (!kSplit) valsOut[dst[j]] = sm.valsOwn[i];
+        }
+      }
+    }
+    if (kSplit) {
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j)
+        if (t0 + 32 * j < valid) sm.vals()[(rank[j / 2] >> (16 * (j & 1))) & 0xFFFFu] = val[j];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j)
+        if (dst[j] < n) valsOut[dst[j]] = sm.vals()[j * THREADS + threadIdx.x];
+    }
+    if (!more) return;
   }
 }
 
+// The passes over bits [beginBit, endBit) between the out and alternate arrays, the last one into the out
+// arrays (outLast) or into the alternate ones.
 template <typename K, int THREADS, int ITEMS>
 int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t *valsIn, uint32_t *valsOut, K *altK,
                     uint32_t *altV, uint32_t *hist, uint32_t *counters, uint32_t *status, uint32_t *err, uint32_t n,
-                    uint32_t beginBit, uint32_t endBit, cudaStream_t s) {
+                    uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate, bool outLast) {
   const size_t smem = sizeof(OnesweepSmem<K, THREADS, ITEMS>);
-  // Ping-pong so that the last pass lands in keysOut/valsOut.
+  const uint32_t grid = min(L.tiles, (uint32_t)(sm_count() * kSortCtas<ITEMS>));
   const K *srcK = keysIn;
   const uint32_t *srcV = valsIn;
   for (uint32_t p = 0; p < L.passes; ++p) {
-    const bool toOut = ((L.passes - 1 - p) % 2) == 0;
+    const bool toOut = (((L.passes - 1 - p) % 2) == 0) == outLast;
     K *dstK = toOut ? keysOut : altK;
     uint32_t *dstV = toOut ? valsOut : altV;
     const uint32_t shift = beginBit + 8 * p;
-    onesweep_kernel<K, THREADS, ITEMS><<<L.tiles, THREADS, smem, s>>>(
-        srcK, dstK, srcV, dstV, n, shift, digit_mask(shift, endBit), hist + p * kRadix, counters + p,
-        status + (size_t)p * L.tiles * kRadix, err);
+    launch_kernel(onesweep_kernel<K, THREADS, ITEMS>, grid, THREADS, smem, s, gate != nullptr, srcK, dstK, srcV, dstV, n,
+                  L.tiles, shift, digit_mask(shift, endBit), hist + p * kRadix, counters + p,
+                  status + (size_t)p * L.tiles * kRadix, err, gate);
     BVHGB_LAUNCH_CHECK("radix onesweep");
     srcK = dstK;
     srcV = dstV;
@@ -297,12 +371,51 @@ int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t
   return BVHGB_OK;
 }
 
+// Histogram, scan and passes; hist, counters, err and status start at zero.
+template <typename K>
+int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn,
+                uint32_t *valsOut, K *altK, uint32_t *altV, uint32_t *hist, uint32_t *counters, uint32_t *status,
+                uint32_t *err, uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate,
+                bool outLast) {
+  const uint32_t hgrid = min(ceil_div(n, kThreads * 8), (uint32_t)sm_count() * 4);
+  const bool early = gate != nullptr;
+  launch_kernel(histogram_kernel<K>, hgrid, kThreads, sizeof(uint32_t) * kRadix * L.passes, s, early, keysIn, n,
+                beginBit, endBit, L.passes, hist, gate);
+  BVHGB_LAUNCH_CHECK("radix histogram");
+  launch_kernel(scan_kernel, L.passes, kRadix, 0, s, early, hist, gate);
+  BVHGB_LAUNCH_CHECK("radix scan");
+  switch (tileKeys) {
+    case 2048:
+      return onesweep_passes<K, 256, 8>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
+                                        beginBit, endBit, s, gate, outLast);
+    case 4096:
+      return onesweep_passes<K, 256, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
+                                         n, beginBit, endBit, s, gate, outLast);
+    default:
+      return onesweep_passes<K, 512, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
+                                         n, beginBit, endBit, s, gate, outLast);
+  }
+}
+
 std::atomic<uint32_t> g_default_tile{kSortTileDefault};
+
+// Keys per CTA of a sort that is given none: small sorts fill few CTAs at the large tiles (30-bit pairs,
+// 2,048 / 8,192 keys: 65,536 pairs 52 / 72 us, 524,288 73 / 80, 1M 95 / 86).
+uint32_t auto_tile(uint32_t n) {
+  return n <= (1u << 19) ? (uint32_t)kMinTile : g_default_tile.load(std::memory_order_relaxed);
+}
+
+// The gated sort's memset: all but the error word, which keeps what an earlier pass found.
+__global__ void clear_kernel(uint32_t *p, uint32_t words, const uint32_t *err, const uint32_t *gate) {
+  if (gate_closed(gate)) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x)
+    if (p + i != err) p[i] = 0u;
+}
 
 template <typename K>
 int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-              uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s) {
-  if (tileKeys == 0) tileKeys = g_default_tile.load(std::memory_order_relaxed);
+              uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate = nullptr) {
+  if (tileKeys == 0) tileKeys = auto_tile(n);
   const Layout L = make_layout(n, sizeof(K), beginBit, endBit, tileKeys);
   const Layout Lmax = make_layout(n, sizeof(K), beginBit, endBit, kMinTile);  // the temp space's layout
   char *t = static_cast<char *>(temp);
@@ -319,25 +432,60 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
     return BVHGB_OK;
   }
   // hist, counters, err and the status words this tile size uses start at zero
-  BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes, s));
-  uint32_t hgrid = min(ceil_div(n, kThreads * 8), (uint32_t)sm_count() * 4);
-  histogram_kernel<K><<<hgrid, kThreads, sizeof(uint32_t) * kRadix * L.passes, s>>>(keysIn, n, beginBit, endBit,
-                                                                                      L.passes, hist);
-  BVHGB_LAUNCH_CHECK("radix histogram");
-  scan_kernel<<<L.passes, kRadix, 0, s>>>(hist);
-  BVHGB_LAUNCH_CHECK("radix scan");
+  const size_t zeroed = Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes;
+  if (gate) {
+    launch_kernel(clear_kernel, min(ceil_div(zeroed, 4096), (uint32_t)sm_count() * 4), 256, 0, s, true,
+                  reinterpret_cast<uint32_t *>(t), (uint32_t)(zeroed / 4), err, gate);
+    BVHGB_LAUNCH_CHECK("radix clear");
+  } else {
+    BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, zeroed, s));
+  }
   int st = sort_prepare();
   if (st) return st;
-  switch (tileKeys) {
-    case 2048:
-      return onesweep_passes<K, 256, 8>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
-                                        beginBit, endBit, s);
-    case 4096:
-      return onesweep_passes<K, 256, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s);
-    default:
-      return onesweep_passes<K, 512, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s);
+  return sort_passes<K>(L, tileKeys, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
+                        beginBit, endBit, s, gate, true);
+}
+
+// ---- 63-bit Morton keys -----------------------------------------------------------------------------
+//
+// sort_morton: the stable order of 63-bit keys from passes over their upper 32 or 40 bits only and one
+// kernel that puts the groups with equal upper bits in order: a group's members stand in their
+// original order, so a member's place is the number of members with a lower key, or an equal one and
+// an earlier position, and every member counts that for itself. A mesh leaves few triangles in one
+// cell of the upper bits; a group of more than kMaxGroup raises the gate, and the full eight-pass
+// sort, whose launches otherwise return at once, makes the order instead. Measured against the eight
+// passes alone: 65,536 keys 96 us against 119, 1M 122 / 153, 4.19M 274 / 441, 33.5M 1,840 / 2,840.
+constexpr int kGroupTile = 1024;  // keys per block, 256 threads
+constexpr int kMaxGroup = 256;
+
+__global__ void __launch_bounds__(256) order_groups_kernel(const uint64_t *__restrict__ keys,
+                                                           const uint32_t *__restrict__ vals, uint32_t n,
+                                                           uint32_t beginBit, uint64_t *__restrict__ keysOut,
+                                                           uint32_t *__restrict__ valsOut, uint32_t *gate) {
+  constexpr int kSpan = kGroupTile + kMaxGroup;
+  __shared__ uint64_t key[kSpan + 1];  // [e + 1]: the tile's keys and the halo behind it; [0]: the key before the tile
+  const uint32_t base = blockIdx.x * kGroupTile;
+  const int valid = (int)min((uint32_t)kSpan, n - base);
+  const bool first = base == 0;
+  for (int e = (int)threadIdx.x - 1; e < valid; e += 256)
+    if (e >= 0 || !first) key[e + 1] = __ldg(keys + base + e);
+  __syncthreads();
+  const uint64_t last = key[min(kGroupTile, valid)] >> beginBit;  // the tile's last group, which the halo may go on with
+  for (int e = threadIdx.x; e < valid; e += 256) {
+    const uint64_t mine = key[e + 1], u = mine >> beginBit;
+    if (e >= kGroupTile && u != last) break;  // sorted: no later one either
+    int lo = e, hi = e + 1;
+    while (lo > 0 && key[lo] >> beginBit == u && e - lo <= kMaxGroup) --lo;
+    if (lo == 0 && !first && key[0] >> beginBit == u && e <= kMaxGroup) continue;  // an earlier tile's group, which orders it
+    while (hi < valid && hi - lo <= kMaxGroup && key[hi + 1] >> beginBit == u) ++hi;  // the halo is as long as a group may be
+    if (hi - lo > kMaxGroup) {
+      *gate = 1u;
+      continue;
+    }
+    int at = lo;
+    for (int j = lo; j < hi; ++j) at += key[j + 1] < mine || (key[j + 1] == mine && j < e) ? 1 : 0;
+    keysOut[base + at] = mine;
+    valsOut[base + at] = __ldg(vals + base + e);
   }
 }
 
@@ -386,6 +534,34 @@ size_t sort_temp_bytes(uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_
 uint32_t *sort_error_word(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit) {
   Layout L = make_layout(n, keyBytes, beginBit, endBit);
   return reinterpret_cast<uint32_t *>(static_cast<char *>(temp) + L.err);
+}
+
+int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
+                uint32_t n, uint32_t *gate, cudaStream_t s) {
+  int st = sort_prepare();
+  if (st) return st;
+  if (n == 0) return BVHGB_OK;
+  // 2^32 cells for up to 8M triangles, 2^40 for more: the densest cells of the benchmark scenes then hold
+  // a few dozen (33.5M triangles in 64 clusters put over 256 into some of 2^32 cells).
+  const uint32_t beginBit = n <= (1u << 23) ? 31u : 23u;
+  const uint32_t tileKeys = auto_tile(n);
+  const Layout L = make_layout(n, 8, beginBit, 63, tileKeys);
+  const Layout Lmax = make_layout(n, 8, 0, 63, kMinTile);  // the temp space's layout
+  char *t = static_cast<char *>(temp);
+  uint32_t *hist = reinterpret_cast<uint32_t *>(t + Lmax.hist);
+  uint32_t *counters = reinterpret_cast<uint32_t *>(t + Lmax.counters);
+  uint32_t *err = reinterpret_cast<uint32_t *>(t + Lmax.err);
+  uint32_t *status = reinterpret_cast<uint32_t *>(t + Lmax.status);
+  uint64_t *altK = reinterpret_cast<uint64_t *>(t + Lmax.altKeys);
+  uint32_t *altV = reinterpret_cast<uint32_t *>(t + Lmax.altVals);
+  BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes, s));
+  BVHGB_CUDA_TRY(cudaMemsetAsync(gate, 0, 4, s));
+  st = sort_passes<uint64_t>(L, tileKeys, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
+                             beginBit, 63, s, nullptr, false);
+  if (st) return st;
+  order_groups_kernel<<<ceil_div(n, kGroupTile), 256, 0, s>>>(altK, altV, n, beginBit, keysOut, valsOut, gate);
+  BVHGB_LAUNCH_CHECK("order groups");
+  return sort_impl<uint64_t>(temp, tileKeys, keysIn, keysOut, valsIn, valsOut, n, 0, 63, s, gate);
 }
 
 void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit) {
@@ -676,9 +852,6 @@ int select_smallest(void *temp, const uint32_t *keys, const uint32_t *vals, uint
   BVHGB_LAUNCH_CHECK("select scan");
   select_scatter_kernel<<<L.tiles, 256, 0, s>>>(keys, vals, n, k, st, tileLt, tileEq, ck, cv, vec);
   BVHGB_LAUNCH_CHECK("select scatter");
-  // A few hundred thousand kept pairs fill few CTAs at the large tiles: the smallest tile spreads
-  // them wider (the order does not depend on the tile).
-  if (tileKeys == 0 && k <= (1u << 18)) tileKeys = 2048;
   return sort_pairs(t + L.sortTemp, ck, ko, cv, valsOut, k, 4, 0, 32, s, tileKeys);
 }
 

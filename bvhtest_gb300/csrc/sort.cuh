@@ -19,6 +19,10 @@ constexpr uint32_t kSortTileDefault = 8192;
 bool sort_tile_valid(uint32_t tileKeys);
 // Polls of an unpublished predecessor before a look-back gives up (0xFFFFFFFF: the default).
 int sort_set_spin_limit(uint32_t limit, uint32_t *previous);
+// The stable ascending sort of n 63-bit Morton keys; temp as for sort_pairs on bits [0, 63). *gate (device)
+// tells afterwards whether the full sort had to run.
+int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
+                uint32_t n, uint32_t *gate, cudaStream_t s);
 // The sort's alternate buffers, (keyBytes + 4) * n bytes of the temp space that hold nothing between sorts.
 void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit);
 int sort_pairs(void *temp, const void *keysIn, void *keysOut, const uint32_t *valsIn, uint32_t *valsOut, uint32_t n,
