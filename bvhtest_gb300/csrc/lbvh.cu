@@ -17,6 +17,8 @@
 //                  kBuildTree + kFixAABBTree, LBVH_CUDA.cu:273-374).
 #include <algorithm>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "lbvh_device.cuh"
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
 //
 // Windows overlap, so a box is a plain minimum and maximum over its leaves. The climb's merge differs
 // from that only where a coordinate is NaN (its result then depends on the order): a block with a NaN
-// among its boxes climbs leaf by leaf.
+// among its boxes merges the children's boxes node by node, in rounds.
 constexpr int kTreelet = 256;
 // Between two neighbouring roots of a block the delta is a strict prefix minimum of the block's deltas
 // or a strict suffix minimum, and a delta is at most 96.
@@ -151,12 +153,12 @@ struct TreeletSmem {
   uint8_t made[T];           // inner record i of the block is one of its own
 };
 
-// The block's leaves are B0 .. B0 + cnt - 1; every thread of the T calls it. box: the thread's leaf's box
-// (t < cnt). keys: the tree's sorted keys (karras mode).
+// The block's leaves are B0 .. B0 + cnt - 1; every thread of the T calls it. key, box: the thread's leaf's
+// (t < cnt). keys: the tree's sorted keys, read for the neighbouring blocks' leaves only (karras mode).
 template <int MODE, int T, typename K>
 __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0, uint32_t n, uint32_t face, const Box &box,
-                                              const K *__restrict__ keys, bvhgb_node *nodes, uint32_t *slots,
-                                              uint2 *__restrict__ roots, uint32_t *rootCount, uint32_t *err) {
+                                              K key, const K *__restrict__ keys, bvhgb_node *nodes,
+                                              uint2 *__restrict__ roots, uint32_t *rootCount) {
   __shared__ int top;
   constexpr int kBits = 8 * (int)sizeof(K);
   const int t = (int)threadIdx.x;
@@ -164,7 +166,7 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
   const bool live = t < cnt;
   const uint32_t i = B0 + (uint32_t)t;
   if (MODE == BVHGB_TOPO_KARRAS) {
-    if (live) sm.key[t + 1] = __ldg(keys + i);
+    if (live) sm.key[t + 1] = key;
     if (t == 0 && B0 > 0) sm.key[0] = __ldg(keys + B0 - 1);
     if (t == 0 && B0 + cnt < n) sm.key[cnt + 1] = __ldg(keys + B0 + cnt);
   }
@@ -179,10 +181,7 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
       nan = nan || isnan(box.mn[k]) || isnan(box.mx[k]);
     }
   }
-  if (__syncthreads_or(nan)) {
-    if (live) lbvh_climb<MODE, K>(i, n, keys, face, box, nodes, slots, err);
-    return;
-  }
+  const bool ordered = __syncthreads_or(nan) != 0;
   // Deltas of the gaps around the block's leaves: gap g (local) at [g + 1], between leaves g and g + 1.
   auto pair_delta = [&](int a) {  // leaves a and a + 1 (local), both in the tree
     if (MODE == BVHGB_TOPO_REFCOMPAT) return __clz((int)((B0 + a) ^ (B0 + a + 1)));
@@ -234,9 +233,38 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
     if (t + 1 == r) sm.parLeaf[t + 1] = parent;
     else sm.parInner[t + 1] = parent;
   }
-  // Boxes: windows of 1, 2, 4 ... leaves.
   Box nb = box;
-  const int level = local ? 31 - __clz(r - l + 1) : -1;
+  if (ordered) {
+    // Node by node: inner boxes in the second buffer, made[slot] = 2 once the box is there.
+    bool done = !local;
+    while (__syncthreads_or(!done)) {
+      const bool now = !done && (l == t || sm.made[t] == 2) && (t + 1 == r || sm.made[t + 1] == 2);
+      Box other = {};
+      if (now) {
+        const int a = l == t ? 0 : 1, b = t + 1 == r ? 0 : 1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          nb.mn[k] = sm.box[a][k][t];
+          nb.mx[k] = sm.box[a][3 + k][t];
+          other.mn[k] = sm.box[b][k][t + 1];
+          other.mx[k] = sm.box[b][3 + k][t + 1];
+        }
+        merge_into(nb, other);
+      }
+      __syncthreads();  // a slot's box and mark appear between two rounds
+      if (now) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          sm.box[1][k][slot] = nb.mn[k];
+          sm.box[1][3 + k][slot] = nb.mx[k];
+        }
+        sm.made[slot] = 2;
+        done = true;
+      }
+    }
+  }
+  // Boxes: windows of 1, 2, 4 ... leaves.
+  const int level = local && !ordered ? 31 - __clz(r - l + 1) : -1;
   int levels = 0;  // block-uniform: the highest level any node needs
   {
     if (t == 0) top = 0;
@@ -343,14 +371,15 @@ __global__ void __launch_bounds__(kTreelet) lbvh_build_kernel(const float *__res
                                                               const K *__restrict__ keys,
                                                               const uint32_t *__restrict__ idx, uint32_t n,
                                                               const float4 *__restrict__ boxes, bvhgb_node *nodes,
-                                                              uint32_t *slots, uint2 *__restrict__ roots,
-                                                              uint32_t *rootCount, uint32_t *err) {
+                                                              uint2 *__restrict__ roots, uint32_t *rootCount) {
   __shared__ TreeletSmem<kTreelet, K> sm;
   const uint32_t B0 = blockIdx.x * kTreelet, i = B0 + threadIdx.x;
   uint32_t face = 0;
+  K key = 0;
   Box box = {};
   if (i < n) {
     face = __ldg(idx + i);
+    if (MODE == BVHGB_TOPO_KARRAS) key = __ldg(keys + i);
     if (boxes) {
       const float4 a = __ldg(boxes + 2 * (size_t)face), c = __ldg(boxes + 2 * (size_t)face + 1);
       box.mn[0] = a.x; box.mn[1] = a.y; box.mn[2] = a.z;
@@ -359,7 +388,162 @@ __global__ void __launch_bounds__(kTreelet) lbvh_build_kernel(const float *__res
       tri_box(vert, faces, face, box, nullptr);
     }
   }
-  treelet_build<MODE, kTreelet, K>(sm, B0, n, face, box, keys, nodes, slots, roots, rootCount, err);
+  treelet_build<MODE, kTreelet, K>(sm, B0, n, face, box, key, keys, nodes, roots, rootCount);
+}
+
+// ---- small meshes in one launch -------------------------------------------------------------------
+//
+// Up to kSmallMesh triangles one block does it all, one triangle per thread: scene box, Morton key, a
+// bitonic sort of (key, face) in registers (shuffles below a stride of 32, shared memory above) and
+// the whole tree as one treelet. It leaves in the workspace what the phases would (scene box, keys,
+// order, box records). Bound: the latency of that chain, 16 us with the launch for 1,000 triangles; twelve
+// launches of a few microseconds each took 59 us.
+constexpr int kSmallMesh = 1024;
+
+template <typename K>
+struct SmallSmem {
+  TreeletSmem<kSmallMesh, K> tree;  // its boxes' place serves the sort first
+  uint32_t scene[6];
+  float red[kSmallMesh / 32][6];
+};
+
+template <int MODE, typename K>
+__global__ void __launch_bounds__(kSmallMesh) lbvh_small_kernel(const float *__restrict__ vert,
+                                                                const uint32_t *__restrict__ faces, uint32_t n,
+                                                                uint32_t *__restrict__ scene,
+                                                                uint32_t *__restrict__ sortErr, K *__restrict__ keys,
+                                                                uint32_t *__restrict__ vals, K *__restrict__ keysSorted,
+                                                                uint32_t *__restrict__ valsSorted,
+                                                                float4 *__restrict__ boxes, bvhgb_node *nodes) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  SmallSmem<K> &sm = *reinterpret_cast<SmallSmem<K> *>(smraw);
+  const uint32_t t = threadIdx.x, warp = t >> 5;
+  const bool live = t < n;
+  Box box = {};
+  float c[3] = {0.0f, 0.0f, 0.0f};
+  if (live) tri_box(vert, faces, t, box, c);
+  // Scene box, from the origin box (lbvh_bounds_kernel).
+  float v[6];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    v[k] = live ? fminf(0.0f, box.mn[k]) : 0.0f;
+    v[3 + k] = live ? fmaxf(0.0f, box.mx[k]) : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v[k] = fminf(v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], o));
+      v[3 + k] = fmaxf(v[3 + k], __shfl_xor_sync(0xFFFFFFFFu, v[3 + k], o));
+    }
+  }
+  if (lane_id() < 6) sm.red[warp][lane_id()] = lane_id() == 0 ? v[0] : lane_id() == 1 ? v[1] : lane_id() == 2 ? v[2]
+                                             : lane_id() == 3 ? v[3] : lane_id() == 4 ? v[4] : v[5];
+  __syncthreads();
+  if (warp < 6) {
+    float m = sm.red[lane_id()][warp];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float x = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+      m = warp < 3 ? fminf(m, x) : fmaxf(m, x);
+    }
+    if (lane_id() == 0) scene[warp] = sm.scene[warp] = f2ord(m);
+  }
+  if (t == 6) scene[6] = *sortErr = 0;  // error words (the sort's may be a larger mesh's)
+  __syncthreads();
+  K key = ~(K)0;
+  uint32_t face = t;  // a padding thread's pair sorts behind every triangle's
+  if (live) {
+    float off[3], sc[3];
+    morton_params(sm.scene, off, sc);
+    key = (K)morton_key<sizeof(K) == 8 ? 63 : 30>(c, off, sc);
+    keys[t] = key;
+    vals[t] = t;
+    if (boxes) {
+      boxes[2 * t] = make_float4(box.mn[0], box.mn[1], box.mn[2], box.mx[0]);
+      boxes[2 * t + 1] = make_float4(box.mx[1], box.mx[2], 0.0f, 0.0f);
+    }
+  }
+  // Bitonic sort by (key, face): the stable order.
+  struct Pair {
+    K key;
+    uint32_t face;
+  };
+  Pair *pair = reinterpret_cast<Pair *>(&sm.tree.box[0][0][0]);
+  static_assert(2 * sizeof(Pair) * kSmallMesh <= sizeof(sm.tree.box), "two pair buffers");
+  int flip = 0;
+  for (uint32_t size = 2; size <= (uint32_t)kSmallMesh; size <<= 1) {
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      K ok;
+      uint32_t of;
+      if (stride >= 32) {
+        pair[flip * kSmallMesh + t] = Pair{key, face};
+        __syncthreads();
+        const Pair o = pair[flip * kSmallMesh + (t ^ stride)];
+        ok = o.key;
+        of = o.face;
+        flip ^= 1;  // the next exchange writes the other buffer: no second barrier
+      } else {
+        ok = __shfl_xor_sync(0xFFFFFFFFu, key, stride);
+        of = __shfl_xor_sync(0xFFFFFFFFu, face, stride);
+      }
+      const bool up = (t & size) == 0, low = (t & stride) == 0;
+      const bool less = ok < key || (ok == key && of < face);  // the other pair comes first
+      if (less == (up == low)) {
+        key = ok;
+        face = of;
+      }
+    }
+  }
+  // The leaf's box: the sorted face's, through shared memory.
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    sm.tree.box[0][k][t] = box.mn[k];
+    sm.tree.box[0][3 + k][t] = box.mx[k];
+  }
+  __syncthreads();
+  if (live) {
+    keysSorted[t] = key;
+    valsSorted[t] = face;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      box.mn[k] = sm.tree.box[0][k][face];
+      box.mx[k] = sm.tree.box[0][3 + k][face];
+    }
+  }
+  __syncthreads();
+  treelet_build<MODE, kSmallMesh, K>(sm.tree, 0u, n, face, box, key, nullptr, nodes, nullptr, nullptr);
+}
+
+template <int MODE, typename K>
+int launch_small(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n, bvhgb_node *nodes,
+                 cudaStream_t s) {
+  ws->slotsArmed = false;
+  lbvh_small_kernel<MODE, K><<<1, kSmallMesh, sizeof(SmallSmem<K>), s>>>(
+      vert, faces, n, ws->scene, sort_error_word(ws->sortTemp, ws->maxFaces, ws->keyBytes, 0, ws->cfg.mortonBits),
+      static_cast<K *>(ws->keys), ws->vals, static_cast<K *>(ws->keysSorted), ws->valsSorted,
+      ws->triBoxes, nodes);
+  BVHGB_LAUNCH_CHECK("lbvh small");
+  return BVHGB_OK;
+}
+
+template <int MODE, typename K>
+cudaError_t set_small_attr() {
+  return cudaFuncSetAttribute(lbvh_small_kernel<MODE, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(SmallSmem<K>));
+}
+
+// Opts in to the small kernel's shared memory, once per context (as sort_prepare).
+int small_prepare() {
+  static std::mutex m;
+  static std::vector<uint64_t> done;
+  const uint64_t ctx = context_id();
+  std::lock_guard<std::mutex> lock(m);
+  if (ctx != 0 && std::find(done.begin(), done.end(), ctx) != done.end()) return BVHGB_OK;
+  BVHGB_CUDA_TRY((set_small_attr<BVHGB_TOPO_REFCOMPAT, uint32_t>()));
+  BVHGB_CUDA_TRY((set_small_attr<BVHGB_TOPO_REFCOMPAT, uint64_t>()));
+  BVHGB_CUDA_TRY((set_small_attr<BVHGB_TOPO_KARRAS, uint32_t>()));
+  BVHGB_CUDA_TRY((set_small_attr<BVHGB_TOPO_KARRAS, uint64_t>()));
+  if (ctx != 0) done.push_back(ctx);
+  return BVHGB_OK;
 }
 
 // Roots a build of n leaves can list at most.
@@ -380,7 +564,7 @@ int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *fa
   uint2 *roots = static_cast<uint2 *>(sort_alternate(ws->sortTemp, n, ws->keyBytes, 0, ws->cfg.mortonBits));
   const K *keys = static_cast<const K *>(ws->keysSorted);
   lbvh_build_kernel<MODE, K><<<ceil_div(n, kTreelet), kTreelet, 0, s>>>(
-      vert, faces, keys, ws->valsSorted, n, ws->triBoxes, nodes, ws->slots, roots, rootCount, ws->scene + 6);
+      vert, faces, keys, ws->valsSorted, n, ws->triBoxes, nodes, roots, rootCount);
   BVHGB_LAUNCH_CHECK("lbvh build");
   if (n <= (uint32_t)kTreelet) return BVHGB_OK;  // one block makes the whole tree
   const uint32_t grid = std::min(ceil_div(max_roots(n), kRootThreads), (uint32_t)sm_count() * 16);
@@ -407,6 +591,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   if ((c.mortonBits != 30 && c.mortonBits != 63) || c.topology > BVHGB_TOPO_KARRAS) return BVHGB_INVALID_ARGUMENT;
   if (maxFaces >= (1u << 30)) return BVHGB_TOO_LARGE;
   int pst = sort_prepare();
+  if (!pst) pst = small_prepare();
   if (pst) return pst;
   auto *ws = new bvhgb_lbvh_workspace();
   ws->maxFaces = maxFaces;
@@ -512,6 +697,16 @@ extern "C" BVHGB_API int bvhgb_lbvh_build(bvhgb_lbvh_workspace *ws, const float 
   if (st) return st;
   if (n == 0) return BVHGB_OK;
   if (!vert || !faces || !nodes) return BVHGB_INVALID_ARGUMENT;
+  if (n <= (uint32_t)kSmallMesh) {
+    if ((st = small_prepare())) return st;
+    cudaStream_t s = as_stream(stream);
+    const bool wide = ws->keyBytes == 8;
+    if (ws->cfg.topology == BVHGB_TOPO_REFCOMPAT)
+      return wide ? launch_small<BVHGB_TOPO_REFCOMPAT, uint64_t>(ws, vert, faces, n, nodes, s)
+                  : launch_small<BVHGB_TOPO_REFCOMPAT, uint32_t>(ws, vert, faces, n, nodes, s);
+    return wide ? launch_small<BVHGB_TOPO_KARRAS, uint64_t>(ws, vert, faces, n, nodes, s)
+                : launch_small<BVHGB_TOPO_KARRAS, uint32_t>(ws, vert, faces, n, nodes, s);
+  }
   if ((st = bvhgb_lbvh_init_tri_data(ws, vert, faces, n, stream))) return st;
   if ((st = bvhgb_lbvh_calc_morton(ws, vert, faces, n, stream))) return st;
   if ((st = bvhgb_lbvh_sort(ws, n, stream))) return st;
@@ -587,9 +782,6 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32
 // and code that must not fail for lack of memory once started. For them the build below takes its
 // working memory from one array in this file, sized for BVHGB_STATIC_MAX_FACES triangles and
 // reserved on every GPU that loads the library until the process exits.
-#include <mutex>
-#include <vector>
-
 namespace bvhgb {
 namespace {
 

@@ -1,13 +1,14 @@
-"""The block-wise tree build gives the nodes of the leaf-by-leaf climb (which the batched build still
-is), byte for byte, around the block size, on equal and comb-like keys, and where a coordinate is
-infinite or no number (a block with one climbs); 63-bit keys against the oracle."""
+"""The block-wise tree build and the one-launch build of small meshes (up to 1,024 triangles) give the
+nodes of the leaf-by-leaf climb (which the batched build still is), byte for byte, around the block
+sizes, on equal and comb-like keys, and where a coordinate is infinite or no number (whose boxes depend
+on the order of the merges); 63-bit keys against the oracle."""
 import numpy as np
 import pytest
 
 from bvhtest_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
-SIZES = [1, 2, 3, 31, 255, 256, 257, 511, 513, 4096, 66049]
+SIZES = [1, 2, 3, 31, 255, 256, 257, 511, 513, 1000, 1024, 1025, 4096, 66049]
 
 
 def _vert(kind, n, seed):
@@ -39,6 +40,14 @@ def test_equals_the_climb(gpu, n, kind, topo):
     got = one.build(v, f)
     again = gpu.empty_nodes(2 * n - 1)
     one.build_tree(v, f, again)  # from the same sorted keys: slots and root counter re-armed
+    phases = gpu.LBVH(n, 30, topo)  # what a build leaves is what the phases leave
+    phases.init_tri_data(v, f)
+    phases.calc_morton(v, f)
+    phases.sort(n)
+    assert np.array_equal(one.scene_box(), phases.scene_box(), equal_nan=True)
+    for done in (False, True):
+        for a, b in zip(one.keys(n, done), phases.keys(n, done)):
+            assert np.array_equal(a, b)
     batch = gpu.Batch([n], topology=topo)
     ref = batch.empty_nodes()
     batch.build(v, f, ref)
@@ -49,7 +58,7 @@ def test_equals_the_climb(gpu, n, kind, topo):
 
 @pytest.mark.parametrize("topo", ["refCompat", "karras"])
 @pytest.mark.parametrize("kind", ["soup", "equal", "runs", "comb"])
-@pytest.mark.parametrize("n", [2, 255, 257, 5000, 66049])
+@pytest.mark.parametrize("n", [2, 255, 257, 1000, 1024, 5000, 66049])
 def test_long_keys(gpu, orc, n, kind, topo):
     import torch
     vert, faces = _vert(kind, n, n + 1)
