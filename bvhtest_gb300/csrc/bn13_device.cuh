@@ -542,12 +542,15 @@ struct PatchKeys {
   }
 };
 
-// One batched search. The frontier's entry e = slot * 32 + lane is live when e < m; the per-lane
-// best is the lane's first entry of its smallest total, the lowest (cost, node) within a round.
+// One batched search. The frontier's entry e = slot * 32 + lane of slots 1 to 3 is live when e < m, slot
+// 0's entries are the lanes of 'live'; the per-lane best is the lane's first entry of its smallest
+// total, the lowest (cost, node) within a round.
 struct BatchedSearch {
   float fc[kFrontier];
   uint32_t fn[kFrontier];
   uint32_t m;         // entries in the frontier (every one is within the bound)
+  uint32_t live;      // lanes that hold one in slot 0 (the lowest min(m, 32), or after a narrow round any)
+  uint32_t src;       // the lane of slot 0's (lane / 2)-th entry, for a narrow round
   uint32_t round;
   float4 rec[3];      // the tree record of slot 0's entry
   float bestCost;     // warp-uniform
@@ -582,7 +585,8 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
   uint32_t roundNode = kNone;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    const bool live = (uint32_t)s * 32u + lane < st.m;  // other lanes compute on what they hold
+    // other lanes compute on what they hold
+    const bool live = s == 0 ? (st.live >> lane) & 1u : (uint32_t)s * 32u + lane < st.m;
     const uint32_t x = st.fn[s];
     float4 q[3];
     if (s == 0) {
@@ -652,6 +656,8 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
   }
   __syncwarp();
   const uint2 *child = reinterpret_cast<const uint2 *>(buf);
+  st.src = lane >> 1;
+  st.live = m >= 32u ? 0xFFFFFFFFu : (1u << m) - 1u;
   if (S <= 2 || m <= kFrontierCap) {
     st.m = m;
     if (lane < m) {  // slot 0 first: its records are on their way while the other slots are read
@@ -734,6 +740,77 @@ __device__ __forceinline__ void batched_round(const Patch &p, const PatchKeys &k
   if (S > 1) __syncwarp();
 }
 
+// A read-only load that is issued where it stands.
+__device__ __forceinline__ float4 ldg_now(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+// One round over at most 16 entries, which may stand in any lanes (st.live), and their at most 32
+// children, one per lane. The children's records are fetched as soon as the entries' links are known,
+// while the entries are evaluated and the round's bound is found: a round then takes little more
+// than a record's round trip. Records of children that are not expanded are fetched for nothing,
+// about as many as of those that are. The survivors stay in their lanes; src tells the next round
+// where they are. The loads are volatile: they must not sink below the evaluation. A chunk's launch
+// went from 18.0 to 17.3 us on 65,536 triangles and from 35.0 to 33.6 us on 4.19M.
+__device__ __forceinline__ void narrow_round(const Patch &p, const PatchKeys &keys, BatchedSearch &st, const Box &nbox,
+                                             float sarea, uint4 *buf, SearchCounters &ctr) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool live = (st.live >> lane) & 1u;
+  ctr.visits += st.m;
+  const uint32_t x = st.fn[0];
+  if (live && x >= p.numNodes) p.bad = true;
+  Box b;
+  b.mn[0] = st.rec[0].x; b.mn[1] = st.rec[0].y; b.mn[2] = st.rec[0].z;
+  b.mx[0] = st.rec[0].w; b.mx[1] = st.rec[1].x; b.mx[2] = st.rec[1].y;
+  uint32_t left = __float_as_uint(st.rec[1].w), right = __float_as_uint(st.rec[2].x);
+  bool leaf = (__float_as_uint(st.rec[2].y) & 0xFFFFu) != 0u;
+  if (live && keys.patched(x)) {
+    NodeP n;
+    p.subset_aabb_from(x, st.rec[0], st.rec[1], st.rec[2], n, b);
+    left = n.left;
+    right = n.right;
+    leaf = n.isLeafFlag != 0;
+  }
+  // the children, and their records
+  const uint32_t inner = __ballot_sync(kFull, live && !leaf);
+  const uint32_t cl = __shfl_sync(kFull, left, st.src), cr = __shfl_sync(kFull, right, st.src);
+  const uint32_t child = lane & 1u ? cr : cl;
+  const bool have = lane < 2u * st.m && ((inner >> st.src) & 1u);
+  {
+    const float4 *q = reinterpret_cast<const float4 *>(p.t + (have && child < p.numNodes ? child : p.root));
+    st.rec[0] = ldg_now(q);
+    st.rec[1] = ldg_now(q + 1);
+    st.rec[2] = ldg_now(q + 2);
+  }
+  // the entries
+  const float ind = fmul(-1.0f, surface_area(b));
+  merge_into(b, nbox);
+  const float total = fadd(st.fc[0], surface_area(b));
+  const float induced = fadd(ind, total);
+  const float cost = live ? total : __int_as_float(0x7f800000);
+  const float kmin = ord2f(__reduce_min_sync(kFull, f2ord(cost)));
+  if (kmin < st.bestCost) st.bestCost = kmin;
+  if (cost < st.myCost) {
+    st.myCost = cost;
+    st.myEntry = st.fc[0];
+    st.myNode = x;
+    st.myRound = st.round;
+  }
+  const uint32_t kids = __ballot_sync(kFull, live && !leaf && fadd(induced, sarea) < st.bestCost);
+  st.fc[0] = __shfl_sync(kFull, induced, st.src);
+  st.fn[0] = child;
+  const bool stays = have && ((kids >> st.src) & 1u);
+  st.live = __ballot_sync(kFull, stays);
+  st.m = __popc(st.live);
+  // two tables in turn: a round's writes never meet the previous round's reads
+  uint32_t *lanes = reinterpret_cast<uint32_t *>(buf + kFrontierCap / 2) + (st.round & 1u) * 32u;
+  if (stays) lanes[__popc(st.live & ((1u << lane) - 1u))] = lane;
+  __syncwarp();
+  st.src = (lane >> 1) < st.m ? lanes[lane >> 1] : 0u;
+}
+
 // findNode1's cost model in batched rounds (every lane of the warp calls it with the same patch).
 __device__ __forceinline__ uint32_t find_node_batched(const Patch &p, uint32_t n, SearchCounters &ctr) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -750,6 +827,8 @@ __device__ __forceinline__ uint32_t find_node_batched(const Patch &p, uint32_t n
   }
   load_entry(p, p.root, st.rec);
   st.m = sarea < kInf ? 1u : 0u;  // the root's bound: 0 + sarea against no best yet
+  st.live = st.m;
+  st.src = 0;
   st.bestCost = kInf;
   st.myCost = st.myEntry = kInf;
   st.myNode = 0;
@@ -760,7 +839,8 @@ __device__ __forceinline__ uint32_t find_node_batched(const Patch &p, uint32_t n
       p.bad = true;
       break;
     }
-    if (st.m <= 32u) batched_round<1>(p, keys, st, nbox, sarea, buf, ctr);
+    if (st.m <= 16u) narrow_round(p, keys, st, nbox, sarea, buf, ctr);
+    else if (st.m <= 32u) batched_round<1>(p, keys, st, nbox, sarea, buf, ctr);
     else if (st.m <= 64u) batched_round<2>(p, keys, st, nbox, sarea, buf, ctr);
     else batched_round<kFrontier>(p, keys, st, nbox, sarea, buf, ctr);
   }
