@@ -28,7 +28,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t maxFaces = 0;
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
-  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, root counter, sort gate
+  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -98,7 +98,6 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
                                                                      float4 *__restrict__ boxes) {
   float off[3], sc[3];
   morton_params(scene, off, sc);
-  if (blockIdx.x == 0 && threadIdx.x == 0) scene[7] = 0;  // the build's root counter
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     Box b;
     float c[3];
@@ -124,14 +123,13 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
 // W_j[r - 2^j + 1]); the windows double level by level, in the order the queries need them. The
 // records are staged in shared memory and written in 16-byte words, neighbours together. What is
 // left, the roots of the block's subtrees (about 2 log2 T of them, at most kTreeletRoots), goes to a
-// list that a second launch climbs from through the global exchange slots (lbvh_climb_from).
+// list in leaf order for the joining launches below.
 //
 // Why: with one climb per leaf every inner node cost an acquire-release exchange, a sibling's box
 // from L2 and three scattered stores in one dependent chain (4.19M leaves: 413 us at 24% of DRAM
-// throughput); here all but one node in seventeen costs none of them. Climbing from the block
-// itself cost more than it saved (450 us): its fences wait for all the records it has just written.
-// Measured, block of 256 / 512 / 1,024 leaves without the climbs: 186 / 209 / 295 us; the climbs of
-// the second launch 79 us (33.5M leaves: 3,050 us as one climb per leaf, 1,413 + 360 now).
+// throughput; 33.5M: 3,050 us); here all but one node in seventeen costs none of them.
+// Measured, block of 256 / 512 / 1,024 leaves: 182 / 209 / 295 us (33.5M, 256: 1,407 us), bound by
+// shared memory's wavefronts (83%; DRAM 50%).
 //
 // Windows overlap, so a box is a plain minimum and maximum over its leaves. The climb's merge differs
 // from that only where a coordinate is NaN (its result then depends on the order): a block with a NaN
@@ -141,17 +139,99 @@ constexpr int kTreelet = 256;
 // or a strict suffix minimum, and a delta is at most 96.
 constexpr int kTreeletRoots = 193;
 
+// Two buffers of T boxes, a component per array: neighbours' loads share a wavefront.
+template <int T>
+struct BoxPair {
+  float v[2][6][T];
+  __device__ __forceinline__ Box get(int buf, int i) const {
+    Box x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x.mn[k] = v[buf][k][i];
+      x.mx[k] = v[buf][3 + k][i];
+    }
+    return x;
+  }
+  __device__ __forceinline__ void put(int buf, int i, const Box &x) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v[buf][k][i] = x.mn[k];
+      v[buf][3 + k][i] = x.mx[k];
+    }
+  }
+};
+
+__device__ __forceinline__ bool has_nan(const Box &b) {
+  bool nan = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) nan = nan || isnan(b.mn[k]) || isnan(b.mx[k]);
+  return nan;
+}
+
 template <int T, typename K>
 struct TreeletSmem {
   union {
-    float box[2][6][T];      // window boxes, ping-pong
+    BoxPair<T> box;          // window boxes, ping-pong
     float4 record[3 * T];    // node records on their way out
   };
   K key[T + 2];              // leaf B0 + i at [i + 1]
   uint32_t parInner[T], parLeaf[T];  // parent | is-left << 31 (an index has 31 bits); kNone: not in this block
   uint8_t gap[T + 1];        // delta of the leaves B0 + i - 1 and B0 + i
   uint8_t made[T];           // inner record i of the block is one of its own
+  uint32_t starts[T / 32];   // bit i: a root of the block's subtrees starts at leaf B0 + i
 };
+
+// Boxes of ranges from windows of 1, 2, 4 ... boxes: thread t's range [l, r] (if it has one; cnt boxes, T
+// threads) comes from the two windows of 2^j boxes that cover it. Buffer 0 holds the boxes, w thread t's own.
+template <int T>
+__device__ __forceinline__ void window_boxes(BoxPair<T> &box, int &top, int cnt, bool has, int l, int r, Box w, Box &nb) {
+  const int t = (int)threadIdx.x;
+  const int level = has ? 31 - __clz(r - l + 1) : -1;
+  // The highest level any thread needs (block-uniform).
+  if (t == 0) top = 0;
+  __syncthreads();
+  const int warpTop = __reduce_max_sync(0xFFFFFFFFu, level);
+  if ((t & 31) == 0 && warpTop > 0) atomicMax(&top, warpTop);
+  __syncthreads();
+  const int levels = top;
+  for (int j = 0; j < levels; ++j) {  // w: window W_j[t]
+    const int half = 1 << j;
+    const float(*cur)[T] = box.v[j & 1];
+    float(*nxt)[T] = box.v[(j + 1) & 1];
+    if (t + half < cnt) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        w.mn[k] = fminf(w.mn[k], cur[k][t + half]);
+        w.mx[k] = fmaxf(w.mx[k], cur[3 + k][t + half]);
+      }
+    }
+    if (t < cnt) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        nxt[k][t] = w.mn[k];
+        nxt[3 + k][t] = w.mx[k];
+      }
+    }
+    __syncthreads();
+    if (level == j + 1) {
+      const int e = r - 2 * half + 1;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        nb.mn[k] = fminf(nxt[k][l], nxt[k][e]);
+        nb.mx[k] = fmaxf(nxt[3 + k][l], nxt[3 + k][e]);
+      }
+    }
+  }
+}
+
+// Set bits below bit 'at' of a mask of W words.
+template <int W>
+__device__ __forceinline__ uint32_t ones_before(const uint32_t *mask, int at) {
+  uint32_t p = __popc(mask[at >> 5] & ((1u << (at & 31)) - 1u));
+#pragma unroll
+  for (int w = 0; w < W; ++w) p += w < (at >> 5) ? __popc(mask[w]) : 0;
+  return p;
+}
 
 // The block's leaves are B0 .. B0 + cnt - 1; every thread of the T calls it. key, box: the thread's leaf's
 // (t < cnt). keys: the tree's sorted keys, read for the neighbouring blocks' leaves only (karras mode).
@@ -174,12 +254,8 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
   sm.made[t] = 0;
   bool nan = false;
   if (live) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      sm.box[0][k][t] = box.mn[k];
-      sm.box[0][3 + k][t] = box.mx[k];
-      nan = nan || isnan(box.mn[k]) || isnan(box.mx[k]);
-    }
+    sm.box.put(0, t, box);
+    nan = has_nan(box);
   }
   const bool ordered = __syncthreads_or(nan) != 0;
   // Deltas of the gaps around the block's leaves: gap g (local) at [g + 1], between leaves g and g + 1.
@@ -241,68 +317,19 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
       const bool now = !done && (l == t || sm.made[t] == 2) && (t + 1 == r || sm.made[t + 1] == 2);
       Box other = {};
       if (now) {
-        const int a = l == t ? 0 : 1, b = t + 1 == r ? 0 : 1;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          nb.mn[k] = sm.box[a][k][t];
-          nb.mx[k] = sm.box[a][3 + k][t];
-          other.mn[k] = sm.box[b][k][t + 1];
-          other.mx[k] = sm.box[b][3 + k][t + 1];
-        }
+        nb = sm.box.get(l == t ? 0 : 1, t);
+        other = sm.box.get(t + 1 == r ? 0 : 1, t + 1);
         merge_into(nb, other);
       }
       __syncthreads();  // a slot's box and mark appear between two rounds
       if (now) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          sm.box[1][k][slot] = nb.mn[k];
-          sm.box[1][3 + k][slot] = nb.mx[k];
-        }
+        sm.box.put(1, slot, nb);
         sm.made[slot] = 2;
         done = true;
       }
     }
   }
-  // Boxes: windows of 1, 2, 4 ... leaves.
-  const int level = local && !ordered ? 31 - __clz(r - l + 1) : -1;
-  int levels = 0;  // block-uniform: the highest level any node needs
-  {
-    if (t == 0) top = 0;
-    __syncthreads();
-    const int warpTop = __reduce_max_sync(0xFFFFFFFFu, level);
-    if ((t & 31) == 0 && warpTop > 0) atomicMax(&top, warpTop);
-    __syncthreads();
-    levels = top;
-  }
-  Box w = box;  // this thread's window W_j[t]
-  for (int j = 0; j < levels; ++j) {
-    const int half = 1 << j;
-    const float(*cur)[T] = sm.box[j & 1];
-    float(*nxt)[T] = sm.box[(j + 1) & 1];
-    if (t + half < cnt) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        w.mn[k] = fminf(w.mn[k], cur[k][t + half]);
-        w.mx[k] = fmaxf(w.mx[k], cur[3 + k][t + half]);
-      }
-    }
-    if (live) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        nxt[k][t] = w.mn[k];
-        nxt[3 + k][t] = w.mx[k];
-      }
-    }
-    __syncthreads();
-    if (level == j + 1) {
-      const int e = r - 2 * half + 1;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        nb.mn[k] = fminf(nxt[k][l], nxt[k][e]);
-        nb.mx[k] = fmaxf(nxt[3 + k][l], nxt[3 + k][e]);
-      }
-    }
-  }
+  window_boxes<T>(sm.box, top, cnt, local && !ordered, l, r, box, nb);
   __syncthreads();  // the windows make room for the records
   auto stage = [&](int at, const Box &b, uint32_t par, uint32_t left, uint32_t rightLink, uint32_t leaf, uint32_t level) {
     const uint32_t isLeft = par == kNone ? 0u : par >> 31, parent = par == kNone ? kNone : par & 0x7FFFFFFFu;
@@ -332,38 +359,207 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
   // The roots of the block's subtrees: (l, r | is-left << 31).
   const bool innerRoot = local && !root && sm.parInner[slot] == kNone;
   const bool leafRoot = live && n > 1 && sm.parLeaf[t] == kNone;
-  if (t == 0) top = 0;
+  if (roots == nullptr) return;  // one block made the whole tree
+  // In the order of the leaves: a root's place is the number of roots that start before it.
+  if (t < T / 32) sm.starts[t] = 0;
   __syncthreads();
-  const uint32_t mine = (innerRoot ? 1u : 0u) + (leafRoot ? 1u : 0u);
-  uint32_t at = mine ? (uint32_t)atomicAdd(&top, (int)mine) : 0u;
+  if (innerRoot) atomicOr(&sm.starts[l >> 5], 1u << (l & 31));
+  if (leafRoot) atomicOr(&sm.starts[t >> 5], 1u << (t & 31));
   __syncthreads();
-  if (t == 0 && top > 0) top = (int)atomicAdd(rootCount, (uint32_t)top);
-  __syncthreads();
-  if (mine) at += (uint32_t)top;
-  if (innerRoot) roots[at++] = make_uint2(B0 + l, (B0 + r) | (right ? 0x80000000u : 0u));
+  uint2 *list = roots + (size_t)(B0 / T) * kTreeletRoots;
+  if (innerRoot) {
+    const uint32_t p = ones_before<T / 32>(sm.starts, l);
+    if (p < (uint32_t)kTreeletRoots) list[p] = make_uint2(B0 + l, (B0 + r) | (right ? 0x80000000u : 0u));
+  }
   if (leafRoot) {
     const bool leafRight = i == 0 ? true : i == n - 1 ? false : sm.gap[t + 1] > sm.gap[t];
-    roots[at] = make_uint2(i, i | (leafRight ? 0x80000000u : 0u));
+    const uint32_t p = ones_before<T / 32>(sm.starts, t);
+    if (p < (uint32_t)kTreeletRoots) list[p] = make_uint2(i, i | (leafRight ? 0x80000000u : 0u));
   }
+  if (t == 0) rootCount[B0 / T] = min(ones_before<T / 32>(sm.starts, T - 1) + (sm.starts[T / 32 - 1] >> 31), (uint32_t)kTreeletRoots);
 }
 
-// Climbs from the listed subtree roots.
-constexpr int kRootThreads = 128;
+// ---- the subtrees of several blocks joined ------------------------------------------------------------
+//
+// The roots of kJoinBlocks neighbouring blocks' subtrees, in leaf order, are to the nodes above them
+// what the leaves are to a block's: a block takes them one per thread (at most kJoin; 15 a block on
+// average) and makes every node whose range lies among them in the same way. A root's place in a
+// comparison is taken by its last leaf, whose bits within the range are every leaf's. The roots of what
+// it made replace the first of the lists it read, and the next launch joins kJoinBlocks of those, until
+// one block makes the tree's root. A list whose roots do not fit one block, or that holds a NaN (whose
+// box depends on the order of the merges), stays as it is, as do the wider ones: a last launch climbs
+// from its roots through the global exchange slots.
+//
+// Why: a climb pays an L2 exchange, a sibling's box and a fence a level, 3.7 us, and its upper levels
+// are one chain; a joining launch makes about five levels in 7 us. Measured, 4.19M leaves: climbs from
+// every block's roots 79 us, one joining launch and climbs from what it leaves 23 + 60, joined to the
+// root 45 + 2 (33.5M: 357, 128 + 77, 169 + 3). Climbs from within the joining block cost more than they
+// save (93 us; 424): a block lives as long as its longest climb.
+constexpr int kJoin = 512, kJoinBlocks = 16;
+
+template <typename K>
+struct JoinSmem {
+  BoxPair<kJoin> box;
+  K key[kJoin + 2];          // of root c's last leaf at [c + 1]; its neighbours outside at both ends
+  uint32_t last[kJoin + 2];  // that leaf
+  uint8_t gap[kJoin + 1];    // delta of the leaves between the roots c - 1 and c
+  uint8_t below[2][kJoin];   // the root (0) or the inner node numbered c (1) has its parent here
+  uint32_t before[kJoinBlocks + 1];
+  uint32_t starts[kJoin / 32];
+};
+
 template <int MODE, typename K>
-__global__ void __launch_bounds__(kRootThreads) lbvh_roots_kernel(const uint2 *__restrict__ roots,
-                                                                  const uint32_t *__restrict__ rootCount, uint32_t n,
-                                                                  const K *__restrict__ keys, bvhgb_node *nodes,
-                                                                  uint32_t *slots, uint32_t *err) {
-  const uint32_t count = min(*rootCount, n);
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-    const uint2 e = __ldg(roots + q);
-    const uint32_t l = e.x, r = e.y & 0x7FFFFFFFu;
-    const bool right = (e.y >> 31) != 0u;
-    const uint32_t node = l == r ? n - 1 + l : right ? r : l;
-    lbvh_climb_from<MODE, K>(l, r, right, load_box_cg(nodes + node), n, keys, nodes, slots, err);
+__global__ void __launch_bounds__(kJoin) lbvh_join_kernel(uint2 *roots, const uint32_t *__restrict__ count,
+                                                          uint32_t *__restrict__ joined, uint32_t lists, size_t pitch,
+                                                          uint32_t n, const K *__restrict__ keys, bvhgb_node *nodes) {
+  __shared__ JoinSmem<K> sm;
+  __shared__ int top;
+  constexpr int kBits = 8 * (int)sizeof(K);
+  const int t = (int)threadIdx.x;
+  const uint32_t b0 = blockIdx.x * kJoinBlocks, own = min((uint32_t)kJoinBlocks, lists - b0);
+  if (t < 32) {
+    uint32_t c = (uint32_t)t < own ? min(__ldg(count + b0 + t), (uint32_t)kJoin + 1u) : 0u;  // kNone: does not fit either
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, c, o);
+      if (t >= o) c += x;
+    }
+    if (t < kJoinBlocks) sm.before[t + 1] = c;
+    if (t == 0) sm.before[0] = 0;
   }
+  sm.below[0][t] = sm.below[1][t] = 0;
+  __syncthreads();
+  const int m = (int)sm.before[kJoinBlocks];
+  auto root_at = [&](int c) {
+    int b = 0;
+#pragma unroll
+    for (int step = kJoinBlocks / 2; step > 0; step >>= 1)
+      if ((uint32_t)c >= sm.before[b + step]) b += step;
+    return __ldcg(roots + (b0 + b) * pitch + ((uint32_t)c - sm.before[b]));
+  };
+  if (m > kJoin) {
+    if (t == 0) joined[blockIdx.x] = kNone;
+    return;
+  }
+  const bool live = t < m;
+  uint2 e = make_uint2(0u, 0u);
+  Box box = {};
+  bool nan = false;
+  if (live) {
+    e = root_at(t);
+    const uint32_t l = e.x, r = e.y & 0x7FFFFFFFu;
+    box = load_box_cg(nodes + (l == r ? n - 1 + l : (e.y >> 31) != 0u ? r : l));
+    sm.last[t + 1] = r;
+    if (t == 0) sm.last[0] = l - 1;
+    if (t == m - 1) sm.last[m + 1] = r + 1;
+    if (MODE == BVHGB_TOPO_KARRAS) {
+      sm.key[t + 1] = __ldg(keys + r);
+      if (t == 0 && l > 0) sm.key[0] = __ldg(keys + l - 1);
+      if (t == m - 1 && r + 1 < n) sm.key[m + 1] = __ldg(keys + r + 1);
+    }
+    if (r + 1 < n) sm.gap[t + 1] = (uint8_t)delta<MODE, K>(keys, r, r + 1);
+    if (t == 0 && l > 0) sm.gap[0] = (uint8_t)delta<MODE, K>(keys, l - 1, l);
+    sm.box.put(0, t, box);
+    nan = has_nan(box);
+  }
+  if (__syncthreads_or(nan)) {
+    if (t == 0) joined[blockIdx.x] = kNone;
+    return;
+  }
+  // The node that splits between the roots t and t + 1: its range, if that lies among the block's.
+  int l = t, r = t;
+  bool local = live && t + 1 < m;
+  if (local) {
+    const int d = sm.gap[t + 1];
+    const uint32_t i = sm.last[t + 1];
+    r = t + 1;
+    const uint32_t mask = MODE == BVHGB_TOPO_REFCOMPAT ? (2u << (31 - d)) - 1u : 0u;
+    const K mine = MODE == BVHGB_TOPO_KARRAS ? sm.key[t + 1] : (K)0;
+    const K bound = d < kBits ? (K)1 << (kBits - d) : (K)1;
+    auto same = [&](int c) {  // root c lies in the node's range
+      if (MODE == BVHGB_TOPO_REFCOMPAT) return ((sm.last[c + 1] ^ i) & ~mask) == 0u;
+      if ((K)(sm.key[c + 1] ^ mine) >= bound) return false;
+      return d < kBits || __clz((int)(sm.last[c + 1] ^ i)) >= d - kBits;
+    };
+#pragma unroll
+    for (int step = kJoin / 2; step > 0; step >>= 1) {
+      if (l - step >= 0 && same(l - step)) l -= step;
+      if (r + step < m && same(r + step)) r += step;
+    }
+    if (l == 0 && sm.last[0] != kNone && same(-1)) local = false;
+    if (r == m - 1 && sm.last[m + 1] < n && same(m)) local = false;
+  }
+  const uint32_t L = local ? sm.last[l] + 1u : 0u, R = local ? sm.last[r + 1] : 0u;
+  const bool root = local && L == 0 && R == n - 1;
+  bool right = false;
+  int slot = 0;  // the root whose first or last leaf numbers the node
+  if (local) {
+    right = L == 0 ? true : R == n - 1 ? false : sm.gap[r + 1] > sm.gap[l];
+    slot = root ? 0 : right ? r : l;
+    sm.below[l == t ? 0 : 1][t] = 1;
+    sm.below[t + 1 == r ? 0 : 1][t + 1] = 1;
+  }
+  Box nb = box;
+  window_boxes<kJoin>(sm.box, top, m, local, l, r, box, nb);
+  const uint32_t index = root ? 0u : right ? R : L, split = local ? sm.last[t + 1] : 0u;
+  const uint32_t a = L == split ? n - 1 + split : split, b = split + 1 == R ? n + split : split + 1;
+  if (local) store_record(nodes + index, nb, root ? 0u : kNone, a, b, 0u, 0u, 0u);
+  __syncthreads();  // every record before its parent's links
+  if (local) {
+    set_parent(nodes + a, index, 1);
+    set_parent(nodes + b, index, 0);
+  }
+  // What is left goes, in leaf order, to the start of the lists this block has read.
+  if (t < kJoin / 32) sm.starts[t] = 0;
+  __syncthreads();
+  const bool rest = live && !sm.below[0][t], innerRest = local && !root && !sm.below[1][slot];
+  if (rest) atomicOr(&sm.starts[t >> 5], 1u << (t & 31));
+  if (innerRest) atomicOr(&sm.starts[l >> 5], 1u << (l & 31));
+  __syncthreads();
+  uint2 *list = roots + b0 * pitch;
+  if (rest) list[ones_before<kJoin / 32>(sm.starts, t)] = e;
+  if (innerRest) list[ones_before<kJoin / 32>(sm.starts, l)] = make_uint2(L, R | (right ? 0x80000000u : 0u));
+  if (t == 0) joined[blockIdx.x] = ones_before<kJoin / 32>(sm.starts, kJoin - 1) + (sm.starts[kJoin / 32 - 1] >> 31);
 }
 
+// Climbs from the lists that were not joined: a warp looks after kJoinBlocks of the blocks' lists, and
+// after the joined list that starts with them if no wider one holds its roots. counts: the blocks', then
+// every joining launch's.
+constexpr int kClimbThreads = 128;
+template <int MODE, typename K>
+__global__ void __launch_bounds__(kClimbThreads) lbvh_roots_kernel(const uint2 *__restrict__ roots,
+                                                                   const uint32_t *__restrict__ counts,
+                                                                   uint32_t blocks, uint32_t n,
+                                                                   const K *__restrict__ keys, bvhgb_node *nodes,
+                                                                   uint32_t *slots, uint32_t *err) {
+  const uint32_t q = (blockIdx.x * kClimbThreads + threadIdx.x) >> 5;
+  if (q * kJoinBlocks >= blocks) return;
+  // The widest joined list over this warp's blocks; it starts with those of warp 'first'.
+  const uint32_t *level = counts + blocks;
+  uint32_t lists = (blocks + kJoinBlocks - 1) / kJoinBlocks, span = 1, first = q, joined = kNone;
+  for (;;) {
+    const uint32_t c = __ldg(level + q / span);
+    if (c == kNone) break;
+    joined = c;
+    first = q / span * span;
+    if (lists == 1) break;
+    level += lists;
+    lists = (lists + kJoinBlocks - 1) / kJoinBlocks;
+    span *= kJoinBlocks;
+  }
+  if (joined != kNone && first != q) return;
+  const uint32_t b0 = q * kJoinBlocks;
+  for (uint32_t b = b0; b < (joined != kNone ? b0 + 1 : min(b0 + kJoinBlocks, blocks)); ++b) {
+    const uint32_t m = min(joined != kNone ? joined : __ldg(counts + b), (uint32_t)kJoin);
+    for (uint32_t c = lane_id(); c < m; c += 32u) {
+      const uint2 e = __ldg(roots + (size_t)b * kTreeletRoots + c);
+      const uint32_t l = e.x, r = e.y & 0x7FFFFFFFu;
+      const bool right = (e.y >> 31) != 0u;
+      const uint32_t node = l == r ? n - 1 + l : right ? r : l;
+      lbvh_climb_from<MODE, K>(l, r, right, load_box_cg(nodes + node), n, keys, nodes, slots, err);
+    }
+  }
+}
 
 template <int MODE, typename K>
 __global__ void __launch_bounds__(kTreelet) lbvh_build_kernel(const float *__restrict__ vert,
@@ -466,7 +662,7 @@ __global__ void __launch_bounds__(kSmallMesh) lbvh_small_kernel(const float *__r
     K key;
     uint32_t face;
   };
-  Pair *pair = reinterpret_cast<Pair *>(&sm.tree.box[0][0][0]);
+  Pair *pair = reinterpret_cast<Pair *>(&sm.tree.box);
   static_assert(2 * sizeof(Pair) * kSmallMesh <= sizeof(sm.tree.box), "two pair buffers");
   int flip = 0;
   for (uint32_t size = 2; size <= (uint32_t)kSmallMesh; size <<= 1) {
@@ -494,20 +690,12 @@ __global__ void __launch_bounds__(kSmallMesh) lbvh_small_kernel(const float *__r
   }
   // The leaf's box: the sorted face's, through shared memory.
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    sm.tree.box[0][k][t] = box.mn[k];
-    sm.tree.box[0][3 + k][t] = box.mx[k];
-  }
+  sm.tree.box.put(0, t, box);
   __syncthreads();
   if (live) {
     keysSorted[t] = key;
     valsSorted[t] = face;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      box.mn[k] = sm.tree.box[0][k][face];
-      box.mx[k] = sm.tree.box[0][3 + k][face];
-    }
+    box = sm.tree.box.get(0, face);
   }
   __syncthreads();
   treelet_build<MODE, kSmallMesh, K>(sm.tree, 0u, n, face, box, key, nullptr, nodes, nullptr, nullptr);
@@ -546,29 +734,39 @@ int small_prepare() {
   return BVHGB_OK;
 }
 
-// Roots a build of n leaves can list at most.
-size_t max_roots(uint32_t n) { return std::min<size_t>(n, (size_t)ceil_div(n, kTreelet) * kTreeletRoots); }
-
 template <int MODE, typename K>
 int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n, bvhgb_node *nodes,
                  cudaStream_t s) {
-  // The exchange slots and the root counter are re-armed by the Morton kernel; a second build from the
-  // same sorted keys re-arms them here.
-  uint32_t *rootCount = ws->scene + 7;
-  if (!ws->slotsArmed) {
-    BVHGB_CUDA_TRY(cudaMemsetAsync(ws->slots, 0xFF, 4ull * n, s));
-    BVHGB_CUDA_TRY(cudaMemsetAsync(rootCount, 0, 4, s));
-  }
+  // The exchange slots are re-armed by the Morton kernel; a second build from the same sorted keys
+  // re-arms them here.
+  if (!ws->slotsArmed) BVHGB_CUDA_TRY(cudaMemsetAsync(ws->slots, 0xFF, 4ull * n, s));
   ws->slotsArmed = false;
-  // The list takes the place of the sort's alternate buffers, which nothing reads after the sort.
-  uint2 *roots = static_cast<uint2 *>(sort_alternate(ws->sortTemp, n, ws->keyBytes, 0, ws->cfg.mortonBits));
+  // The lists of roots take the place of the sort's alternate buffers, which nothing reads after the
+  // sort. 8 n bytes hold them: 193 places of 8 bytes per 256 leaves, and the counts at the end
+  // (4 (b + b / 15 + 8) bytes for b blocks at most).
+  const uint32_t blocks = ceil_div(n, kTreelet);
+  static_assert(8 * (kTreelet - kTreeletRoots) >= 2 * 4 * 2 + 4 * 8, "room for the counts beside the roots");
+  char *lists = static_cast<char *>(sort_alternate(ws->sortTemp, n, ws->keyBytes, 0, ws->cfg.mortonBits));
+  uint2 *roots = blocks > 1 ? reinterpret_cast<uint2 *>(lists) : nullptr;
+  uint32_t words = blocks;  // counts: the blocks', then every joining launch's
+  for (uint32_t m = blocks; m > 1;) words += m = ceil_div(m, kJoinBlocks);
+  uint32_t *counts = reinterpret_cast<uint32_t *>(lists + 8ull * n) - words;
   const K *keys = static_cast<const K *>(ws->keysSorted);
-  lbvh_build_kernel<MODE, K><<<ceil_div(n, kTreelet), kTreelet, 0, s>>>(
-      vert, faces, keys, ws->valsSorted, n, ws->triBoxes, nodes, roots, rootCount);
+  lbvh_build_kernel<MODE, K><<<blocks, kTreelet, 0, s>>>(
+      vert, faces, keys, ws->valsSorted, n, ws->triBoxes, nodes, roots, counts);
   BVHGB_LAUNCH_CHECK("lbvh build");
-  if (n <= (uint32_t)kTreelet) return BVHGB_OK;  // one block makes the whole tree
-  const uint32_t grid = std::min(ceil_div(max_roots(n), kRootThreads), (uint32_t)sm_count() * 16);
-  lbvh_roots_kernel<MODE, K><<<grid, kRootThreads, 0, s>>>(roots, rootCount, n, keys, nodes, ws->slots, ws->scene + 6);
+  if (blocks == 1) return BVHGB_OK;  // one block makes the whole tree
+  size_t pitch = kTreeletRoots;
+  uint32_t *in = counts;
+  for (uint32_t m = blocks; m > 1; pitch *= kJoinBlocks) {
+    const uint32_t joins = ceil_div(m, kJoinBlocks);
+    lbvh_join_kernel<MODE, K><<<joins, kJoin, 0, s>>>(roots, in, in + m, m, pitch, n, keys, nodes);
+    BVHGB_LAUNCH_CHECK("lbvh join");
+    in += m;
+    m = joins;
+  }
+  lbvh_roots_kernel<MODE, K><<<ceil_div(ceil_div(blocks, kJoinBlocks), kClimbThreads / 32), kClimbThreads, 0, s>>>(
+      roots, counts, blocks, n, keys, nodes, ws->slots, ws->scene + 6);
   BVHGB_LAUNCH_CHECK("lbvh roots");
   return BVHGB_OK;
 }

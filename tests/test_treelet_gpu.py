@@ -68,3 +68,48 @@ def test_long_keys(gpu, orc, n, kind, topo):
     ref, _, _ = orc.lbvh_build(vert, faces, 63, 0 if topo == "refCompat" else 1)
     assert np.array_equal(gpu.nodes_to_numpy(got).view(np.uint8), ref.view(np.uint8))
     assert b.errors() == 0
+
+
+def _from_keys(keys):
+    """One degenerate triangle per 63-bit key, in the middle of its Morton cell, and the two that hold the
+    scene box at [0, 1]."""
+    cell = np.zeros((keys.size, 3), np.int64)
+    for bit in range(21):
+        for axis in range(3):
+            cell[:, axis] |= ((keys >> (3 * bit + 2 - axis)) & 1) << bit
+    p = ((cell + 0.5) / 2097152.0).astype(np.float32)
+    p = np.concatenate([p, np.ones((1, 3), np.float32), np.zeros((1, 3), np.float32)])
+    return np.repeat(p, 3, 0), np.arange(3 * len(p), dtype=np.uint32).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("kind", ["peaks", "one nan"])
+def test_lists_that_are_not_joined(gpu, orc, kind):
+    """A comb on both sides of every 256th leaf leaves more roots than a joining block takes, over a part of
+    the leaves; one NaN keeps a part of the lists, and the wider ones over it, from being joined."""
+    import torch
+    if kind == "peaks":
+        g = np.random.default_rng(5)
+        step, mid, bit = 2 ** 56, int("01" * 27, 2), 2 ** np.arange(54, dtype=np.int64)
+        runs = [g.integers(1, step // 8, 227)]  # with the cell at the origin and 28 of a comb: 256
+        for c in range(1, 41):  # deltas fall away from the middle, which is a block's first leaf, on both sides
+            runs += [c * step + mid - bit[::2], [c * step + mid], c * step + mid + bit[1::2],
+                     c * step + g.integers(step // 3, step // 2, 201)]
+        vert, faces = _from_keys(np.concatenate(runs + [g.integers(48 * step, 120 * step, 60000)]))
+    else:
+        vert, faces = _vert("soup", 66049, 3)
+        vert[3 * 20000 + 1, 2] = np.nan
+    n = len(faces)
+    bits = 63 if kind == "peaks" else 30
+    b = gpu.LBVH(n, bits, "karras")
+    v, f = torch.from_numpy(vert).cuda(), torch.from_numpy(faces.view(np.int32)).cuda()
+    got = b.build(v, f)
+    torch.cuda.synchronize()
+    if kind == "peaks":
+        ref, _, _ = orc.lbvh_build(vert, faces, 63, 1)
+        assert np.array_equal(gpu.nodes_to_numpy(got).view(np.uint8), ref.view(np.uint8))
+    else:
+        batch = gpu.Batch([n], topology="karras")
+        ref = batch.empty_nodes()
+        batch.build(v, f, ref)
+        assert torch.equal(got, ref)
+    assert b.errors() == 0
