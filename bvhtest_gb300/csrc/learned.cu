@@ -43,15 +43,19 @@ __device__ __forceinline__ float gelu_both(float z, float &slope) {
 // errors near 2^-22 each), which leaves an absolute error of about 2e-7, far below the BF16 step
 // the activations are rounded to; the infinite or zero exponential saturates it to +-1. Training
 // keeps tanhf (its gradients are checked against float64).
-__device__ __forceinline__ float tanh_fast(float u) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(u * 2.8853900817779268f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return fmaf(-2.0f, r, 1.0f);
-}
-__device__ __forceinline__ float gelu_fast(float z) {
-  const float u = kGeluC * (z + kGeluA * z * z * z);
-  return 0.5f * z * (1.0f + tanh_fast(u));
+// Two at a time; both halves of a packed operation are rounded as a single one.
+__device__ __forceinline__ float2 gelu_fast(float2 z) {
+  const float2 cube = fma2(mul2(mul2(make_float2(kGeluA, kGeluA), z), z), z, z);
+  const float2 u = mul2(make_float2(kGeluC, kGeluC), cube);
+  const float2 v = mul2(u, make_float2(2.8853900817779268f, 2.8853900817779268f));
+  float2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(v.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(v.y));
+  e = add2(make_float2(1.0f, 1.0f), e);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(e.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(e.y));
+  const float2 t = fma2(make_float2(-2.0f, -2.0f), r, make_float2(1.0f, 1.0f));
+  return mul2(mul2(make_float2(0.5f, 0.5f), z), add2(make_float2(1.0f, 1.0f), t));
 }
 // Two values to BF16 in one conversion, packed low | high << 16.
 __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
@@ -62,15 +66,22 @@ __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
 // ---- inference on the 5th-generation tensor cores (tcgen05) ----------------------------------------
 // Persistent CTAs of 4 warps; a tile is 128 rows. Layer 1: D1[128 x 64] = X[128 x 32] * W1^T (the 24
 // features padded to K = 32), layer 2: D2[128 x 64] = A1[128 x 64] * W2^T, both BF16 operands in
-// shared memory and FP32 accumulators in tensor memory (columns 0-63 and 64-127 of a 128-column
-// allocation). Thread 0 issues the MMAs and commits them to an mbarrier; each warp then reads its 32
+// shared memory and FP32 accumulators in tensor memory (64 columns that the layers take in turn: a
+// layer's MMAs start after every warp has read the other's). Thread 0 issues the MMAs and commits them to an mbarrier; each warp then reads its 32
 // accumulator rows (TMEM lanes 32w .. 32w + 31) with tcgen05.ld, adds the bias, applies GELU and
 // rounds to BF16 (layer 1 into the next A operand, layer 2 straight into the 64 -> 1 dot product).
 // Operand layout: the no-swizzle K-major canonical layout of 8-row x 16-byte core matrices, core
 // (r8, k8) at r8 * SBO + k8 * LBO with LBO = 128 bytes (next 8 K-elements) and SBO = K * 16 bytes
 // (next 8 rows); an MMA consumes K = 16, so its descriptors advance by 2 * LBO per step.
+//
+// Bound: instruction issue and the special function unit, an exponential and a reciprocal for each of
+// the 128 GELUs of a row; the MMAs are a few percent. So the epilogues' arithmetic is packed two values
+// an instruction (16 issue slots a GELU before, 11 now), and with one accumulator for both layers six
+// CTAs fit an SM instead of four, whose epilogues cover each other's MMAs and loads. Measured, 4.19M rows:
+// 326 us, now 278; the special functions alone take 232.
 constexpr int kTcRows = 128;
-constexpr uint32_t kTcCols = 128;        // tensor-memory columns per CTA
+constexpr uint32_t kTcCols = 64;         // tensor-memory columns per CTA: both layers' accumulator
+constexpr int kTcCtas = 6;               // CTAs per SM (38 KB of shared memory each)
 constexpr int kTcK1 = 32;                // layer-1 K (24 features + zero padding)
 constexpr uint32_t kTcWaitLimit = 1u << 22;
 
@@ -79,7 +90,7 @@ struct TcSmem {
   alignas(128) uint8_t b1[kH * kTcK1 * 2];       // W1 (N = 64 rows x K = 32), 4 KB
   alignas(128) uint8_t a2[kTcRows * kH * 2];     // layer-1 activations, 16 KB
   alignas(128) uint8_t b2[kH * kH * 2];          // W2 (64 x 64), 8 KB
-  float b1f[kH], b2f[kH], w3f[kH], b3f;
+  alignas(8) float b1f[kH], b2f[kH], w3f[kH], b3f;
   alignas(8) uint64_t bar;
   uint32_t tmem;
   uint32_t fail;
@@ -159,7 +170,7 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 template <bool KEYS>
-__global__ void __launch_bounds__(128, 4) mlp_forward_tc_kernel(const __nv_bfloat16 *__restrict__ w,
+__global__ void __launch_bounds__(128, kTcCtas) mlp_forward_tc_kernel(const __nv_bfloat16 *__restrict__ w,
                                                                 const uint16_t *__restrict__ x, uint32_t n,
                                                                 float *__restrict__ y,
                                                                 const uint32_t *__restrict__ inner,
@@ -247,9 +258,9 @@ __global__ void __launch_bounds__(128, 4) mlp_forward_tc_kernel(const __nv_bfloa
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           const int j0 = 32 * half + 8 * c + 2 * h;
-          const float g0 = gelu_fast(v[8 * c + 2 * h] + sm.b1f[j0]);
-          const float g1 = gelu_fast(v[8 * c + 2 * h + 1] + sm.b1f[j0 + 1]);
-          u[h] = bf16x2_bits(g0, g1);
+          const float2 g = gelu_fast(add2(make_float2(v[8 * c + 2 * h], v[8 * c + 2 * h + 1]),
+                                          *reinterpret_cast<const float2 *>(sm.b1f + j0)));
+          u[h] = bf16x2_bits(g.x, g.y);
         }
         *reinterpret_cast<uint4 *>(sm.a2 + core_off(tid, 32 * half + 8 * c, kH)) = make_uint4(u[0], u[1], u[2], u[3]);
       }
@@ -261,7 +272,7 @@ __global__ void __launch_bounds__(128, 4) mlp_forward_tc_kernel(const __nv_bfloa
     if (tid == 0) {
 #pragma unroll
       for (int k = 0; k < kH / 16; ++k)
-        tc_mma(tmem + 64u, tc_smem_desc(a2 + 256u * k, 128u, kH * 16u), tc_smem_desc(b2 + 256u * k, 128u, kH * 16u),
+        tc_mma(tmem, tc_smem_desc(a2 + 256u * k, 128u, kH * 16u), tc_smem_desc(b2 + 256u * k, 128u, kH * 16u),
                k > 0);
       tc_commit(&sm.bar);
     }
@@ -276,11 +287,12 @@ __global__ void __launch_bounds__(128, 4) mlp_forward_tc_kernel(const __nv_bfloa
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       float v[32];
-      tc_ld32(tmem + lanebase + 64u + 32u * half, v);
+      tc_ld32(tmem + lanebase + 32u * half, v);
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
-        const uint32_t u = bf16x2_bits(gelu_fast(v[i] + sm.b2f[32 * half + i]),
-                                       gelu_fast(v[i + 1] + sm.b2f[32 * half + i + 1]));
+        const float2 g = gelu_fast(add2(make_float2(v[i], v[i + 1]),
+                                        *reinterpret_cast<const float2 *>(sm.b2f + 32 * half + i)));
+        const uint32_t u = bf16x2_bits(g.x, g.y);
         out += sm.w3f[32 * half + i] * __uint_as_float(u << 16);
         out += sm.w3f[32 * half + i + 1] * __uint_as_float(u & 0xFFFF0000u);
       }
@@ -981,9 +993,9 @@ __global__ void features_pack_kernel(const uint4 *__restrict__ pend, const uint3
   }
 }
 
-// Persistent tensor-core CTAs: up to four per SM (4 x 128 of the 512 tensor-memory columns).
+// Persistent tensor-core CTAs.
 uint32_t tc_grid(uint32_t rows) {
-  return std::max(1u, std::min(ceil_div(rows, kTcRows), (uint32_t)sm_count() * 4));
+  return std::max(1u, std::min(ceil_div(rows, kTcRows), (uint32_t)sm_count() * kTcCtas));
 }
 
 uint32_t grid_for(uint32_t n, uint32_t block) {
@@ -1054,18 +1066,21 @@ int lr_features(LrScratch &s, const bvhgb_node *nodes, uint32_t numNodes, uint32
     depth_jump_kernel<<<gi, 256, 0, st>>>(inner, numInner, numNodes, root, s.ad);
     BVHGB_LAUNCH_CHECK("lr depth jump");
   }
+  // One node or row per thread: a thread with several waits for the longest climb of its warp each time
+  // (4.19M leaves: 150 us, 95 so; the feature rows 226 and 209, their ranks 59 and 53). The jumps and the
+  // first pass, whose threads all do alike, are faster with several.
   BVHGB_CUDA_TRY(cudaMemsetAsync(s.acc, 0, 8ull * numNodes, st));
-  leaf_count_kernel<<<g, 256, 0, st>>>(s.par, numNodes, root, s.leafCount, s.acc, lr_error_word(s));
+  leaf_count_kernel<<<ceil_div(numNodes, 256), 256, 0, st>>>(s.par, numNodes, root, s.leafCount, s.acc, lr_error_word(s));
   BVHGB_LAUNCH_CHECK("lr leaf count");
   BVHGB_CUDA_TRY(cudaMemsetAsync(s.hist, 0, 4 * kHistPrefix, st));
-  features_raw_kernel<<<gi, 256, 0, st>>>(nodes, inner, numInner, numNodes, root, s.ad, s.leafCount, s.sa, s.par,
+  features_raw_kernel<<<ceil_div(numInner, 256), 256, 0, st>>>(nodes, inner, numInner, numNodes, root, s.ad, s.leafCount, s.sa, s.par,
                                           invLog2Leaves, s.x, s.pend, s.hist, lr_error_word(s));
   BVHGB_LAUNCH_CHECK("lr features");
   hist_reduce_kernel<<<grid_for(kRankBins, 256), 256, 0, st>>>(s.hist);
   BVHGB_LAUNCH_CHECK("lr rank reduce");
   hist_scan_kernel<<<4, 1024, 0, st>>>(s.hist);
   BVHGB_LAUNCH_CHECK("lr rank scan");
-  features_pack_kernel<<<gi, 256, 0, st>>>(s.pend, s.hist, numInner, s.x);
+  features_pack_kernel<<<ceil_div(numInner, 256), 256, 0, st>>>(s.pend, s.hist, numInner, s.x);
   BVHGB_LAUNCH_CHECK("lr features pack");
   return BVHGB_OK;
 }

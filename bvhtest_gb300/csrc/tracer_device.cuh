@@ -18,24 +18,6 @@ struct RayPre {
   int kx, ky, kz;
 };
 
-// Two single-precision operations in one instruction, each half rounded on its own.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n"
-      " mov.b64 {%0, %1}, z;\n}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n"
-      " mov.b64 {%0, %1}, z;\n}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
 __device__ __forceinline__ void setup_ray(RayPre &r) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) r.inv[k] = fdiv(1.0f, r.d[k]);
@@ -86,15 +68,6 @@ __device__ __forceinline__ bool ray_tri(const RayPre &r, const float *v0, const 
   if (!(t > tmin) || !(t <= tmax)) return false;
   tout = t;
   return true;
-}
-
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
-      " fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;\n}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
 }
 
 // Robust slab test; sign-selected planes make 0 * inf NaNs drop out of the min/max. The six plane
