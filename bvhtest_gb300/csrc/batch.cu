@@ -8,7 +8,7 @@
 //   - build  : the single-mesh leaf climb on each sorted segment (node arrays at per-mesh offsets,
 //              leaves store the face index within their mesh);
 //   - Bittner13 : per iteration, one sort of (mesh << 32 | ~order(inefficiency)) gives every mesh's
-//              selection; chunk c of every mesh runs in the same four launches (meshes share nothing,
+//              selection (of the nodes that the chunks read, where they are few); chunk c of every mesh runs in the same four launches (meshes share nothing,
 //              so this equals running each mesh's chunks one after another);
 //   - trace  : random rays per mesh (origins uniform in the mesh box grown 1.5x about its centre,
 //              directions uniform on the sphere), closest hit in that mesh's tree.
@@ -36,6 +36,10 @@ struct bvhgb_batch_workspace {
   float4 *triBoxes = nullptr;
   void *sortTemp = nullptr;
   bvhgb::WideNode *wide = nullptr;  // the tracer's wide records, one per inner node; null where they do not fit
+  // The selection of every mesh's first numChunks * chunk nodes (sel.tiles = 0: all are sorted).
+  bvhgb::SegSelect sel{};
+  uint32_t kept = 0;            // nodes selected in all
+  uint32_t *selWords = nullptr;  // the device arrays of sel
   // optimizer
   uint32_t *todo = nullptr, *valid = nullptr, *toFix = nullptr, *owner = nullptr, *counter = nullptr;
   unsigned long long *mail = nullptr;  // refit mail slots, three words per node, empty between launches
@@ -198,6 +202,35 @@ __global__ void __launch_bounds__(kBatchThreads) batch_cost_kernel(const bvhgb_n
   }
 }
 
+// The same keys without the mesh, a block per tile of one mesh, and the histogram of their upper 11 bits
+// that the selection starts from.
+__global__ void __launch_bounds__(kSegThreads) batch_tile_cost_kernel(const bvhgb_node *__restrict__ nodes,
+                                                                      const uint32_t *__restrict__ nodeOff, SegSelect q,
+                                                                      uint32_t *__restrict__ keys,
+                                                                      uint32_t *__restrict__ hist) {
+  __shared__ uint32_t sh[kSegBins];
+  const SegTile t = q.tile[blockIdx.x];
+  const uint32_t row = q.row[t.seg];
+  if (row != kNone)
+    for (uint32_t b = threadIdx.x; b < kSegBins; b += kSegThreads) sh[b] = 0;
+  __syncthreads();
+  const bvhgb_node *mesh = nodes + __ldg(nodeOff + t.seg);
+  for (uint32_t base = 0; base < t.len; base += kSegThreads) {
+    const uint32_t j = base + threadIdx.x;
+    uint32_t bin = 0xFFFFFFFFu;
+    if (j < t.len) {
+      const uint32_t key = ~f2ord(inefficiency(mesh, t.local + j));
+      keys[t.start + j] = key;
+      bin = key >> 21;
+    }
+    if (row != kNone) count_bin(sh, bin);
+  }
+  __syncthreads();
+  if (row != kNone)
+    for (uint32_t b = threadIdx.x; b < kSegBins; b += kSegThreads)
+      if (sh[b]) atomicAdd(&hist[(size_t)row * kSegBins + b], sh[b]);
+}
+
 struct MeshItem {
   uint32_t m, k;  // mesh, rank of the item within the mesh's chunk
 };
@@ -211,7 +244,7 @@ __global__ void __launch_bounds__(kWarpItemsPerBlock * 32, 5) batch_patch_kernel
     const bvhgb_node *__restrict__ nodes, const uint32_t *__restrict__ todo, const uint32_t *__restrict__ itemMesh,
     const uint32_t *__restrict__ itemOff, const uint32_t *__restrict__ chunkSize,
     const uint32_t *__restrict__ faceOff, const uint32_t *__restrict__ nodeOff,
-    const uint32_t *__restrict__ innerOff, uint32_t items, uint32_t chunk, PatchOut *__restrict__ out,
+    const uint32_t *__restrict__ todoOff, uint32_t items, uint32_t chunk, PatchOut *__restrict__ out,
     uint32_t *__restrict__ valid, uint32_t *__restrict__ toFix, uint32_t *__restrict__ owner,
     unsigned long long *__restrict__ stats, uint32_t *__restrict__ err) {
   const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -221,7 +254,7 @@ __global__ void __launch_bounds__(kWarpItemsPerBlock * 32, 5) batch_patch_kernel
   const uint32_t numNodes = 2 * n - 1, numInner = n - 1, nb = __ldg(nodeOff + it.m);
   const uint32_t pos = chunk * __ldg(chunkSize + it.m) + it.k;
   const bool ok = pos < numInner;
-  const uint32_t node = ok ? __ldg(todo + __ldg(innerOff + it.m) + pos) : kNone;
+  const uint32_t node = ok ? __ldg(todo + __ldg(todoOff + it.m) + pos) : kNone;
   warp_patch_item(nodes + nb, 0u, numNodes, node, ok, it.k, out + q, valid + q, toFix + 3 * (size_t)q, owner + nb,
                   stats, err);
 }
@@ -416,12 +449,25 @@ int batch_build(bvhgb_batch_workspace *ws, const float *vert, const uint32_t *fa
 int batch_iteration(bvhgb_batch_workspace *ws, bvhgb_node *nodes, cudaStream_t s) {
   const uint32_t M = ws->numMeshes, I = ws->totalInner, T = ws->items;
   if (I == 0) return BVHGB_OK;
-  batch_cost_kernel<<<grid_of(I, kBatchThreads), kBatchThreads, off_smem(M), s>>>(nodes, ws->innerOff, ws->nodeOff, M,
-                                                                                   I, ws->keys, ws->vals);
-  BVHGB_LAUNCH_CHECK("batch cost");
-  int st = sort_pairs(ws->sortTemp, ws->keys, ws->keysSorted, ws->vals, ws->todo, I, 8, 0, 32 + ws->meshBits, s,
+  if (ws->sel.tiles) {
+    uint32_t *keys = reinterpret_cast<uint32_t *>(ws->keys), *hist = reinterpret_cast<uint32_t *>(ws->keysSorted);
+    uint64_t *kept = ws->keys + (I + 1u) / 2u;  // behind the keys, of 4 bytes each
+    if (ws->sel.rows) BVHGB_CUDA_TRY(cudaMemsetAsync(hist, 0, 4ull * kSegBins * ws->sel.rows, s));
+    batch_tile_cost_kernel<<<ws->sel.tiles, kSegThreads, 0, s>>>(nodes, ws->nodeOff, ws->sel, keys, hist);
+    BVHGB_LAUNCH_CHECK("batch cost");
+    int st = select_segments(ws->sel, keys, hist, kept, ws->vals, s);
+    if (!st)
+      st = sort_pairs(ws->sortTemp, kept, ws->keysSorted, ws->vals, ws->todo, ws->kept, 8, 0, 32 + ws->meshBits, s,
                       ws->cfg.sortTileKeys);
-  if (st) return st;
+    if (st) return st;
+  } else {
+    batch_cost_kernel<<<grid_of(I, kBatchThreads), kBatchThreads, off_smem(M), s>>>(nodes, ws->innerOff, ws->nodeOff, M,
+                                                                                     I, ws->keys, ws->vals);
+    BVHGB_LAUNCH_CHECK("batch cost");
+    int st = sort_pairs(ws->sortTemp, ws->keys, ws->keysSorted, ws->vals, ws->todo, I, 8, 0, 32 + ws->meshBits, s,
+                        ws->cfg.sortTileKeys);
+    if (st) return st;
+  }
   if (T == 0) return BVHGB_OK;
   const uint32_t bs = ws->cfg.refitBlock;
   // climbs per warp: the fewest that fit in one wave of resident warps
@@ -435,7 +481,7 @@ int batch_iteration(bvhgb_batch_workspace *ws, bvhgb_node *nodes, cudaStream_t s
   const uint32_t pc = perWarp((const void *)batch_count_kernel), pr = perWarp((const void *)batch_refit_kernel);
   for (uint32_t c = 0; c < ws->cfg.numChunks; ++c) {
     batch_patch_kernel<<<ceil_div(T, kWarpItemsPerBlock), kWarpItemsPerBlock * 32, 0, s>>>(
-        nodes, ws->todo, ws->itemMesh, ws->itemOff, ws->chunk, ws->faceOff, ws->nodeOff, ws->innerOff, T, c,
+        nodes, ws->todo, ws->itemMesh, ws->itemOff, ws->chunk, ws->faceOff, ws->nodeOff, ws->sel.tiles ? ws->sel.outOff : ws->innerOff, T, c,
         ws->patches, ws->valid, ws->toFix, ws->owner, ws->stats, ws->err);
     BVHGB_LAUNCH_CHECK("batch patch");
     batch_apply_kernel<<<ceil_div(T, bs), bs, 0, s>>>(nodes, ws->patches, ws->valid, ws->toFix, ws->owner,
@@ -485,6 +531,71 @@ bool valid_config(const bvhgb_batch_config &c) {
   const bool refit = c.refitBlock >= 32 && c.refitBlock <= 1024 && c.refitBlock % 32 == 0;
   const bool trace = c.traceBlock >= 32 && c.traceBlock <= 1024 && c.traceBlock % 32 == 0;
   return tile && refit && trace && c.numChunks > 0 && c.topology <= BVHGB_TOPO_KARRAS && c.mortonBits == 30;
+}
+
+// Plans the selection of the nodes that the chunks read (the rest of the sorted order is never looked
+// at). Meshes of up to kSelectWhole inner nodes keep all of them, which costs less than three
+// histograms.
+//
+// Why: six passes over all nodes for the order of 2% of them were the iteration's second largest part.
+// Measured, 256 meshes of 20.1M triangles: costs and sort 360 + 1,130 us an iteration, costs and selection
+// 332 + 200. Per iteration of 64 meshes, sorted / selected, in us: 262,144 triangles 1,264 / 1,268,
+// 524,288 1,422 / 1,393, 2.1M 1,922 / 1,895; with 24% of the nodes kept 524,288 1,996 / 2,011, 1.05M
+// 2,989 / 3,022, 2.1M 5,603 / 5,590, 8.4M 21,039 / 20,772.
+constexpr uint32_t kSelectWhole = 2048, kSelectLeast = 1u << 19, kSelectMany = 1u << 21;
+cudaError_t plan_selection(bvhgb_batch_workspace *ws) {
+  const uint32_t M = ws->numMeshes;
+  std::vector<uint32_t> tileOff(M + 1), row(M), rowSeg, keep(M), outOff(M + 1);
+  std::vector<SegTile> tile;
+  uint64_t kept = 0;
+  for (uint32_t m = 0; m < M; ++m) {
+    const uint32_t base = ws->hInnerOff[m], n = ws->hInnerOff[m + 1] - base;
+    const uint64_t want = (uint64_t)ws->hChunk[m] * ws->cfg.numChunks;
+    const bool select = n > kSelectWhole && want > 0 && want < n;
+    tileOff[m] = (uint32_t)tile.size();
+    row[m] = select ? (uint32_t)rowSeg.size() : kNone;
+    if (select) rowSeg.push_back(m);
+    keep[m] = select ? (uint32_t)want : want ? n : 0u;
+    outOff[m] = (uint32_t)kept;
+    kept += keep[m];
+    if (keep[m])
+      for (uint32_t at = 0; at < n; at += kSegTile) tile.push_back({m, base + at, std::min(kSegTile, n - at), at});
+  }
+  tileOff[M] = (uint32_t)tile.size();
+  outOff[M] = (uint32_t)kept;
+  const uint32_t most = ws->totalInner / (ws->totalInner < kSelectMany ? 16 : 4);
+  if (ws->totalInner < kSelectLeast || kept == 0 || kept > most) return cudaSuccess;
+  SegSelect q{};
+  q.segs = M;
+  q.tiles = (uint32_t)tile.size();
+  q.rows = (uint32_t)rowSeg.size();
+  // One allocation: tiles, then the words, then the two pair arrays.
+  const size_t words = 4 * (size_t)q.tiles + (M + 1) + M + std::max(q.rows, 1u) + M + (M + 1);
+  const size_t pairs = (words + 1) & ~(size_t)1;
+  cudaError_t e = dev_malloc(&ws->selWords, 4 * (pairs + 2 * (size_t)q.rows + 2 * (size_t)q.tiles));
+  if (e != cudaSuccess) return e;
+  std::vector<uint32_t> host(words, 0u);
+  size_t at = 0;
+  auto put = [&](const void *src, size_t n) {
+    std::copy_n(static_cast<const uint32_t *>(src), n, host.begin() + (ptrdiff_t)at);
+    const uint32_t *p = ws->selWords + at;
+    at += n;
+    return p;
+  };
+  q.tile = reinterpret_cast<const SegTile *>(put(tile.data(), 4 * tile.size()));
+  q.tileOff = put(tileOff.data(), M + 1);
+  q.row = put(row.data(), M);
+  q.rowSeg = put(rowSeg.data(), rowSeg.size());
+  q.keep = put(keep.data(), M);
+  q.outOff = put(outOff.data(), M + 1);
+  q.state = reinterpret_cast<uint2 *>(ws->selWords + pairs);
+  q.count = q.state + q.rows;
+  e = cudaMemcpy(ws->selWords, host.data(), 4 * words, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    ws->sel = q;
+    ws->kept = (uint32_t)kept;
+  }
+  return e;
 }
 
 void drop_graph(bvhgb_batch_workspace *ws) {
@@ -580,6 +691,7 @@ extern "C" BVHGB_API int bvhgb_batch_create(uint32_t numMeshes, const uint32_t *
   alloc(&ws->counter, 4 * N);
   alloc(&ws->mail, 24 * N);
   alloc(&ws->stats, sizeof(unsigned long long) * S_COUNT);
+  if (e == cudaSuccess) e = plan_selection(ws);
   // Where the wide records do not fit, rays go through the node arrays.
   if (e == cudaSuccess && dev_malloc(&ws->wide, sizeof(WideNode) * std::max<size_t>(inner, 1)) != cudaSuccess) {
     ws->wide = nullptr;
@@ -612,7 +724,7 @@ extern "C" BVHGB_API int bvhgb_batch_destroy(bvhgb_batch_workspace *ws) {
                   (void *)ws->itemMesh, (void *)ws->scene, (void *)ws->err, (void *)ws->keys, (void *)ws->keysSorted,
                   (void *)ws->vals, (void *)ws->valsSorted, (void *)ws->slots, (void *)ws->triBoxes, ws->sortTemp,
                   (void *)ws->todo, (void *)ws->valid, (void *)ws->toFix, (void *)ws->patches, (void *)ws->owner,
-                  (void *)ws->counter, (void *)ws->mail, (void *)ws->stats, (void *)ws->wide})
+                  (void *)ws->counter, (void *)ws->mail, (void *)ws->stats, (void *)ws->wide, (void *)ws->selWords})
     cudaFree(p);
   delete ws;
   return BVHGB_OK;

@@ -855,6 +855,164 @@ int select_smallest(void *temp, const uint32_t *keys, const uint32_t *vals, uint
   return sort_pairs(t + L.sortTemp, ck, ko, cv, valsOut, k, 4, 0, 32, s, tileKeys);
 }
 
+// ---- the selection over many segments --------------------------------------------------------------
+//
+// select_smallest's steps, a block per tile of one segment, thresholds and counts per segment. The
+// first histogram (of the upper 11 bits) comes from the kernel that makes the keys. Bound: reading the
+// keys four times (20M keys in 256 segments: histograms 40 us each, counts 20, scatter 38; the stable
+// sort of all of them by segment and key took 1,130).
+namespace {
+
+__global__ void __launch_bounds__(kSegThreads) seg_hist_kernel(SegSelect q, const uint32_t *__restrict__ keys,
+                                                               uint32_t *__restrict__ hist, int pass) {
+  __shared__ uint32_t sh[kSegBins];
+  const SegTile t = q.tile[blockIdx.x];
+  const uint32_t row = q.row[t.seg];
+  if (row == kNone) return;
+  for (uint32_t b = threadIdx.x; b < kSegBins; b += kSegThreads) sh[b] = 0;
+  __syncthreads();
+  const uint32_t shift = sel_shift(pass), mask = (1u << sel_bits(pass)) - 1u, hi = shift + sel_bits(pass);
+  const uint32_t prefix = q.state[row].x;
+  for (uint32_t base = 0; base < t.len; base += kSegThreads) {
+    const uint32_t j = base + threadIdx.x;
+    uint32_t bin = 0xFFFFFFFFu;
+    if (j < t.len) {
+      const uint32_t key = __ldg(keys + t.start + j);
+      if ((key >> hi) == prefix) bin = (key >> shift) & mask;
+    }
+    if (__ballot_sync(0xFFFFFFFFu, bin != 0xFFFFFFFFu) != 0u) count_bin(sh, bin);  // most warps have none
+  }
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < kSegBins; b += kSegThreads)
+    if (sh[b]) atomicAdd(&hist[(size_t)row * kSegBins + b], sh[b]);
+}
+
+__global__ void __launch_bounds__(kSegBins / 2) seg_find_kernel(SegSelect q, uint32_t *__restrict__ hist, int pass) {
+  __shared__ uint32_t warpSums[33];
+  const uint32_t row = blockIdx.x, b0 = 2u * threadIdx.x;
+  uint32_t *h = hist + (size_t)row * kSegBins;
+  const uint32_t h0 = h[b0], h1 = h[b0 + 1];
+  const uint2 st = pass ? q.state[row] : make_uint2(0u, 0u);
+  uint32_t total;
+  const uint32_t ex = block_exclusive_sum(h0 + h1, warpSums, total);  // its barriers: every thread has read the state
+  const uint32_t need = q.keep[q.rowSeg[row]] - st.y;  // rank (from 1) of the wanted key among those with the prefix
+  if (ex < need && need <= ex + h0) q.state[row] = make_uint2((st.x << sel_bits(pass)) | b0, st.y + ex);
+  else if (ex + h0 < need && need <= ex + h0 + h1) q.state[row] = make_uint2((st.x << sel_bits(pass)) | (b0 + 1u), st.y + ex + h0);
+  h[b0] = h[b0 + 1] = 0u;
+}
+
+__global__ void __launch_bounds__(kSegThreads) seg_count_kernel(SegSelect q, const uint32_t *__restrict__ keys) {
+  __shared__ uint32_t warpSums[33];
+  const SegTile t = q.tile[blockIdx.x];
+  const uint32_t row = q.row[t.seg];
+  if (row == kNone) {
+    if (threadIdx.x == 0) q.count[blockIdx.x] = make_uint2(t.len, 0u);
+    return;
+  }
+  const uint32_t T = q.state[row].x;
+  uint32_t c = 0;  // at T: upper half (a tile has at most kSegTile of either)
+  for (uint32_t j = threadIdx.x; j < t.len; j += kSegThreads) {
+    const uint32_t key = __ldg(keys + t.start + j);
+    c += (key < T ? 1u : 0u) + (key == T ? 1u << 16 : 0u);
+  }
+  uint32_t total;
+  block_exclusive_sum(c, warpSums, total);
+  if (threadIdx.x == 0) q.count[blockIdx.x] = make_uint2(total & 0xFFFFu, total >> 16);
+}
+
+// Exclusive prefixes of a segment's tile counts, in place, one block per segment.
+__global__ void __launch_bounds__(256) seg_scan_kernel(SegSelect q) {
+  __shared__ uint32_t warpSums[33];
+  const uint32_t first = q.tileOff[blockIdx.x], last = q.tileOff[blockIdx.x + 1];
+  uint2 carry = make_uint2(0u, 0u);
+  for (uint32_t c = first; c < last; c += 256u) {
+    const uint32_t i = c + threadIdx.x;
+    const uint2 v = i < last ? q.count[i] : make_uint2(0u, 0u);
+    uint32_t sumLt, sumEq;
+    const uint32_t lt = block_exclusive_sum(v.x, warpSums, sumLt), eq = block_exclusive_sum(v.y, warpSums, sumEq);
+    if (i < last) q.count[i] = make_uint2(carry.x + lt, carry.y + eq);
+    carry.x += sumLt;
+    carry.y += sumEq;
+  }
+}
+
+__global__ void __launch_bounds__(kSegThreads) seg_scatter_kernel(SegSelect q, const uint32_t *__restrict__ keys,
+                                                                  uint64_t *__restrict__ outKeys,
+                                                                  uint32_t *__restrict__ outVals) {
+  __shared__ uint32_t warpSums[33];
+  constexpr uint32_t kPer = kSegTile / kSegThreads;
+  const SegTile t = q.tile[blockIdx.x];
+  const uint32_t row = q.row[t.seg], keep = q.keep[t.seg], out = q.outOff[t.seg];
+  const uint64_t high = (uint64_t)t.seg << 32;
+  uint2 before = q.count[blockIdx.x];
+  if (row == kNone) {
+    for (uint32_t j = threadIdx.x; j < t.len; j += kSegThreads) {
+      outKeys[out + before.x + j] = high | __ldg(keys + t.start + j);
+      outVals[out + before.x + j] = t.local + j;
+    }
+    return;
+  }
+  const uint2 st = q.state[row];
+  const uint32_t T = st.x, need = keep - st.y;
+  // A warp takes 32 consecutive keys at a time, a thread's 16 are 32 apart: a lane's place among the
+  // warp's keys comes from ballots.
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, ltMask = (1u << lane) - 1u;
+  const uint32_t j0 = warp * 32u * kPer + lane;
+  uint32_t key[kPer], c = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kPer; ++j) {
+    const bool live = j0 + 32u * j < t.len;
+    key[j] = live ? __ldg(keys + t.start + j0 + 32u * j) : 0xFFFFFFFFu;
+    c += (live && key[j] < T ? 1u : 0u) + (live && key[j] == T ? 1u << 16 : 0u);
+  }
+  // The counts before this warp: lane 0's place in the block's order of (warp, lane).
+  uint32_t total;
+  const uint32_t ex = block_exclusive_sum(c, warpSums, total);
+  const uint32_t warpEx = __shfl_sync(0xFFFFFFFFu, ex, 0);
+  before.x += warpEx & 0xFFFFu;
+  before.y += warpEx >> 16;
+#pragma unroll
+  for (uint32_t j = 0; j < kPer; ++j) {
+    const bool live = j0 + 32u * j < t.len;
+    const bool lt = live && key[j] < T, eq = live && key[j] == T;
+    const uint32_t lts = __ballot_sync(0xFFFFFFFFu, lt), eqs = __ballot_sync(0xFFFFFFFFu, eq);
+    const uint32_t myLt = before.x + __popc(lts & ltMask), myEq = before.y + __popc(eqs & ltMask);
+    if (lt || (eq && myEq < need)) {
+      const uint32_t pos = myLt + min(myEq, need);
+      if (pos < keep) {  // always, unless the keys changed between the passes
+        outKeys[out + pos] = high | key[j];
+        outVals[out + pos] = t.local + j0 + 32u * j;
+      }
+    }
+    before.x += __popc(lts);
+    before.y += __popc(eqs);
+  }
+}
+
+}  // namespace
+
+int select_segments(const SegSelect &q, const uint32_t *keys, uint32_t *hist, uint64_t *outKeys, uint32_t *outVals,
+                    cudaStream_t s) {
+  static_assert(kSegBins == 1u << sel_bits(0) && kSegTile < 1u << 16, "one digit per row, counts in 16 bits");
+  if (q.rows) {
+    for (int pass = 0; pass < 3; ++pass) {
+      if (pass) {
+        seg_hist_kernel<<<q.tiles, kSegThreads, 0, s>>>(q, keys, hist, pass);
+        BVHGB_LAUNCH_CHECK("segment histogram");
+      }
+      seg_find_kernel<<<q.rows, kSegBins / 2, 0, s>>>(q, hist, pass);
+      BVHGB_LAUNCH_CHECK("segment find");
+    }
+  }
+  seg_count_kernel<<<q.tiles, kSegThreads, 0, s>>>(q, keys);
+  BVHGB_LAUNCH_CHECK("segment count");
+  seg_scan_kernel<<<q.segs, 256, 0, s>>>(q);
+  BVHGB_LAUNCH_CHECK("segment scan");
+  seg_scatter_kernel<<<q.tiles, kSegThreads, 0, s>>>(q, keys, outKeys, outVals);
+  BVHGB_LAUNCH_CHECK("segment scatter");
+  return BVHGB_OK;
+}
+
 }  // namespace bvhgb
 
 extern "C" BVHGB_API int bvhgb_radix_sort_pairs(void *temp, size_t *tempBytes, const void *keysIn, void *keysOut,

@@ -33,4 +33,30 @@ int sort_pairs(void *temp, const void *keysIn, void *keysOut, const uint32_t *va
 size_t select_temp_bytes(uint32_t n, uint32_t k);
 int select_smallest(void *temp, const uint32_t *keys, const uint32_t *vals, uint32_t n, uint32_t k, uint32_t *valsOut,
                     cudaStream_t s, uint32_t tileKeys = 0);
+
+// The same for many segments of one key array at once: segment g keeps its keep[g] smallest keys (ties
+// in index order), in index order, as (g << 32 | key, index within the segment) from place outOff[g] on.
+// A stable sort of the kept pairs is then every segment's prefix of its own stable sort. Segments
+// without a row keep all their keys. All arrays are on the device.
+constexpr uint32_t kSegTile = 8192, kSegThreads = 512, kSegBins = 2048;
+struct SegTile {
+  uint32_t seg, start, len, local;  // keys [start, start + len); 'local' is the first one's index in its segment
+};
+struct SegSelect {
+  uint32_t segs, tiles, rows;  // rows: segments that select
+  const SegTile *tile;         // in order, tileOff[g] .. tileOff[g + 1] - 1 for segment g
+  const uint32_t *tileOff, *row, *rowSeg, *keep, *outOff;  // row[g] or kNone; rowSeg[row] = g
+  uint2 *state;                // per row: digits of the threshold found so far, keys below them
+  uint2 *count;                // per tile: keys below and at the threshold
+};
+// hist: rows x kSegBins counts of the keys' upper 11 bits (cleared on return).
+int select_segments(const SegSelect &q, const uint32_t *keys, uint32_t *hist, uint64_t *outKeys, uint32_t *outVals,
+                    cudaStream_t s);
+#ifdef __CUDACC__
+// Adds one key per lane (bin 0xFFFFFFFF: none) to a block's counts; lanes with the same bin add together.
+__device__ __forceinline__ void count_bin(uint32_t *bins, uint32_t bin) {
+  const uint32_t peers = __match_any_sync(0xFFFFFFFFu, bin);
+  if (bin != 0xFFFFFFFFu && (peers & ((1u << (threadIdx.x & 31u)) - 1u)) == 0u) atomicAdd(&bins[bin], (uint32_t)__popc(peers));
+}
+#endif
 }  // namespace bvhgb
