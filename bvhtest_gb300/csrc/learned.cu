@@ -76,7 +76,7 @@ __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi) {
 //
 // Bound: instruction issue and the special function unit, an exponential and a reciprocal for each of
 // the 128 GELUs of a row; the MMAs are a few percent. So the epilogues' arithmetic is packed two values
-// an instruction (16 issue slots a GELU before, 11 now), and with one accumulator for both layers six
+// an instruction (16 issue slots a GELU otherwise), and with one accumulator for both layers six
 // CTAs fit an SM instead of four, whose epilogues cover each other's MMAs and loads. Measured, 4.19M rows:
 // 326 us, now 278; the special functions alone take 232.
 constexpr int kTcRows = 128;
