@@ -8,8 +8,9 @@
 //   - build  : the single-mesh leaf climb on each sorted segment (node arrays at per-mesh offsets,
 //              leaves store the face index within their mesh);
 //   - Bittner13 : per iteration, one sort of (mesh << 32 | ~order(inefficiency)) gives every mesh's
-//              selection (of the nodes that the chunks read, where they are few); chunk c of every mesh runs in the same four launches (meshes share nothing,
-//              so this equals running each mesh's chunks one after another);
+//              selection (of the nodes that the chunks read, where they are few); chunk c of every mesh
+//              runs in the same four launches (meshes share nothing, so this equals running each mesh's
+//              chunks one after another);
 //   - trace  : random rays per mesh (origins uniform in the mesh box grown 1.5x about its centre,
 //              directions uniform on the sphere), closest hit in that mesh's tree.
 // Mesh-level indices are found by binary search over the offset arrays held in shared memory.

@@ -1,20 +1,19 @@
 // Parallel Bittner13 SAH optimizer (lib/builder/Bittner13CUDA.cu, lib/base/BVHPatch.hpp).
 //
 // One iteration = select + numChunks chunks. Selection: inefficiency of every inner node, then the
-// onesweep sort on (~order(cost), node) gives the stable descending order of the reference's
-// SortPairsDescending. Each chunk runs four kernels:
-//   patch  : one thread per batch item removes its node and reinserts both children into a private
+// nodes the chunks read in the stable descending order of the reference's SortPairsDescending
+// (select_smallest on ~order(cost)). Each chunk runs three kernels:
+//   patch  : one warp per batch item removes its node and reinserts both children into a private
 //            10-slot copy-on-write patch, finding each position by branch and bound over the induced
-//            cost (findNode1 with the standard-library heap discipline), then claims every node it
-//            patched with atomicMin(owner, rank);
+//            cost (a whole frontier per round; searchMode heap and alt run the reference's searches,
+//            one thread per item), then claims every node it patched with atomicMin(owner, rank);
 //   apply  : an item whose every node is still owned by its own rank writes its patch; all others
-//            count as skipped. Lower rank = higher cost wins, so the result does not depend on
-//            scheduling (the reference locks first-come and is not deterministic);
-//   count  : owners are released and each dirty path (grand parent, both reused nodes) counts its
-//            arrivals on the way to the root (kFixTree3_1);
-//   refit  : the last arrival at a node recomputes its box from its children (kFixTree3_2); the
-//            counters are relaxed and a rewritten child box reaches the last arrival through a
-//            self-validating mail slot, so no box is read before it is final.
+//   + count  count as skipped. Lower rank = higher cost wins, so the result does not depend on
+//            scheduling (the reference locks first-come and is not deterministic). The same launch
+//            marks the dirty paths (grand parent, both reused nodes) up to the root (kFixTree3_1);
+//   release: the claims are cleared; the last arrival at a node recomputes its box from its children
+//   + refit  (kFixTree3_2); arrivals are relaxed and a rewritten child box reaches the last one through
+//            a self-validating mail slot, so no box is read before it is final.
 // bvhgb_bn13_run captures one iteration into a CUDA graph and replays it. With a learned scorer
 // set, iteration i selects by the scorer unless plainEvery > 0 and i % plainEvery == plainEvery - 1,
 // in which case it selects by the inefficiency (one graph per kind of iteration).

@@ -1,4 +1,4 @@
-// LBVH build: scene box, Morton codes, onesweep sort, and a fused bottom-up topology + refit.
+// LBVH build: scene box, Morton codes, onesweep sort, and topology + refit block by block.
 //
 // Reference: lib/builder/LBVH_CUDA.cu. Kernel plan (HBM-bound, no tensor cores):
 //   lbvh_bounds  : per-triangle box (+-FLT_EPSILON) reduced into the scene box, whose initial value
@@ -10,10 +10,14 @@
 //   sort         : sort.cu (replaces cub::DeviceRadixSort, LBVH_CUDA.cu:185-193).
 //   lbvh_build   : a block makes the inner nodes among its 256 sorted leaves in shared memory and lists
 //                  the roots of its subtrees (treelet_build).
-//   lbvh_roots   : climbs from those roots (Apetrei 2014 style): at each step a climb picks the parent
-//                  from the two neighbouring key deltas, meets its sibling through one acq_rel exchange
-//                  on the split's slot, and the second to arrive merges the boxes and writes the parent.
-//                  Both give the nodes the Karras index the reference assigns (kGenLeafNodes +
+//   lbvh_join    : a block makes the nodes over 16 neighbouring lists of roots in the same way, launch by
+//                  launch up to the tree's root.
+//   lbvh_roots   : climbs from the lists that could not be joined (Apetrei 2014 style): at each step a
+//                  climb picks the parent from the two neighbouring key deltas, meets its sibling through
+//                  one acq_rel exchange on the split's slot, and the second to arrive merges the boxes
+//                  and writes the parent.
+//   lbvh_small   : all of it in one launch for up to 1,024 triangles.
+//                  All give the nodes the Karras index the reference assigns (kGenLeafNodes +
 //                  kBuildTree + kFixAABBTree, LBVH_CUDA.cu:273-374).
 #include <algorithm>
 #include <cstring>

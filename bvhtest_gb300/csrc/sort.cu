@@ -4,8 +4,8 @@
 // SortPairsDescending (lib/builder/Bittner13CUDA.cu:674-680). Design (Adinets & Merrill 2022):
 //   1. one read of all keys builds the digit histograms of every pass;
 //   2. a tiny scan turns them into global digit offsets;
-//   3. per pass, one kernel: each CTA takes the next tile index from an atomic counter (so the
-//      tiles it looks back on are already running), ranks its 8192 keys stably (per item, the lanes
+//   3. per pass, one kernel: each CTA takes tile indices from an atomic counter until none is left (so
+//      the tiles it looks back on are already running), ranks its keys stably (per item, the lanes
 //      holding the same digit are found with 9 ballots and a warp-private counter per digit is
 //      advanced by one shared-memory atomic of the lowest such lane; the atomics of all items are
 //      issued before any result is used), publishes per-digit counts, resolves its exclusive prefix
