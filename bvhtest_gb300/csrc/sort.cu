@@ -21,6 +21,7 @@
 #include "sort.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <vector>
 
@@ -145,7 +146,7 @@ struct OnesweepSmem {
 // stage, write) are a chain of latencies with barriers between them, so a second CTA per SM is what
 // fills them: 64 registers per thread (ranks kept as 16-bit pairs, values read when the keys are out
 // of the way) and one staging buffer for keys and then values (82 KB for 8,192 64-bit keys). A pass of
-// 4.19M / 33.5M pairs of 64-bit keys: 45 / 310 us; with one CTA per SM and 124 registers 49 / 336;
+// 4.19M / 33.5M pairs of 64-bit keys in tiles of 8,192: 45 / 310 us (39.5 for 4.19M in tiles of 7,168); with one CTA per SM and 124 registers 49 / 336;
 // with the look-back before the staging 50 / 298, in the lower warps while the upper ones stage 48 /
 // 374; 32 predecessors per round trip 46 / 334; digits matched by match.any 58 / 397.
 template <typename K, int THREADS, int ITEMS>
@@ -159,7 +160,8 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
   constexpr int kWarps = Smem::kWarps, kTile = Smem::kTile;
   constexpr bool kSplit = Smem::kSplit, kLate = THREADS == 512;
   static_assert(THREADS >= kRadix, "one thread per digit in the look-back");
-  static_assert(ITEMS % 4 == 0 && kTile <= 65536, "ranks in groups of four, as 16-bit pairs");
+  constexpr int kGroup = ITEMS % 4 == 0 ? 4 : 2;  // items ranked together
+  static_assert(ITEMS % 2 == 0 && kTile <= 65536, "ranks as 16-bit pairs");
   extern __shared__ __align__(16) unsigned char smraw[];
   Smem &sm = *reinterpret_cast<Smem *>(smraw);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -183,14 +185,14 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
     }
     // Stable rank within the warp: items in order, lanes in order. Peers of an item are the lanes
     // with the same digit (8 ballots, and one for the padding bin in the last tile); the lowest of
-    // them advances the warp's counter for that digit by their number. The atomics of four items are
+    // them advances the warp's counter for that digit by their number. The atomics of a group of items are
     // issued, in item order (__syncwarp orders them), before their results are used.
     uint32_t rank[ITEMS / 2];
 #pragma unroll
-    for (int j0 = 0; j0 < ITEMS; j0 += 4) {
-      uint32_t old[4], peers[4];
+    for (int j0 = 0; j0 < ITEMS; j0 += kGroup) {
+      uint32_t old[kGroup], peers[kGroup];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < kGroup; ++q) {
         const int j = j0 + q;
         const bool in = t0 + 32 * j < valid;
         const uint32_t d = in ? (uint32_t)(key[j] >> shift) & mask : (uint32_t)kRadix;
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
         __syncwarp();
       }
 #pragma unroll
-      for (int q = 0; q < 4; q += 2) {
+      for (int q = 0; q < kGroup; q += 2) {
         const uint32_t a = __shfl_sync(0xFFFFFFFFu, old[q], __ffs(peers[q]) - 1) + __popc(peers[q] & ltMask);
         const uint32_t b = __shfl_sync(0xFFFFFFFFu, old[q + 1], __ffs(peers[q + 1]) - 1) + __popc(peers[q + 1] & ltMask);
         rank[(j0 + q) / 2] = a | (b << 16);
@@ -391,6 +393,12 @@ int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut,
     case 4096:
       return onesweep_passes<K, 256, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
                                          n, beginBit, endBit, s, gate, outLast);
+    case 6144:
+      return onesweep_passes<K, 512, 12>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
+                                         n, beginBit, endBit, s, gate, outLast);
+    case 7168:
+      return onesweep_passes<K, 512, 14>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
+                                         n, beginBit, endBit, s, gate, outLast);
     default:
       return onesweep_passes<K, 512, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
                                          n, beginBit, endBit, s, gate, outLast);
@@ -399,10 +407,28 @@ int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut,
 
 std::atomic<uint32_t> g_default_tile{kSortTileDefault};
 
-// Keys per CTA of a sort that is given none: small sorts fill few CTAs at the large tiles (30-bit pairs,
-// 2,048 / 8,192 keys: 65,536 pairs 52 / 72 us, 524,288 73 / 80, 1M 95 / 86).
+// Keys per CTA of a sort that is given none. Small sorts fill few CTAs at the large tiles (63-bit keys,
+// 2,048 / 4,096 / 8,192: 262,144 pairs 81 / 88 / 104 us, 524,288 100 / 91 / 109). From there to 8M pairs
+// the tile is the one whose SMs are done first: w tiles an SM take about (w + ceil(w)) / 2 times a tile's
+// time, which grows with its items and, for 16 of them, the registers they spill. 63-bit keys, tiles of
+// 4,096 / 6,144 / 7,168 / 8,192: 1M 122 / 124 / 114 / 121 us, 1.5M 154 / 137 / 142 / 154, 2.49M 190 / 191 /
+// 199 / 175, 4.19M 297 / 266 / 249 / 272, 8.39M 546 / 479 / 466 / 474. Beyond, where the arrays do not fit
+// L2, the longer runs of the largest tile count: 12M 895 / 768 / 757 / 720, 33.5M 2,424 / 2,067 / 1,983 / 1,852.
 uint32_t auto_tile(uint32_t n) {
-  return n <= (1u << 19) ? (uint32_t)kMinTile : g_default_tile.load(std::memory_order_relaxed);
+  const uint32_t given = g_default_tile.load(std::memory_order_relaxed);
+  if (n <= (1u << 18)) return (uint32_t)kMinTile;
+  if (given != kSortTileDefault || n > (1u << 23)) return given;
+  constexpr uint32_t shapes[4][2] = {{4096, 12}, {6144, 16}, {7168, 18}, {8192, 22}};  // keys, a tile's time
+  uint32_t best = 0;
+  float least = 0.0f;
+  for (const auto &t : shapes) {
+    const float w = (float)ceil_div(n, t[0]) / (float)sm_count(), cost = (w + std::ceil(w)) * (float)t[1];
+    if (best == 0 || cost < least) {
+      best = t[0];
+      least = cost;
+    }
+  }
+  return best;
 }
 
 // The gated sort's memset: all but the error word, which keeps what an earlier pass found.
@@ -454,7 +480,7 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
 // an earlier position, and every member counts that for itself. A mesh leaves few triangles in one
 // cell of the upper bits; a group of more than kMaxGroup raises the gate, and the full eight-pass
 // sort, whose launches otherwise return at once, makes the order instead. Measured against the eight
-// passes alone: 65,536 keys 96 us against 119, 1M 122 / 153, 4.19M 274 / 441, 33.5M 1,840 / 2,840.
+// passes alone: 65,536 keys 96 us against 119, 1M 114 / 153, 4.19M 249 / 441, 33.5M 1,840 / 2,840.
 constexpr int kGroupTile = 1024;  // keys per block, 256 threads
 constexpr int kMaxGroup = 256;
 
@@ -508,9 +534,13 @@ int sort_prepare() {
   if (ctx != 0 && std::find(done.begin(), done.end(), ctx) != done.end()) return BVHGB_OK;
   BVHGB_CUDA_TRY((set_smem_attr<uint32_t, 256, 8>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint32_t, 256, 16>()));
+  BVHGB_CUDA_TRY((set_smem_attr<uint32_t, 512, 12>()));
+  BVHGB_CUDA_TRY((set_smem_attr<uint32_t, 512, 14>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint32_t, 512, 16>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 256, 8>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 256, 16>()));
+  BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 12>()));
+  BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 14>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 16>()));
   if (ctx != 0) done.push_back(ctx);
   return BVHGB_OK;

@@ -198,7 +198,7 @@ BVHGB_API int bvhgb_select_smallest_pairs(void *temp, size_t *tempBytes, const u
 
 /* Keys per CTA of the onesweep passes (2048, 4096 or 8192) for sorts that are not given one: the
  * LBVH build's and the optimizer's selection sort, launched (or captured into a graph) after the
- * call. tileKeys = 0 only reads the setting. *previous (may be NULL) receives the old value. The
+ * call. The default, 8192, leaves the choice to the sort's size. tileKeys = 0 only reads the setting. *previous (may be NULL) receives the old value. The
  * results do not depend on it. No counterpart in the reference (cub picks its own tiles). */
 BVHGB_API int bvhgb_sort_set_default_tile(uint32_t tileKeys, uint32_t *previous);
 /* Diagnostics of the failure paths (no counterpart in the reference). bvhgb_sort_set_spin_limit:
