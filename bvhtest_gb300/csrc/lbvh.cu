@@ -32,7 +32,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t maxFaces = 0;
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
-  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate
+  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate, heavy-cell flag
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -40,6 +40,9 @@ struct bvhgb_lbvh_workspace {
   uint32_t *slots = nullptr;
   float4 *triBoxes = nullptr;  // 2 x float4 per face (mn.xyz mx.x | mx.yz 0 0); null: gather the triangle
   bool slotsArmed = false;  // slots hold kNone (set by the Morton kernel)
+  // Sampled counts of the Morton cells, 2^cellBits (63-bit keys; null: none); cleared with the scene box.
+  uint32_t *cells = nullptr;
+  uint32_t cellBits = 0;
   void *sortTemp = nullptr;
   size_t sortTempBytes = 0;
 };
@@ -57,7 +60,9 @@ __global__ void lbvh_init_kernel(uint32_t *scene) {
 
 __global__ void __launch_bounds__(kBoundsThreads) lbvh_bounds_kernel(const float *__restrict__ vert,
                                                                      const uint32_t *__restrict__ faces, uint32_t n,
-                                                                     uint32_t *scene) {
+                                                                     uint32_t *scene, uint32_t *__restrict__ cells,
+                                                                     uint32_t cellWords) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cellWords; i += gridDim.x * blockDim.x) cells[i] = 0u;
   // Starting the local box at the origin is the same as merging the reduction's initial value.
   float mn[3] = {0.0f, 0.0f, 0.0f}, mx[3] = {0.0f, 0.0f, 0.0f};
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -99,7 +104,8 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
                                                                      uint32_t *__restrict__ scene, void *keysOut,
                                                                      uint32_t *__restrict__ vals,
                                                                      uint32_t *__restrict__ slots,
-                                                                     float4 *__restrict__ boxes) {
+                                                                     float4 *__restrict__ boxes,
+                                                                     uint32_t *__restrict__ cells, uint32_t cellBits) {
   float off[3], sc[3];
   morton_params(scene, off, sc);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -107,7 +113,14 @@ __global__ void __launch_bounds__(kMortonThreads) lbvh_morton_kernel(const float
     float c[3];
     tri_box(vert, faces, (uint32_t)i, b, c);
     if (BITS == 30) static_cast<uint32_t *>(keysOut)[i] = (uint32_t)morton_key<30>(c, off, sc);
-    else static_cast<uint64_t *>(keysOut)[i] = morton_key<63>(c, off, sc);
+    else {
+      const uint64_t key = morton_key<63>(c, off, sc);
+      static_cast<uint64_t *>(keysOut)[i] = key;
+      if (cells && i % cell_sample(n) == 0) {
+        const uint64_t h = (key >> morton_cell_bit(n)) * 0x9E3779B97F4A7C15ull;
+        atomicAdd(cells + (h >> (64u - cellBits)), 1u);  // nobody waits for it
+      }
+    }
     vals[i] = (uint32_t)i;
     if (i + 1 < n) slots[i] = kNone;
     if (boxes) {
@@ -810,6 +823,11 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   if (e == cudaSuccess) e = dev_malloc(&ws->slots, 4 * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->triBoxes, 32 * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->sortTemp, ws->sortTempBytes ? ws->sortTempBytes : 256);
+  if (ws->keyBytes == 8) {  // two places a sample
+    for (ws->cellBits = 10; ws->cellBits < 22 && (1u << ws->cellBits) < maxFaces / (cell_sample(maxFaces) / 2);) ++ws->cellBits;
+    if (e == cudaSuccess) e = dev_malloc(&ws->cells, 4ull << ws->cellBits);
+    if (e == cudaSuccess) e = cudaMemset(ws->cells, 0, 4ull << ws->cellBits);
+  }
   if (e != cudaSuccess) {
     set_last_error("bvhgb_lbvh_create", e);
     bvhgb_lbvh_destroy(ws);
@@ -828,6 +846,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_destroy(bvhgb_lbvh_workspace *ws) {
   cudaFree(ws->valsSorted);
   cudaFree(ws->slots);
   cudaFree(ws->triBoxes);
+  cudaFree(ws->cells);
   cudaFree(ws->sortTemp);
   delete ws;
   return BVHGB_OK;
@@ -843,7 +862,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_init_tri_data(bvhgb_lbvh_workspace *ws, cons
   if (n == 0) return BVHGB_OK;
   if (!vert || !faces) return BVHGB_INVALID_ARGUMENT;
   uint32_t grid = min(ceil_div(n, kBoundsThreads * 4), (uint32_t)sm_count() * 8);
-  lbvh_bounds_kernel<<<grid, kBoundsThreads, 0, s>>>(vert, faces, n, ws->scene);
+  lbvh_bounds_kernel<<<grid, kBoundsThreads, 0, s>>>(vert, faces, n, ws->scene, ws->cells,
+                                                     ws->cells ? 1u << ws->cellBits : 0u);
   BVHGB_LAUNCH_CHECK("lbvh bounds");
   return BVHGB_OK;
 }
@@ -858,10 +878,10 @@ extern "C" BVHGB_API int bvhgb_lbvh_calc_morton(bvhgb_lbvh_workspace *ws, const 
   uint32_t grid = ceil_div(n, kMortonThreads * 2);
   if (ws->cfg.mortonBits == 30)
     lbvh_morton_kernel<30><<<grid, kMortonThreads, 0, s>>>(vert, faces, n, ws->scene, ws->keys, ws->vals, ws->slots,
-                                                           ws->triBoxes);
+                                                           ws->triBoxes, nullptr, 0u);
   else
     lbvh_morton_kernel<63><<<grid, kMortonThreads, 0, s>>>(vert, faces, n, ws->scene, ws->keys, ws->vals, ws->slots,
-                                                           ws->triBoxes);
+                                                           ws->triBoxes, ws->cells, ws->cellBits);
   BVHGB_LAUNCH_CHECK("lbvh morton");
   ws->slotsArmed = true;
   return BVHGB_OK;
@@ -872,7 +892,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_sort(bvhgb_lbvh_workspace *ws, uint32_t n, b
   if (st) return st;
   if (ws->keyBytes == 8) {
     return sort_morton(ws->sortTemp, static_cast<const uint64_t *>(ws->keys), static_cast<uint64_t *>(ws->keysSorted),
-                       ws->vals, ws->valsSorted, n, ws->scene + 8, as_stream(stream));
+                       ws->vals, ws->valsSorted, n, ws->scene + 8,
+                       MortonCells{ws->cells, ws->cells ? 1u << ws->cellBits : 0u, ws->cells ? ws->scene + 9 : nullptr}, as_stream(stream));
   }
   return sort_pairs(ws->sortTemp, ws->keys, ws->keysSorted, ws->vals, ws->valsSorted, n, ws->keyBytes, 0,
                     ws->cfg.mortonBits, as_stream(stream));

@@ -73,26 +73,16 @@ Layout make_layout(uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t en
   return L;
 }
 
-// A kernel given a gate word does its work only where that is not zero (null: always). The launches of a
-// gated sort start while the one before is still draining, so that a closed gate costs little.
-__device__ __forceinline__ bool gate_closed(const uint32_t *gate) {
-  if (!gate) return false;
-  grid_release();
-  grid_wait();
-  return __ldcg(gate) == 0u;
-}
+// A kernel given this word does nothing where it is set (null: it always works).
+__device__ __forceinline__ bool skipped(const uint32_t *word) { return word && __ldcg(word) != 0u; }
 
 template <typename K>
-__global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict__ keys, uint32_t n,
-                                                             uint32_t beginBit, uint32_t endBit, uint32_t passes,
-                                                             uint32_t *__restrict__ hist,
-                                                             const uint32_t *gate) {
-  if (gate_closed(gate)) return;
-  extern __shared__ uint32_t sh[];  // passes * 256
+__device__ __forceinline__ void histogram_all(const K *keys, uint32_t n, uint32_t beginBit, uint32_t endBit,
+                                              uint32_t passes, uint32_t *hist, uint32_t *sh) {  // sh: passes * 256 words
   for (uint32_t i = threadIdx.x; i < passes * kRadix; i += blockDim.x) sh[i] = 0;
   __syncthreads();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    K k = keys[i];
+    K k = __ldcg(keys + i);
     for (uint32_t p = 0; p < passes; ++p) {
       const uint32_t sh0 = beginBit + 8 * p;
       uint32_t d = (uint32_t)(k >> sh0) & digit_mask(sh0, endBit);
@@ -104,9 +94,19 @@ __global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
+template <typename K>
+__global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict__ keys, uint32_t n,
+                                                             uint32_t beginBit, uint32_t endBit, uint32_t passes,
+                                                             uint32_t *__restrict__ hist, MortonCells cells) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cells.words; i += gridDim.x * blockDim.x)
+    if (__ldg(cells.count + i) >= heavy_cell(n)) *cells.heavy = 1u;
+  extern __shared__ uint32_t histSm[];
+  histogram_all(keys, n, beginBit, endBit, passes, hist, histSm);
+}
+
 // Exclusive scan of each pass's 256 counts, in place. One CTA per pass.
-__global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint32_t *gate) {
-  if (gate_closed(gate)) return;
+__global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint32_t *skip) {
+  if (skipped(skip)) return;
   __shared__ uint32_t s[kRadix];
   uint32_t *h = hist + blockIdx.x * kRadix;
   uint32_t v = h[threadIdx.x];
@@ -149,21 +149,24 @@ struct OnesweepSmem {
 // 4.19M / 33.5M pairs of 64-bit keys in tiles of 8,192: 45 / 310 us (39.5 for 4.19M in tiles of 7,168); with one CTA per SM and 124 registers 49 / 336;
 // with the look-back before the staging 50 / 298, in the lower warps while the upper ones stage 48 /
 // 374; 32 predecessors per round trip 46 / 334; digits matched by match.any 58 / 397.
-template <typename K, int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
-    const K *__restrict__ keysIn, K *__restrict__ keysOut, const uint32_t *__restrict__ valsIn,
-    uint32_t *__restrict__ valsOut, uint32_t n, uint32_t tiles, uint32_t shift, uint32_t mask,
-    const uint32_t *__restrict__ offsets, uint32_t *tileCounter, uint32_t *status, uint32_t *err,
-    const uint32_t *gate) {
-  if (gate_closed(gate)) return;
+// FRESH: the pairs and offsets were written in this launch (the loads go past L1); otherwise by an earlier
+// one (33.5M 64-bit pairs, a pass: read-only loads 310 us, past L1 336).
+template <bool FRESH, typename T>
+__device__ __forceinline__ T load_once(const T *p) {
+  return FRESH ? __ldcg(p) : __ldg(p);
+}
+
+template <typename K, int THREADS, int ITEMS, bool FRESH>
+__device__ __forceinline__ void onesweep_tiles(OnesweepSmem<K, THREADS, ITEMS> &sm, const K *keysIn, K *keysOut,
+                                               const uint32_t *valsIn, uint32_t *valsOut, uint32_t n, uint32_t tiles,
+                                               uint32_t shift, uint32_t mask, const uint32_t *offsets,
+                                               uint32_t *tileCounter, uint32_t *status, uint32_t *err) {
   using Smem = OnesweepSmem<K, THREADS, ITEMS>;
   constexpr int kWarps = Smem::kWarps, kTile = Smem::kTile;
   constexpr bool kSplit = Smem::kSplit, kLate = THREADS == 512;
   static_assert(THREADS >= kRadix, "one thread per digit in the look-back");
   constexpr int kGroup = ITEMS % 4 == 0 ? 4 : 2;  // items ranked together
   static_assert(ITEMS % 2 == 0 && kTile <= 65536, "ranks as 16-bit pairs");
-  extern __shared__ __align__(16) unsigned char smraw[];
-  Smem &sm = *reinterpret_cast<Smem *>(smraw);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t ltMask = (1u << lane) - 1u;
   if (threadIdx.x == 0) sm.tileIdx = atomicAdd(tileCounter, 1u);
@@ -180,8 +183,8 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
     uint32_t val[ITEMS];
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-      key[j] = t0 + 32 * j < valid ? keysIn[base + t0 + 32 * j] : (K)0;
-      if (!kSplit) val[j] = t0 + 32 * j < valid ? valsIn[base + t0 + 32 * j] : 0u;
+      key[j] = t0 + 32 * j < valid ? load_once<FRESH>(keysIn + base + t0 + 32 * j) : (K)0;
+      if (!kSplit) val[j] = t0 + 32 * j < valid ? load_once<FRESH>(valsIn + base + t0 + 32 * j) : 0u;
     }
     // Stable rank within the warp: items in order, lanes in order. Peers of an item are the lanes
     // with the same digit (8 ballots, and one for the padding bin in the last tile); the lowest of
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
         }
         st_relaxed(status + (size_t)tile * kRadix + d, kFlagInc | (excl + count));
       }
-      sm.globalBase[d] = offsets[d] + excl;
+      sm.globalBase[d] = load_once<FRESH>(offsets + d) + excl;
     };
     uint32_t count = 0, incl = 0;
     if (threadIdx.x < kRadix) {
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
     if (more && threadIdx.x == THREADS - 1) sm.tileIdx = atomicAdd(tileCounter, 1u);
     if (kSplit) {
 #pragma unroll
-      for (int j = 0; j < ITEMS; ++j) val[j] = t0 + 32 * j < valid ? valsIn[base + t0 + 32 * j] : 0u;
+      for (int j = 0; j < ITEMS; ++j) val[j] = t0 + 32 * j < valid ? load_once<FRESH>(valsIn + base + t0 + 32 * j) : 0u;
     }
     __syncthreads();
     uint32_t dst[ITEMS];
@@ -348,12 +351,24 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
   }
 }
 
+template <typename K, int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
+    const K *__restrict__ keysIn, K *__restrict__ keysOut, const uint32_t *__restrict__ valsIn,
+    uint32_t *__restrict__ valsOut, uint32_t n, uint32_t tiles, uint32_t shift, uint32_t mask,
+    const uint32_t *__restrict__ offsets, uint32_t *tileCounter, uint32_t *status, uint32_t *err,
+    const uint32_t *skip) {
+  if (skipped(skip)) return;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  onesweep_tiles<K, THREADS, ITEMS, false>(*reinterpret_cast<OnesweepSmem<K, THREADS, ITEMS> *>(smraw), keysIn, keysOut, valsIn,
+                                    valsOut, n, tiles, shift, mask, offsets, tileCounter, status, err);
+}
+
 // The passes over bits [beginBit, endBit) between the out and alternate arrays, the last one into the out
 // arrays (outLast) or into the alternate ones.
 template <typename K, int THREADS, int ITEMS>
 int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t *valsIn, uint32_t *valsOut, K *altK,
                     uint32_t *altV, uint32_t *hist, uint32_t *counters, uint32_t *status, uint32_t *err, uint32_t n,
-                    uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate, bool outLast) {
+                    uint32_t beginBit, uint32_t endBit, cudaStream_t s, bool outLast, const uint32_t *skip) {
   const size_t smem = sizeof(OnesweepSmem<K, THREADS, ITEMS>);
   const uint32_t grid = min(L.tiles, (uint32_t)(sm_count() * kSortCtas<ITEMS>));
   const K *srcK = keysIn;
@@ -363,9 +378,9 @@ int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t
     K *dstK = toOut ? keysOut : altK;
     uint32_t *dstV = toOut ? valsOut : altV;
     const uint32_t shift = beginBit + 8 * p;
-    launch_kernel(onesweep_kernel<K, THREADS, ITEMS>, grid, THREADS, smem, s, gate != nullptr, srcK, dstK, srcV, dstV, n,
-                  L.tiles, shift, digit_mask(shift, endBit), hist + p * kRadix, counters + p,
-                  status + (size_t)p * L.tiles * kRadix, err, gate);
+    onesweep_kernel<K, THREADS, ITEMS><<<grid, THREADS, smem, s>>>(
+        srcK, dstK, srcV, dstV, n, L.tiles, shift, digit_mask(shift, endBit), hist + p * kRadix, counters + p,
+        status + (size_t)p * L.tiles * kRadix, err, skip);
     BVHGB_LAUNCH_CHECK("radix onesweep");
     srcK = dstK;
     srcV = dstV;
@@ -377,31 +392,30 @@ int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t
 template <typename K>
 int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn,
                 uint32_t *valsOut, K *altK, uint32_t *altV, uint32_t *hist, uint32_t *counters, uint32_t *status,
-                uint32_t *err, uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate,
-                bool outLast) {
+                uint32_t *err, uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s, bool outLast,
+                const MortonCells &cells = {}) {
   const uint32_t hgrid = min(ceil_div(n, kThreads * 8), (uint32_t)sm_count() * 4);
-  const bool early = gate != nullptr;
-  launch_kernel(histogram_kernel<K>, hgrid, kThreads, sizeof(uint32_t) * kRadix * L.passes, s, early, keysIn, n,
-                beginBit, endBit, L.passes, hist, gate);
+  histogram_kernel<K><<<hgrid, kThreads, sizeof(uint32_t) * kRadix * L.passes, s>>>(keysIn, n, beginBit, endBit,
+                                                                                    L.passes, hist, cells);
   BVHGB_LAUNCH_CHECK("radix histogram");
-  launch_kernel(scan_kernel, L.passes, kRadix, 0, s, early, hist, gate);
+  scan_kernel<<<L.passes, kRadix, 0, s>>>(hist, cells.heavy);
   BVHGB_LAUNCH_CHECK("radix scan");
   switch (tileKeys) {
     case 2048:
       return onesweep_passes<K, 256, 8>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
-                                        beginBit, endBit, s, gate, outLast);
+                                        beginBit, endBit, s, outLast, cells.heavy);
     case 4096:
       return onesweep_passes<K, 256, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s, gate, outLast);
+                                         n, beginBit, endBit, s, outLast, cells.heavy);
     case 6144:
       return onesweep_passes<K, 512, 12>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s, gate, outLast);
+                                         n, beginBit, endBit, s, outLast, cells.heavy);
     case 7168:
       return onesweep_passes<K, 512, 14>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s, gate, outLast);
+                                         n, beginBit, endBit, s, outLast, cells.heavy);
     default:
       return onesweep_passes<K, 512, 16>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err,
-                                         n, beginBit, endBit, s, gate, outLast);
+                                         n, beginBit, endBit, s, outLast, cells.heavy);
   }
 }
 
@@ -431,16 +445,9 @@ uint32_t auto_tile(uint32_t n) {
   return best;
 }
 
-// The gated sort's memset: all but the error word, which keeps what an earlier pass found.
-__global__ void clear_kernel(uint32_t *p, uint32_t words, const uint32_t *err, const uint32_t *gate) {
-  if (gate_closed(gate)) return;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x)
-    if (p + i != err) p[i] = 0u;
-}
-
 template <typename K>
 int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-              uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s, const uint32_t *gate = nullptr) {
+              uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s) {
   if (tileKeys == 0) tileKeys = auto_tile(n);
   const Layout L = make_layout(n, sizeof(K), beginBit, endBit, tileKeys);
   const Layout Lmax = make_layout(n, sizeof(K), beginBit, endBit, kMinTile);  // the temp space's layout
@@ -459,17 +466,11 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
   }
   // hist, counters, err and the status words this tile size uses start at zero
   const size_t zeroed = Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes;
-  if (gate) {
-    launch_kernel(clear_kernel, min(ceil_div(zeroed, 4096), (uint32_t)sm_count() * 4), 256, 0, s, true,
-                  reinterpret_cast<uint32_t *>(t), (uint32_t)(zeroed / 4), err, gate);
-    BVHGB_LAUNCH_CHECK("radix clear");
-  } else {
-    BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, zeroed, s));
-  }
+  BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, zeroed, s));
   int st = sort_prepare();
   if (st) return st;
   return sort_passes<K>(L, tileKeys, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
-                        beginBit, endBit, s, gate, true);
+                        beginBit, endBit, s, true);
 }
 
 // ---- 63-bit Morton keys -----------------------------------------------------------------------------
@@ -481,13 +482,20 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
 // cell of the upper bits; a group of more than kMaxGroup raises the gate, and the full eight-pass
 // sort, whose launches otherwise return at once, makes the order instead. Measured against the eight
 // passes alone: 65,536 keys 96 us against 119, 1M 114 / 153, 4.19M 249 / 441, 33.5M 1,840 / 2,840.
+//
+// Where a cell is that full (a detailed object in a large scene), the passes over the upper bits would be
+// for nothing, so the kernel that makes the keys samples its cells (MortonCells) and a full one sends all keys to
+// the full sort at once. With a quarter of the triangles in one cell, before / sampled / the eight passes as
+// they were: 65,536 keys 182 / 110 / 127 us, 1M 317 / 180 / 154, 4.19M 687 / 435 / 445, 16.8M 2,647 / 1,531 / 1,471.
 constexpr int kGroupTile = 1024;  // keys per block, 256 threads
 constexpr int kMaxGroup = 256;
 
 __global__ void __launch_bounds__(256) order_groups_kernel(const uint64_t *__restrict__ keys,
                                                            const uint32_t *__restrict__ vals, uint32_t n,
                                                            uint32_t beginBit, uint64_t *__restrict__ keysOut,
-                                                           uint32_t *__restrict__ valsOut, uint32_t *gate) {
+                                                           uint32_t *__restrict__ valsOut, uint32_t *gate,
+                                                           const uint32_t *skip) {
+  if (skipped(skip)) return;
   constexpr int kSpan = kGroupTile + kMaxGroup;
   __shared__ uint64_t key[kSpan + 1];  // [e + 1]: the tile's keys and the halo behind it; [0]: the key before the tile
   const uint32_t base = blockIdx.x * kGroupTile;
@@ -513,6 +521,103 @@ __global__ void __launch_bounds__(256) order_groups_kernel(const uint64_t *__res
     keysOut[base + at] = mine;
     valsOut[base + at] = __ldg(vals + base + e);
   }
+}
+
+// The full sort of 63-bit keys behind the gate: every step in one cooperative launch, which returns at
+// once where the gate is closed (a chain of ten launches that did so took 22 us of a 4.19M build, this
+// one 2.5). The blocks, all resident, meet at bounded barriers between the steps.
+struct FullSort {
+  const uint64_t *keysIn;
+  const uint32_t *valsIn;
+  uint64_t *keysOut, *altK;
+  uint32_t *valsOut, *altV, *words, *hist, *counters, *status, *err, *barrier;
+  uint32_t n, tiles, passes, zeroed;  // words[0, zeroed) are cleared, but for the error and barrier words
+  const uint32_t *gate, *heavy;
+};
+
+__device__ __forceinline__ bool grid_barrier(const FullSort &f, uint32_t target) {
+  int ok = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(f.barrier, 1u);
+    for (uint32_t spins = 0; ld_relaxed(f.barrier) < target; ++spins) {
+      if (spins > kSpinLimit) {
+        atomicOr(f.err, kErrTimeout);
+        ok = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    __threadfence();
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) full_sort_kernel(const __grid_constant__ FullSort f) {
+  if (__ldcg(f.gate) == 0u && !skipped(f.heavy)) return;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  auto &sm = *reinterpret_cast<OnesweepSmem<uint64_t, THREADS, ITEMS> *>(smraw);
+  uint32_t *sh = reinterpret_cast<uint32_t *>(smraw);
+  static_assert(sizeof(sm) >= 8 * kRadix * sizeof(uint32_t), "room for the histograms of eight passes");
+  uint32_t met = 0;
+  for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < f.zeroed; i += gridDim.x * THREADS)
+    if (f.words + i != f.err && f.words + i != f.barrier) f.words[i] = 0u;
+  if (!grid_barrier(f, met += gridDim.x)) return;
+  histogram_all(f.keysIn, f.n, 0u, 63u, f.passes, f.hist, sh);
+  if (!grid_barrier(f, met += gridDim.x)) return;
+  // Exclusive scans, a pass per block (or more): one warp, eight digits a lane.
+  for (uint32_t p = blockIdx.x; p < f.passes && threadIdx.x < 32u; p += gridDim.x) {
+    uint32_t v[kRadix / 32], sum = 0;
+#pragma unroll
+    for (int q = 0; q < kRadix / 32; ++q) sum += v[q] = __ldcg(f.hist + p * kRadix + threadIdx.x * (kRadix / 32) + q);
+    uint32_t at = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o);
+      if (threadIdx.x >= (uint32_t)o) at += y;
+    }
+    at -= sum;
+#pragma unroll
+    for (int q = 0; q < kRadix / 32; ++q) {
+      f.hist[p * kRadix + threadIdx.x * (kRadix / 32) + q] = at;
+      at += v[q];
+    }
+  }
+  const uint64_t *srcK = f.keysIn;
+  const uint32_t *srcV = f.valsIn;
+  for (uint32_t p = 0; p < f.passes; ++p) {
+    if (!grid_barrier(f, met += gridDim.x)) return;
+    const bool toOut = (f.passes - 1 - p) % 2 == 0;
+    uint64_t *dstK = toOut ? f.keysOut : f.altK;
+    uint32_t *dstV = toOut ? f.valsOut : f.altV;
+    onesweep_tiles<uint64_t, THREADS, ITEMS, true>(sm, srcK, dstK, srcV, dstV, f.n, f.tiles, 8 * p, digit_mask(8 * p, 63u),
+                                             f.hist + p * kRadix, f.counters + p,
+                                             f.status + (size_t)p * f.tiles * kRadix, f.err);
+    srcK = dstK;
+    srcV = dstV;
+  }
+}
+
+template <int THREADS, int ITEMS>
+int launch_full_sort(const FullSort &f, cudaStream_t s) {
+  int perSm = 0;
+  const size_t smem = sizeof(OnesweepSmem<uint64_t, THREADS, ITEMS>);
+  BVHGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, full_sort_kernel<THREADS, ITEMS>, THREADS, smem));
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min(f.tiles, (uint32_t)(perSm * sm_count())));
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  BVHGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, full_sort_kernel<THREADS, ITEMS>, f));
+  BVHGB_LAUNCH_CHECK("full sort");
+  return BVHGB_OK;
 }
 
 template <typename K, int THREADS, int ITEMS>
@@ -542,6 +647,10 @@ int sort_prepare() {
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 12>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 14>()));
   BVHGB_CUDA_TRY((set_smem_attr<uint64_t, 512, 16>()));
+  BVHGB_CUDA_TRY(cudaFuncSetAttribute(full_sort_kernel<256, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(OnesweepSmem<uint64_t, 256, 8>)));
+  BVHGB_CUDA_TRY(cudaFuncSetAttribute(full_sort_kernel<512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(OnesweepSmem<uint64_t, 512, 16>)));
   if (ctx != 0) done.push_back(ctx);
   return BVHGB_OK;
 }
@@ -567,13 +676,11 @@ uint32_t *sort_error_word(void *temp, uint32_t n, uint32_t keyBytes, uint32_t be
 }
 
 int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-                uint32_t n, uint32_t *gate, cudaStream_t s) {
+                uint32_t n, uint32_t *gate, const MortonCells &cells, cudaStream_t s) {
   int st = sort_prepare();
   if (st) return st;
   if (n == 0) return BVHGB_OK;
-  // 2^32 cells for up to 8M triangles, 2^40 for more: the densest cells of the benchmark scenes then hold
-  // a few dozen (33.5M triangles in 64 clusters put over 256 into some of 2^32 cells).
-  const uint32_t beginBit = n <= (1u << 23) ? 31u : 23u;
+  const uint32_t beginBit = morton_cell_bit(n);
   const uint32_t tileKeys = auto_tile(n);
   const Layout L = make_layout(n, 8, beginBit, 63, tileKeys);
   const Layout Lmax = make_layout(n, 8, 0, 63, kMinTile);  // the temp space's layout
@@ -585,13 +692,20 @@ int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uin
   uint64_t *altK = reinterpret_cast<uint64_t *>(t + Lmax.altKeys);
   uint32_t *altV = reinterpret_cast<uint32_t *>(t + Lmax.altVals);
   BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes, s));
-  BVHGB_CUDA_TRY(cudaMemsetAsync(gate, 0, 4, s));
+  BVHGB_CUDA_TRY(cudaMemsetAsync(gate, 0, 8, s));  // and the flag behind it
   st = sort_passes<uint64_t>(L, tileKeys, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
-                             beginBit, 63, s, nullptr, false);
+                             beginBit, 63, s, false, cells);
   if (st) return st;
-  order_groups_kernel<<<ceil_div(n, kGroupTile), 256, 0, s>>>(altK, altV, n, beginBit, keysOut, valsOut, gate);
+  order_groups_kernel<<<ceil_div(n, kGroupTile), 256, 0, s>>>(altK, altV, n, beginBit, keysOut, valsOut, gate,
+                                                                    cells.heavy);
   BVHGB_LAUNCH_CHECK("order groups");
-  return sort_impl<uint64_t>(temp, tileKeys, keysIn, keysOut, valsIn, valsOut, n, 0, 63, s, gate);
+  // The full sort, in small tiles or in large ones.
+  const bool small = tileKeys == (uint32_t)kMinTile;
+  const Layout F = make_layout(n, 8, 0, 63, small ? kMinTile : 8192);
+  const FullSort f{keysIn, valsIn, keysOut, altK, valsOut, altV, reinterpret_cast<uint32_t *>(t), hist, counters, status,
+                   err, err + 1, n, F.tiles, F.passes,
+                   (uint32_t)(Lmax.status / 4 + kRadix * (size_t)F.tiles * F.passes), gate, cells.heavy};
+  return small ? launch_full_sort<256, 8>(f, s) : launch_full_sort<512, 16>(f, s);
 }
 
 void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit) {

@@ -19,10 +19,22 @@ constexpr uint32_t kSortTileDefault = 8192;
 bool sort_tile_valid(uint32_t tileKeys);
 // Polls of an unpublished predecessor before a look-back gives up (0xFFFFFFFF: the default).
 int sort_set_spin_limit(uint32_t limit, uint32_t *previous);
+// The lowest bit of a Morton cell: 2^32 cells for up to 8M triangles, 2^40 for more (the densest cells of the
+// benchmark scenes then hold a few dozen; 33.5M triangles in 64 clusters put over 256 into some of 2^32).
+__host__ __device__ constexpr uint32_t morton_cell_bit(uint32_t n) { return n <= (1u << 23) ? 31u : 23u; }
+// A hashed table that the kernel making the keys counts every cell_sample(n)-th one's cell in. The sort raises
+// *heavy where a count is heavy_cell(n) or more (groups of about 320, 448 and 640 keys). Null and 0: none.
+__host__ __device__ constexpr uint32_t cell_sample(uint32_t n) { return n <= (1u << 20) ? 16u : n <= (1u << 23) ? 32u : 64u; }
+__host__ __device__ constexpr uint32_t heavy_cell(uint32_t n) { return n <= (1u << 20) ? 20u : n <= (1u << 23) ? 14u : 10u; }
+struct MortonCells {
+  const uint32_t *count = nullptr;
+  uint32_t words = 0;
+  uint32_t *heavy = nullptr;
+};
 // The stable ascending sort of n 63-bit Morton keys; temp as for sort_pairs on bits [0, 63). *gate (device)
-// tells afterwards whether the full sort had to run.
+// tells afterwards whether a group of equal upper bits was too long; cells.heavy, if any, is the word behind it.
 int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-                uint32_t n, uint32_t *gate, cudaStream_t s);
+                uint32_t n, uint32_t *gate, const MortonCells &cells, cudaStream_t s);
 // The sort's alternate buffers, (keyBytes + 4) * n bytes of the temp space that hold nothing between sorts.
 void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit);
 int sort_pairs(void *temp, const void *keysIn, void *keysOut, const uint32_t *valsIn, uint32_t *valsOut, uint32_t n,

@@ -73,3 +73,27 @@ def test_many_keys(gpu):
     p = torch.rand((n, 1, 3), generator=g, device="cuda")
     p[: n // 2] = p[: n // 2] * 0.01
     _check(gpu, p.expand(n, 3, 3).cpu().numpy())
+
+
+@pytest.mark.parametrize("n", [1025, 5000, 262144, 1100000])
+@pytest.mark.parametrize("full", [0.02, 0.5])
+def test_full_cells(gpu, n, full):
+    """A part of the triangles in one cell of the upper bits: the sort of all bits at once, and again from the
+    same keys; then an even mesh in the same workspace, whose cells are counted afresh."""
+    import torch
+    b = gpu.LBVH(n, 63, "karras")
+    for part in (full, 0.0):
+        g = np.random.default_rng(n)
+        p = g.random((n, 1, 3))
+        p[:int(part * n)] = 0.3 + 1e-4 * p[:int(part * n)]
+        v = torch.from_numpy(np.repeat(p, 3, 1).reshape(-1, 3).astype(np.float32)).cuda()
+        f = torch.arange(3 * n, dtype=torch.int32, device="cuda").reshape(-1, 3)
+        b.init_tri_data(v, f)
+        b.calc_morton(v, f)
+        keys, _ = b.keys(n, False)
+        order = np.argsort(keys, kind="stable")
+        for _ in range(2):
+            b.sort(n)
+            k, i = b.keys(n, True)
+            assert np.array_equal(k, keys[order]) and np.array_equal(i, order.astype(np.uint32))
+    assert b.errors() == 0
