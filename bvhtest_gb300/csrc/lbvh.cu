@@ -816,6 +816,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   ws->sortTempBytes = sort_temp_bytes(maxFaces, ws->keyBytes, 0, c.mortonBits);
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = dev_malloc(&ws->scene, 256);
+  if (e == cudaSuccess) e = cudaMemset(ws->scene, 0, 256);
   if (e == cudaSuccess) e = dev_malloc(&ws->keys, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->keysSorted, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->vals, 4 * m);

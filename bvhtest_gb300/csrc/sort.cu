@@ -3,15 +3,14 @@
 // Replaces cub::DeviceRadixSort::SortPairs (lib/builder/LBVH_CUDA.cu:185-193) and
 // SortPairsDescending (lib/builder/Bittner13CUDA.cu:674-680). Design (Adinets & Merrill 2022):
 //   1. one read of all keys builds the digit histograms of every pass;
-//   2. a tiny scan turns them into global digit offsets;
-//   3. per pass, one kernel: each CTA takes tile indices from an atomic counter until none is left (so
-//      the tiles it looks back on are already running), ranks its keys stably (per item, the lanes
-//      holding the same digit are found with 9 ballots and a warp-private counter per digit is
-//      advanced by one shared-memory atomic of the lowest such lane; the atomics of all items are
-//      issued before any result is used), publishes per-digit counts, resolves its exclusive prefix
-//      by decoupled look-back (kLook predecessors per round trip, bounded spin), stages the tile in
-//      shared memory in digit order and writes it out in runs, so each digit's run is a contiguous
-//      store.
+//   2. per pass, one kernel: each CTA makes the digits' global offsets from the pass's histogram (a tiny
+//      scan launch does for the large tiles) and takes tile indices from an atomic counter until none is left (so the tiles it looks back on are
+//      already running). It ranks a tile's keys stably (per item, the lanes holding the same digit are
+//      found with 9 ballots and a warp-private counter per digit is advanced by one shared-memory
+//      atomic of the lowest such lane; the atomics of all items are issued before any result is
+//      used), publishes per-digit counts, resolves its exclusive prefix by decoupled look-back (kLook
+//      predecessors per round trip, bounded spin), stages the tile in shared memory in digit order and
+//      writes it out in runs, so each digit's run is a contiguous store.
 // A status word holds a flag and a count together and nothing else is read through it, so it is
 // published and polled with relaxed gpu-scope accesses (no fences); the next pass reads the keys
 // this pass wrote only after the kernel boundary.
@@ -104,7 +103,9 @@ __global__ void __launch_bounds__(kThreads) histogram_kernel(const K *__restrict
   histogram_all(keys, n, beginBit, endBit, passes, hist, histSm);
 }
 
-// Exclusive scan of each pass's 256 counts, in place. One CTA per pass.
+// Exclusive scan of each pass's 256 counts, in place. One CTA per pass. For the tile shapes whose CTAs do not
+// scan their pass's counts themselves: the large ones, which have no registers to spare for it (a pass of
+// 4.19M pairs 39 us, 41 so; the launch saved is worth 2 us of a small sort).
 __global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint32_t *skip) {
   if (skipped(skip)) return;
   __shared__ uint32_t s[kRadix];
@@ -122,6 +123,9 @@ __global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint
 }
 
 // CTAs per SM of a tile shape.
+template <int THREADS>
+constexpr bool kScans = THREADS == 256;  // the CTAs scan their pass's counts themselves
+
 template <int ITEMS>
 constexpr int kSortCtas = ITEMS <= 8 ? 3 : 2;
 
@@ -132,6 +136,7 @@ struct OnesweepSmem {
   uint32_t warpHist[kWarps][kBins];
   uint32_t tileStart[kRadix];
   uint32_t globalBase[kRadix];
+  uint32_t digitBase[kScans<THREADS> ? kRadix : 1], digitTot[kRadix / 32];  // keys of lower digits in the same 32, and of each 32
   uint32_t scanTot[kRadix / 32];
   uint32_t tileIdx;
   // The tile in digit order; its values beside the keys or, where two CTAs would not fit then, in their
@@ -159,7 +164,7 @@ __device__ __forceinline__ T load_once(const T *p) {
 template <typename K, int THREADS, int ITEMS, bool FRESH>
 __device__ __forceinline__ void onesweep_tiles(OnesweepSmem<K, THREADS, ITEMS> &sm, const K *keysIn, K *keysOut,
                                                const uint32_t *valsIn, uint32_t *valsOut, uint32_t n, uint32_t tiles,
-                                               uint32_t shift, uint32_t mask, const uint32_t *offsets,
+                                               uint32_t shift, uint32_t mask, const uint32_t *hist,
                                                uint32_t *tileCounter, uint32_t *status, uint32_t *err) {
   using Smem = OnesweepSmem<K, THREADS, ITEMS>;
   constexpr int kWarps = Smem::kWarps, kTile = Smem::kTile;
@@ -170,6 +175,17 @@ __device__ __forceinline__ void onesweep_tiles(OnesweepSmem<K, THREADS, ITEMS> &
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t ltMask = (1u << lane) - 1u;
   if (threadIdx.x == 0) sm.tileIdx = atomicAdd(tileCounter, 1u);
+  if (kScans<THREADS> && threadIdx.x < kRadix) {  // where each digit's keys begin, from the pass's histogram
+    const uint32_t v = load_once<FRESH>(hist + threadIdx.x);
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    sm.digitBase[threadIdx.x] = incl - v;
+    if (lane == 31) sm.digitTot[warp] = incl;
+  }
   for (;;) {
     for (uint32_t i = lane; i < kBins; i += 32) sm.warpHist[warp][i] = 0;
     __syncthreads();
@@ -266,7 +282,14 @@ __device__ __forceinline__ void onesweep_tiles(OnesweepSmem<K, THREADS, ITEMS> &
         }
         st_relaxed(status + (size_t)tile * kRadix + d, kFlagInc | (excl + count));
       }
-      sm.globalBase[d] = load_once<FRESH>(offsets + d) + excl;
+      if (kScans<THREADS>) {
+        excl += sm.digitBase[d];
+#pragma unroll
+        for (uint32_t w = 0; w < kRadix / 32; ++w) excl += w < d / 32 ? sm.digitTot[w] : 0u;
+        sm.globalBase[d] = excl;
+      } else {
+        sm.globalBase[d] = load_once<FRESH>(hist + d) + excl;
+      }
     };
     uint32_t count = 0, incl = 0;
     if (threadIdx.x < kRadix) {
@@ -355,12 +378,12 @@ template <typename K, int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) onesweep_kernel(
     const K *__restrict__ keysIn, K *__restrict__ keysOut, const uint32_t *__restrict__ valsIn,
     uint32_t *__restrict__ valsOut, uint32_t n, uint32_t tiles, uint32_t shift, uint32_t mask,
-    const uint32_t *__restrict__ offsets, uint32_t *tileCounter, uint32_t *status, uint32_t *err,
+    const uint32_t *__restrict__ hist, uint32_t *tileCounter, uint32_t *status, uint32_t *err,
     const uint32_t *skip) {
   if (skipped(skip)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   onesweep_tiles<K, THREADS, ITEMS, false>(*reinterpret_cast<OnesweepSmem<K, THREADS, ITEMS> *>(smraw), keysIn, keysOut, valsIn,
-                                    valsOut, n, tiles, shift, mask, offsets, tileCounter, status, err);
+                                    valsOut, n, tiles, shift, mask, hist, tileCounter, status, err);
 }
 
 // The passes over bits [beginBit, endBit) between the out and alternate arrays, the last one into the out
@@ -388,7 +411,7 @@ int onesweep_passes(const Layout &L, const K *keysIn, K *keysOut, const uint32_t
   return BVHGB_OK;
 }
 
-// Histogram, scan and passes; hist, counters, err and status start at zero.
+// Histogram and passes; hist, counters, err and status start at zero.
 template <typename K>
 int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn,
                 uint32_t *valsOut, K *altK, uint32_t *altV, uint32_t *hist, uint32_t *counters, uint32_t *status,
@@ -398,8 +421,10 @@ int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut,
   histogram_kernel<K><<<hgrid, kThreads, sizeof(uint32_t) * kRadix * L.passes, s>>>(keysIn, n, beginBit, endBit,
                                                                                     L.passes, hist, cells);
   BVHGB_LAUNCH_CHECK("radix histogram");
-  scan_kernel<<<L.passes, kRadix, 0, s>>>(hist, cells.heavy);
-  BVHGB_LAUNCH_CHECK("radix scan");
+  if (tileKeys > 4096) {  // the shapes of 512 threads
+    scan_kernel<<<L.passes, kRadix, 0, s>>>(hist, cells.heavy);
+    BVHGB_LAUNCH_CHECK("radix scan");
+  }
   switch (tileKeys) {
     case 2048:
       return onesweep_passes<K, 256, 8>(L, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
@@ -532,7 +557,7 @@ struct FullSort {
   uint64_t *keysOut, *altK;
   uint32_t *valsOut, *altV, *words, *hist, *counters, *status, *err, *barrier;
   uint32_t n, tiles, passes, zeroed;  // words[0, zeroed) are cleared, but for the error and barrier words
-  const uint32_t *gate, *heavy;
+  uint32_t *gate, *heavy;  // both 0 between sorts
 };
 
 __device__ __forceinline__ bool grid_barrier(const FullSort &f, uint32_t target) {
@@ -565,24 +590,30 @@ __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) full_sort_kernel(co
   for (uint32_t i = blockIdx.x * THREADS + threadIdx.x; i < f.zeroed; i += gridDim.x * THREADS)
     if (f.words + i != f.err && f.words + i != f.barrier) f.words[i] = 0u;
   if (!grid_barrier(f, met += gridDim.x)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // every block has read them: closed for the next sort
+    *f.gate = 0u;
+    if (f.heavy) *f.heavy = 0u;
+  }
   histogram_all(f.keysIn, f.n, 0u, 63u, f.passes, f.hist, sh);
-  if (!grid_barrier(f, met += gridDim.x)) return;
-  // Exclusive scans, a pass per block (or more): one warp, eight digits a lane.
-  for (uint32_t p = blockIdx.x; p < f.passes && threadIdx.x < 32u; p += gridDim.x) {
-    uint32_t v[kRadix / 32], sum = 0;
+  if constexpr (!kScans<THREADS>) {
+    if (!grid_barrier(f, met += gridDim.x)) return;
+    // Exclusive scans, a pass per block (or more): one warp, eight digits a lane.
+    for (uint32_t p = blockIdx.x; p < f.passes && threadIdx.x < 32u; p += gridDim.x) {
+      uint32_t v[kRadix / 32], sum = 0;
 #pragma unroll
-    for (int q = 0; q < kRadix / 32; ++q) sum += v[q] = __ldcg(f.hist + p * kRadix + threadIdx.x * (kRadix / 32) + q);
-    uint32_t at = sum;
+      for (int q = 0; q < kRadix / 32; ++q) sum += v[q] = __ldcg(f.hist + p * kRadix + threadIdx.x * (kRadix / 32) + q);
+      uint32_t at = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o);
-      if (threadIdx.x >= (uint32_t)o) at += y;
-    }
-    at -= sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o);
+        if (threadIdx.x >= (uint32_t)o) at += y;
+      }
+      at -= sum;
 #pragma unroll
-    for (int q = 0; q < kRadix / 32; ++q) {
-      f.hist[p * kRadix + threadIdx.x * (kRadix / 32) + q] = at;
-      at += v[q];
+      for (int q = 0; q < kRadix / 32; ++q) {
+        f.hist[p * kRadix + threadIdx.x * (kRadix / 32) + q] = at;
+        at += v[q];
+      }
     }
   }
   const uint64_t *srcK = f.keysIn;
@@ -692,7 +723,6 @@ int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uin
   uint64_t *altK = reinterpret_cast<uint64_t *>(t + Lmax.altKeys);
   uint32_t *altV = reinterpret_cast<uint32_t *>(t + Lmax.altVals);
   BVHGB_CUDA_TRY(cudaMemsetAsync(t, 0, Lmax.status + sizeof(uint32_t) * kRadix * (size_t)L.tiles * L.passes, s));
-  BVHGB_CUDA_TRY(cudaMemsetAsync(gate, 0, 8, s));  // and the flag behind it
   st = sort_passes<uint64_t>(L, tileKeys, keysIn, keysOut, valsIn, valsOut, altK, altV, hist, counters, status, err, n,
                              beginBit, 63, s, false, cells);
   if (st) return st;

@@ -31,8 +31,8 @@ struct MortonCells {
   uint32_t words = 0;
   uint32_t *heavy = nullptr;
 };
-// The stable ascending sort of n 63-bit Morton keys; temp as for sort_pairs on bits [0, 63). *gate (device)
-// tells afterwards whether a group of equal upper bits was too long; cells.heavy, if any, is the word behind it.
+// The stable ascending sort of n 63-bit Morton keys; temp as for sort_pairs on bits [0, 63). *gate
+// and *cells.heavy (device) are 0 before and after.
 int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
                 uint32_t n, uint32_t *gate, const MortonCells &cells, cudaStream_t s);
 // The sort's alternate buffers, (keyBytes + 4) * n bytes of the temp space that hold nothing between sorts.
