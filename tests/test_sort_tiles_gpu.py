@@ -1,5 +1,5 @@
 """The tile that a sort picks by its size (2,048 to 8,192 keys, for whole and ragged last tiles): keys and
-values against a stable sort."""
+values against a stable sort; and a few keys, which are placed by counting."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -19,3 +19,24 @@ def test_stable_order(gpu, n, bytes_):
     ref, order = torch.sort(keys, stable=True)
     assert torch.equal(k, ref)
     assert torch.equal(v, order.to(torch.int32))
+
+
+@pytest.mark.parametrize("bytes_", [4, 8])
+@pytest.mark.parametrize("bits", [(0, None), (8, 20), (3, 4)])
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 255, 500, 1025, 4095, 4096, 4097])
+def test_few_keys(gpu, n, bits, bytes_):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    dtype = torch.int32 if bytes_ == 4 else torch.int64
+    keys = torch.randint(0, 2 ** 31 - 1, (n,), generator=g, device="cuda", dtype=dtype)
+    keys[n // 3:n // 2] = -1  # the highest key
+    vals = torch.randint(0, 2 ** 31 - 1, (n,), generator=g, device="cuda", dtype=torch.int32)
+    k, v = gpu.radix_sort_pairs(keys, vals, *bits)
+    end = 8 * bytes_ if bits[1] is None else bits[1]
+    digits = (keys.to(torch.int64) & 0xFFFFFFFF if bytes_ == 4 else keys) >> bits[0] & 2 ** min(end - bits[0], 62) - 1
+    if bytes_ == 8 and bits[1] is None:
+        digits = torch.where(keys < 0, torch.full_like(keys, 2 ** 62), keys)  # read as unsigned
+    order = torch.sort(digits, stable=True)[1]
+    assert torch.equal(k, keys[order])
+    assert torch.equal(v, vals[order])
