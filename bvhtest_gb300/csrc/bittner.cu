@@ -18,6 +18,7 @@
 // set, iteration i selects by the scorer unless plainEvery > 0 and i % plainEvery == plainEvery - 1,
 // in which case it selects by the inefficiency (one graph per kind of iteration).
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "bn13_device.cuh"
@@ -312,9 +313,56 @@ __global__ void __launch_bounds__(kWarpItemsPerBlock * 32) gain_warp_kernel(
   if (target) target[k] = copysignf(log1pf(fmul(fabsf(v), targetScale)), v);
 }
 
-__global__ void init_inner_kernel(const bvhgb_node *__restrict__ t, uint32_t n, uint32_t *__restrict__ flag) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    flag[i] = __ldg(&t[i].isLeafFlag) == 0 ? 1u : 0u;
+// The inner nodes in ascending index order (initData, Bittner13CUDA.cu:939-987): counts per tile, their
+// prefix, and the list. The host reads the number of them only; listing them there took a copy of a flag per node
+// and a loop over them.
+constexpr uint32_t kInnerTile = 1024;
+__device__ __forceinline__ bool is_inner(const bvhgb_node *__restrict__ t, uint32_t n, uint32_t i) {
+  return i < n && __ldg(&t[i].isLeafFlag) == 0;
+}
+__global__ void __launch_bounds__(kInnerTile) inner_count_kernel(const bvhgb_node *__restrict__ t, uint32_t n,
+                                                                 uint32_t *__restrict__ count) {
+  const int c = __syncthreads_count(is_inner(t, n, blockIdx.x * kInnerTile + threadIdx.x));
+  if (threadIdx.x == 0) count[blockIdx.x] = (uint32_t)c;
+}
+// Exclusive prefix in place; count[tiles] receives the sum. One block.
+__global__ void __launch_bounds__(1024) inner_scan_kernel(uint32_t *count, uint32_t tiles) {
+  __shared__ uint32_t warpSum[32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < tiles; base += 1024u) {
+    const uint32_t i = base + threadIdx.x, v = i < tiles ? count[i] : 0u;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) warpSum[warp] = incl;
+    __syncthreads();
+    uint32_t below = 0, all = 0;
+    for (uint32_t w = 0; w < 32; ++w) {
+      below += w < warp ? warpSum[w] : 0u;
+      all += warpSum[w];
+    }
+    if (i < tiles) count[i] = carry + below + incl - v;
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) count[tiles] = carry;
+}
+__global__ void __launch_bounds__(kInnerTile) inner_list_kernel(const bvhgb_node *__restrict__ t, uint32_t n,
+                                                                const uint32_t *__restrict__ first,
+                                                                uint32_t *__restrict__ list) {
+  __shared__ uint32_t warpCount[32];
+  const uint32_t i = blockIdx.x * kInnerTile + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const bool inner = is_inner(t, n, i);
+  const uint32_t m = __ballot_sync(0xFFFFFFFFu, inner);
+  if (lane == 0) warpCount[warp] = __popc(m);
+  __syncthreads();
+  uint32_t at = first[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+  for (uint32_t w = 0; w < warp; ++w) at += warpCount[w];
+  if (inner) list[at] = i;
 }
 
 }  // namespace
@@ -325,6 +373,7 @@ using namespace bvhgb;
 struct bvhgb_bn13_workspace {
   bvhgb_bn13_config cfg{};
   uint32_t numNodes = 0, root = 0, numInner = 0, numChunks = 0, chunkSize = 0;
+  unsigned char *block = nullptr;  // the allocation that holds all arrays
   uint32_t *inner = nullptr, *keys = nullptr, *vals = nullptr, *todo = nullptr;
   void *sortTemp = nullptr;
   PatchOut *patches = nullptr;
@@ -507,52 +556,64 @@ extern "C" BVHGB_API int bvhgb_bn13_create(const bvhgb_node *nodes, uint32_t num
   ws->chunkSize = ws->cfg.chunkSize ? ws->cfg.chunkSize : lNum / ws->numChunks;
   cudaStream_t s = as_stream(stream);
 
-  // initData (Bittner13CUDA.cu:939-987): inner nodes in ascending index order.
-  std::vector<uint32_t> hflags(numNodes);
-  uint32_t *dflag = nullptr;
-  cudaError_t e = dev_malloc(&dflag, 4ull * numNodes);
+  // The number of inner nodes, which the arrays are sized by.
+  const uint32_t tiles = ceil_div(numNodes, kInnerTile);
+  uint32_t *count = nullptr;
+  cudaError_t e = dev_malloc(&count, 4ull * (tiles + 1));
   if (e == cudaSuccess) {
-    init_inner_kernel<<<min(ceil_div(numNodes, 256), 4096u), 256, 0, s>>>(nodes, numNodes, dflag);
+    inner_count_kernel<<<tiles, kInnerTile, 0, s>>>(nodes, numNodes, count);
+    inner_scan_kernel<<<1, 1024, 0, s>>>(count, tiles);
+    count_launch(2);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&ws->numInner, count + tiles, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  const size_t ni = ws->numInner ? ws->numInner : 1;
+  const size_t cs = ws->chunkSize ? ws->chunkSize : 1;
+  const size_t sortBytes = select_temp_bytes(ws->numInner, selection_count(ws));
+  // Only the heap search keeps a queue in global memory (entries beyond the shared-memory top).
+  const size_t heapItems = ws->cfg.searchMode == BVHGB_SEARCH_HEAP ? cs * ws->cfg.heapCapacity : 1;
+  // One allocation; what starts as zeros stands together, and what starts as ones.
+  size_t bytes = 0;
+  auto place = [&](size_t size) {
+    const size_t at = bytes;
+    bytes = (bytes + size + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t oCounter = place(4ull * numNodes), oErr = place(4), oStats = place(sizeof(unsigned long long) * S_COUNT);
+  const size_t zeros = bytes;
+  const size_t oMail = place(24ull * numNodes), oOwner = place(4ull * numNodes);
+  const size_t ones = bytes;
+  const size_t oInner = place(4 * ni), oKeys = place(4 * ni), oVals = place(4 * ni), oTodo = place(4 * ni);
+  const size_t oSort = place(sortBytes ? sortBytes : 256), oPatches = place(sizeof(PatchOut) * cs);
+  const size_t oValid = place(4 * cs), oFix = place(12 * cs), oHeaps = place(sizeof(HeapItem) * heapItems);
+  if (e == cudaSuccess) e = dev_malloc(&ws->block, bytes);
+  if (e == cudaSuccess) {
+    auto at = [&](auto **p, size_t o) { *p = reinterpret_cast<std::remove_reference_t<decltype(**p)> *>(ws->block + o); };
+    at(&ws->counter, oCounter);
+    at(&ws->err, oErr);
+    at(&ws->stats, oStats);
+    at(&ws->mail, oMail);
+    at(&ws->owner, oOwner);
+    at(&ws->inner, oInner);
+    at(&ws->keys, oKeys);
+    at(&ws->vals, oVals);
+    at(&ws->todo, oTodo);
+    ws->sortTemp = ws->block + oSort;
+    at(&ws->patches, oPatches);
+    at(&ws->valid, oValid);
+    at(&ws->toFix, oFix);
+    at(&ws->heaps, oHeaps);
+    inner_list_kernel<<<tiles, kInnerTile, 0, s>>>(nodes, numNodes, count, ws->inner);
     count_launch();
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hflags.data(), dflag, 4ull * numNodes, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(dflag);
-  std::vector<uint32_t> inner;
-  inner.reserve(numNodes / 2 + 1);
-  for (uint32_t i = 0; i < numNodes; ++i)
-    if (hflags[i]) inner.push_back(i);
-  ws->numInner = (uint32_t)inner.size();
-  const size_t ni = inner.size() ? inner.size() : 1;
-  const size_t cs = ws->chunkSize ? ws->chunkSize : 1;
-  const size_t sortBytes = select_temp_bytes(ws->numInner, selection_count(ws));
-  if (e == cudaSuccess) e = dev_malloc(&ws->inner, 4 * ni);
-  if (e == cudaSuccess) e = dev_malloc(&ws->keys, 4 * ni);
-  if (e == cudaSuccess) e = dev_malloc(&ws->vals, 4 * ni);
-  if (e == cudaSuccess) e = dev_malloc(&ws->todo, 4 * ni);
-  if (e == cudaSuccess) e = dev_malloc(&ws->sortTemp, sortBytes ? sortBytes : 256);
-  if (e == cudaSuccess) e = dev_malloc(&ws->patches, sizeof(PatchOut) * cs);
-  if (e == cudaSuccess) e = dev_malloc(&ws->valid, 4 * cs);
-  if (e == cudaSuccess) e = dev_malloc(&ws->toFix, 12 * cs);
-  if (e == cudaSuccess) e = dev_malloc(&ws->owner, 4ull * numNodes);
-  if (e == cudaSuccess) e = dev_malloc(&ws->counter, 4ull * numNodes);
-  if (e == cudaSuccess) e = dev_malloc(&ws->mail, 24ull * numNodes);
-  if (e == cudaSuccess) e = dev_malloc(&ws->err, 4);
-  // Only the heap search keeps a queue in global memory (entries beyond the shared-memory top).
-  const size_t heapItems = ws->cfg.searchMode == BVHGB_SEARCH_HEAP ? cs * ws->cfg.heapCapacity : 1;
-  if (e == cudaSuccess) e = dev_malloc(&ws->heaps, sizeof(HeapItem) * heapItems);
-  if (e == cudaSuccess) e = dev_malloc(&ws->stats, sizeof(unsigned long long) * S_COUNT);
-  if (e == cudaSuccess && inner.size())
-    e = cudaMemcpyAsync(ws->inner, inner.data(), 4 * inner.size(), cudaMemcpyHostToDevice, s);
   ws->countClimbsPerWarp = climbs_per_warp((const void *)apply_count_kernel, 3ull * cs);
   ws->refitClimbsPerWarp = climbs_per_warp((const void *)release_refit_kernel, 3ull * cs);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws->counter, 0, 4ull * numNodes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws->mail, 0xFF, 24ull * numNodes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws->owner, 0xFF, 4ull * numNodes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws->err, 0, 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws->stats, 0, sizeof(unsigned long long) * S_COUNT, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ws->block, 0, zeros, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ws->block + zeros, 0xFF, ones - zeros, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(count);
   if (e == cudaSuccess && ws->cfg.profileKernels) {
     ws->evStart.assign(ws->numChunks, nullptr);
     ws->evStop.assign(ws->numChunks, nullptr);
@@ -577,20 +638,7 @@ extern "C" BVHGB_API int bvhgb_bn13_destroy(bvhgb_bn13_workspace *ws) {
     if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : ws->evStop)
     if (ev) cudaEventDestroy(ev);
-  cudaFree(ws->inner);
-  cudaFree(ws->keys);
-  cudaFree(ws->vals);
-  cudaFree(ws->todo);
-  cudaFree(ws->sortTemp);
-  cudaFree(ws->patches);
-  cudaFree(ws->valid);
-  cudaFree(ws->toFix);
-  cudaFree(ws->owner);
-  cudaFree(ws->counter);
-  cudaFree(ws->mail);
-  cudaFree(ws->err);
-  cudaFree(ws->heaps);
-  cudaFree(ws->stats);
+  cudaFree(ws->block);
   lr_scratch_free(ws->lr);
   delete ws;
   return BVHGB_OK;

@@ -1009,18 +1009,29 @@ float lr_inv_log2_leaves(uint32_t numLeaves) { return 1.0f / std::log2((float)st
 int lr_scratch_alloc(LrScratch &s, uint32_t numNodes) {
   lr_scratch_free(s);
   const size_t n = std::max(numNodes, 1u), ni = n / 2 + 1;
-  cudaError_t e = cudaSuccess;
-  e = dev_malloc(&s.ad, 8 * n);
-  if (e == cudaSuccess) e = dev_malloc(&s.leafCount, 4 * n);
-  if (e == cudaSuccess) e = dev_malloc(&s.sa, 4 * n);
-  if (e == cudaSuccess) e = dev_malloc(&s.par, 4 * n);
-  if (e == cudaSuccess) e = dev_malloc(&s.acc, 8 * n);
-  if (e == cudaSuccess) e = dev_malloc(&s.err, 4);
-  if (e == cudaSuccess) e = dev_malloc(&s.hist, 4 * kHistWords);
-  if (e == cudaSuccess) e = dev_malloc(&s.pend, 16 * ni);
-  if (e == cudaSuccess) e = dev_malloc(&s.x, 2ull * kIn * ni);
-  if (e == cudaSuccess) e = dev_malloc(&s.y, 4 * ni);
-  if (e == cudaSuccess) e = cudaMemset(s.err, 0, 4);
+  size_t bytes = 0;  // one allocation
+  auto place = [&](size_t size) {
+    const size_t at = bytes;
+    bytes = (bytes + size + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t oAd = place(8 * n), oLeaf = place(4 * n), oSa = place(4 * n), oPar = place(4 * n), oAcc = place(8 * n);
+  const size_t oErr = place(4), oHist = place(4 * kHistWords), oPend = place(16 * ni), oX = place(2ull * kIn * ni);
+  const size_t oY = place(4 * ni);
+  cudaError_t e = dev_malloc(&s.block, bytes);
+  if (e == cudaSuccess) {
+    s.ad = reinterpret_cast<unsigned long long *>(s.block + oAd);
+    s.leafCount = reinterpret_cast<uint32_t *>(s.block + oLeaf);
+    s.sa = reinterpret_cast<float *>(s.block + oSa);
+    s.par = reinterpret_cast<uint32_t *>(s.block + oPar);
+    s.acc = reinterpret_cast<unsigned long long *>(s.block + oAcc);
+    s.err = reinterpret_cast<uint32_t *>(s.block + oErr);
+    s.hist = reinterpret_cast<uint32_t *>(s.block + oHist);
+    s.pend = reinterpret_cast<uint4 *>(s.block + oPend);
+    s.x = reinterpret_cast<uint16_t *>(s.block + oX);
+    s.y = reinterpret_cast<float *>(s.block + oY);
+    e = cudaMemset(s.err, 0, 4);
+  }
   if (e != cudaSuccess) {
     set_last_error("lr_scratch_alloc", e);
     lr_scratch_free(s);
@@ -1031,25 +1042,8 @@ int lr_scratch_alloc(LrScratch &s, uint32_t numNodes) {
 }
 
 void lr_scratch_free(LrScratch &s) {
-  cudaFree(s.ad);
-  s.ad = nullptr;
-  cudaFree(s.leafCount);
-  cudaFree(s.sa);
-  cudaFree(s.par);
-  s.sa = nullptr;
-  s.par = nullptr;
-  cudaFree(s.acc);
-  cudaFree(s.err);
-  cudaFree(s.hist);
-  cudaFree(s.pend);
-  cudaFree(s.x);
-  cudaFree(s.y);
-  s.leafCount = s.hist = s.err = nullptr;
-  s.acc = nullptr;
-  s.pend = nullptr;
-  s.y = nullptr;
-  s.x = nullptr;
-  s.numNodes = 0;
+  cudaFree(s.block);
+  s = LrScratch{};
 }
 
 uint32_t *lr_error_word(LrScratch &s) { return s.err; }

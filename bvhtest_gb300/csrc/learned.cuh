@@ -20,6 +20,7 @@ constexpr float kTargetEps = 0.16f;           // target = sign(g) ln(1 + |g| num
 // Device scratch for the features of one tree (sized for numNodes nodes).
 struct LrScratch {
   uint32_t numNodes = 0;
+  unsigned char *block = nullptr;  // the allocation that holds all arrays
   unsigned long long *ad = nullptr;  // depth pointer jumping: distance << 32 | ancestor
   uint32_t *leafCount = nullptr, *hist = nullptr, *err = nullptr;
   float *sa = nullptr;        // per-node surface area (compact copy)
