@@ -382,7 +382,8 @@ __global__ void __launch_bounds__(kBatchThreads) batch_wide_kernel(const bvhgb_n
   stage_offsets(shOff, innerOff, numMeshes);
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < totalInner; q += gridDim.x * blockDim.x) {
     const uint32_t m = segment_of(shOff, numMeshes, q), n = shOff[m + 1] - shOff[m] + 1u;
-    build_wide(nodes + __ldg(nodeOff + m), 2 * n - 1, q - shOff[m], wide + shOff[m], err);
+    const bvhgb_node *tree = nodes + __ldg(nodeOff + m);
+    build_wide(tree, 2 * n - 1, q - shOff[m], wide_size(tree, 0u), wide + shOff[m], err);
   }
 }
 

@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(32, kWideWarps) trace_rays_wide_kernel(
       sc, n, run,
       [&](uint32_t i, bool valid, RayPre &r) {
         if (valid) load_ray(org, dir, i, r);
-        return valid;
+        // Without a direction the triangle test's shears are NaN: nothing is hit.
+        return valid && (r.d[0] != 0.0f || r.d[1] != 0.0f || r.d[2] != 0.0f);
       },
       [&](uint32_t i, const Hit &h) { store_hit(hits + i, h); }, &g_trace_errors);
 }
@@ -387,11 +388,12 @@ __global__ void __launch_bounds__(128) trace_ray_image_kernel(const bvhgb_node *
   }
 }
 
-__global__ void build_trav_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, TravNode *__restrict__ out,
-                                  WideNode *__restrict__ wide) {
+__global__ void build_trav_kernel(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, uint32_t root,
+                                  TravNode *__restrict__ out, WideNode *__restrict__ wide) {
+  const WideSize size = wide_size(nodes, root);
   for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < numNodes; x += gridDim.x * blockDim.x) {
     build_trav(nodes, numNodes, x, out, &g_trace_errors);
-    if (wide) build_wide(nodes, numNodes, x, wide, &g_trace_errors);
+    if (wide) build_wide(nodes, numNodes, x, size, wide, &g_trace_errors);
   }
 }
 
@@ -598,7 +600,7 @@ extern "C" BVHGB_API int bvhgb_tracer_update(bvhgb_tracer *tr, const bvhgb_node 
   tr->numNodes = numNodes;
   tr->root = root;
   build_trav_kernel<<<std::min(ceil_div(numNodes, 256), (uint32_t)sm_count() * 16), 256, 0, as_stream(stream)>>>(
-      nodes, numNodes, tr->trav, tr->wide);
+      nodes, numNodes, root, tr->trav, tr->wide);
   BVHGB_LAUNCH_CHECK("tracer records");
   return BVHGB_OK;
 }

@@ -332,9 +332,27 @@ constexpr uint32_t kLeafNode = 0x80000000u;
 constexpr int kWideSteps = 8;       // records per lane between two rounds of leaf tests
 constexpr int kWideStack = kStack * 3 / 2 + 3 * kWideSteps;
 
+// A tree's size is the largest coordinate of its root's box. No grid step is finer than kWideFinest of it, and
+// boxes that reach twice as far are on no grid (nested boxes don't): that bounds every plane distance of a ray,
+// and what a slab test may say about a ray that is all but parallel to the slab (limit_reciprocals).
+constexpr float kWideFinest = 9.0949470e-13f;  // 2^-40
+struct WideSize {
+  float size;
+  bool finite;  // false: the root's box is not, 'size' is any
+  __device__ __forceinline__ WideSize(float4 a, float4 b) {
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))), fmaxf(fabsf(b.x), fabsf(b.y)));
+    finite = m < 1e37f;  // a NaN component drops out
+    size = finite ? fmaxf(m, 2.7755576e-17f) : 1.1529215e18f;  // 2^-55, 2^60
+  }
+};
+__device__ __forceinline__ WideSize wide_size(const bvhgb_node *__restrict__ nodes, uint32_t root) {
+  const float4 *p = reinterpret_cast<const float4 *>(nodes + root);
+  return WideSize(__ldg(p), __ldg(p + 1));
+}
+
 // Node x's wide record (none for a leaf).
 __device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, uint32_t x,
-                                           WideNode *__restrict__ out, uint32_t *err) {
+                                           const WideSize &tree, WideNode *__restrict__ out, uint32_t *err) {
   const float4 *p = reinterpret_cast<const float4 *>(nodes + x);
   const float4 xb = __ldg(p + 1), xc = __ldg(p + 2);
   if (__float_as_uint(xc.y) & 0xFFFFu) return;
@@ -401,10 +419,11 @@ __device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes,
     }
     // The step: 240 of them span the boxes, and none is finer than two units in the last place of
     // the largest coordinate, so that the differences below are exact to a fraction of a step.
-    const float need = fmaxf((hi - lo) * (1.0f / 240.0f), fmaxf(fabsf(lo), fabsf(hi)) * 4.76837158e-7f);
+    const float far = fmaxf(fabsf(lo), fabsf(hi));
+    const float need = fmaxf(fmaxf((hi - lo) * (1.0f / 240.0f), far * 4.76837158e-7f), tree.finite ? tree.size * kWideFinest : 0.0f);
     uint32_t e = (__float_as_uint(need) >> 23) + 1u;  // the next power of two above
     n.lo[k] = n.hi[k] = 0u;
-    if (!finite || !(need < 1e37f) || kinds == 0u) {
+    if (!finite || !(far <= 2.0f * tree.size) || kinds == 0u) {
       // Not on any grid: a step of infinity makes every plane distance NaN, which drops out of the
       // slab test, so the slots pass on this axis.
       n.o[k] = 0.0f;
@@ -538,6 +557,26 @@ struct WideScene {
   __device__ __forceinline__ uint32_t root() const { return rootNode; }
 };
 
+// The largest reciprocal of a direction component that the slab tests of a ray use, and what takes the place of
+// larger ones.
+//   - Beyond 2^116 over the tree's size (and a thousandth of the ray's reach) products with the largest grid
+//     step or the origin's distance can overflow, and a distance that is infinite on one side would drop a
+//     box: there the reciprocal is infinite, the distances are NaN, and every box passes on that axis.
+//   - A ray parallel to an axis is to be kept out of the slabs beside it: for a component below 2^-80 of the
+//     largest the limit itself serves. A ray inside a slab is an eighth of a step or more from its planes, which
+//     then are as far away as 2^77 steps along the ray; and such a component moves the ray by a thirty-second
+//     of a step at most on its first 2^75 steps. A step is kWideFinest of the size or more, so this holds
+//     while the origin is within 2^35 sizes (2^-45 of the limit times the largest component).
+__device__ __forceinline__ void limit_reciprocals(RayPre &r, const WideSize &tree) {
+  const float reach = fmaxf(fmaxf(fabsf(r.o[0]), fabsf(r.o[1])), fabsf(r.o[2])) + tree.size;
+  const float most = fminf(1.2089258e24f * fabsf(r.sz), __fdividef(8.3076750e34f, fmaf(reach, 0.0009765625f, tree.size)));
+  const bool near = tree.finite && reach <= tree.size * (most * fabsf(pick(r.d, r.kz)) * 2.8421709e-14f);  // 2^-45
+  const float beyond = near ? most : __int_as_float(0x7f800000);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (fabsf(r.inv[k]) > most) r.inv[k] = copysignf(beyond, r.d[k]);
+}
+
 // Block b's run is rays [b * run, ...) of 'total' (< 2^31). gen(i, valid, r), which
 // the whole warp calls for 32 rays in a row from a multiple of 32, sets r.o and r.d of a valid ray and
 // returns whether there is one to trace; emit(i, hit) takes every ray's result (no hit for those gen
@@ -597,6 +636,7 @@ __device__ __forceinline__ void trace_wide(const Scene &sc, uint32_t total, uint
           } else if (!live) {
             emit(i, Hit{kNone, sc.tmax});
           }
+          limit_reciprocals(g, WideSize(a, b));
         } else if (i < end) {
           emit(i, Hit{kNone, sc.tmax});
         }
@@ -607,9 +647,7 @@ __device__ __forceinline__ void trace_wide(const Scene &sc, uint32_t total, uint
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
             sm.org[k][s] = g.o[k];
-            // A direction component near zero counts as 2^-80: products with the reciprocal stay
-            // finite, so a ray parallel to an axis is still kept out of the slabs beside it.
-            sm.inv[k][s] = fabsf(g.d[k]) < 8.271806e-25f ? copysignf(1.2089258e24f, g.d[k]) : g.inv[k];
+            sm.inv[k][s] = g.inv[k];
           }
           sm.shear[0][s] = g.sx;
           sm.shear[1][s] = g.sy;
