@@ -37,6 +37,8 @@ struct bvhgb_batch_workspace {
   float4 *triBoxes = nullptr;
   void *sortTemp = nullptr;
   bvhgb::WideNode *wide = nullptr;  // the tracer's wide records, one per inner node; null where they do not fit
+  uint32_t *wideSkip = nullptr;     // behind them, per mesh and for any: the last trace whose records missed a node
+  uint32_t traces = 0;              // traces on the records so far: the number of the last one
   // The selection of every mesh's first numChunks * chunk nodes (sel.tiles = 0: all are sorted).
   bvhgb::SegSelect sel{};
   uint32_t kept = 0;            // nodes selected in all
@@ -351,14 +353,12 @@ __device__ __forceinline__ void batch_store(bvhgb_hit *out, const Hit &h) {
   *out = o;
 }
 
-// On the node arrays, one thread per ray.
-__global__ void batch_trace_kernel(const bvhgb_node *__restrict__ nodes, const float *__restrict__ vert,
-                                   const uint32_t *__restrict__ faces, const uint32_t *__restrict__ faceOff,
-                                   const uint32_t *__restrict__ nodeOff, uint32_t numMeshes, uint32_t raysPerMesh,
-                                   uint64_t seed, bvhgb_hit *__restrict__ hits, float *__restrict__ rayOrg,
-                                   float *__restrict__ rayDir, uint32_t *__restrict__ err) {
-  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= (uint64_t)numMeshes * raysPerMesh) return;
+// Ray r on its mesh's nodes.
+__device__ __forceinline__ void batch_trace_ray(const bvhgb_node *__restrict__ nodes, const float *__restrict__ vert,
+                                                const uint32_t *__restrict__ faces, const uint32_t *__restrict__ faceOff,
+                                                const uint32_t *__restrict__ nodeOff, uint32_t raysPerMesh, uint64_t r,
+                                                uint64_t seed, bvhgb_hit *__restrict__ hits, float *__restrict__ rayOrg,
+                                                float *__restrict__ rayDir, uint32_t *__restrict__ err) {
   const uint32_t m = (uint32_t)(r / raysPerMesh);
   const uint32_t fb = __ldg(faceOff + m), n = __ldg(faceOff + m + 1) - fb;
   const bvhgb_node *t = nodes + __ldg(nodeOff + m);
@@ -370,20 +370,49 @@ __global__ void batch_trace_kernel(const bvhgb_node *__restrict__ nodes, const f
   batch_store(hits + r, h);
 }
 
+// On the node arrays, one thread per ray.
+__global__ void batch_trace_kernel(const bvhgb_node *__restrict__ nodes, const float *__restrict__ vert,
+                                   const uint32_t *__restrict__ faces, const uint32_t *__restrict__ faceOff,
+                                   const uint32_t *__restrict__ nodeOff, uint32_t numMeshes, uint32_t raysPerMesh,
+                                   uint64_t seed, bvhgb_hit *__restrict__ hits, float *__restrict__ rayOrg,
+                                   float *__restrict__ rayDir, uint32_t *__restrict__ err) {
+  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < (uint64_t)numMeshes * raysPerMesh)
+    batch_trace_ray(nodes, vert, faces, faceOff, nodeOff, raysPerMesh, r, seed, hits, rayOrg, rayDir, err);
+}
+
+// The rays of the meshes that the records of this trace do not cover, on the node arrays, in place of what the
+// records gave: a launch of its own, which mostly returns at once (2 us), because the traversal's code beside the
+// records' costs every ray registers (16.7M rays 22.7 ms, as a call from their kernel 24.3).
+__global__ void __launch_bounds__(kBatchThreads) batch_trace_rest_kernel(
+    const bvhgb_node *__restrict__ nodes, const float *__restrict__ vert, const uint32_t *__restrict__ faces,
+    const uint32_t *__restrict__ faceOff, const uint32_t *__restrict__ nodeOff, uint32_t numMeshes, uint32_t raysPerMesh,
+    uint64_t seed, const uint32_t *__restrict__ skip, uint32_t trace, bvhgb_hit *__restrict__ hits,
+    float *__restrict__ rayOrg, float *__restrict__ rayDir, uint32_t *__restrict__ err) {
+  grid_wait();
+  if (__ldcg(skip + numMeshes) != trace) return;
+  for (uint64_t r = (uint64_t)blockIdx.x * kBatchThreads + threadIdx.x; r < (uint64_t)numMeshes * raysPerMesh;
+       r += (uint64_t)gridDim.x * kBatchThreads)
+    if (__ldg(skip + (uint32_t)(r / raysPerMesh)) == trace)
+      batch_trace_ray(nodes, vert, faces, faceOff, nodeOff, raysPerMesh, r, seed, hits, rayOrg, rayDir, err);
+}
+
 // Wide records of every mesh's inner nodes, at the meshes' inner offsets (an LBVH's inner nodes are
-// [0, n - 1) and stay inner, so a record's references are offsets into its mesh's records).
+// [0, n - 1) and stay inner, so a record's references are offsets into its mesh's records). A mesh whose tree is in
+// another order (an inner node from n - 1 on has no record), or has a bad link, is noted under the trace's number: its
+// records lead to no other mesh's, and its rays are traced again on the nodes.
 __global__ void __launch_bounds__(kBatchThreads) batch_wide_kernel(const bvhgb_node *__restrict__ nodes,
                                                                    const uint32_t *__restrict__ innerOff,
                                                                    const uint32_t *__restrict__ nodeOff,
                                                                    uint32_t numMeshes, uint32_t totalInner,
                                                                    WideNode *__restrict__ wide,
-                                                                   uint32_t *__restrict__ err) {
+                                                                   uint32_t *__restrict__ skip, uint32_t trace) {
   extern __shared__ uint32_t shOff[];
   stage_offsets(shOff, innerOff, numMeshes);
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < totalInner; q += gridDim.x * blockDim.x) {
     const uint32_t m = segment_of(shOff, numMeshes, q), n = shOff[m + 1] - shOff[m] + 1u;
     const bvhgb_node *tree = nodes + __ldg(nodeOff + m);
-    build_wide(tree, 2 * n - 1, q - shOff[m], wide_size(tree, 0u), wide + shOff[m], err);
+    if (!build_wide(tree, 2 * n - 1, n - 1, q - shOff[m], wide_size(tree, 0u), wide + shOff[m])) skip[m] = skip[numMeshes] = trace;
   }
 }
 
@@ -500,17 +529,20 @@ int batch_iteration(bvhgb_batch_workspace *ws, bvhgb_node *nodes, cudaStream_t s
   return BVHGB_OK;
 }
 
+// built: the trees are the workspace's own, in the order of an LBVH build.
 int batch_trace(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
-                uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, cudaStream_t s) {
+                uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, cudaStream_t s,
+                bool built) {
   const uint64_t R = (uint64_t)ws->numMeshes * raysPerMesh;
   if (R == 0) return BVHGB_OK;
   // Making the records costs 43 us per million inner nodes and tracing on them saves 0.48 ms per million
   // rays (256 meshes, 20M triangles, 16.7M rays: 25.6 ms on the node arrays, 17.6 on the records), so
   // they are made from one ray per 8 nodes on.
   if (ws->wide && R < (1ull << 31) && R >= ws->totalInner / 8) {
+    const uint32_t trace = ++ws->traces ? ws->traces : ++ws->traces;  // 0: none
     if (ws->totalInner) {
       batch_wide_kernel<<<grid_of(ws->totalInner, kBatchThreads), kBatchThreads, off_smem(ws->numMeshes), s>>>(
-          nodes, ws->innerOff, ws->nodeOff, ws->numMeshes, ws->totalInner, ws->wide, ws->err);
+          nodes, ws->innerOff, ws->nodeOff, ws->numMeshes, ws->totalInner, ws->wide, ws->wideSkip, trace);
       BVHGB_LAUNCH_CHECK("batch wide records");
     }
     const BatchScene sc{nodes, ws->wide, faces, vert, ws->faceOff, ws->nodeOff, ws->innerOff, raysPerMesh, ws->totalNodes,
@@ -518,6 +550,12 @@ int batch_trace(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float 
     const uint32_t run = wide_run(R);
     batch_trace_wide_kernel<<<ceil_div(R, run), 32, 0, s>>>(sc, (uint32_t)R, run, seed, hits, rayOrg, rayDir, ws->err);
     BVHGB_LAUNCH_CHECK("batch trace");
+    if (!built) {  // given trees; it starts while the records' launch drains
+      BVHGB_CUDA_TRY(launch_kernel(batch_trace_rest_kernel, std::min(ceil_div(R, kBatchThreads), (uint32_t)sm_count() * 4),
+                                   kBatchThreads, 0, s, true, nodes, vert, faces, ws->faceOff, ws->nodeOff, ws->numMeshes,
+                                   raysPerMesh, seed, ws->wideSkip, trace, hits, rayOrg, rayDir, ws->err));
+      BVHGB_LAUNCH_CHECK("batch trace rest");
+    }
     return BVHGB_OK;
   }
   const uint32_t bs = ws->cfg.traceBlock;
@@ -695,9 +733,14 @@ extern "C" BVHGB_API int bvhgb_batch_create(uint32_t numMeshes, const uint32_t *
   alloc(&ws->stats, sizeof(unsigned long long) * S_COUNT);
   if (e == cudaSuccess) e = plan_selection(ws);
   // Where the wide records do not fit, rays go through the node arrays.
-  if (e == cudaSuccess && dev_malloc(&ws->wide, sizeof(WideNode) * std::max<size_t>(inner, 1)) != cudaSuccess) {
+  if (e == cudaSuccess &&
+      dev_malloc(&ws->wide, sizeof(WideNode) * (size_t)inner + 4 * ((size_t)numMeshes + 1)) != cudaSuccess) {
     ws->wide = nullptr;
     cudaGetLastError();
+  }
+  if (ws->wide) {
+    ws->wideSkip = reinterpret_cast<uint32_t *>(ws->wide + inner);
+    e = cudaMemset(ws->wideSkip, 0, 4 * ((size_t)numMeshes + 1));
   }
   if (e == cudaSuccess) e = cudaMemcpy(ws->faceOff, ws->hFaceOff.data(), 4 * (numMeshes + 1), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(ws->nodeOff, ws->hNodeOff.data(), 4 * (numMeshes + 1), cudaMemcpyHostToDevice);
@@ -784,7 +827,7 @@ extern "C" BVHGB_API int bvhgb_batch_trace_random(bvhgb_batch_workspace *ws, con
   if ((rayOrg == nullptr) != (rayDir == nullptr)) return BVHGB_INVALID_ARGUMENT;
   for (uint32_t m = 0; m < ws->numMeshes; ++m)
     if (raysPerMesh && ws->hFaceOff[m + 1] == ws->hFaceOff[m]) return BVHGB_INVALID_ARGUMENT;  // an empty mesh
-  return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, as_stream(stream));
+  return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, as_stream(stream), false);
 }
 
 extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float *vert, const uint32_t *faces,
@@ -809,7 +852,7 @@ extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float 
     if (e == cudaSuccess) {
       st = batch_build(ws, vert, faces, nodes, cap);
       for (uint32_t i = 0; i < iterations && st == BVHGB_OK; ++i) st = batch_iteration(ws, nodes, cap);
-      if (st == BVHGB_OK) st = batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, cap);
+      if (st == BVHGB_OK) st = batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, cap, true);
       e = cudaStreamEndCapture(cap, &g);
     }
     const uint64_t kernels = bvhgb_launch_count() - before;
@@ -920,7 +963,7 @@ extern "C" BVHGB_API int bvhgb_batch_autotune(bvhgb_batch_workspace *ws, const f
   bestMs = 3.4e38f;
   for (int i = 0; i < 3 && !st && raysPerMesh; ++i) {
     ws->cfg.traceBlock = traces[i];
-    st = timed([&] { return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, s); },
+    st = timed([&] { return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, s, true); },
                report->traceBlockMs[i]);
     report->traceBlock[i] = traces[i];
     if (!st && report->traceBlockMs[i] < bestMs) {

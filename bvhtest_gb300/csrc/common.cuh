@@ -158,8 +158,8 @@ uint64_t context_id();
 // Launch; early: it may start while the stream's previous kernel drains, and the kernel calls grid_wait()
 // before it touches anything that kernel (or one before it) wrote or reads.
 template <typename... P, typename... A>
-inline void launch_kernel(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, bool early,
-                          A &&...args) {
+inline cudaError_t launch_kernel(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, bool early,
+                                 A &&...args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -170,7 +170,7 @@ inline void launch_kernel(void (*kernel)(P...), uint32_t grid, uint32_t block, s
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = early ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 // cudaMalloc through the library's allocation-failure injection (bvhgb_debug_fail_allocations).
 cudaError_t dev_malloc(void **p, size_t bytes);

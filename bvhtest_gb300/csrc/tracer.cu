@@ -393,7 +393,7 @@ __global__ void build_trav_kernel(const bvhgb_node *__restrict__ nodes, uint32_t
   const WideSize size = wide_size(nodes, root);
   for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < numNodes; x += gridDim.x * blockDim.x) {
     build_trav(nodes, numNodes, x, out, &g_trace_errors);
-    if (wide) build_wide(nodes, numNodes, x, size, wide, &g_trace_errors);
+    if (wide && !build_wide(nodes, numNodes, numNodes, x, size, wide)) atomicOr(&g_trace_errors, kErrBadIndex);
   }
 }
 

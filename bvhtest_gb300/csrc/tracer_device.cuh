@@ -350,12 +350,13 @@ __device__ __forceinline__ WideSize wide_size(const bvhgb_node *__restrict__ nod
   return WideSize(__ldg(p), __ldg(p + 1));
 }
 
-// Node x's wide record (none for a leaf).
-__device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, uint32_t x,
-                                           const WideSize &tree, WideNode *__restrict__ out, uint32_t *err) {
+// Node x's wide record (none for a leaf). False: a link leads out of the tree, or to an inner node that has no
+// record (nodes [0, records) have one); no slot of the record is ever opened then.
+__device__ __forceinline__ bool build_wide(const bvhgb_node *__restrict__ nodes, uint32_t numNodes, uint32_t records,
+                                           uint32_t x, const WideSize &tree, WideNode *__restrict__ out) {
   const float4 *p = reinterpret_cast<const float4 *>(nodes + x);
   const float4 xb = __ldg(p + 1), xc = __ldg(p + 2);
-  if (__float_as_uint(xc.y) & 0xFFFFu) return;
+  if (__float_as_uint(xc.y) & 0xFFFFu) return true;
   const uint32_t child[2] = {__float_as_uint(xb.w), __float_as_uint(xc.x)};
   float mn[4][3], mx[4][3];
   uint32_t ref[4] = {0u, 0u, 0u, 0u}, kinds = 0;
@@ -391,16 +392,14 @@ __device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes,
       if (!(__float_as_uint(h.y) & 0xFFFFu)) {
         kinds |= 1u << s;
         ref[s] = g[k];
+        ok = ok && g[k] < records;
       } else if (count != 0u) {
         kinds |= 16u << s;
         ref[s] = count == 1u && __float_as_uint(f.w) < kLeafNode ? __float_as_uint(f.w) : g[k] | kLeafNode;
       }
     }
   }
-  if (!ok) {  // no slot is ever opened
-    atomicOr(err, kErrBadIndex);
-    kinds = 0;
-  }
+  if (!ok) kinds = 0;
   WideNode n;
   n.meta = kinds << 24;
   n.pad[0] = n.pad[1] = 0u;
@@ -447,6 +446,7 @@ __device__ __forceinline__ void build_wide(const bvhgb_node *__restrict__ nodes,
   uint4 *dst = reinterpret_cast<uint4 *>(out + x);
 #pragma unroll
   for (int w = 0; w < 4; ++w) dst[w] = src[w];
+  return ok;
 }
 
 // A plane's byte in the middle of the mantissa of 1.0: 1 + q 2^-15, exactly, in one byte permute.
