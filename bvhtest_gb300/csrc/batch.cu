@@ -15,7 +15,9 @@
 //              directions uniform on the sphere), closest hit in that mesh's tree.
 // Mesh-level indices are found by binary search over the offset arrays held in shared memory.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 #include "bn13_device.cuh"
@@ -38,7 +40,9 @@ struct bvhgb_batch_workspace {
   void *sortTemp = nullptr;
   bvhgb::WideNode *wide = nullptr;  // the tracer's wide records, one per inner node; null where they do not fit
   uint32_t *wideSkip = nullptr;     // behind them, per mesh and for any: the last trace whose records missed a node
-  uint32_t traces = 0;              // traces on the records so far: the number of the last one
+  std::atomic<uint32_t> traces{0};  // traces on the records so far: the number of the last one
+  std::mutex wideLock;              // held while a trace on the records is launched
+  cudaEvent_t wideFree = nullptr;   // the end of the last one
   // The selection of every mesh's first numChunks * chunk nodes (sel.tiles = 0: all are sorted).
   bvhgb::SegSelect sel{};
   uint32_t kept = 0;            // nodes selected in all
@@ -53,6 +57,7 @@ struct bvhgb_batch_workspace {
   const void *gVert = nullptr, *gFaces = nullptr, *gNodes = nullptr, *gHits = nullptr;
   uint32_t gIterations = 0, gRays = 0;
   uint64_t gSeed = 0, graphKernels = 0;
+  bool gRecords = false;
 };
 
 namespace bvhgb {
@@ -529,41 +534,82 @@ int batch_iteration(bvhgb_batch_workspace *ws, bvhgb_node *nodes, cudaStream_t s
   return BVHGB_OK;
 }
 
-// built: the trees are the workspace's own, in the order of an LBVH build.
-int batch_trace(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
-                uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, cudaStream_t s,
-                bool built) {
+// Making the records costs 43 us per million inner nodes and tracing on them saves 0.48 ms per million
+// rays (256 meshes, 20M triangles, 16.7M rays: 25.6 ms on the node arrays, 17.6 on the records), so
+// they are made from one ray per 8 nodes on.
+bool pays_for_records(const bvhgb_batch_workspace *ws, uint32_t raysPerMesh) {
+  const uint64_t R = (uint64_t)ws->numMeshes * raysPerMesh;
+  return ws->wide && R > 0 && R < (1ull << 31) && R >= ws->totalInner / 8;
+}
+
+// Records, then rays. built: the trees are the workspace's own, in the order of an LBVH build.
+int trace_on_records(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
+                     uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, bool built,
+                     cudaStream_t s) {
+  const uint64_t R = (uint64_t)ws->numMeshes * raysPerMesh;
+  uint32_t trace = ++ws->traces;
+  if (trace == 0) trace = ++ws->traces;  // 0: none
+  if (ws->totalInner) {
+    batch_wide_kernel<<<grid_of(ws->totalInner, kBatchThreads), kBatchThreads, off_smem(ws->numMeshes), s>>>(
+        nodes, ws->innerOff, ws->nodeOff, ws->numMeshes, ws->totalInner, ws->wide, ws->wideSkip, trace);
+    BVHGB_LAUNCH_CHECK("batch wide records");
+  }
+  const BatchScene sc{nodes, ws->wide, faces, vert, ws->faceOff, ws->nodeOff, ws->innerOff, raysPerMesh, ws->totalNodes,
+                      0.0f, INFINITY, false};
+  const uint32_t run = wide_run(R);
+  batch_trace_wide_kernel<<<ceil_div(R, run), 32, 0, s>>>(sc, (uint32_t)R, run, seed, hits, rayOrg, rayDir, ws->err);
+  BVHGB_LAUNCH_CHECK("batch trace");
+  if (!built) {  // given trees; it starts while the records' launch drains
+    BVHGB_CUDA_TRY(launch_kernel(batch_trace_rest_kernel, std::min(ceil_div(R, kBatchThreads), (uint32_t)sm_count() * 4),
+                                 kBatchThreads, 0, s, true, nodes, vert, faces, ws->faceOff, ws->nodeOff, ws->numMeshes,
+                                 raysPerMesh, seed, ws->wideSkip, trace, hits, rayOrg, rayDir, ws->err));
+    BVHGB_LAUNCH_CHECK("batch trace rest");
+  }
+  return BVHGB_OK;
+}
+
+int trace_on_nodes(const bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
+                   uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, cudaStream_t s) {
   const uint64_t R = (uint64_t)ws->numMeshes * raysPerMesh;
   if (R == 0) return BVHGB_OK;
-  // Making the records costs 43 us per million inner nodes and tracing on them saves 0.48 ms per million
-  // rays (256 meshes, 20M triangles, 16.7M rays: 25.6 ms on the node arrays, 17.6 on the records), so
-  // they are made from one ray per 8 nodes on.
-  if (ws->wide && R < (1ull << 31) && R >= ws->totalInner / 8) {
-    const uint32_t trace = ++ws->traces ? ws->traces : ++ws->traces;  // 0: none
-    if (ws->totalInner) {
-      batch_wide_kernel<<<grid_of(ws->totalInner, kBatchThreads), kBatchThreads, off_smem(ws->numMeshes), s>>>(
-          nodes, ws->innerOff, ws->nodeOff, ws->numMeshes, ws->totalInner, ws->wide, ws->wideSkip, trace);
-      BVHGB_LAUNCH_CHECK("batch wide records");
-    }
-    const BatchScene sc{nodes, ws->wide, faces, vert, ws->faceOff, ws->nodeOff, ws->innerOff, raysPerMesh, ws->totalNodes,
-                        0.0f, INFINITY, false};
-    const uint32_t run = wide_run(R);
-    batch_trace_wide_kernel<<<ceil_div(R, run), 32, 0, s>>>(sc, (uint32_t)R, run, seed, hits, rayOrg, rayDir, ws->err);
-    BVHGB_LAUNCH_CHECK("batch trace");
-    if (!built) {  // given trees; it starts while the records' launch drains
-      BVHGB_CUDA_TRY(launch_kernel(batch_trace_rest_kernel, std::min(ceil_div(R, kBatchThreads), (uint32_t)sm_count() * 4),
-                                   kBatchThreads, 0, s, true, nodes, vert, faces, ws->faceOff, ws->nodeOff, ws->numMeshes,
-                                   raysPerMesh, seed, ws->wideSkip, trace, hits, rayOrg, rayDir, ws->err));
-      BVHGB_LAUNCH_CHECK("batch trace rest");
-    }
-    return BVHGB_OK;
-  }
   const uint32_t bs = ws->cfg.traceBlock;
   batch_trace_kernel<<<(uint32_t)((R + bs - 1) / bs), bs, 0, s>>>(nodes, vert, faces, ws->faceOff, ws->nodeOff,
                                                                   ws->numMeshes, raysPerMesh, seed, hits, rayOrg,
                                                                   rayDir, ws->err);
   BVHGB_LAUNCH_CHECK("batch trace");
   return BVHGB_OK;
+}
+
+// The records belong to one trace at a time: work that makes and reads them waits on its stream for the last
+// such work, whatever stream and thread that came from.
+template <typename Fn>
+int in_turn(bvhgb_batch_workspace *ws, cudaStream_t s, Fn &&work) {
+  std::lock_guard<std::mutex> lock(ws->wideLock);
+  BVHGB_CUDA_TRY(cudaStreamWaitEvent(s, ws->wideFree, 0));
+  const int st = work();
+  BVHGB_CUDA_TRY(cudaEventRecord(ws->wideFree, s));
+  return st;
+}
+
+// A captured call cannot wait for work outside its graph, and its replays come when they come: it has no turn
+// at the records and traces on the nodes.
+bool is_captured(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
+int batch_trace(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
+                uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, bool built,
+                cudaStream_t s) {
+  if (!pays_for_records(ws, raysPerMesh) || is_captured(s))
+    return trace_on_nodes(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, s);
+  return in_turn(ws, s, [&] {
+    return trace_on_records(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, built, s);
+  });
 }
 
 bool valid_config(const bvhgb_batch_config &c) {
@@ -740,7 +786,8 @@ extern "C" BVHGB_API int bvhgb_batch_create(uint32_t numMeshes, const uint32_t *
   }
   if (ws->wide) {
     ws->wideSkip = reinterpret_cast<uint32_t *>(ws->wide + inner);
-    e = cudaMemset(ws->wideSkip, 0, 4 * ((size_t)numMeshes + 1));
+    e = cudaEventCreateWithFlags(&ws->wideFree, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMemset(ws->wideSkip, 0, 4 * ((size_t)numMeshes + 1));
   }
   if (e == cudaSuccess) e = cudaMemcpy(ws->faceOff, ws->hFaceOff.data(), 4 * (numMeshes + 1), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(ws->nodeOff, ws->hNodeOff.data(), 4 * (numMeshes + 1), cudaMemcpyHostToDevice);
@@ -765,6 +812,7 @@ extern "C" BVHGB_API int bvhgb_batch_create(uint32_t numMeshes, const uint32_t *
 extern "C" BVHGB_API int bvhgb_batch_destroy(bvhgb_batch_workspace *ws) {
   if (!ws) return BVHGB_OK;
   drop_graph(ws);
+  if (ws->wideFree) cudaEventDestroy(ws->wideFree);
   for (void *p : {(void *)ws->faceOff, (void *)ws->nodeOff, (void *)ws->innerOff, (void *)ws->itemOff, (void *)ws->chunk,
                   (void *)ws->itemMesh, (void *)ws->scene, (void *)ws->err, (void *)ws->keys, (void *)ws->keysSorted,
                   (void *)ws->vals, (void *)ws->valsSorted, (void *)ws->slots, (void *)ws->triBoxes, ws->sortTemp,
@@ -827,7 +875,7 @@ extern "C" BVHGB_API int bvhgb_batch_trace_random(bvhgb_batch_workspace *ws, con
   if ((rayOrg == nullptr) != (rayDir == nullptr)) return BVHGB_INVALID_ARGUMENT;
   for (uint32_t m = 0; m < ws->numMeshes; ++m)
     if (raysPerMesh && ws->hFaceOff[m + 1] == ws->hFaceOff[m]) return BVHGB_INVALID_ARGUMENT;  // an empty mesh
-  return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, as_stream(stream), false);
+  return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, false, as_stream(stream));
 }
 
 extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float *vert, const uint32_t *faces,
@@ -837,8 +885,10 @@ extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float 
   for (uint32_t m = 0; m < ws->numMeshes; ++m)
     if (raysPerMesh && ws->hFaceOff[m + 1] == ws->hFaceOff[m]) return BVHGB_INVALID_ARGUMENT;
   cudaStream_t s = as_stream(stream);
+  const bool records = pays_for_records(ws, raysPerMesh) && !is_captured(s);
   const bool same = ws->graph && ws->gVert == vert && ws->gFaces == faces && ws->gNodes == nodes && ws->gHits == hits &&
-                    ws->gIterations == iterations && ws->gRays == raysPerMesh && ws->gSeed == seed;
+                    ws->gIterations == iterations && ws->gRays == raysPerMesh && ws->gSeed == seed &&
+                    ws->gRecords == records;
   if (!same) {
     drop_graph(ws);
     int pst = sort_prepare();
@@ -852,7 +902,9 @@ extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float 
     if (e == cudaSuccess) {
       st = batch_build(ws, vert, faces, nodes, cap);
       for (uint32_t i = 0; i < iterations && st == BVHGB_OK; ++i) st = batch_iteration(ws, nodes, cap);
-      if (st == BVHGB_OK) st = batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, cap, true);
+      if (st == BVHGB_OK)
+        st = records ? trace_on_records(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, true, cap)
+                     : trace_on_nodes(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, cap);
       e = cudaStreamEndCapture(cap, &g);
     }
     const uint64_t kernels = bvhgb_launch_count() - before;
@@ -873,11 +925,16 @@ extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float 
     ws->gIterations = iterations;
     ws->gRays = raysPerMesh;
     ws->gSeed = seed;
+    ws->gRecords = records;
     ws->graphKernels = kernels;
   }
-  BVHGB_CUDA_TRY(cudaGraphLaunch(ws->graph, s));
-  count_launch((uint32_t)ws->graphKernels);
-  return BVHGB_OK;
+  auto launch = [&]() -> int {
+    BVHGB_CUDA_TRY(cudaGraphLaunch(ws->graph, s));
+    return BVHGB_OK;
+  };
+  const int st = records ? in_turn(ws, s, launch) : launch();
+  if (st == BVHGB_OK) count_launch((uint32_t)ws->graphKernels);
+  return st;
 }
 
 extern "C" BVHGB_API int bvhgb_batch_get_stats(bvhgb_batch_workspace *ws, bvhgb_bn13_stats *stats, uint32_t *errors,
@@ -963,7 +1020,7 @@ extern "C" BVHGB_API int bvhgb_batch_autotune(bvhgb_batch_workspace *ws, const f
   bestMs = 3.4e38f;
   for (int i = 0; i < 3 && !st && raysPerMesh; ++i) {
     ws->cfg.traceBlock = traces[i];
-    st = timed([&] { return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, s, true); },
+    st = timed([&] { return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, true, s); },
                report->traceBlockMs[i]);
     report->traceBlock[i] = traces[i];
     if (!st && report->traceBlockMs[i] < bestMs) {

@@ -409,7 +409,9 @@ BVHGB_API int bvhgb_batch_optimize(bvhgb_batch_workspace *ws, bvhgb_node *nodes,
  * directions uniform on the sphere, from a counter hash of seed), closest hit in the mesh's tree:
  * hits[m * raysPerMesh + j] = (face index within the mesh, t). rayOrg / rayDir (float3 per ray, both
  * or neither) receive the rays. A mesh's nodes may stand in any order (root 0); in the order of the build
- * its rays are traced on records of the inner nodes. */
+ * its rays are traced on records of the inner nodes. The workspace holds the records of one trace: traces
+ * on several streams are independent calls, but the parts that use the records follow each other. A call
+ * under stream capture traces on the nodes. */
 BVHGB_API int bvhgb_batch_trace_random(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert,
                                        const uint32_t *faces, uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits,
                                        float *rayOrg, float *rayDir, bvhgb_stream stream);
