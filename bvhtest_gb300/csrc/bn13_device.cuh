@@ -402,7 +402,7 @@ __device__ __forceinline__ bool remove_node(Patch &p, uint32_t x, uint32_t ins[2
   NodeRec rs = tree_rec(p.t, p.chk(s));
   NodeP ng = tree_node(p.t, p.chk(gi));
   const uint32_t other = np.isLeft ? ng.right : ng.left;  // the grand parent's other child
-  const uint32_t ggi = ng.parent;
+  const uint32_t ggi = gi == p.root ? gi : ng.parent;  // what the root's link holds is not looked at
   const Box ob = tree_box(p.t, p.chk(other));
   const NodeP ngg = tree_node(p.t, p.chk(ggi));
   if (np.isLeft) ng.left = s;
