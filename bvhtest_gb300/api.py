@@ -149,8 +149,9 @@ def radix_sort_pairs(keys: torch.Tensor, vals: torch.Tensor, begin_bit=0, end_bi
 
 
 def sort_default_tile(tile_keys: int = 0) -> int:
-    """Sets the onesweep tile (2048, 4096 or 8192 keys per CTA) of the sorts that are not given one
-    (LBVH build, optimizer selection) and returns the previous setting; 0 only reads it."""
+    """Sets the onesweep tile (2048, 4096 or 8192 keys per CTA, or 1: chosen by the number of pairs, the
+    initial setting) of the sorts that are not given one (LBVH build, optimizer selection) and returns the
+    previous setting; 0 only reads it."""
     prev = C.c_uint32()
     check(load().bvhgb_sort_set_default_tile(int(tile_keys), C.byref(prev)), "bvhgb_sort_set_default_tile")
     return prev.value

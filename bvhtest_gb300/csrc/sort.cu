@@ -444,9 +444,10 @@ int sort_passes(const Layout &L, uint32_t tileKeys, const K *keysIn, K *keysOut,
   }
 }
 
-std::atomic<uint32_t> g_default_tile{kSortTileDefault};
+std::atomic<uint32_t> g_default_tile{BVHGB_SORT_TILE_AUTO};
 
-// Keys per CTA of a sort that is given none. Small sorts fill few CTAs at the large tiles (63-bit keys,
+// Keys per CTA of a sort that is given none: the process-wide setting or, where that leaves the choice
+// (BVHGB_SORT_TILE_AUTO), by the number of pairs. Small sorts fill few CTAs at the large tiles (63-bit keys,
 // 2,048 / 4,096 / 8,192: 262,144 pairs 81 / 88 / 104 us, 524,288 100 / 91 / 109). From there to 8M pairs
 // the tile is the one whose SMs are done first: w tiles an SM take about (w + ceil(w)) / 2 times a tile's
 // time, which grows with its items and, for 16 of them, the registers they spill. 63-bit keys, tiles of
@@ -455,8 +456,9 @@ std::atomic<uint32_t> g_default_tile{kSortTileDefault};
 // L2, the longer runs of the largest tile count: 12M 895 / 768 / 757 / 720, 33.5M 2,424 / 2,067 / 1,983 / 1,852.
 uint32_t auto_tile(uint32_t n) {
   const uint32_t given = g_default_tile.load(std::memory_order_relaxed);
+  if (given != BVHGB_SORT_TILE_AUTO) return given;
   if (n <= (1u << 18)) return (uint32_t)kMinTile;
-  if (given != kSortTileDefault || n > (1u << 23)) return given;
+  if (n > (1u << 23)) return kSortTileDefault;
   constexpr uint32_t shapes[4][2] = {{4096, 12}, {6144, 16}, {7168, 18}, {8192, 22}};  // keys, a tile's time
   uint32_t best = 0;
   float least = 0.0f;
@@ -1269,7 +1271,7 @@ extern "C" BVHGB_API int bvhgb_select_smallest_pairs(void *temp, size_t *tempByt
 }
 
 extern "C" BVHGB_API int bvhgb_sort_set_default_tile(uint32_t tileKeys, uint32_t *previous) {
-  if (tileKeys != 0 && !bvhgb::sort_tile_valid(tileKeys)) return BVHGB_INVALID_ARGUMENT;
+  if (tileKeys != 0 && tileKeys != BVHGB_SORT_TILE_AUTO && !bvhgb::sort_tile_valid(tileKeys)) return BVHGB_INVALID_ARGUMENT;
   const uint32_t old = tileKeys ? bvhgb::g_default_tile.exchange(tileKeys) : bvhgb::g_default_tile.load();
   if (previous) *previous = old;
   return BVHGB_OK;

@@ -14,8 +14,8 @@ size_t sort_temp_bytes(uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_
 uint32_t *sort_error_word(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit);
 // Stable ascending sort; temp must hold sort_temp_bytes(...) bytes. tileKeys = keys per CTA of the
 // onesweep passes (2048, 4096 or 8192; the result does not depend on it); 0 takes the process-wide
-// default (kSortTileDefault unless bvhgb_sort_set_default_tile changed it).
-constexpr uint32_t kSortTileDefault = 8192;
+// setting (bvhgb_sort_set_default_tile), which leaves the choice to the number of pairs unless it was changed.
+constexpr uint32_t kSortTileDefault = 8192;  // the batched pipeline's, and the choice for the largest sorts
 bool sort_tile_valid(uint32_t tileKeys);
 // Polls of an unpublished predecessor before a look-back gives up (0xFFFFFFFF: the default).
 int sort_set_spin_limit(uint32_t limit, uint32_t *previous);

@@ -198,8 +198,11 @@ BVHGB_API int bvhgb_select_smallest_pairs(void *temp, size_t *tempBytes, const u
 
 /* Keys per CTA of the onesweep passes (2048, 4096 or 8192) for sorts that are not given one: the
  * LBVH build's and the optimizer's selection sort, launched (or captured into a graph) after the
- * call. The default, 8192, leaves the choice to the sort's size. tileKeys = 0 only reads the setting. *previous (may be NULL) receives the old value. The
- * results do not depend on it. No counterpart in the reference (cub picks its own tiles). */
+ * call. BVHGB_SORT_TILE_AUTO, the initial setting, leaves the choice to the number of pairs; up to 4,096 pairs it
+ * (and 2048) makes no passes at all. tileKeys = 0 only reads the setting. *previous (may be NULL)
+ * receives the old one. The results do not depend on it. No counterpart in the reference (cub picks its own
+ * tiles). */
+#define BVHGB_SORT_TILE_AUTO 1u
 BVHGB_API int bvhgb_sort_set_default_tile(uint32_t tileKeys, uint32_t *previous);
 /* Diagnostics of the failure paths (no counterpart in the reference). bvhgb_sort_set_spin_limit:
  * how many times a sort tile polls a predecessor that has not published its digit counts before it
