@@ -109,6 +109,12 @@ class LBVH:
         check(self.lib.bvhgb_lbvh_read_errors(self.ws, C.byref(v), _stream(stream)), "read_errors")
         return v.value
 
+    def sort_route(self, stream=None) -> int:
+        """How the last 63-bit sort went: 0 upper bits and groups, 1 all bits after a long group, 2 all bits at once."""
+        v = C.c_uint32()
+        check(self.lib.bvhgb_lbvh_read_sort_route(self.ws, C.byref(v), _stream(stream)), "read_sort_route")
+        return v.value
+
     def keys(self, n, sorted_: bool, stream=None):
         k = np.zeros(n, np.uint32 if self.cfg.mortonBits == 30 else np.uint64)
         idx = np.zeros(n, np.uint32)

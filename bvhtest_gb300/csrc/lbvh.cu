@@ -32,7 +32,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t maxFaces = 0;
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
-  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate, heavy-cell flag
+  uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate, heavy-cell flag, sort route
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -40,9 +40,13 @@ struct bvhgb_lbvh_workspace {
   uint32_t *slots = nullptr;
   float4 *triBoxes = nullptr;  // 2 x float4 per face (mn.xyz mx.x | mx.yz 0 0); null: gather the triangle
   bool slotsArmed = false;  // slots hold kNone (set by the Morton kernel)
-  // Sampled counts of the Morton cells, 2^cellBits (63-bit keys; null: none); cleared with the scene box.
+  // Sampled counts of the Morton cells, 2^cellBits (63-bit keys; null: none). The Morton phase adds to them; the
+  // kernel of the scene box clears them, and the Morton phase itself where that has not run since (in the same
+  // capture, if any: 0 is none).
   uint32_t *cells = nullptr;
   uint32_t cellBits = 0;
+  bool cellsClear = false;
+  unsigned long long cellsClearIn = 0;
   void *sortTemp = nullptr;
   size_t sortTempBytes = 0;
 };
@@ -788,6 +792,17 @@ int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *fa
   return BVHGB_OK;
 }
 
+// The capture that s is in (0: none; all ones where that cannot be told).
+unsigned long long capture_of(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return ~0ull;
+  }
+  return status == cudaStreamCaptureStatusNone ? 0ull : id;
+}
+
 int check_ws(const bvhgb_lbvh_workspace *ws, uint32_t n) {
   if (!ws) return BVHGB_INVALID_ARGUMENT;
   if (n > ws->maxFaces) return BVHGB_TOO_LARGE;
@@ -827,7 +842,6 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   if (ws->keyBytes == 8) {  // two places a sample
     for (ws->cellBits = 10; ws->cellBits < 22 && (1u << ws->cellBits) < maxFaces / (cell_sample(maxFaces) / 2);) ++ws->cellBits;
     if (e == cudaSuccess) e = dev_malloc(&ws->cells, 4ull << ws->cellBits);
-    if (e == cudaSuccess) e = cudaMemset(ws->cells, 0, 4ull << ws->cellBits);
   }
   if (e != cudaSuccess) {
     set_last_error("bvhgb_lbvh_create", e);
@@ -866,6 +880,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_init_tri_data(bvhgb_lbvh_workspace *ws, cons
   lbvh_bounds_kernel<<<grid, kBoundsThreads, 0, s>>>(vert, faces, n, ws->scene, ws->cells,
                                                      ws->cells ? 1u << ws->cellBits : 0u);
   BVHGB_LAUNCH_CHECK("lbvh bounds");
+  ws->cellsClear = true;
+  ws->cellsClearIn = capture_of(s);
   return BVHGB_OK;
 }
 
@@ -877,6 +893,11 @@ extern "C" BVHGB_API int bvhgb_lbvh_calc_morton(bvhgb_lbvh_workspace *ws, const 
   if (!vert || !faces) return BVHGB_INVALID_ARGUMENT;
   cudaStream_t s = as_stream(stream);
   uint32_t grid = ceil_div(n, kMortonThreads * 2);
+  if (ws->cells) {
+    if (!ws->cellsClear || ws->cellsClearIn != capture_of(s))
+      BVHGB_CUDA_TRY(cudaMemsetAsync(ws->cells, 0, 4ull << ws->cellBits, s));
+    ws->cellsClear = false;
+  }
   if (ws->cfg.mortonBits == 30)
     lbvh_morton_kernel<30><<<grid, kMortonThreads, 0, s>>>(vert, faces, n, ws->scene, ws->keys, ws->vals, ws->slots,
                                                            ws->triBoxes, nullptr, 0u);
@@ -893,7 +914,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_sort(bvhgb_lbvh_workspace *ws, uint32_t n, b
   if (st) return st;
   if (ws->keyBytes == 8) {
     return sort_morton(ws->sortTemp, static_cast<const uint64_t *>(ws->keys), static_cast<uint64_t *>(ws->keysSorted),
-                       ws->vals, ws->valsSorted, n, ws->scene + 8,
+                       ws->vals, ws->valsSorted, n, ws->scene + 8, ws->scene + 10,
                        MortonCells{ws->cells, ws->cells ? 1u << ws->cellBits : 0u, ws->cells ? ws->scene + 9 : nullptr}, as_stream(stream));
   }
   return sort_pairs(ws->sortTemp, ws->keys, ws->keysSorted, ws->vals, ws->valsSorted, n, ws->keyBytes, 0,
@@ -995,6 +1016,14 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32
   BVHGB_CUDA_TRY(cudaMemcpyAsync(&b, se, 4, cudaMemcpyDeviceToHost, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   *flags = a | b;
+  return BVHGB_OK;
+}
+
+extern "C" BVHGB_API int bvhgb_lbvh_read_sort_route(bvhgb_lbvh_workspace *ws, uint32_t *route, bvhgb_stream stream) {
+  if (!ws || !route) return BVHGB_INVALID_ARGUMENT;
+  cudaStream_t s = as_stream(stream);
+  BVHGB_CUDA_TRY(cudaMemcpyAsync(route, ws->scene + 10, 4, cudaMemcpyDeviceToHost, s));
+  BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   return BVHGB_OK;
 }
 

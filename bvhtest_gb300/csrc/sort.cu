@@ -607,6 +607,7 @@ struct FullSort {
   uint32_t *valsOut, *altV, *words, *hist, *counters, *status, *err, *barrier;
   uint32_t n, tiles, passes, zeroed;  // words[0, zeroed) are cleared, but for the error and barrier words
   uint32_t *gate, *heavy;  // both 0 between sorts
+  uint32_t *route;         // receives what they were
 };
 
 __device__ __forceinline__ bool grid_barrier(const FullSort &f, uint32_t target) {
@@ -630,7 +631,9 @@ __device__ __forceinline__ bool grid_barrier(const FullSort &f, uint32_t target)
 
 template <int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, kSortCtas<ITEMS>) full_sort_kernel(const __grid_constant__ FullSort f) {
-  if (__ldcg(f.gate) == 0u && !skipped(f.heavy)) return;
+  const bool gate = __ldcg(f.gate) != 0u, heavy = skipped(f.heavy);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *f.route = heavy ? 2u : gate ? 1u : 0u;
+  if (!gate && !heavy) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   auto &sm = *reinterpret_cast<OnesweepSmem<uint64_t, THREADS, ITEMS> *>(smraw);
   uint32_t *sh = reinterpret_cast<uint32_t *>(smraw);
@@ -756,7 +759,7 @@ uint32_t *sort_error_word(void *temp, uint32_t n, uint32_t keyBytes, uint32_t be
 }
 
 int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-                uint32_t n, uint32_t *gate, const MortonCells &cells, cudaStream_t s) {
+                uint32_t n, uint32_t *gate, uint32_t *route, const MortonCells &cells, cudaStream_t s) {
   int st = sort_prepare();
   if (st) return st;
   if (n == 0) return BVHGB_OK;
@@ -784,7 +787,7 @@ int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uin
   const Layout F = make_layout(n, 8, 0, 63, small ? kMinTile : 8192);
   const FullSort f{keysIn, valsIn, keysOut, altK, valsOut, altV, reinterpret_cast<uint32_t *>(t), hist, counters, status,
                    err, err + 1, n, F.tiles, F.passes,
-                   (uint32_t)(Lmax.status / 4 + kRadix * (size_t)F.tiles * F.passes), gate, cells.heavy};
+                   (uint32_t)(Lmax.status / 4 + kRadix * (size_t)F.tiles * F.passes), gate, cells.heavy, route};
   return small ? launch_full_sort<256, 8>(f, s) : launch_full_sort<512, 16>(f, s);
 }
 

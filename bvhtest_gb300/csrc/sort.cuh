@@ -32,9 +32,11 @@ struct MortonCells {
   uint32_t *heavy = nullptr;
 };
 // The stable ascending sort of n 63-bit Morton keys; temp as for sort_pairs on bits [0, 63). *gate
-// and *cells.heavy (device) are 0 before and after.
+// and *cells.heavy (device) are 0 after; where they are not before, the full sort makes the order. *route
+// receives how it was made: 0 by the upper bits and their groups, 1 by the full sort after a long group, 2 by the full
+// sort at once, for a full cell (not written up to 4,096 pairs).
 int sort_morton(void *temp, const uint64_t *keysIn, uint64_t *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
-                uint32_t n, uint32_t *gate, const MortonCells &cells, cudaStream_t s);
+                uint32_t n, uint32_t *gate, uint32_t *route, const MortonCells &cells, cudaStream_t s);
 // The sort's alternate buffers, (keyBytes + 4) * n bytes of the temp space that hold nothing between sorts.
 void *sort_alternate(void *temp, uint32_t n, uint32_t keyBytes, uint32_t beginBit, uint32_t endBit);
 int sort_pairs(void *temp, const void *keysIn, void *keysOut, const uint32_t *valsIn, uint32_t *valsOut, uint32_t n,

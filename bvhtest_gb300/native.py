@@ -98,6 +98,7 @@ PROTOS = {
     "bvhgb_lbvh_set_scene_box": (I32, [VP, C.POINTER(Aabb), VP]),
     "bvhgb_lbvh_read_keys": (I32, [VP, I32, VP, VP, U32, VP]),
     "bvhgb_lbvh_read_errors": (I32, [VP, C.POINTER(U32), VP]),
+    "bvhgb_lbvh_read_sort_route": (I32, [VP, C.POINTER(U32), VP]),
     "bvhgb_radix_sort_pairs": (I32, [VP, C.POINTER(SZ), VP, VP, VP, VP, U32, U32, U32, U32, VP]),
     "bvhgb_select_smallest_pairs": (I32, [VP, C.POINTER(SZ), VP, VP, VP, U32, U32, VP]),
     "bvhgb_sort_set_default_tile": (I32, [U32, C.POINTER(U32)]),

@@ -180,6 +180,10 @@ BVHGB_API int bvhgb_lbvh_static_read_errors(const bvhgb_lbvh_config *cfg, uint32
 /* Device error bits of the last build (4 = an inconsistent exchange slot was met and the build
  * stopped; 1 = the sort's look-back gave up); synchronous on 'stream'. 0 = the build is valid. */
 BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32_t *flags, bvhgb_stream stream);
+/* How the last sort of more than 4,096 63-bit keys went (diagnostics; the order is the same): 0 = by the keys'
+ * upper bits and the groups that share them, 1 = by all bits, because a group was too long, 2 = by all
+ * bits at once, because a sample of the keys found a full cell. Synchronous on 'stream'. */
+BVHGB_API int bvhgb_lbvh_read_sort_route(bvhgb_lbvh_workspace *ws, uint32_t *route, bvhgb_stream stream);
 
 /* ---- radix sort (used by the build and the optimizer; exposed for tests) --------------------- */
 
