@@ -803,6 +803,18 @@ unsigned long long capture_of(cudaStream_t s) {
   return status == cudaStreamCaptureStatusNone ? 0ull : id;
 }
 
+// Cleared when it returns. A cudaMemset would be queued behind the default stream's work and run later, beside
+// what a caller's non-blocking stream does with the memory by then.
+cudaError_t clear_now(void *p, size_t bytes) {
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(p, 0, bytes, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  return e != cudaSuccess ? e : done;
+}
+
 int check_ws(const bvhgb_lbvh_workspace *ws, uint32_t n) {
   if (!ws) return BVHGB_INVALID_ARGUMENT;
   if (n > ws->maxFaces) return BVHGB_TOO_LARGE;
@@ -831,7 +843,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   ws->sortTempBytes = sort_temp_bytes(maxFaces, ws->keyBytes, 0, c.mortonBits);
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = dev_malloc(&ws->scene, 256);
-  if (e == cudaSuccess) e = cudaMemset(ws->scene, 0, 256);
+  if (e == cudaSuccess) e = clear_now(ws->scene, 256);
   if (e == cudaSuccess) e = dev_malloc(&ws->keys, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->keysSorted, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->vals, 4 * m);
