@@ -332,22 +332,23 @@ __device__ __forceinline__ void treelet_build(TreeletSmem<T, K> &sm, uint32_t B0
   }
   Box nb = box;
   if (ordered) {
-    // Node by node: inner boxes in the second buffer, made[slot] = 2 once the box is there.
+    // Node by node: inner boxes in the second buffer, made[slot] = 2 once the box is there. A round makes the nodes
+    // whose children are there; one that makes none is the last (all are made, or the keys are in no order, which the
+    // sort has reported: their nodes wait for children that nobody makes).
     bool done = !local;
-    while (__syncthreads_or(!done)) {
+    __syncthreads();
+    for (;;) {
       const bool now = !done && (l == t || sm.made[t] == 2) && (t + 1 == r || sm.made[t + 1] == 2);
-      Box other = {};
+      if (!__syncthreads_or(now)) break;  // every thread has read the marks
       if (now) {
         nb = sm.box.get(l == t ? 0 : 1, t);
-        other = sm.box.get(t + 1 == r ? 0 : 1, t + 1);
+        const Box other = sm.box.get(t + 1 == r ? 0 : 1, t + 1);
         merge_into(nb, other);
-      }
-      __syncthreads();  // a slot's box and mark appear between two rounds
-      if (now) {
         sm.box.put(1, slot, nb);
         sm.made[slot] = 2;
         done = true;
       }
+      __syncthreads();
     }
   }
   window_boxes<T>(sm.box, top, cnt, local && !ordered, l, r, box, nb);
