@@ -33,6 +33,7 @@ struct bvhgb_lbvh_workspace {
   bvhgb_lbvh_config cfg{};
   uint32_t keyBytes = 4;
   uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate, heavy-cell flag, sort route
+  bool sceneReady = false;    // they have been written
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -57,9 +58,11 @@ namespace {
 constexpr int kBoundsThreads = 256;
 constexpr int kMortonThreads = 256;
 
+constexpr uint32_t kSceneWords = 11;
+
 __global__ void lbvh_init_kernel(uint32_t *scene) {
   if (threadIdx.x < 6) scene[threadIdx.x] = f2ord(0.0f);  // origin box [(0,0,0),(0,0,0)]
-  if (threadIdx.x == 6) scene[6] = 0;                     // error word
+  else if (threadIdx.x < kSceneWords) scene[threadIdx.x] = 0;
 }
 
 __global__ void __launch_bounds__(kBoundsThreads) lbvh_bounds_kernel(const float *__restrict__ vert,
@@ -664,7 +667,8 @@ __global__ void __launch_bounds__(kSmallMesh) lbvh_small_kernel(const float *__r
     }
     if (lane_id() == 0) scene[warp] = sm.scene[warp] = f2ord(m);
   }
-  if (t == 6) scene[6] = *sortErr = 0;  // error words (the sort's may be a larger mesh's)
+  if (t >= 6 && t < kSceneWords) scene[t] = 0;
+  if (t == 6) *sortErr = 0;  // which may be a larger mesh's
   __syncthreads();
   K key = ~(K)0;
   uint32_t face = t;  // a padding thread's pair sorts behind every triangle's
@@ -727,6 +731,7 @@ template <int MODE, typename K>
 int launch_small(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n, bvhgb_node *nodes,
                  cudaStream_t s) {
   ws->slotsArmed = false;
+  ws->sceneReady = true;
   lbvh_small_kernel<MODE, K><<<1, kSmallMesh, sizeof(SmallSmem<K>), s>>>(
       vert, faces, n, ws->scene, sort_error_word(ws->sortTemp, ws->maxFaces, ws->keyBytes, 0, ws->cfg.mortonBits),
       static_cast<K *>(ws->keys), ws->vals, static_cast<K *>(ws->keysSorted), ws->valsSorted,
@@ -804,16 +809,12 @@ unsigned long long capture_of(cudaStream_t s) {
   return status == cudaStreamCaptureStatusNone ? 0ull : id;
 }
 
-// Cleared when it returns. A cudaMemset would be queued behind the default stream's work and run later, beside
-// what a caller's non-blocking stream does with the memory by then.
-cudaError_t clear_now(void *p, size_t bytes) {
-  cudaStream_t s = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(p, 0, bytes, s);
-  const cudaError_t done = cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
-  return e != cudaSuccess ? e : done;
+// The scene words hold nothing until a build's first phase writes all of them, on its stream; a call that comes
+// before any such phase clears them there.
+int scene_ready(bvhgb_lbvh_workspace *ws, cudaStream_t s) {
+  if (!ws->sceneReady) BVHGB_CUDA_TRY(cudaMemsetAsync(ws->scene, 0, 4 * kSceneWords, s));
+  ws->sceneReady = true;
+  return BVHGB_OK;
 }
 
 int check_ws(const bvhgb_lbvh_workspace *ws, uint32_t n) {
@@ -844,7 +845,6 @@ extern "C" BVHGB_API int bvhgb_lbvh_create(uint32_t maxFaces, const bvhgb_lbvh_c
   ws->sortTempBytes = sort_temp_bytes(maxFaces, ws->keyBytes, 0, c.mortonBits);
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = dev_malloc(&ws->scene, 256);
-  if (e == cudaSuccess) e = clear_now(ws->scene, 256);
   if (e == cudaSuccess) e = dev_malloc(&ws->keys, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->keysSorted, ws->keyBytes * m);
   if (e == cudaSuccess) e = dev_malloc(&ws->vals, 4 * m);
@@ -887,6 +887,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_init_tri_data(bvhgb_lbvh_workspace *ws, cons
   cudaStream_t s = as_stream(stream);
   lbvh_init_kernel<<<1, 32, 0, s>>>(ws->scene);
   BVHGB_LAUNCH_CHECK("lbvh init");
+  ws->sceneReady = true;
   if (n == 0) return BVHGB_OK;
   if (!vert || !faces) return BVHGB_INVALID_ARGUMENT;
   uint32_t grid = min(ceil_div(n, kBoundsThreads * 4), (uint32_t)sm_count() * 8);
@@ -905,6 +906,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_calc_morton(bvhgb_lbvh_workspace *ws, const 
   if (n == 0) return BVHGB_OK;
   if (!vert || !faces) return BVHGB_INVALID_ARGUMENT;
   cudaStream_t s = as_stream(stream);
+  if ((st = scene_ready(ws, s))) return st;
   uint32_t grid = ceil_div(n, kMortonThreads * 2);
   if (ws->cells) {
     if (!ws->cellsClear || ws->cellsClearIn != capture_of(s))
@@ -925,6 +927,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_calc_morton(bvhgb_lbvh_workspace *ws, const 
 extern "C" BVHGB_API int bvhgb_lbvh_sort(bvhgb_lbvh_workspace *ws, uint32_t n, bvhgb_stream stream) {
   int st = check_ws(ws, n);
   if (st) return st;
+  if ((st = scene_ready(ws, as_stream(stream)))) return st;
   if (ws->keyBytes == 8) {
     return sort_morton(ws->sortTemp, static_cast<const uint64_t *>(ws->keys), static_cast<uint64_t *>(ws->keysSorted),
                        ws->vals, ws->valsSorted, n, ws->scene + 8, ws->scene + 10,
@@ -975,6 +978,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_scene_box(bvhgb_lbvh_workspace *ws, bvh
   if (!ws || !scene) return BVHGB_INVALID_ARGUMENT;
   uint32_t h[6];
   cudaStream_t s = as_stream(stream);
+  int st = scene_ready(ws, s);
+  if (st) return st;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(h, ws->scene, sizeof(h), cudaMemcpyDeviceToHost, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   float f[6];
@@ -1001,6 +1006,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_set_scene_box(bvhgb_lbvh_workspace *ws, cons
     h[k] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
   }
   cudaStream_t s = as_stream(stream);
+  int st = scene_ready(ws, s);
+  if (st) return st;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(ws->scene, h, sizeof(h), cudaMemcpyHostToDevice, s));
   // The copy reads pageable host memory, so it is staged before the call returns.
   return BVHGB_OK;
@@ -1024,6 +1031,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32
   if (!ws || !flags) return BVHGB_INVALID_ARGUMENT;
   uint32_t a = 0, b = 0;
   cudaStream_t s = as_stream(stream);
+  int st = scene_ready(ws, s);
+  if (st) return st;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(&a, ws->scene + 6, 4, cudaMemcpyDeviceToHost, s));
   const uint32_t *se = sort_error_word(ws->sortTemp, ws->maxFaces, ws->keyBytes, 0, ws->cfg.mortonBits);
   BVHGB_CUDA_TRY(cudaMemcpyAsync(&b, se, 4, cudaMemcpyDeviceToHost, s));
@@ -1035,6 +1044,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32
 extern "C" BVHGB_API int bvhgb_lbvh_read_sort_route(bvhgb_lbvh_workspace *ws, uint32_t *route, bvhgb_stream stream) {
   if (!ws || !route) return BVHGB_INVALID_ARGUMENT;
   cudaStream_t s = as_stream(stream);
+  int st = scene_ready(ws, s);
+  if (st) return st;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(route, ws->scene + 10, 4, cudaMemcpyDeviceToHost, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   return BVHGB_OK;
@@ -1104,6 +1115,7 @@ int static_workspace(const bvhgb_lbvh_config &c, bvhgb_lbvh_workspace &ws) {
     return p;
   };
   ws.scene = reinterpret_cast<uint32_t *>(take(256));
+  ws.sceneReady = true;  // the array starts as zeros
   ws.keys = take(ws.keyBytes * m);
   ws.keysSorted = take(ws.keyBytes * m);
   ws.vals = reinterpret_cast<uint32_t *>(take(4 * m));
@@ -1137,8 +1149,8 @@ extern "C" BVHGB_API int bvhgb_lbvh_build_static(const float *vert, const uint32
   if (st) return st;
   // The same phases as bvhgb_lbvh_build; every scratch word that must start at a known value is
   // written by the phase that uses it (scene box init kernel, which also clears the build's error
-  // word; slot reset in the Morton kernel; the sort's memset of its counters and error word), so
-  // the previous call's contents do not matter.
+  // word and the sort's gate; slot reset in the Morton kernel; the sort's memset of its counters and error
+  // word), so the previous call's contents do not matter.
   if ((st = bvhgb_lbvh_init_tri_data(&ws, vert, faces, numFaces, stream))) return st;
   if ((st = bvhgb_lbvh_calc_morton(&ws, vert, faces, numFaces, stream))) return st;
   if ((st = bvhgb_lbvh_sort(&ws, numFaces, stream))) return st;

@@ -28,3 +28,15 @@ def test_build_beside_a_busy_default_stream(gpu, n, bits):
     torch.cuda.synchronize()
     assert np.array_equal(b.scene_box(stream=side), box)
     assert torch.equal(nodes, expected) and b.errors(stream=side) == 0
+
+
+def test_calls_before_any_build(gpu):
+    """A new workspace has an empty box and no errors, whatever its memory held."""
+    import torch
+    junk = [torch.full((64,), -1, dtype=torch.int32, device="cuda") for _ in range(2000)]
+    del junk
+    torch.cuda.empty_cache()
+    for _ in range(20):
+        b = gpu.LBVH(5000, 63, "karras")
+        assert b.errors() == 0 and b.sort_route() == 0
+        b.close()
