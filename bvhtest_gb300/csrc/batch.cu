@@ -961,8 +961,9 @@ extern "C" BVHGB_API int bvhgb_batch_get_stats(bvhgb_batch_workspace *ws, bvhgb_
 // ---- autotuner ------------------------------------------------------------------------------------
 // Coordinate search over the three knobs, each timed with CUDA events on the caller's stream on
 // the caller's data (the results do not depend on them): the sort tile on the build, the refit block
-// on one optimizer iteration, the trace block on the random rays. Each candidate runs twice, the
-// faster run counts. The workspace keeps the best; the report lists every measurement.
+// on one optimizer iteration, the trace block on the random rays where these go through the node arrays
+// (the records' launch has blocks of one warp). Each candidate runs twice, the faster run counts. The workspace
+// keeps the best; the report lists every measurement, 0 for what was not measured.
 
 extern "C" BVHGB_API int bvhgb_batch_autotune(bvhgb_batch_workspace *ws, const float *vert, const uint32_t *faces,
                                               bvhgb_node *nodes, uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits,
@@ -1018,11 +1019,16 @@ extern "C" BVHGB_API int bvhgb_batch_autotune(bvhgb_batch_workspace *ws, const f
   }
   ws->cfg.refitBlock = best.refitBlock;
   bestMs = 3.4e38f;
-  for (int i = 0; i < 3 && !st && raysPerMesh; ++i) {
+  const bool records = pays_for_records(ws, raysPerMesh);
+  if (records && !st) {
+    st = batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, true, s);
+    if (!st && cudaStreamSynchronize(s) != cudaSuccess) st = BVHGB_CUDA_ERROR;
+  }
+  for (int i = 0; i < 3 && raysPerMesh; ++i) report->traceBlock[i] = traces[i];
+  for (int i = 0; i < 3 && !st && raysPerMesh && !records; ++i) {
     ws->cfg.traceBlock = traces[i];
     st = timed([&] { return batch_trace(ws, nodes, vert, faces, raysPerMesh, seed, hits, nullptr, nullptr, true, s); },
                report->traceBlockMs[i]);
-    report->traceBlock[i] = traces[i];
     if (!st && report->traceBlockMs[i] < bestMs) {
       bestMs = report->traceBlockMs[i];
       best.traceBlock = traces[i];

@@ -437,7 +437,7 @@ typedef struct bvhgb_batch_tune_report {
   uint32_t refitBlock[3];
   float refitBlockMs[3]; /* one optimizer iteration with each apply / count / refit block */
   uint32_t traceBlock[3];
-  float traceBlockMs[3]; /* the random-ray trace with each tracer block */
+  float traceBlockMs[3]; /* the random-ray trace with each tracer block (0: rays on records, which use none) */
   bvhgb_batch_config chosen;
 } bvhgb_batch_tune_report;
 
