@@ -78,7 +78,6 @@ __device__ __forceinline__ NodeRec tree_rec(const bvhgb_node *t, uint32_t x) {
   return r;
 }
 __device__ __forceinline__ float tree_sa(const bvhgb_node *t, uint32_t x) { return __ldg(&t[x].surfaceArea); }
-__device__ __forceinline__ bool tree_leaf(const bvhgb_node *t, uint32_t x) { return __ldg(&t[x].isLeafFlag) != 0; }
 
 // The storage of a BVHPatch: its node slots and patched boxes. Every lane of a warp that runs one
 // item holds the same patch, so the warp kernels keep one copy per warp in shared memory (a copy
@@ -147,10 +146,6 @@ struct Patch {
     d->idx[from] = kNone;
     d->nd[to] = d->nd[from];
     return to;
-  }
-  __device__ uint32_t sibling(const NodeP &n) const {
-    NodeP p = get(n.parent);
-    return n.isLeft == 0 ? p.left : p.right;
   }
   // get_subset(x) and get_aabb(x) given the tree's 48-byte record of x (a, m, c: its three float4).
   __device__ void subset_aabb_from(uint32_t x, const float4 &a, const float4 &m, const float4 &c, NodeP &n,

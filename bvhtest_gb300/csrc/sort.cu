@@ -122,11 +122,10 @@ __global__ void __launch_bounds__(kRadix) scan_kernel(uint32_t *hist, const uint
   h[threadIdx.x] = s[threadIdx.x] - v;
 }
 
-// CTAs per SM of a tile shape.
 template <int THREADS>
 constexpr bool kScans = THREADS == 256;  // the CTAs scan their pass's counts themselves
 
-template <int ITEMS>
+template <int ITEMS>  // CTAs per SM of a tile shape
 constexpr int kSortCtas = ITEMS <= 8 ? 3 : 2;
 
 template <typename K, int THREADS, int ITEMS>
