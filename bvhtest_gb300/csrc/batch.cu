@@ -581,7 +581,8 @@ int trace_on_nodes(const bvhgb_batch_workspace *ws, const bvhgb_node *nodes, con
 }
 
 // The records belong to one trace at a time: work that makes and reads them waits on its stream for the last
-// such work, whatever stream and thread that came from.
+// such work, whatever stream and thread that came from. A captured call cannot wait for work outside its graph, and
+// its replays come when they come: it has no turn and traces on the nodes.
 template <typename Fn>
 int in_turn(bvhgb_batch_workspace *ws, cudaStream_t s, Fn &&work) {
   std::lock_guard<std::mutex> lock(ws->wideLock);
@@ -591,21 +592,10 @@ int in_turn(bvhgb_batch_workspace *ws, cudaStream_t s, Fn &&work) {
   return st;
 }
 
-// A captured call cannot wait for work outside its graph, and its replays come when they come: it has no turn
-// at the records and traces on the nodes.
-bool is_captured(cudaStream_t s) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
-    cudaGetLastError();
-    return true;
-  }
-  return status != cudaStreamCaptureStatusNone;
-}
-
 int batch_trace(bvhgb_batch_workspace *ws, const bvhgb_node *nodes, const float *vert, const uint32_t *faces,
                 uint32_t raysPerMesh, uint64_t seed, bvhgb_hit *hits, float *rayOrg, float *rayDir, bool built,
                 cudaStream_t s) {
-  if (!pays_for_records(ws, raysPerMesh) || is_captured(s))
+  if (!pays_for_records(ws, raysPerMesh) || capture_of(s) != 0)
     return trace_on_nodes(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, s);
   return in_turn(ws, s, [&] {
     return trace_on_records(ws, nodes, vert, faces, raysPerMesh, seed, hits, rayOrg, rayDir, built, s);
@@ -885,7 +875,7 @@ extern "C" BVHGB_API int bvhgb_batch_run(bvhgb_batch_workspace *ws, const float 
   for (uint32_t m = 0; m < ws->numMeshes; ++m)
     if (raysPerMesh && ws->hFaceOff[m + 1] == ws->hFaceOff[m]) return BVHGB_INVALID_ARGUMENT;
   cudaStream_t s = as_stream(stream);
-  const bool records = pays_for_records(ws, raysPerMesh) && !is_captured(s);
+  const bool records = pays_for_records(ws, raysPerMesh) && capture_of(s) == 0;
   const bool same = ws->graph && ws->gVert == vert && ws->gFaces == faces && ws->gNodes == nodes && ws->gHits == hits &&
                     ws->gIterations == iterations && ws->gRays == raysPerMesh && ws->gSeed == seed &&
                     ws->gRecords == records;

@@ -155,6 +155,16 @@ inline cudaStream_t as_stream(bvhgb_stream s) { return reinterpret_cast<cudaStre
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 int sm_count();
 uint64_t context_id();
+// The capture that s is in (0: none; all ones where that cannot be told).
+inline unsigned long long capture_of(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return ~0ull;
+  }
+  return status == cudaStreamCaptureStatusNone ? 0ull : id;
+}
 // Launch; early: it may start while the stream's previous kernel drains, and the kernel calls grid_wait()
 // before it touches anything that kernel (or one before it) wrote or reads.
 template <typename... P, typename... A>

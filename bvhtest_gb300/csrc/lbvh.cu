@@ -798,17 +798,6 @@ int launch_build(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *fa
   return BVHGB_OK;
 }
 
-// The capture that s is in (0: none; all ones where that cannot be told).
-unsigned long long capture_of(cudaStream_t s) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) {
-    cudaGetLastError();
-    return ~0ull;
-  }
-  return status == cudaStreamCaptureStatusNone ? 0ull : id;
-}
-
 // The scene words hold nothing until a build's first phase writes all of them, on its stream; a call that comes
 // before any such phase clears them there.
 int scene_ready(bvhgb_lbvh_workspace *ws, cudaStream_t s) {

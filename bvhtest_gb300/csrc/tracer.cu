@@ -11,6 +11,7 @@
 //    hit is never culled; closest-hit ties resolve to the smallest primitive index;
 //  * each hit also yields (primId, t).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "common.cuh"
@@ -537,6 +538,15 @@ struct bvhgb_tracer {
   uint32_t numNodes = 0, root = 0;
   bvhgb::TravNode *trav = nullptr;  // both children per record: images (their pixels count the visits)
   bvhgb::WideNode *wide = nullptr;  // four grandchildren per record: rays that only want the hit
+  // The second kind doubles what an update writes (4.19M triangles: 122 us, 222 with it), for nothing where only
+  // pictures are traced. So an update leaves it out once the tracer has traced images and neither rays nor bounces;
+  // these then go through the nodes until the next update, which makes it.
+  mutable std::atomic<bool> images{false}, rays{false};  // traced so far
+  bool stale = false;  // the last update left the second kind out
+  const bvhgb::WideNode *ray_records() const {
+    rays.store(true, std::memory_order_relaxed);
+    return stale ? nullptr : wide;
+  }
 };
 
 using namespace bvhgb;
@@ -599,8 +609,13 @@ extern "C" BVHGB_API int bvhgb_tracer_update(bvhgb_tracer *tr, const bvhgb_node 
   tr->nodes = nodes;
   tr->numNodes = numNodes;
   tr->root = root;
-  build_trav_kernel<<<std::min(ceil_div(numNodes, 256), (uint32_t)sm_count() * 16), 256, 0, as_stream(stream)>>>(
-      nodes, numNodes, root, tr->trav, tr->wide);
+  // A captured update is replayed after calls that are still to come: it makes both, and the records are as
+  // current as the last call that ran has left them.
+  const cudaStream_t s = as_stream(stream);
+  const bool captured = capture_of(s) != 0, both = captured || tr->rays || !tr->images;
+  if (!captured) tr->stale = !both;
+  build_trav_kernel<<<std::min(ceil_div(numNodes, 256), (uint32_t)sm_count() * 16), 256, 0, s>>>(
+      nodes, numNodes, root, tr->trav, both ? tr->wide : nullptr);
   BVHGB_LAUNCH_CHECK("tracer records");
   return BVHGB_OK;
 }
@@ -609,6 +624,7 @@ extern "C" BVHGB_API int bvhgb_tracer_trace_image(const bvhgb_tracer *tr, const 
                                                   const bvhgb_camera *cam, const bvhgb_trace_config *cfg,
                                                   bvhgb_pixel *img, bvhgb_hit *hits, bvhgb_stream stream) {
   if (!tr || !tr->nodes || !vert || !faces || !cam || !img) return BVHGB_INVALID_ARGUMENT;
+  tr->images.store(true, std::memory_order_relaxed);
   return launch_image(tr->nodes, tr->trav, tr->numNodes, tr->root, vert, faces, cam, cfg, img, hits, as_stream(stream));
 }
 
@@ -616,7 +632,7 @@ extern "C" BVHGB_API int bvhgb_tracer_trace_rays(const bvhgb_tracer *tr, const f
                                                  const float *org, const float *dir, uint32_t n,
                                                  const bvhgb_trace_config *cfg, bvhgb_hit *hits, bvhgb_stream stream) {
   if (!tr || !tr->nodes || !vert || !faces) return BVHGB_INVALID_ARGUMENT;
-  return launch_rays(tr->nodes, tr->wide, tr->numNodes, tr->root, vert, faces, org, dir, n, cfg, hits,
+  return launch_rays(tr->nodes, tr->ray_records(), tr->numNodes, tr->root, vert, faces, org, dir, n, cfg, hits,
                      as_stream(stream));
 }
 
@@ -625,7 +641,7 @@ extern "C" BVHGB_API int bvhgb_tracer_trace_bounce(const bvhgb_tracer *tr, const
                                                    float offset, const bvhgb_hit *primary, bvhgb_hit *bounce,
                                                    float *rayOrg, float *rayDir, bvhgb_stream stream) {
   if (!tr || !tr->nodes || !vert || !faces || !cam) return BVHGB_INVALID_ARGUMENT;
-  return launch_bounce(tr->nodes, tr->wide, tr->numNodes, tr->root, vert, faces, cam, cfg, seed, offset, primary,
+  return launch_bounce(tr->nodes, tr->ray_records(), tr->numNodes, tr->root, vert, faces, cam, cfg, seed, offset, primary,
                        bounce, rayOrg, rayDir, as_stream(stream));
 }
 

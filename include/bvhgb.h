@@ -493,8 +493,9 @@ BVHGB_API int bvhgb_trace_bounce(const bvhgb_node *nodes, uint32_t numNodes, uin
  * array): bvhgb_tracer_update builds traversal records once, and every trace call on the tracer
  * reuses them: for images both children's boxes and references per inner node, for rays and bounces
  * its grandchildren's, 64 bytes each, maxNodes of either kind allocated at create (the second kind
- * where there is memory for it). The node array must stay as it was at the last update while traces
- * run. Same hits as the calls above. */
+ * where there is memory for it). An update leaves the second kind out once the tracer has traced images and
+ * neither rays nor bounces, which then go through the node array until the next update. The node array must
+ * stay as it was at the last update while traces run. Same hits as the calls above. */
 typedef struct bvhgb_tracer bvhgb_tracer;
 BVHGB_API int bvhgb_tracer_create(uint32_t maxNodes, bvhgb_tracer **out);
 BVHGB_API int bvhgb_tracer_destroy(bvhgb_tracer *tr);
