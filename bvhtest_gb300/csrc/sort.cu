@@ -511,10 +511,20 @@ __global__ void __launch_bounds__((int)kRankThreads) rank_sort_kernel(const K *_
   valsOut[before] = __ldg(valsIn + e);
 }
 
+// In and out arrays that share memory: the counting sort's blocks read all keys while others write, and one tile of
+// the largest shape reads everything before it writes where several small ones would not.
+bool shares_memory(const void *in, const void *out, size_t inBytes, size_t outBytes) {
+  const auto a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
+  return a < b + outBytes && b < a + inBytes;
+}
+
 template <typename K>
 int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const uint32_t *valsIn, uint32_t *valsOut,
               uint32_t n, uint32_t beginBit, uint32_t endBit, cudaStream_t s) {
-  if (tileKeys == 0) tileKeys = auto_tile(n);
+  const size_t keyBytes = sizeof(K) * (size_t)n, valBytes = 4 * (size_t)n;
+  const bool shared = shares_memory(keysIn, keysOut, keyBytes, keyBytes) || shares_memory(keysIn, valsOut, keyBytes, valBytes) ||
+                      shares_memory(valsIn, keysOut, valBytes, keyBytes) || shares_memory(valsIn, valsOut, valBytes, valBytes);
+  if (tileKeys == 0) tileKeys = shared ? kSortTileDefault : auto_tile(n);
   const Layout L = make_layout(n, sizeof(K), beginBit, endBit, tileKeys);
   const Layout Lmax = make_layout(n, sizeof(K), beginBit, endBit, kMinTile);  // the temp space's layout
   char *t = static_cast<char *>(temp);
@@ -530,7 +540,7 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
     BVHGB_CUDA_TRY(cudaMemcpyAsync(valsOut, valsIn, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
     return BVHGB_OK;
   }
-  if (tileKeys == (uint32_t)kMinTile && n <= kRankSort) {
+  if (tileKeys == (uint32_t)kMinTile && n <= kRankSort && !shared) {
     const K mask = endBit - beginBit >= 8 * sizeof(K) ? ~(K)0 : ((K)1 << (endBit - beginBit)) - 1;
     rank_sort_kernel<K><<<ceil_div(n, kRankThreads / kRankParts), kRankThreads, 0, s>>>(keysIn, keysOut, valsIn, valsOut, n,
                                                                               beginBit, mask, err);
