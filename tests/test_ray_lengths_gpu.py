@@ -9,9 +9,10 @@ from bvhtest_gb300 import scenes
 pytestmark = pytest.mark.gpu
 
 
-def _scene(gpu):
+def _scene(gpu, scale=1.0, offset=0.0):
     import torch
     vert, faces = scenes.uniform_soup(3000, sigma=0.05, seed=71)
+    vert = ((vert + np.float32(offset)) * np.float32(scale)).astype(np.float32)
     v = torch.from_numpy(vert).cuda()
     f = torch.from_numpy(faces.view(np.int32)).cuda()
     return vert, faces, v, f, gpu.LBVH(3000, 30, "refCompat").build(v, f)
@@ -22,8 +23,8 @@ def _same(got, ref):
     assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
 
 
-def _hits(gpu, orc, org, d, least):
-    vert, faces, v, f, nodes = _scene(gpu)
+def _hits(gpu, orc, org, d, least, **scene):
+    vert, faces, v, f, nodes = _scene(gpu, **scene)
     tr = gpu.Tracer(nodes.shape[0]).update(nodes)
     got = gpu.hits_to_numpy(tr.trace_rays(v, f, org, d))
     ref = orc.trace_brute(org, d, vert, faces)
@@ -84,3 +85,14 @@ def test_no_direction(gpu, orc):
     d[::3] = 0.0
     d[1::6] = -0.0
     _hits(gpu, orc, org, d, 0.1)
+
+
+@pytest.mark.parametrize("scale,offset", [(1e-18, 0.0), (1e-3, 0.0), (1e9, 0.0), (1e12, 0.0), (1.0, 1000.0), (1e-6, 5e5)])
+@pytest.mark.parametrize("length", [1e-20, 1.0, 1e20])
+def test_scenes_of_every_size(gpu, orc, scale, offset, length):
+    """Every kind of direction in scenes of every size, at the origin and far from it."""
+    g = np.random.default_rng(8)
+    n = 3000
+    org = ((g.uniform(-0.5, 1.5, (n, 3)) + offset) * scale).astype(np.float32)
+    d = (_directions(g, n) * length).astype(np.float32)
+    _hits(gpu, orc, org, d, 0.05 if scale >= 1e-6 else 0.0, scale=scale, offset=offset)
