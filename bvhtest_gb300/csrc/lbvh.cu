@@ -34,6 +34,7 @@ struct bvhgb_lbvh_workspace {
   uint32_t keyBytes = 4;
   uint32_t *scene = nullptr;  // 6 order-mapped floats, error word, (free), sort gate, heavy-cell flag, sort route
   bool sceneReady = false;    // they have been written
+  bool sorted = false;        // the sort's error word has been
   void *keys = nullptr;
   void *keysSorted = nullptr;
   uint32_t *vals = nullptr;
@@ -731,7 +732,7 @@ template <int MODE, typename K>
 int launch_small(bvhgb_lbvh_workspace *ws, const float *vert, const uint32_t *faces, uint32_t n, bvhgb_node *nodes,
                  cudaStream_t s) {
   ws->slotsArmed = false;
-  ws->sceneReady = true;
+  ws->sceneReady = ws->sorted = true;
   lbvh_small_kernel<MODE, K><<<1, kSmallMesh, sizeof(SmallSmem<K>), s>>>(
       vert, faces, n, ws->scene, sort_error_word(ws->sortTemp, ws->maxFaces, ws->keyBytes, 0, ws->cfg.mortonBits),
       static_cast<K *>(ws->keys), ws->vals, static_cast<K *>(ws->keysSorted), ws->valsSorted,
@@ -917,6 +918,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_sort(bvhgb_lbvh_workspace *ws, uint32_t n, b
   int st = check_ws(ws, n);
   if (st) return st;
   if ((st = scene_ready(ws, as_stream(stream)))) return st;
+  ws->sorted = ws->sorted || n != 0;
   if (ws->keyBytes == 8) {
     return sort_morton(ws->sortTemp, static_cast<const uint64_t *>(ws->keys), static_cast<uint64_t *>(ws->keysSorted),
                        ws->vals, ws->valsSorted, n, ws->scene + 8, ws->scene + 10,
@@ -1024,7 +1026,7 @@ extern "C" BVHGB_API int bvhgb_lbvh_read_errors(bvhgb_lbvh_workspace *ws, uint32
   if (st) return st;
   BVHGB_CUDA_TRY(cudaMemcpyAsync(&a, ws->scene + 6, 4, cudaMemcpyDeviceToHost, s));
   const uint32_t *se = sort_error_word(ws->sortTemp, ws->maxFaces, ws->keyBytes, 0, ws->cfg.mortonBits);
-  BVHGB_CUDA_TRY(cudaMemcpyAsync(&b, se, 4, cudaMemcpyDeviceToHost, s));
+  if (ws->sorted) BVHGB_CUDA_TRY(cudaMemcpyAsync(&b, se, 4, cudaMemcpyDeviceToHost, s));
   BVHGB_CUDA_TRY(cudaStreamSynchronize(s));
   *flags = a | b;
   return BVHGB_OK;
@@ -1104,7 +1106,7 @@ int static_workspace(const bvhgb_lbvh_config &c, bvhgb_lbvh_workspace &ws) {
     return p;
   };
   ws.scene = reinterpret_cast<uint32_t *>(take(256));
-  ws.sceneReady = true;  // the array starts as zeros
+  ws.sceneReady = ws.sorted = true;  // the array starts as zeros
   ws.keys = take(ws.keyBytes * m);
   ws.keysSorted = take(ws.keyBytes * m);
   ws.vals = reinterpret_cast<uint32_t *>(take(4 * m));
