@@ -306,8 +306,7 @@ __global__ void __launch_bounds__(32, kWideWarps) trace_rays_wide_kernel(
       sc, n, run,
       [&](uint32_t i, bool valid, RayPre &r) {
         if (valid) load_ray(org, dir, i, r);
-        // Without a direction the triangle test's shears are NaN: nothing is hit.
-        return valid && (r.d[0] != 0.0f || r.d[1] != 0.0f || r.d[2] != 0.0f);
+        return valid;
       },
       [&](uint32_t i, const Hit &h) { store_hit(hits + i, h); }, &g_trace_errors);
 }

@@ -336,11 +336,14 @@ constexpr int kWideStack = kStack * 3 / 2 + 3 * kWideSteps;
 // boxes that reach twice as far are on no grid (nested boxes don't): that bounds every plane distance of a ray,
 // and what a slab test may say about a ray that is all but parallel to the slab (limit_reciprocals).
 constexpr float kWideFinest = 9.0949470e-13f;  // 2^-40
+__device__ __forceinline__ float wide_extent(float4 a, float4 b) {
+  return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))), fmaxf(fabsf(b.x), fabsf(b.y)));
+}
 struct WideSize {
   float size;
   bool finite;  // false: the root's box is not, 'size' is any
   __device__ __forceinline__ WideSize(float4 a, float4 b) {
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))), fmaxf(fabsf(b.x), fabsf(b.y)));
+    const float m = wide_extent(a, b);
     finite = m < 1e37f;  // a NaN component drops out
     size = finite ? fmaxf(m, 2.7755576e-17f) : 1.1529215e18f;  // 2^-55, 2^60
   }
@@ -557,24 +560,34 @@ struct WideScene {
   __device__ __forceinline__ uint32_t root() const { return rootNode; }
 };
 
-// The largest reciprocal of a direction component that the slab tests of a ray use, and what takes the place of
-// larger ones.
-//   - Beyond 2^116 over the tree's size (and a thousandth of the ray's reach) products with the largest grid
-//     step or the origin's distance can overflow, and a distance that is infinite on one side would drop a
-//     box: there the reciprocal is infinite, the distances are NaN, and every box passes on that axis.
-//   - A ray parallel to an axis is to be kept out of the slabs beside it: for a component below 2^-80 of the
-//     largest the limit itself serves. A ray inside a slab is an eighth of a step or more from its planes, which
-//     then are as far away as 2^77 steps along the ray; and such a component moves the ray by a thirty-second
-//     of a step at most on its first 2^75 steps. A step is kWideFinest of the size or more, so this holds
-//     while the origin is within 2^35 sizes (2^-45 of the limit times the largest component).
-__device__ __forceinline__ void limit_reciprocals(RayPre &r, const WideSize &tree) {
-  const float reach = fmaxf(fmaxf(fabsf(r.o[0]), fabsf(r.o[1])), fabsf(r.o[2])) + tree.size;
-  const float most = fminf(1.2089258e24f * fabsf(r.sz), __fdividef(8.3076750e34f, fmaf(reach, 0.0009765625f, tree.size)));
-  const bool near = tree.finite && reach <= tree.size * (most * fabsf(pick(r.d, r.kz)) * 2.8421709e-14f);  // 2^-45
-  const float beyond = near ? most : __int_as_float(0x7f800000);
+// Reciprocals of direction components beyond 2^116 over the tree's size (and a thousandth of the ray's reach), which a
+// ray all but parallel to an axis has, are not used as they are: products with the largest grid step or the origin's
+// distance could overflow, and a distance that is infinite on one side only would drop a box.
+//   - An infinite one makes the distances NaN, and every box passes on that axis: true, but nothing is culled.
+//   - To keep the ray out of the slabs beside it, 2^80 over the largest component serves (or that limit). A ray
+//     inside a slab is an eighth of a step or more from its planes, which then are as far away as 2^77 steps along
+//     the ray; and the component moves the ray by a thirty-second of a step at most on its first 2^75 steps. A
+//     step is kWideFinest of the size or more, so this holds while the origin is within 2^35 sizes (2^-45 of
+//     the reciprocal times the largest component).
+// Other rays pass one test (a: the root's box with b.x, b.y): a set-up is as long as its instructions are cold.
+__device__ __forceinline__ void limit_reciprocals(RayPre &r, float4 a, float4 b) {
+  const float origin = fmaxf(fmaxf(fabsf(r.o[0]), fabsf(r.o[1])), fabsf(r.o[2]));
+  const float most = fmaxf(fmaxf(fabsf(r.inv[0]), fabsf(r.inv[1])), fabsf(r.inv[2]));
+  if (__builtin_expect(most * fmaxf(origin, wide_extent(a, b)) <= 1.1258999e15f, 1)) return;  // 2^50
+  if (pick(r.d, r.kz) == 0.0f) {
+    // No direction at all: the triangle test's shears are NaN and nothing is hit, so every box lies behind the ray.
+    r.o[0] = 3e38f;
+    r.inv[0] = r.inv[1] = r.inv[2] = 1.0f;
+    return;
+  }
+  const WideSize tree(a, b);
+  const float reach = origin + tree.size;
+  const float limit = __fdividef(8.3076750e34f, fmaf(reach, 0.0009765625f, tree.size));
+  const float stand = fminf(1.2089258e24f * fabsf(r.sz), limit);
+  const bool near = tree.finite && reach <= tree.size * (stand * fabsf(pick(r.d, r.kz)) * 2.8421709e-14f);  // 2^-45
 #pragma unroll
   for (int k = 0; k < 3; ++k)
-    if (fabsf(r.inv[k]) > most) r.inv[k] = copysignf(beyond, r.d[k]);
+    if (fabsf(r.inv[k]) > limit) r.inv[k] = copysignf(near ? stand : __int_as_float(0x7f800000), r.d[k]);
 }
 
 // Block b's run is rays [b * run, ...) of 'total' (< 2^31). gen(i, valid, r), which
@@ -636,7 +649,7 @@ __device__ __forceinline__ void trace_wide(const Scene &sc, uint32_t total, uint
           } else if (!live) {
             emit(i, Hit{kNone, sc.tmax});
           }
-          limit_reciprocals(g, WideSize(a, b));
+          limit_reciprocals(g, a, b);
         } else if (i < end) {
           emit(i, Hit{kNone, sc.tmax});
         }
