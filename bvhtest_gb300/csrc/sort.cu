@@ -4,8 +4,8 @@
 // SortPairsDescending (lib/builder/Bittner13CUDA.cu:674-680). Design (Adinets & Merrill 2022):
 //   1. one read of all keys builds the digit histograms of every pass;
 //   2. per pass, one kernel: each CTA makes the digits' global offsets from the pass's histogram (a tiny
-//      scan launch does for the large tiles) and takes tile indices from an atomic counter until none is left (so the tiles it looks back on are
-//      already running). It ranks a tile's keys stably (per item, the lanes holding the same digit are
+//      scan launch does for the large tiles) and takes tile indices from an atomic counter until none is left
+//      (so the tiles it looks back on are already running). It ranks a tile's keys stably (per item, the lanes holding the same digit are
 //      found with 9 ballots and a warp-private counter per digit is advanced by one shared-memory
 //      atomic of the lowest such lane; the atomics of all items are issued before any result is
 //      used), publishes per-digit counts, resolves its exclusive prefix by decoupled look-back (kLook
@@ -563,8 +563,9 @@ int sort_impl(void *temp, uint32_t tileKeys, const K *keysIn, K *keysOut, const 
 // original order, so a member's place is the number of members with a lower key, or an equal one and
 // an earlier position, and every member counts that for itself. A mesh leaves few triangles in one
 // cell of the upper bits; a group of more than kMaxGroup raises the gate, and the full eight-pass
-// sort, whose launches otherwise return at once, makes the order instead. Measured against the eight
-// passes alone: 65,536 keys 96 us against 119, 1M 114 / 153, 4.19M 249 / 441, 33.5M 1,840 / 2,840.
+// sort, whose launch otherwise returns at once, makes the order instead. Measured, launched one after the
+// other (65,536 keys / 262,144 / 1M / 4.19M / 33.5M): 55 / 65 / 96 / 225 / 1,822 us; eight passes over tiles of 8,192 keys,
+// one per SM, as the sort was before this: 120 / 129 / 150 / 442 / 2,855.
 //
 // Where a cell is that full (a detailed object in a large scene), the passes over the upper bits would be
 // for nothing, so the kernel that makes the keys samples its cells (MortonCells) and a full one sends all keys to

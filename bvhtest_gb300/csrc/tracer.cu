@@ -537,7 +537,7 @@ struct bvhgb_tracer {
   uint32_t numNodes = 0, root = 0;
   bvhgb::TravNode *trav = nullptr;  // both children per record: images (their pixels count the visits)
   bvhgb::WideNode *wide = nullptr;  // four grandchildren per record: rays that only want the hit
-  // The second kind doubles what an update writes (4.19M triangles: 122 us, 222 with it), for nothing where only
+  // The second kind doubles what an update writes (4.19M triangles: 125 us, 222 with it), for nothing where only
   // pictures are traced. So an update leaves it out once the tracer has traced images and neither rays nor bounces;
   // these then go through the nodes until the next update, which makes it. Rays are worth it however few they are:
   // an update and 1,000 rays 606 us, 998 without it (the longest ray's chain is half as long).

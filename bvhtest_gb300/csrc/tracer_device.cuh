@@ -315,7 +315,8 @@ __device__ __forceinline__ uint32_t traverse_records(const RayPre &r, const bvhg
 // plane on a power-of-two grid of the record's own, in one 64-byte line. A ray reads one such line
 // where it reads three of the binary records (192 bytes), and its chain of dependent loads halves.
 // Every plane is rounded outwards, so a box only grows and the closest hit, which does not depend
-// on which further boxes are opened, stays the same (the smallest t, then the smallest primitive).
+// on which further boxes are opened, stays the same (the smallest t, then the smallest primitive). Wide trees
+// with quantised boxes are the compressed wide BVHs of Ylitie, Karras and Laine (HPG 2017).
 struct __align__(64) WideNode {
   float o[3];       // the grid's origin
   uint32_t meta;    // byte k < 3: the exponent of axis k's grid step (biased); bits 24-27: slots with an
@@ -466,8 +467,8 @@ __device__ __forceinline__ float wide_plane(uint32_t packed, int slot) {
 // changes a hit: the closest one does not depend on when a triangle is tested, only on which
 // records are skipped, and those lie behind a hit already found.
 //
-// Bound: the latency of the record loads (long scoreboard 9.6 of 15 cycles per instruction; L1 hits
-// 53%, shared with the stacks). 4.19M rays in 33.5M triangles / the 1080p bounce in 4.19M, in ms:
+// Bound: the latency of the record loads (long scoreboard 5.4 of 10.3 cycles per instruction; L1 hits
+// 58%, shared with the stacks). 4.19M rays in 33.5M triangles / the 1080p bounce in 4.19M, in ms:
 // one thread per ray on binary records 8.6 / 4.2; four-wide records alone 8.4 / 4.3; with refill and
 // queued leaves 4.9 / 2.7 (128 rays per run; 64: 5.4 / 2.9, 256: 5.2 / 2.9; 4 or 12 records between
 // leaf tests: 5.0 / 2.9, 4.9 / 2.7); with stolen runs 5.0 / 2.5; with 24 warps per SM and 12 stack
